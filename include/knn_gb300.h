@@ -33,13 +33,14 @@ extern "C" {
 
 /* kernel families */
 #define KNNS_ALGO_AUTO 0 /* tensor cores when the shape allows, else CUDA cores */
-#define KNNS_ALGO_TC 1   /* tcgen05 tensor cores: BF16 keys for data exact in BF16, else 3xTF32; D <= 128
+#define KNNS_ALGO_TC 1   /* tcgen05 tensor cores: BF16 keys for data exact in BF16, else split FP16 or 3xTF32; D <= 128
                             with shortlists <= 128 on any corpus, any D (to 2048) and shortlists up to 512
-                            on corpora of at least 16384 rows (the 3xTF32 threshold scan) */
+                            on corpora of at least 16384 rows (the split-key threshold scan) */
 #define KNNS_ALGO_SIMT 2 /* CUDA-core FP32 fused distance + shortlist (any D, shortlist <= 512) */
 
 /* precision of the ranking keys */
-#define KNNS_PREC_EXACT 0 /* FP32-accurate keys (BF16 products when the data are BF16-exact, else 3xTF32) */
+#define KNNS_PREC_EXACT 0 /* FP32-accurate keys (BF16 products when the data are BF16-exact, else split FP16: x = hi + lo,
+                             11 + 11 bits, or 3xTF32 where the shortlist has no margin) */
 #define KNNS_PREC_BF16 1  /* BF16 keys pick a shortlist of c*k per query, re-ranked by exact distance
                              (tensor cores, D <= 256; c*k <= 128, or up to 512 on corpora of at least
                              16384 rows, where the threshold scan keeps the shortlist) */
@@ -50,14 +51,14 @@ extern "C" {
 
 /* threshold scan: the tensor-core pass keeps no shortlist on chip; per-query thresholds
    seeded from nested corpus samples let it collect only the keys that can still enter the
-   top-kp (results are the same).  It runs on BF16 / E4M3 keys, or in the exact form on 3xTF32
+   top-kp (results are the same).  It runs on BF16 / E4M3 keys, or in the exact form on split
    keys for data that are not exact in BF16 (the choice is made on the device). */
 #define KNNS_SCAN_AUTO 0 /* N >= 131072: BF16 keys for BF16-exact data (always in the BF16 / FP8
-                            forms), 3xTF32 keys otherwise; exact form with 16384 <= N < 131072
-                            (and re-rank on): the 3xTF32 scan for any data */
-#define KNNS_SCAN_ON 1   /* as AUTO, with the BF16 / 3xTF32 pair from N >= 16384 */
+                            forms), split keys otherwise; exact form with 16384 <= N < 131072
+                            (and re-rank on): the split-key scan for any data */
+#define KNNS_SCAN_ON 1   /* as AUTO, with the BF16 / split-key pair from N >= 16384 */
 #define KNNS_SCAN_OFF 2  /* never used */
-#define KNNS_SCAN_TF32 3 /* exact form: the 3xTF32 threshold scan alone for any data when N >= 16384
+#define KNNS_SCAN_TF32 3 /* exact form: the split-key threshold scan alone for any data when N >= 16384
                             (by default it also serves rows wider than 128 and k above 128); same results */
 
 typedef struct knns_options {
@@ -77,7 +78,7 @@ typedef struct knns_options {
                         per device block; 0 = automatic: the whole corpus when it fits in free device memory,
                         else blocks sized to it.  Each block is searched and merged into the running top-k
                         by (distance, index): results are identical to one search over the whole corpus */
-    int tf32_only;   /* exact form: 1 = 3xTF32 keys even for data that are exact in BF16 (the BF16
+    int tf32_only;   /* exact form: 1 = split keys even for data that are exact in BF16 (the BF16
                         tensor-core shortcut and the threshold scan stand down); results are the same,
                         the kernels slower -- a measurement switch for comparing the two key types */
     int scan_accs;   /* threshold scan: tensor-memory accumulators, 2 (tiles of 224 corpus rows; 192
@@ -101,7 +102,7 @@ typedef struct knns_stats {
     int scan_splits; /* corpus splits of the main threshold scan */
     int scan_cap;    /* candidate slots per (query, split half) of the main threshold scan */
     int scan_ring;   /* ring slots x boxes per slot, as 100 * slots + boxes */
-    int scan_keys;   /* threshold scans launched: 1 BF16 / E4M3 keys, 2 3xTF32 keys, 3 both (the exact
+    int scan_keys;   /* threshold scans launched: 1 BF16 / E4M3 keys, 2 split keys, 3 both (the exact
                         form then runs the one that matches the data: BF16 keys for BF16-exact data) */
 } knns_stats;
 
@@ -158,7 +159,7 @@ int knns_last_fixups(int64_t *out);
 /*
  * Stage timings of the searches run with opt->timing = 1 since the last
  * collection, from CUDA events recorded on each search's stream:
- * ms[0] preparation (norms, TF32 split), ms[1] fused distance + shortlist
+ * ms[0] preparation (norms, split), ms[1] fused distance + shortlist
  * kernel, ms[2] shortlist merge / re-rank.  Synchronises the device; *count
  * receives the number of searches summed.  Resets the accumulator.
  * (The reference kept the same split in knntimes dst_time / srch_time,
@@ -212,7 +213,7 @@ int knns_noalloc_prepare(void);
  * Resident index (no counterpart in the reference, whose drivers copy the corpus
  * to the device on every call, src/cuknnBitonic.cu:493-512).  knns_index_create
  * prepares a device corpus once -- BF16 copy, row norms, the exactness and
- * integrality flags and, with KNNS_INDEX_TF32, the TF32 hi/lo copies the exact
+ * integrality flags and, with KNNS_INDEX_TF32, the hi/lo copies the exact
  * form needs for data that are not BF16-exact -- and synchronises `stream`.
  * The caller keeps the FP32 corpus alive and unchanged while the index is used;
  * searches on it skip the corpus preparation.  D <= 256.
@@ -233,7 +234,7 @@ void knns_index_destroy(knns_index *index);
  * shortlist factors c = 2, 4, 8 (while c*k <= 512), and returns in *c_out the
  * smallest c whose recall@k against the exact form reaches `target` (else the
  * largest tried), its recall in *recall_out.  Synchronises `stream`; needs an
- * index with TF32 copies unless the data are BF16-exact.
+ * index with the hi/lo copies unless the data are BF16-exact.
  */
 int knns_autotune_shortlist(knns_index *index, const float *queries, int64_t Q, int64_t ldq, int k, int precision,
                             double target, int *c_out, double *recall_out, void *stream);
@@ -312,7 +313,7 @@ int knns_debug_prep(const float *x, int64_t n, int64_t ld, int D, float *norms, 
 
 /* The threshold scan's plan for an exact-form search (default options), computed on the host
  * alone (no GPU is touched): the seeding levels, coarsest first, and the main pass.  tf32 = 1
- * gives the 3xTF32 scan's plan, 0 the BF16 scan's; sms is the GPU's SM count. */
+ * gives the split-key scan's plan, 0 the BF16 scan's; sms is the GPU's SM count. */
 #define KNNS_MAX_SEED_LEVELS 6
 typedef struct knns_scan_plan_info {
     int kp;                                      /* shortlist length */

@@ -8,6 +8,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 namespace knn {
@@ -64,6 +65,32 @@ __device__ __forceinline__ float exact_dist_row(const float* __restrict__ q,
     }
     return __fadd_rn(__fadd_rn(__fadd_rn(p[0], p[1]), __fadd_rn(p[2], p[3])),
                      __fadd_rn(__fadd_rn(p[4], p[5]), __fadd_rn(p[6], p[7])));
+}
+
+// ---------------------------------------------------------------------------
+// FP16 split of FP32 rows (operands of the exact form's tensor-core keys)
+// ---------------------------------------------------------------------------
+
+// Scale of a row whose largest |x| is mx: the power of two that puts mx into [2^14, 2^15) (within
+// 2^-126..2^126; 1 when mx is not finite), and its reciprocal, both exact.
+__device__ __forceinline__ float row_scale(float mx, float& inv)
+{
+    const int e = (int)(__float_as_uint(mx) >> 23);  // biased exponent, mx >= 0
+    const int b = e == 255 ? 127 : min(max(268 - e, 1), 253);
+    inv = __uint_as_float((uint32_t)(254 - b) << 23);
+    return __uint_as_float((uint32_t)b << 23);
+}
+
+// s x0, s x1 as hi + lo FP16 pairs; returns whether a low part is nonzero.  A value that is not
+// finite leaves NaN in lo (inf - inf), so its keys are NaN and enter no segment.
+__device__ __forceinline__ uint32_t split_pair(float x0, float x1, float sc, uint32_t& hi, uint32_t& lo)
+{
+    const float y0 = __fmul_rn(x0, sc), y1 = __fmul_rn(x1, sc);
+    const __half2 h = __floats2half2_rn(y0, y1);
+    const __half2 l = __floats2half2_rn(__fsub_rn(y0, __low2float(h)), __fsub_rn(y1, __high2float(h)));
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+    return lo & 0x7fff7fffu;
 }
 
 // ---------------------------------------------------------------------------

@@ -1,6 +1,6 @@
 // engine.cu -- host engine and the status-returning C ABI (include/knn_gb300.h).
 //
-// One engine per CUDA device holds a grow-only workspace (norms, TF32 hi/lo
+// One engine per CUDA device holds a grow-only workspace (norms, hi/lo
 // copies of the corpus, per-split shortlists, staging for host calls) so a
 // search allocates nothing once warm.  It replaces the reference's per-call
 // set-up in gpuknnsBitonic / gpuknnsHeap (src/cuknnBitonic.cu:422-547,
@@ -152,10 +152,10 @@ static int encode_rows(CUtensorMap* m, const float* base, int64_t rows, int64_t 
     return KNNS_OK;
 }
 
-// 2-D bf16 matrix [rows][cols] (rows `pitch` elements apart), box {64 cols (128 B), box_rows rows},
-// 128B swizzle
+// 2-D matrix [rows][cols] of 16-bit values (BF16 unless `type` says FP16; rows `pitch` elements
+// apart), box {64 cols (128 B), box_rows rows}, 128B swizzle; columns past `cols` read as zeros
 static int encode_rows_bf16(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t pitch = 0,
-                            int box_rows = kTileN)
+                            int box_rows = kTileN, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16)
 {
     EncodeTiledFn fn;
     int rc = get_encode_fn(&fn);
@@ -164,11 +164,18 @@ static int encode_rows_bf16(CUtensorMap* m, const void* base, int64_t rows, int6
     cuuint64_t strides[1] = {(cuuint64_t)(pitch > 0 ? pitch : cols) * 2};
     cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    CUresult r = fn(m, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return set_error(KNNS_ERR_CUDA, "cuTensorMapEncodeTiled (bf16) failed (%d)", (int)r);
+    if (r != CUDA_SUCCESS) return set_error(KNNS_ERR_CUDA, "cuTensorMapEncodeTiled (16-bit) failed (%d)", (int)r);
     return KNNS_OK;
+}
+
+// One half (hi or lo) of the FP16 split of rows of D columns: every stride-th row, `rows` of them
+static int encode_split(CUtensorMap* m, const void* base, int64_t rows, int D, int64_t stride, int box_rows)
+{
+    const int hp = split_pitch(D);
+    return encode_rows_bf16(m, base, rows, hp, stride * hp, box_rows, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
 }
 
 // Norm parts [rows][kNormParts] BF16 (rows `pitch` elements apart), box {kNormParts, box_rows},
@@ -193,16 +200,23 @@ static int encode_np(CUtensorMap* m, const void* base, int64_t rows, int64_t pit
 // smallest corpus the threshold scan runs on when asked to (KNNS_SCAN_ON, long shortlists)
 constexpr int64_t kScanMinRowsForced = 16384;
 // Corpus size from which the BF16 / E4M3 threshold scan runs by default; below it the exact
-// form runs the 3xTF32 threshold scan (from kScanMinRowsForced rows) for data of any kind.
+// form runs the split-key threshold scan (from kScanMinRowsForced rows) for data of any kind.
 constexpr int64_t kScanMinRowsAuto = 131072;
 // accumulators of the threshold scan when the options leave it open
 constexpr int kScanAccsAuto = 2;
-// widest rows the 3xTF32 scan takes: its K loop has no limit, the selection's re-rank stages
+// widest rows the FP16-split scan takes: its K loop has no limit, the selection's re-rank stages
 // candidate rows in shared memory (four rows of 2048 values per warp)
-constexpr int kTscanMaxDp = 2048;
+constexpr int kTscanMaxD = 2048;
 static inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int round32(int x) { return (x + 31) & ~31; }
 static inline int round16(int x) { return (x + 15) & ~15; }
+
+// Entries a shortlist must hold beyond k for the FP16-split keys to serve the exact form.  Their
+// rounding differs from the 3xTF32 keys' (it is smaller: rms over row norms 0.5 to 0.8 of it at
+// every width measured), so a shortlist without a margin, whose last entries decide the result,
+// could end in another row; results there, and distances read off the keys (rerank = 0), stay those of
+// the 3xTF32 keys.  With 8 entries to spare no result depends on the keys' rounding.
+constexpr int kKeyMargin = 8;
 
 // Shortlist length: k plus a re-rank margin of max(8, k/8), in multiples of 16.
 int auto_kp(int k, int rerank)
@@ -257,7 +271,6 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
                              "%s shortlist of %d entries needs the threshold scan (N >= %d, scan not off); "
                              "at most %d entries otherwise", name, c->kp, kScanMinRowsForced, kMaxKpTC);
         c->algo = KNNS_ALGO_TC;
-        c->dp = kChunkK;  // TF32 operands unused
         c->dpb = dpb;
         c->stages = std::min(4, tc_max_stages(c->kp));
         c->qtile = kTileQ;
@@ -278,16 +291,17 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
     int algo = o.algo;
     const int dp = (int)round32(D);
     const bool tc_ok = E.cc >= 100 && dp <= kMaxDpTC;
-    // The 3xTF32 threshold scan alone (no BF16 path beside it) on corpora large enough to seed
+    // The split-key threshold scan alone (no BF16 path beside it) on corpora large enough to seed
     // its thresholds: rows wider than 128 or k above 128 (the shortlist kernel's limits),
     // corpora below the BF16 scan's default size, or on request
-    const bool wide = dp > kMaxDpTC || round16(k) > kMaxKpTC;
+    const bool wide = D > kMaxDpTC || round16(k) > kMaxKpTC;
     const bool small = o.scan == KNNS_SCAN_AUTO && N < kScanMinRowsAuto && c->rerank;
-    const bool tscan_ok = E.cc >= 100 && o.scan != KNNS_SCAN_OFF && N >= kScanMinRowsForced && dp <= kTscanMaxDp &&
+    const bool tscan_ok = E.cc >= 100 && o.scan != KNNS_SCAN_OFF && N >= kScanMinRowsForced && D <= kTscanMaxD &&
                           c->kp <= kMaxKpScan && (wide || small || o.scan == KNNS_SCAN_TF32);
     if ((algo == KNNS_ALGO_AUTO || algo == KNNS_ALGO_TC) && tscan_ok) {
         c->algo = KNNS_ALGO_TC;
         c->tscan = true;
+        c->tf32 = !c->rerank || c->kp < k + kKeyMargin;
         c->dp = dp;
         c->dpb = (D + 63) & ~63;
         c->qtile = kTileQ;
@@ -304,6 +318,7 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
         if (!tc_ok) return set_error(KNNS_ERR_UNSUPPORTED, "tensor-core path needs sm_100+ and D <= %d", kMaxDpTC);
         if (c->kp > kMaxKpTC)
             return set_error(KNNS_ERR_UNSUPPORTED, "tensor-core path holds at most %d shortlist entries", kMaxKpTC);
+        c->tf32 = !c->rerank || c->kp < k + kKeyMargin;
         c->dp = dp;
         c->dpb = (D + 63) & ~63;
         c->stages = std::min(4, tc_max_stages(c->kp));
@@ -311,7 +326,6 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
     } else if (algo == KNNS_ALGO_SIMT) {
         if (c->kp > 512) return set_error(KNNS_ERR_UNSUPPORTED, "shortlist of %d entries exceeds 512", c->kp);
         c->qtile = c->kp <= 128 ? 128 : 32;
-        c->dp = D;
         c->stages = 0;
     } else {
         return set_error(KNNS_ERR_INVALID, "unknown algo %d", algo);
@@ -423,15 +437,22 @@ static int seg_cap(double per_seg, double sigmas)
 
 static int seed_rank(double m) { return (int)std::ceil(2.0 * m + 4.0 * std::sqrt(m)) + 1; }
 
-// tf32: the plan of the 3xTF32 scan (tiles of 128 rows, 32 columns per segment; fix-up on the
-// CUDA-core kernel); otherwise of the BF16 / E4M3 scan of row width dpb.
+// keys kKeyF16 / kKeyTf32: the plan of the scan on split keys (fix-up on the CUDA-core kernel; dpb
+// only decides its tile: the row width rounded up to 64); otherwise of the BF16 / E4M3 scan of row
+// width dpb.
+enum ScanKeys { kKeyBf16, kKeyF8, kKeyF16, kKeyTf32 };
 static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, const knns_options& o, ScanPlan* P,
-                     bool fp8, bool tf32 = false)
+                     ScanKeys keys)
 {
     if (o.scan_accs != 0 && o.scan_accs != 2 && o.scan_accs != 4)
         return set_error(KNNS_ERR_INVALID, "threshold scan: %d accumulators (2 or 4)", o.scan_accs);
     int tn = 128, pc = 32;
-    if (tf32) {
+    const bool split = keys == kKeyF16 || keys == kKeyTf32, fp8 = keys == kKeyF8;
+    if (keys == kKeyF16) {
+        P->ring = fscan_ring(dpb);
+        tn = fscan_tile_rows(dpb);
+        pc = fscan_part_cols(dpb);
+    } else if (keys == kKeyTf32) {
         P->accs = 4;
         P->ring = tscan_ring(dpb <= 128);  // rows of up to 128 columns: queries in tensor memory
     } else {
@@ -513,7 +534,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     // fix-up of failed queries: up to 512 on a full wave, the rest (rare) on 8 splits; shortlists
     // above the tensor-core kernel's kMaxKpTC go to the CUDA-core kernel in tiles of 32 queries
     // (exact FP32 keys): the first 32 failed queries on a wave of splits, the rest on 8
-    P->simt_fix = kp > kMaxKpTC || tf32;
+    P->simt_fix = kp > kMaxKpTC || split;
     const int ft = P->simt_fix ? kSimtTileN : kTileN;
     const int fq = P->simt_fix ? 32 : kTileQ;
     const int64_t tilesF = cdiv(N, ft);
@@ -529,14 +550,21 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     return KNNS_OK;
 }
 
-// ---------------------------------------------------------------- 3xTF32 threshold scan
-// The stages of the 3xTF32 threshold scan over prepared corpus operands (norms, TF32 hi / lo
-// copies and their tile flags) and query norms: the queries' TF32 split, threshold seeding over
+// ---------------------------------------------------------------- threshold scan on split keys
+// The stages of the threshold scan on split keys -- FP16 (scan_f16.cu), or 3xTF32 (scan_tf32.cu)
+// where the shortlist has no margin -- over prepared corpus operands (norms, hi / lo copies, row
+// scales of the FP16 ones, tile flags) and query norms: the queries' split, threshold seeding over
 // nested corpus samples, the main scan, the selection with the exact re-rank, and the CUDA-core
 // fix-up of the queries the scan could not answer.  With run_if set, every kernel that writes
 // thresholds, candidates or results returns at once unless *run_if != 0 (the exact form's
-// device-side choice between BF16 and TF32 keys); its failed-query list is its own (fail), so
+// device-side choice between BF16 and split keys); its failed-query list is its own (fail), so
 // the other path's fix-up never sees it.
+struct SplitCopies {
+    const void* hi;
+    const void* lo;
+    const float* rs;         // FP16 copies: row scales
+    const uint32_t* flags;   // 128-row tiles with a low part
+};
 struct TscanStages {
     Engine& E;
     const Config& c;
@@ -547,9 +575,7 @@ struct TscanStages {
     int64_t Q, ldq;
     int D, k;
     const float* cn;
-    const float* hi;
-    const float* lo;
-    const uint32_t* cflags;
+    SplitCopies cp;
     const float* qn;
     float* dist;
     int32_t* idx;
@@ -561,19 +587,22 @@ struct TscanStages {
     cudaStream_t s;
     int launches = 0;
     TscanArgs a;
+    FscanArgs f;
     const float* T = nullptr;
 
     // buffers of the queries and of the plan (the corpus side is the caller's)
     int ensure()
     {
-        const int dp = c.dp;
-        int rc = E.qhi.ensure((size_t)Q * dp * sizeof(float));
-        if (!rc) rc = E.qlo.ensure((size_t)Q * dp * sizeof(float));
-        if (!rc) rc = E.qlof.ensure(((size_t)cdiv(Q, 128) + 4) * sizeof(uint32_t));
+        const size_t qb = c.tf32 ? (size_t)Q * c.dp * sizeof(float) : (size_t)Q * split_pitch(D) * 2;
+        int rc = E.qhi.ensure(qb);
+        if (!rc) rc = E.qlo.ensure(qb);
+        if (!rc) rc = E.qrs.ensure(Q * sizeof(float));
+        if (!rc) rc = E.qlof.ensure(((size_t)cdiv(Q, kTileRows) + 4) * sizeof(uint32_t));
         if (!rc) rc = E.tq.ensure((size_t)2 * Q * sizeof(float));
         if (!rc) rc = E.cand.ensure(sp.cand_words * sizeof(uint64_t));
         if (!rc) rc = E.cnt.ensure(sp.cnt_words * sizeof(uint32_t));
         if (!rc) rc = E.cnv.ensure(sp.norm_words * sizeof(float));
+        if (!rc) rc = E.csv.ensure(sp.norm_words * sizeof(float));
         if (!rc) rc = fail.ensure((size_t)(Q + 1) * sizeof(uint32_t));
         if (!rc) rc = E.part.ensure(sp.part_words * sizeof(uint64_t));
         if (!rc) rc = thr2.ensure(Q * sizeof(uint32_t));
@@ -581,51 +610,89 @@ struct TscanStages {
     }
     size_t workspace() const
     {
-        return E.qhi.cap + E.qlo.cap + E.qlof.cap + E.tq.cap + E.cand.cap + E.cnt.cap + E.cnv.cap + fail.cap +
-               E.part.cap + thr2.cap;
+        return E.qhi.cap + E.qlo.cap + E.qrs.cap + E.qlof.cap + E.tq.cap + E.cand.cap + E.cnt.cap + E.cnv.cap +
+               E.csv.cap + fail.cap + E.part.cap + thr2.cap;
     }
-    // the queries' TF32 hi / lo copies and the tensor maps of the scan's query operand
+    // the queries' split and the scan's query operands
     int split_queries()
     {
-        memset(&a, 0, sizeof(a));
-        if (c.dp <= 128) {
-            // the kernel splits the queries into tensor memory itself
-            a.tmem_a = 1;
-            a.queries = queries;
-            a.ldq = ldq;
-            a.D = D;
-        } else {
-            KNN_CUDA(launch_split(queries, Q, ldq, D, c.dp, (float*)E.qhi.p, (float*)E.qlo.p, (uint32_t*)E.qlof.p,
-                                  q_any_lo, run_if, s));
-            ++launches;
-            int rc = encode_rows(&a.tm_qhi, (const float*)E.qhi.p, Q, c.dp, c.dp);
-            if (!rc) rc = encode_rows(&a.tm_qlo, (const float*)E.qlo.p, Q, c.dp, c.dp);
-            if (rc) return rc;
-            a.qlo_flags = (const uint32_t*)E.qlof.p;
+        if (c.tf32) {
+            memset(&a, 0, sizeof(a));
+            if (c.dp <= 128) {
+                // the kernel splits the queries into tensor memory itself
+                a.tmem_a = 1;
+                a.queries = queries;
+                a.ldq = ldq;
+                a.D = D;
+            } else {
+                KNN_CUDA(launch_split_tf32(queries, Q, ldq, D, c.dp, (float*)E.qhi.p, (float*)E.qlo.p,
+                                           (uint32_t*)E.qlof.p, q_any_lo, run_if, s));
+                ++launches;
+                int rc = encode_rows(&a.tm_qhi, (const float*)E.qhi.p, Q, c.dp, c.dp);
+                if (!rc) rc = encode_rows(&a.tm_qlo, (const float*)E.qlo.p, Q, c.dp, c.dp);
+                if (rc) return rc;
+                a.qlo_flags = (const uint32_t*)E.qlof.p;
+            }
+            a.cand = (uint64_t*)E.cand.p;
+            a.cnt = (uint32_t*)E.cnt.p;
+            a.err = (int*)E.err.p;
+            a.Q = Q;
+            a.dp = c.dp;
+            a.ring = sp.ring;
+            a.run_if = run_if;
+            return KNNS_OK;
         }
-        a.cand = (uint64_t*)E.cand.p;
-        a.cnt = (uint32_t*)E.cnt.p;
-        a.err = (int*)E.err.p;
-        a.Q = Q;
-        a.dp = c.dp;
-        a.ring = sp.ring;
-        a.run_if = run_if;
+        memset(&f, 0, sizeof(f));
+        KNN_CUDA(launch_split_f16(queries, Q, ldq, D, E.qhi.p, E.qlo.p, (float*)E.qrs.p, Q, (uint32_t*)E.qlof.p,
+                                  q_any_lo, run_if, s));
+        ++launches;
+        if (D > kFscanTmemD) {
+            int rc = encode_split(&f.tm_qhi, E.qhi.p, Q, D, 1, kTileQ);
+            if (!rc) rc = encode_split(&f.tm_qlo, E.qlo.p, Q, D, 1, kTileQ);
+            if (rc) return rc;
+        }
+        f.qhi = (const uint16_t*)E.qhi.p;
+        f.qlo = (const uint16_t*)E.qlo.p;
+        f.qs = (const float*)E.qrs.p;
+        f.qlo_flags = (const uint32_t*)E.qlof.p;
+        f.cand = (uint64_t*)E.cand.p;
+        f.cnt = (uint32_t*)E.cnt.p;
+        f.err = (int*)E.err.p;
+        f.Q = Q;
+        f.D = D;
+        f.hp = split_pitch(D);
+        f.run_if = run_if;
         return KNNS_OK;
     }
     // one scan over rows 0, stride, 2*stride, ... of the corpus (nview of them)
-    int pass(int64_t nview, int64_t stride, const float* cn_view, const float* thr, int splits, int64_t split_len,
-             int cap, const uint32_t* flags)
+    int pass(int64_t nview, int64_t stride, const float* cn_view, const float* cs_view, const float* thr, int splits,
+             int64_t split_len, int cap, const uint32_t* flags)
     {
-        int r = encode_rows(&a.tm_chi, hi, nview, c.dp, stride * c.dp);
-        if (!r) r = encode_rows(&a.tm_clo, lo, nview, c.dp, stride * c.dp);
-        if (r) return r;
-        a.cn = cn_view;
-        a.thr = thr;
-        a.N = nview;
-        a.split_len = split_len;
-        a.cap = cap;
-        a.clo_flags = flags;
-        KNN_CUDA(launch_tscan(a, splits, s));
+        int r;
+        if (c.tf32) {
+            r = encode_rows(&a.tm_chi, (const float*)cp.hi, nview, c.dp, stride * c.dp);
+            if (!r) r = encode_rows(&a.tm_clo, (const float*)cp.lo, nview, c.dp, stride * c.dp);
+            if (r) return r;
+            a.cn = cn_view;
+            a.thr = thr;
+            a.N = nview;
+            a.split_len = split_len;
+            a.cap = cap;
+            a.clo_flags = flags;
+            KNN_CUDA(launch_tscan(a, splits, s));
+        } else {
+            r = encode_split(&f.tm_chi, cp.hi, nview, D, stride, fscan_tile_rows(D));
+            if (!r) r = encode_split(&f.tm_clo, cp.lo, nview, D, stride, fscan_tile_rows(D));
+            if (r) return r;
+            f.cn = cn_view;
+            f.cs = cs_view;
+            f.thr = thr;
+            f.N = nview;
+            f.split_len = split_len;
+            f.cap = cap;
+            f.clo_flags = flags;
+            KNN_CUDA(launch_fscan(f, splits, s));
+        }
         ++launches;
         return KNNS_OK;
     }
@@ -645,12 +712,13 @@ struct TscanStages {
     {
         float* Tbuf[2] = {(float*)E.tq.p, (float*)E.tq.p + Q};
         float* cnv = (float*)E.cnv.p;
+        float* csv = (float*)E.csv.p;
         CandSelect cs = cand_select();
         T = nullptr;
         for (int l = 0; l < sp.levels; ++l) {
             const ScanLevel& v = sp.lv[l];
-            KNN_CUDA(launch_gather_norms(cn, v.n, v.stride, cnv, v.n_pad, s, std::numeric_limits<float>::infinity(), run_if));
-            int rc = pass(v.n, v.stride, cnv, T, v.S, v.len, v.cap, nullptr);
+            KNN_CUDA(launch_gather_norms(cn, v.n, v.stride, cnv, v.n_pad, s, run_if, cp.rs, cp.rs ? csv : nullptr));
+            int rc = pass(v.n, v.stride, cnv, csv, T, v.S, v.len, v.cap, nullptr);
             if (rc) return rc;
             cs.nseg = kScanParts * v.S;
             cs.cap = v.cap;
@@ -661,10 +729,11 @@ struct TscanStages {
             launches += 2;
             T = Tbuf[l & 1];
             cnv += v.n_pad;
+            csv += v.n_pad;
         }
         return KNNS_OK;
     }
-    int main_pass() { return pass(N, 1, cn, T, sp.S, sp.len, sp.cap, cflags); }
+    int main_pass() { return pass(N, 1, cn, cp.rs, T, sp.S, sp.len, sp.cap, cp.flags); }
     int select()
     {
         uint32_t* fail_cnt = (uint32_t*)fail.p;
@@ -719,23 +788,56 @@ struct TscanStages {
     }
 };
 
-// The exact form on TF32 keys alone (rows wider than 128, k above 128, corpora below the BF16
-// scan's size, or on request): corpus and query norms and TF32 copies, then the stages above.
+// The corpus's hi / lo copies in this engine's buffers: space, and the split itself (skip_unless: as
+// launch_split_f16); any_lo is a word of the search's flags.
+static int ensure_split(Engine& E, const Config& c, int64_t N, int D, int64_t n_pad)
+{
+    const size_t b = c.tf32 ? (size_t)N * c.dp * sizeof(float) : (size_t)N * split_pitch(D) * 2;
+    int rc = E.hi.ensure(b);
+    if (!rc) rc = E.lo.ensure(b);
+    if (!rc && !c.tf32) rc = E.rs.ensure(n_pad * sizeof(float));
+    return rc;
+}
+
+static int split_corpus(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, int D, int64_t n_pad,
+                        uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
+{
+    uint32_t* flags = (uint32_t*)E.loflags.p;
+    if (c.tf32)
+        KNN_CUDA(launch_split_tf32(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, flags, any_lo,
+                                   skip_unless, s));
+    else
+        KNN_CUDA(launch_split_f16(corpus, N, ldc, D, E.hi.p, E.lo.p, (float*)E.rs.p, n_pad, flags, any_lo,
+                                  skip_unless, s));
+    return KNNS_OK;
+}
+
+// the copies a search reads: the index's or the engine's
+static SplitCopies split_copies(const Engine& E, const Config& c, const PreparedCorpus* pc)
+{
+    if (c.tf32)
+        return pc ? SplitCopies{pc->thi.p, pc->tlo.p, nullptr, (const uint32_t*)pc->ttiles.p}
+                  : SplitCopies{E.hi.p, E.lo.p, nullptr, (const uint32_t*)E.loflags.p};
+    return pc ? SplitCopies{pc->hi.p, pc->lo.p, (const float*)pc->rs.p, (const uint32_t*)pc->tiles.p}
+              : SplitCopies{E.hi.p, E.lo.p, (const float*)E.rs.p, (const uint32_t*)E.loflags.p};
+}
+
+// The exact form on split keys alone (rows wider than 128, k above 128, corpora below the BF16
+// scan's size, or on request): corpus and query norms and FP16 copies, then the stages above.
 static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, const float* queries,
                      int64_t Q, int64_t ldq, int D, int k, float* dist, int32_t* idx, float* idx_f,
                      const knns_options& o, cudaStream_t s, knns_stats* st, const PreparedCorpus* pc, bool capture)
 {
     ScanPlan sp;
-    int rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp, false, true);
+    int rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp, c.tf32 ? kKeyTf32 : kKeyF16);
     if (rc) return rc;
-    const int dp = c.dp;
-    if (pc && (!pc->tf32 || pc->dp != dp))
+    if (pc && !pc->tf32)
         return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies of this width");
+    if (pc && c.tf32 && (rc = prepare_tf32(pc, s, capture))) return rc;
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     if (!pc) {
         rc = E.cn.ensure(n_pad * sizeof(float));
-        if (!rc) rc = E.hi.ensure((size_t)N * dp * sizeof(float));
-        if (!rc) rc = E.lo.ensure((size_t)N * dp * sizeof(float));
+        if (!rc) rc = ensure_split(E, c, N, D, n_pad);
         if (!rc) rc = E.loflags.ensure(((size_t)cdiv(N, 128) + 4) * sizeof(uint32_t));
         if (rc) return rc;
     }
@@ -744,12 +846,9 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     if (rc) return rc;
     uint32_t* words = (uint32_t*)E.words.p;
     float* cn = (float*)(pc ? pc->cn.p : E.cn.p);
-    uint32_t* cflags = (uint32_t*)(pc ? pc->tiles.p : E.loflags.p);
-    TscanStages ts{E, c, sp, corpus, N, ldc, queries, Q, ldq, D, k, cn,
-                   (const float*)(pc ? pc->hi.p : E.hi.p), (const float*)(pc ? pc->lo.p : E.lo.p), cflags,
-                   (const float*)E.qn.p, dist, idx, idx_f, nullptr, words + 1, E.fail, E.thr2, s};
+    TscanStages ts{E, c, sp, corpus, N, ldc, queries, Q, ldq, D, k, cn, split_copies(E, c, pc), (const float*)E.qn.p, dist, idx, idx_f, nullptr, words + 1, E.fail, E.thr2, s};
     if ((rc = ts.ensure())) return rc;
-    const size_t ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.loflags.cap) + E.qn.cap + ts.workspace();
+    const size_t ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap + E.loflags.cap) + E.qn.cap + ts.workspace();
 
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
     cudaEvent_t tv[Engine::kTimingEvents] = {};
@@ -762,7 +861,7 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     KNN_CUDA(cudaMemsetAsync(words, 0, 4 * sizeof(uint32_t), s));
     if (!pc) {
         KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, 0, nullptr, cn, n_pad, nullptr, s));
-        KNN_CUDA(launch_split(corpus, N, ldc, D, dp, (float*)E.hi.p, (float*)E.lo.p, cflags, words, nullptr, s));
+        if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, words, nullptr, s))) return rc;
         ts.launches += 2;
     }
     KNN_CUDA(launch_prep_rows(queries, Q, ldq, D, 0, nullptr, (float*)E.qn.p, Q, nullptr, s));
@@ -826,25 +925,27 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
 
     // The threshold scan serves BF16 keys on large corpora: always in the BF16
     // precision form, and in the exact form when the data turn out BF16-exact; otherwise the
-    // exact form runs the 3xTF32 threshold scan (decided on the device: the kernels of the path
+    // exact form runs the split-key threshold scan (decided on the device: the kernels of the path
     // that does not match the data return at once).
     ScanPlan sp, sp_tf;
     bool scan = false;
     if (c.algo == KNNS_ALGO_TC && o.scan != KNNS_SCAN_OFF && E.cc >= 100 && c.dpb <= 256 && c.rerank) {
         const int64_t min_n = (o.scan == KNNS_SCAN_ON || c.kp > kMaxKpTC) ? kScanMinRowsForced : kScanMinRowsAuto;
         if (N >= min_n) {
-            rc = plan_scan(E, N, Q, c.fp8 ? c.dpf : c.dpb, c.kp, o, &sp, c.fp8);
+            rc = plan_scan(E, N, Q, c.fp8 ? c.dpf : c.dpb, c.kp, o, &sp, c.fp8 ? kKeyF8 : kKeyBf16);
             if (rc) return rc;
             scan = true;
         }
     }
     // E4M3 keys exist only on the scan: without it the form falls back to BF16 keys
     const bool f8 = scan && c.fp8;
-    // beside the BF16 scan, the exact form's TF32 keys run on the 3xTF32 scan; without the scan,
+    // beside the BF16 scan, the exact form's split keys run on the split-key scan; without the scan,
     // on the shortlist kernel
     const bool tf_scan = scan && !bf16_only;
     const bool run_old = !scan;
-    if (tf_scan && (rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp_tf, false, true))) return rc;
+    // the shortlist kernel's split keys are 3xTF32
+    if (run_old) c.tf32 = true;
+    if (tf_scan && (rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp_tf, c.tf32 ? kKeyTf32 : kKeyF16))) return rc;
     if (pc != nullptr) {
         // (the CUDA-core kernel uses the index's norms only)
         if (pc->corpus != corpus || pc->N != N || pc->ldc != ldc || pc->D != D ||
@@ -853,8 +954,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         if (f8 && !pc->fp8) return set_error(KNNS_ERR_INVALID, "the FP8 form needs an index prepared with E4M3 copies");
         if (c.algo == KNNS_ALGO_TC && !bf16_only && !pc->tf32)
             return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies");
-        if (c.algo == KNNS_ALGO_TC && !bf16_only && pc->dp != c.dp)
-            return set_error(KNNS_ERR_INVALID, "prepared corpus has TF32 copies of another width");
+        if (c.algo == KNNS_ALGO_TC && !bf16_only && c.tf32 && (rc = prepare_tf32(pc, s, capture))) return rc;
     }
 
     // norms padded with +inf at least one tile (of any kernel) past the corpus
@@ -911,15 +1011,14 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     }
     if (c.algo == KNNS_ALGO_TC && !pc) {
         if (!bf16_only) {
-            rc = E.hi.ensure((size_t)N * c.dp * sizeof(float));
-            if (!rc) rc = E.lo.ensure((size_t)N * c.dp * sizeof(float));
+            rc = ensure_split(E, c, N, D, n_pad);
             if (rc) return rc;
         }
         rc = E.bf.ensure((size_t)N * c.dpb * 2);
         if (rc) return rc;
         rc = E.loflags.ensure(((size_t)cdiv(N, 128) + 4) * sizeof(uint32_t));
         if (rc) return rc;
-        ws += E.hi.cap + E.lo.cap + E.bf.cap + E.loflags.cap;
+        ws += E.hi.cap + E.lo.cap + E.rs.cap + E.bf.cap + E.loflags.cap;
         if (f8) {
             rc = E.f8.ensure((size_t)N * c.dpf * 2);
             if (!rc) rc = E.cs.ensure(n_pad * sizeof(float));
@@ -941,8 +1040,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     }
     // corpus-side buffers: the index's, or this engine's
     const void* bf_p = pc ? pc->bf.p : E.bf.p;
-    const float* hi_p = (const float*)(pc ? pc->hi.p : E.hi.p);
-    const float* lo_p = (const float*)(pc ? pc->lo.p : E.lo.p);
+    const SplitCopies cp = split_copies(E, c, pc);
     const void* f8_p = pc ? pc->f8.p : E.f8.p;
     const float* cs_p = (const float*)(pc ? pc->cs.p : E.cs.p);
     // BF16 keys on the scan: the corpus norm parts (the scan's last K step)
@@ -963,18 +1061,16 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         ws += E.qbf.cap + E.cand.cap + E.cnt.cap + E.tq.cap + E.cnv.cap + E.fail.cap;
     }
     ws += E.part.cap + E.thr2.cap;
-    // the 3xTF32 scan beside the BF16 one (its buffers are shared with it but for its queries'
-    // TF32 copies and its failed-query list: only one of the two paths runs)
+    // the split-key scan beside the BF16 one (its buffers are shared with it but for its queries'
+    // split and its failed-query list: only one of the two paths runs)
     const float* cn_ts = (const float*)(pc ? pc->cn.p : E.cn.p);
-    TscanStages ts{E, c, sp_tf, corpus, N, ldc, queries, Q, ldq, D, k, cn_ts,
-                   (const float*)(pc ? pc->hi.p : E.hi.p), (const float*)(pc ? pc->lo.p : E.lo.p),
-                   (const uint32_t*)(pc ? pc->tiles.p : E.loflags.p), (const float*)E.qn.p, dist, idx, idx_f,
+    TscanStages ts{E, c, sp_tf, corpus, N, ldc, queries, Q, ldq, D, k, cn_ts, cp, (const float*)E.qn.p, dist, idx, idx_f,
                    (const uint32_t*)E.words.p + 1, (uint32_t*)E.words.p + 5, E.tfail, E.tthr2, s};
     if (tf_scan) {
         if ((rc = ts.ensure())) return rc;
-        ws += E.qhi.cap + E.qlo.cap + E.qlof.cap + E.tfail.cap + E.tthr2.cap;
+        ws += E.qhi.cap + E.qlo.cap + E.qrs.cap + E.qlof.cap + E.tfail.cap + E.tthr2.cap;
     }
-    // Resident corpora (one stream otherwise): the 3xTF32 scan runs on a side stream beside the
+    // Resident corpora (one stream otherwise): the split-key scan runs on a side stream beside the
     // BF16 path, so that the launches of whichever path does not match the data (they return at
     // once) overlap the other path's kernels instead of adding to the search.  The two paths
     // share no buffer that both write: candidates, thresholds and results are written by the
@@ -1034,7 +1130,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
     // ordering events: [0] start, [1] sample landed, [2 + b] block b landed, [2 + nblk + b]
     // block b prepared, [2 + 2 nblk + b] block b scanned, [2 + 3 nblk] flag words cleared,
-    // [3 + 3 nblk] thresholds seeded, [4 + 3 nblk] the TF32 scan done
+    // [3 + 3 nblk] thresholds seeded, [4 + 3 nblk] the split-key scan done
     auto oev = [&](int i) -> cudaEvent_t { return E.order_event(i); };
     if (host_corpus != nullptr || blocked) {
         if (!oev(5 + 3 * nblk) || !E.copy_stream() || (blocked && (!E.prep_stream() || !E.worker_stream(0) ||
@@ -1078,21 +1174,21 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     float* qn = (!c.rerank || scan) ? (float*)E.qn.p : nullptr;
     uint64_t* part = (uint64_t*)E.part.p;
     uint32_t* thr_g = (uint32_t*)E.thr.p;
-    // flag words of this search: [0] TF32 low part in the corpus, [1] corpus or queries not
+    // flag words of this search: [0] low part in the corpus' split, [1] corpus or queries not
     // BF16-exact, [2..3] integrality / max |x| of corpus and queries, [4] always zero
     uint32_t* words = (uint32_t*)E.words.p;
     uint32_t* any_lo = words;
     uint32_t* not_exact = words + 1;
     uint32_t* int_stats = words + 2;
     const uint32_t* zero_word = words + 4;
-    uint32_t* flags = c.algo == KNNS_ALGO_TC ? (uint32_t*)(pc ? pc->tiles.p : E.loflags.p) : nullptr;
+    const uint32_t* flags = c.algo == KNNS_ALGO_TC ? cp.flags : nullptr;
     if (pc) {
         KNN_CUDA(cudaMemcpyAsync(words, pc->words.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
         KNN_CUDA(cudaMemsetAsync(words + 4, 0, 2 * sizeof(uint32_t), s));
     } else {
         KNN_CUDA(cudaMemsetAsync(words, 0, 6 * sizeof(uint32_t), s));
     }
-    // 3xTF32 keys on request: the data count as not BF16-exact (the preparation only ORs into the word)
+    // split keys on request: the data count as not BF16-exact (the preparation only ORs into the word)
     if (o.tf32_only && !bf16_only) KNN_CUDA(cudaMemsetAsync(words + 1, 0x01, 1, s));
     if (blocked) {
         // the corpus blocks, prepared on the preparation stream as they land (their flag words
@@ -1131,12 +1227,11 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                                       int_stats));
         ++launches;
         if (!bf16_only && !pc && !blocked) {
-            // the TF32 split runs only for data that is not BF16-exact
-            KNN_CUDA(launch_split(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, flags, any_lo, not_exact,
-                                  s));
+            // the split runs only for data that is not BF16-exact
+            if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, any_lo, not_exact, s))) return rc;
             ++launches;
         }
-        if (tf_scan && !blocked && (rc = ts.split_queries())) return rc;
+        if (tf_scan && !blocked && !ts_side && (rc = ts.split_queries())) return rc;
     } else {
         if (!pc) {
             KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, 0, nullptr, cn, n_pad, nullptr, s));
@@ -1160,8 +1255,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             memset(&a, 0, sizeof(a));
             int r = 0;
             if (!bf16_only) {
-                r = encode_rows(&a.tm_hi, hi_p, nview, c.dp, stride * c.dp);
-                if (!r) r = encode_rows(&a.tm_lo, lo_p, nview, c.dp, stride * c.dp);
+                r = encode_rows(&a.tm_hi, (const float*)cp.hi, nview, c.dp, stride * c.dp);
+                if (!r) r = encode_rows(&a.tm_lo, (const float*)cp.lo, nview, c.dp, stride * c.dp);
             }
             if (!r) r = encode_rows_bf16(&a.tm_bf, bf_p, nview, c.dpb, stride * c.dpb);
             if (r) return r;
@@ -1330,9 +1425,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             if (f8) {
                 // norms and scales of the sample rows: 0 scales for padding, whose +inf norms keep
                 // their keys at +inf (BF16 keys take the norm parts in place)
-                KNN_CUDA(launch_gather_norms(lv_cn, v.n, v.stride / lv_div, cnv, v.n_pad, s));
-                KNN_CUDA(launch_gather_norms(lv_cs, v.n, v.stride / lv_div, csv, v.n_pad, s, 0.f));
-                launches += 2;
+                KNN_CUDA(launch_gather_norms(lv_cn, v.n, v.stride / lv_div, cnv, v.n_pad, s, nullptr, lv_cs, csv));
+                ++launches;
             }
             if ((rc = scan_pass(key_src, lv_np, v.n, v.stride / lv_div, cnv, csv, T, v.S, v.len, v.cap))) return rc;
             cs.nseg = kScanParts * v.S;
@@ -1346,14 +1440,14 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             cnv += v.n_pad;
             if (csv) csv += v.n_pad;
         }
-        // (the TF32 scan's seeding reuses the sample norms and threshold buffers: the BF16
+        // (the split-key scan's seeding reuses the sample norms and threshold buffers: the BF16
         // levels, run or skipped, are done with them)
         if (ts_side) {
-            // the whole TF32 scan on the side stream, from the prepared inputs on
+            // the whole split-key scan on the side stream, from the prepared inputs on
             KNN_CUDA(cudaEventRecord(E.order_event(0), s));
             KNN_CUDA(cudaStreamWaitEvent(ts_stream, E.order_event(0), 0));
             ts.s = ts_stream;
-            if ((rc = ts.seed()) || (rc = ts.main_pass()) || (rc = ts.select()) || (rc = ts.fix())) return rc;
+            if ((rc = ts.split_queries()) || (rc = ts.seed()) || (rc = ts.main_pass()) || (rc = ts.select()) || (rc = ts.fix())) return rc;
             KNN_CUDA(cudaEventRecord(E.order_event(1), ts_stream));
         } else if (tf_scan && !blocked && (rc = ts.seed())) {
             return rc;
@@ -1376,7 +1470,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                     return rc;
                 KNN_CUDA(cudaEventRecord(oev(2 + 2 * nblk + b), w));
             }
-            // What needs the whole corpus, the TF32 copies and the TF32 scan (gated on the data's
+            // What needs the whole corpus, the split copies and the split-key scan (gated on the data's
             // BF16-exactness in the exact form), runs on the preparation stream: the copies (their own
             // buffers) once the last block is prepared, the flag then final; the scan, which writes
             // the thresholds and candidate segments the BF16 path also uses, once every block is
@@ -1385,8 +1479,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             for (int b = 0; b < nblk; ++b) KNN_CUDA(cudaStreamWaitEvent(s, oev(2 + 2 * nblk + b), 0));
             if (tf_scan) {
                 cudaStream_t ps = E.prep_stream();
-                KNN_CUDA(launch_split(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, flags, any_lo,
-                                      not_exact, ps));
+                if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, any_lo, not_exact, ps))) return rc;
                 ++launches;
                 ts.s = ps;
                 if ((rc = ts.split_queries())) return rc;
@@ -1498,7 +1591,11 @@ void PreparedCorpus::release()
     bf.release();
     hi.release();
     lo.release();
+    rs.release();
     tiles.release();
+    thi.release();
+    tlo.release();
+    ttiles.release();
     words.release();
     f8.release();
     cs.release();
@@ -1511,15 +1608,19 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     if (!pc || !corpus || N <= 0 || D <= 0 || ldc < D) return set_error(KNNS_ERR_INVALID, "invalid corpus");
     if (N > 0x7fffffffLL) return set_error(KNNS_ERR_UNSUPPORTED, "corpus larger than 2^31-1 rows");
     if (E.cc < 100) return set_error(KNNS_ERR_UNSUPPORTED, "a prepared corpus needs sm_100+");
-    const int dpb = (D + 63) & ~63, dp = (D + 31) & ~31;
+    const int dpb = (D + 63) & ~63;
     if (dpb > 256) return set_error(KNNS_ERR_UNSUPPORTED, "a prepared corpus needs D <= 256");
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     int rc = pc->cn.ensure(n_pad * sizeof(float));
     if (!rc) rc = pc->bf.ensure((size_t)N * dpb * 2);
     if (!rc) rc = pc->words.ensure(8 * sizeof(uint32_t));
     if (!rc) rc = pc->tiles.ensure(((size_t)cdiv(N, 128) + 1) * sizeof(uint32_t));
-    if (!rc && tf32) rc = pc->hi.ensure((size_t)N * dp * sizeof(float));
-    if (!rc && tf32) rc = pc->lo.ensure((size_t)N * dp * sizeof(float));
+    // FP16 hi / lo for corpora that the scans take; smaller ones (and the rare searches that need
+    // 3xTF32 keys, see prepare_tf32) keep TF32 hi / lo
+    const bool f16 = tf32 && N >= kScanMinRowsForced;
+    if (!rc && f16) rc = pc->hi.ensure((size_t)N * split_pitch(D) * 2);
+    if (!rc && f16) rc = pc->lo.ensure((size_t)N * split_pitch(D) * 2);
+    if (!rc && f16) rc = pc->rs.ensure(n_pad * sizeof(float));
     const int dpf = ((D + 127) & ~127) / 2;
     if (!rc && fp8) rc = pc->f8.ensure((size_t)N * dpf * 2);
     if (!rc && fp8) rc = pc->cs.ensure(n_pad * sizeof(float));
@@ -1529,9 +1630,9 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     KNN_CUDA(cudaMemsetAsync(w, 0, 8 * sizeof(uint32_t), s));
     KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, dpb, pc->bf.p, (float*)pc->cn.p, n_pad, w + 1, s, w + 2,
                               fp8 ? pc->f8.p : nullptr, 2 * dpf, fp8 ? (float*)pc->cs.p : nullptr, pc->np.p));
-    if (tf32)
-        KNN_CUDA(launch_split(corpus, N, ldc, D, dp, (float*)pc->hi.p, (float*)pc->lo.p, (uint32_t*)pc->tiles.p, w,
-                              nullptr, s));
+    if (f16)
+        KNN_CUDA(launch_split_f16(corpus, N, ldc, D, pc->hi.p, pc->lo.p, (float*)pc->rs.p, n_pad, (uint32_t*)pc->tiles.p,
+                                  w, nullptr, s));
     pc->corpus = corpus;
     pc->N = N;
     pc->ldc = ldc;
@@ -1539,8 +1640,27 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     pc->dpb = dpb;
     pc->dpf = dpf;
     pc->fp8 = fp8;
-    pc->dp = dp;
     pc->tf32 = tf32;
+    pc->f16 = f16;
+    return tf32 && !f16 ? prepare_tf32(pc, s, false) : KNNS_OK;
+}
+
+int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture)
+{
+    std::lock_guard<std::mutex> lk(pc->tmu);
+    if (pc->thi_ready) return KNNS_OK;
+    if (capture) return set_error(KNNS_ERR_INVALID, "the index's TF32 copies have to exist before a capture");
+    const int dp = round32(pc->D);
+    const size_t b = (size_t)pc->N * dp * sizeof(float);
+    int rc = pc->thi.ensure(b);
+    if (!rc) rc = pc->tlo.ensure(b);
+    if (!rc) rc = pc->ttiles.ensure(((size_t)cdiv(pc->N, kTileRows) + 1) * sizeof(uint32_t));
+    if (rc) return rc;
+    KNN_CUDA(launch_split_tf32(pc->corpus, pc->N, pc->ldc, pc->D, dp, (float*)pc->thi.p, (float*)pc->tlo.p,
+                               (uint32_t*)pc->ttiles.p, pc->f16 ? nullptr : (uint32_t*)pc->words.p, nullptr, s));
+    // once per index: later searches on any stream see the copies
+    KNN_CUDA(cudaStreamSynchronize(s));
+    pc->thi_ready = true;
     return KNNS_OK;
 }
 
@@ -1566,8 +1686,8 @@ static int64_t host_block_rows(Engine& E, int64_t N, int64_t Q, int D, int k, in
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return N;
     const double avail = 0.6 * (double)(fr + E.in_corpus.cap + E.bf.cap + E.hi.cap + E.lo.cap + E.cn.cap);
-    // FP32 input, BF16 copy, TF32 hi/lo, norms and flags per row; query-side workspace
-    const double per_row = (double)D * (4 + 2 + 8) + 32;
+    // FP32 input, BF16 copy, FP16 hi / lo, norms, scales and flags per row; query-side workspace
+    const double per_row = (double)D * (4 + 2 + 4) + 96;
     const double fixed = (double)Q * ((double)D * 8 + 8192) + 256.0 * (1 << 20);
     const double rows = (avail - fixed) / per_row;
     if (rows >= (double)N) return N;
@@ -2052,11 +2172,14 @@ int knns_debug_scan_plan(int64_t N, int64_t Q, int D, int k, int sms, int tf32, 
     int kp = auto_kp(k, 1);
     if (kp > 512) kp = std::max(round16(k), 32);  // no margin at the limit (as resolve_config)
     ScanPlan P;
-    const int rc = plan_scan(E, N, Q, (D + 63) & ~63, kp, o, &P, false, tf32 != 0);
+    const ScanKeys keys = !tf32 ? kKeyBf16 : kp < k + kKeyMargin ? kKeyTf32 : kKeyF16;
+    const int rc = plan_scan(E, N, Q, (D + 63) & ~63, kp, o, &P, keys);
     if (rc) return rc;
     memset(out, 0, sizeof(*out));
     out->kp = kp;
-    out->tile_rows = tf32 ? 128 : scan_tile_rows((D + 63) & ~63, P.accs);
+    out->tile_rows = keys == kKeyF16    ? fscan_tile_rows(D)
+                     : keys == kKeyTf32 ? kTileN
+                                        : scan_tile_rows((D + 63) & ~63, P.accs);
     out->levels = P.levels;
     for (int l = 0; l < P.levels; ++l) {
         out->level_rows[l] = P.lv[l].n;
@@ -2100,7 +2223,7 @@ int knns_debug_tc_dot_tile(const float* corpus, int64_t N, const float* queries,
     KNN_CUDA(cudaMemsetAsync(not_exact, 0, sizeof(uint32_t), s));
     KNN_CUDA(launch_bf16(corpus, n_use, D, D, dpb, E->bf.p, not_exact, s));
     KNN_CUDA(launch_bf16(queries, q_use, D, D, dpb, nullptr, not_exact, s));
-    KNN_CUDA(launch_split(corpus, n_use, D, D, dp, (float*)E->hi.p, (float*)E->lo.p, nullptr, nullptr, nullptr, s));
+    KNN_CUDA(launch_split_tf32(corpus, n_use, D, D, dp, (float*)E->hi.p, (float*)E->lo.p, nullptr, nullptr, nullptr, s));
     TcArgs a;
     memset(&a, 0, sizeof(a));
     if ((rc = encode_rows(&a.tm_hi, (const float*)E->hi.p, n_use, dp))) return rc;

@@ -33,8 +33,10 @@ struct Config {
     // E4M3 keys (KNNS_PREC_FP8): the scan's row width in 16-bit units, (D rounded up to 128) / 2
     bool fp8 = false;
     int dpf = 0;
-    // exact form on the 3xTF32 threshold scan (rows wider than 128, or shortlists over 128)
+    // exact form on the split-key threshold scan (rows wider than 128, or shortlists over 128)
     bool tscan = false;
+    // split keys are 3xTF32 (shortlists without a margin, rerank = 0, the shortlist kernel), else FP16
+    bool tf32 = false;
 };
 
 struct Engine {
@@ -43,19 +45,19 @@ struct Engine {
     int cc = 0;
     std::mutex mu;
     cudaEvent_t last_done = nullptr;
-    DevBuf cn, qn, part, hi, lo, bf, err, thr, loflags, cn_s, thr2, redo;
+    DevBuf cn, qn, part, hi, lo, rs, bf, err, thr, loflags, cn_s, thr2, redo;
     // threshold-scan path: BF16 queries, candidate segments and counts, seeded
     // thresholds, sample norms, failed-query list
     DevBuf qbf, cand, cnt, tq, cnv, fail;
     // E4M3 keys: corpus codes and row scales, query scales, sample scales
     DevBuf f8, cs, qs, csv;
-    // 3xTF32 scan: the queries' TF32 hi / lo copies and the low-part flags of their tiles; the
+    // split-key scan: the queries' hi / lo copies, row scales and the low-part flags of their tiles; the
     // failed-query list and fix-up thresholds of the scan when it runs beside the BF16 scan
     // (exact form)
-    DevBuf qhi, qlo, qlof, tfail, tthr2;
-    // per-search flag words: [0] some corpus tile has a TF32 low part, [1] corpus or
+    DevBuf qhi, qlo, qrs, qlof, tfail, tthr2;
+    // per-search flag words: [0] some corpus tile has a low part, [1] corpus or
     // queries not BF16-exact, [2] some value not an integer, [3] max |x| (float bits), [4] zero,
-    // [5] some query tile has a TF32 low part
+    // [5] some query tile has a low part
     DevBuf words;
     DevBuf in_corpus, in_queries, out_dist, out_idx;
     // corpus blocks of host-buffer searches: two running top-k lists (distances, indices)
@@ -91,16 +93,22 @@ struct Engine {
 };
 
 // A corpus prepared once and kept resident (the serving index): BF16 copy,
-// norms, optional TF32 hi/lo copies with their per-tile low-part flags,
+// norms, optional FP16 hi/lo copies with row scales and per-tile low-part flags,
 // optional E4M3 codes with per-row scales, and the corpus half of the flag words ([0] low part, [1] not BF16-exact,
 // [2] not integer, [3] max |x| bits).  The caller keeps the FP32 corpus alive
 // and unchanged while the index is used.
 struct PreparedCorpus {
     const float* corpus = nullptr;
     int64_t N = 0, ldc = 0;
-    int D = 0, dpb = 0, dp = 0, dpf = 0;
+    int D = 0, dpb = 0, dpf = 0;
     bool tf32 = false, fp8 = false;
-    DevBuf cn, bf, hi, lo, tiles, words, f8, cs, np;
+    DevBuf cn, bf, hi, lo, rs, tiles, words, f8, cs, np;
+    // FP16 copies present (hi, lo, rs, tiles); TF32 copies, made by the first search that needs them
+    // (prepare_tf32)
+    bool f16 = false;
+    mutable std::mutex tmu;
+    mutable bool thi_ready = false;
+    mutable DevBuf thi, tlo, ttiles;
     void release();
 };
 
@@ -124,6 +132,9 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                const float* host_corpus = nullptr);
 int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N, int64_t ldc, int D, bool tf32,
                    cudaStream_t s, bool fp8 = false);
+// TF32 hi / lo copies of a prepared corpus (nothing when they exist; an error while capturing).
+// Synchronises s when it makes them.
+int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture);
 int check_device_error(Engine& E, cudaStream_t s);
 int search_host(const float* corpus, int64_t N, const float* queries, int64_t Q, int D, int k, float* dist,
                 int32_t* idx, float* idx_f_host, const knns_options& o, double* seconds, knns_stats* st);

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
                             for (int kk = 0; kk < 4; ++kk) {
                                 const uint64_t db = ptx::desc_sw128_kmajor(hi_addr + bx * kHalfBytes + kk * 32);
                                 const uint32_t acol = tmem + box * 32u + (uint32_t)(kk * 8);
-                                ptx::mma_bf16_ts(d_tmem, acol, db, kIdescBf16, (c | bx | kk) != 0);
+                                ptx::mma_f16_ts(d_tmem, acol, db, kIdescBf16, (c | bx | kk) != 0);
                             }
                         }
                     } else {

@@ -2,7 +2,6 @@
 #pragma once
 
 #include <cstdint>
-#include <limits>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -28,10 +27,19 @@ enum DeviceError : int {
 
 cudaError_t launch_norms(const float* x, int64_t n, int64_t ld, int D, float* out, int64_t n_pad,
                          cudaStream_t s);
+// FP16 split of every row: hi = fp16(s x), lo = fp16(s x - hi), s the power of two that puts the
+// row's largest |x| into [2^14, 2^15); hi / lo are [n][hp] FP16 (hp = split_pitch(D), zero padded),
+// rs[0..n_pad) the reciprocals 1 / s (0 for n <= i < n_pad).  lo_flags[tile of 128 rows] = any lo
+// != 0 (may be null); *any_lo (zeroed by the caller, may be null) becomes 1 when some tile has a
+// low part.  When skip_unless is given and *skip_unless == 0 at run time, the kernel does nothing.
+constexpr int kTileRows = 128;
+__host__ __device__ constexpr int split_pitch(int D) { return (D + 7) & ~7; }  // rows of whole 16-byte words
+cudaError_t launch_split_f16(const float* x, int64_t n, int64_t ld, int D, void* hi, void* lo, float* rs, int64_t n_pad,
+                         uint32_t* lo_flags, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s);
 // TF32 hi/lo split into [n][dp] arrays; lo_flags[tile of 128 rows] = any lo != 0 (may be null);
 // *any_lo (zeroed by the caller, may be null) becomes 1 when some tile has a low part.  When
 // skip_unless is given and *skip_unless == 0 at run time, the kernel does nothing.
-cudaError_t launch_split(const float* x, int64_t n, int64_t ld, int D, int dp, float* hi, float* lo,
+cudaError_t launch_split_tf32(const float* x, int64_t n, int64_t ld, int D, int dp, float* hi, float* lo,
                          uint32_t* lo_flags, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s);
 // BF16 copy into [n][dpb] (out may be null: check only); *not_exact |= 1 when some element
 // is not exactly representable in BF16.
@@ -186,6 +194,39 @@ size_t tscan_smem_bytes(int ring, bool tmem_a);
 int tscan_ring(bool tmem_a);
 cudaError_t launch_tscan(const TscanArgs& a, int splits, cudaStream_t s);
 
+// Tensor-core FP16-split threshold scan (csrc/scan_f16.cu): 128 queries x fscan_tile_rows(D)-row
+// corpus tiles, K in chunks of 64 FP16 columns; the candidate segments are those of the BF16 scan
+// (kScanParts per split, fscan_part_cols(D) columns of every tile each).  Operands as launch_split_f16
+// writes them.
+constexpr int kFscanTmemD = 256;  // widest rows whose queries sit in tensor memory
+struct FscanArgs {
+    CUtensorMap tm_qhi, tm_qlo;   // D > kFscanTmemD: queries hi / lo [Q][hp] fp16, box {64, 128}, 128B swizzle
+    CUtensorMap tm_chi, tm_clo;   // corpus hi / lo view [N][hp] fp16, box {64, tile rows}, 128B swizzle
+    const uint16_t* qhi;          // queries hi / lo [Q][hp] fp16 (D <= kFscanTmemD)
+    const uint16_t* qlo;
+    const float* qs;              // [Q] query row scales
+    const float* cn;              // [>= N + tile rows] corpus norms of the view, +inf padding
+    const float* cs;              // [>= N + tile rows] corpus row scales of the view, 0 padding
+    const float* thr;             // [Q] thresholds (null: +inf, every key collected)
+    const uint32_t* qlo_flags;    // D > kFscanTmemD: [query tiles] 1 when the tile has a low part (null: all)
+    const uint32_t* clo_flags;    // [128-row tiles of the view, + 1] same for the corpus (null: all)
+    uint64_t* cand;               // [splits*kScanParts][Q][cap]
+    uint32_t* cnt;                // [splits*kScanParts][Q]
+    int* err;                     // device error word
+    int64_t Q;
+    int64_t N;
+    int64_t split_len;            // multiple of the tile rows
+    int cap;
+    int D;
+    int hp;                       // row pitch of the queries' copies
+    int split0;                   // first split of this launch
+    const uint32_t* run_if;       // optional: the kernel returns at once when *run_if == 0
+};
+int fscan_tile_rows(int D);
+int fscan_part_cols(int D);
+int fscan_ring(int D);
+cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st);
+
 // Merge of the per-split shortlists, optional exact re-rank, final top-k.
 // Extra modes (all optional):
 //  * thr_out: instead of results, write the order-mapped key of the merged
@@ -271,10 +312,11 @@ cudaError_t launch_merge_topk(const float* run_d, const int32_t* run_i, int have
                               const int32_t* blk_i, int kb, int32_t offset, int64_t Q, int k, float* out_d,
                               int32_t* out_i, float* out_idx_f, cudaStream_t s);
 
-// out[i] = src[i * stride] for i < n, pad for n <= i < n_pad (+inf: norms of padding rows), the
+// out[i] = src[i * stride] for i < n, +inf for n <= i < n_pad (norms of padding rows), the
 // norms of a strided corpus sample; nothing when skip_unless is given and *skip_unless == 0.
+// With scales / out_scales the row scales of the sample are gathered too (padding 0).
 cudaError_t launch_gather_norms(const float* src, int64_t n, int64_t stride, float* out, int64_t n_pad,
-                                cudaStream_t s, float pad = std::numeric_limits<float>::infinity(),
-                                const uint32_t* skip_unless = nullptr);
+                                cudaStream_t s, const uint32_t* skip_unless = nullptr,
+                                const float* scales = nullptr, float* out_scales = nullptr);
 
 }  // namespace knn

@@ -1,4 +1,4 @@
-// prep.cu -- corpus/query preparation: row norms and the TF32 hi/lo split.
+// prep.cu -- corpus/query preparation: row norms, BF16 / E4M3 copies and the FP16 hi/lo split.
 //
 // Replaces the reference's norm kernels crpdot2_* / dot4_* (include/utils.h:72-357,
 // 516-766), which reduce x_d^2 in float with a warp-synchronous tree.  Here a
@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 #include "common.cuh"
@@ -79,7 +80,7 @@ __global__ void bf16_tiles_kernel(const float* __restrict__ x, int64_t n, int64_
 // One block per 128-row tile, one warp per row at a time (eight rows in flight per block), each
 // lane a float4 of columns: coalesced 16-byte loads and stores.  lo_flags[tile] = 1 when any lo
 // in the tile is nonzero (the tensor-core kernels skip the correction products otherwise).
-__global__ void __launch_bounds__(256) split_tiles_kernel(const float* __restrict__ x, int64_t n, int64_t ld, int D,
+__global__ void __launch_bounds__(256) split_tf32_kernel(const float* __restrict__ x, int64_t n, int64_t ld, int D,
                                                           int dp, float* __restrict__ hi, float* __restrict__ lo,
                                                           uint32_t* __restrict__ lo_flags,
                                                           uint32_t* __restrict__ any_lo,
@@ -129,13 +130,76 @@ __global__ void __launch_bounds__(256) split_tiles_kernel(const float* __restric
     }
 }
 
+// FP16 split (launch_split_f16): one block per 128-row tile, one warp per row at a time, each lane
+// four columns of a 128-column chunk; a row is read twice (its maximum, then the split).
+__global__ void __launch_bounds__(256) split_f16_kernel(const float* __restrict__ x, int64_t n, int64_t ld, int D,
+                                                          int hp, __half* __restrict__ hi, __half* __restrict__ lo,
+                                                          float* __restrict__ rs, int64_t n_pad,
+                                                          uint32_t* __restrict__ lo_flags,
+                                                          uint32_t* __restrict__ any_lo,
+                                                          const uint32_t* __restrict__ skip_unless)
+{
+    // BF16-exact inputs are searched by the BF16 kernels: nothing to prepare
+    if (skip_unless && *skip_unless == 0u) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t r0 = (int64_t)blockIdx.x * kTileRows;
+    // 16-byte loads when every row starts 16-byte aligned and holds whole float4s
+    const bool vec = (ld % 4 == 0) && (D % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
+    uint32_t any = 0;
+    for (int rr = warp; rr < kTileRows; rr += 8) {
+        const int64_t r = r0 + rr;
+        if (r >= n) break;  // warp-uniform
+        const float* row = x + r * ld;
+        auto load = [&](int c, float (&v)[4]) {
+            if (vec) {
+                float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (c < D) t = __ldg(reinterpret_cast<const float4*>(row + c));
+                v[0] = t.x;
+                v[1] = t.y;
+                v[2] = t.z;
+                v[3] = t.w;
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = c + i < D ? __ldg(row + c + i) : 0.f;
+            }
+        };
+        float mx = 0.f, v[4];
+        for (int c = 4 * lane; c < hp; c += 128) {
+            load(c, v);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mx = fmaxf(mx, fabsf(v[i]));
+        }
+        mx = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
+        float inv;
+        const float sc = row_scale(mx, inv);
+        for (int c = 4 * lane; c < hp; c += 128) {
+            load(c, v);
+            uint2 h, l;
+            any |= split_pair(v[0], v[1], sc, h.x, l.x);
+            any |= split_pair(v[2], v[3], sc, h.y, l.y);
+            *reinterpret_cast<uint2*>(hi + r * hp + c) = h;
+            *reinterpret_cast<uint2*>(lo + r * hp + c) = l;
+        }
+        if (lane == 0) rs[r] = inv;
+    }
+    if (blockIdx.x == gridDim.x - 1)
+        for (int64_t i = n + threadIdx.x; i < n_pad; i += blockDim.x) rs[i] = 0.f;
+    any = __syncthreads_or(any != 0u);
+    if (threadIdx.x == 0) {
+        if (lo_flags) lo_flags[blockIdx.x] = any ? 1u : 0u;
+        if (any && any_lo) atomicOr(any_lo, 1u);
+    }
+}
+
 __global__ void gather_norms_kernel(const float* __restrict__ src, int64_t n, int64_t stride, float* __restrict__ out,
-                                    int64_t n_pad, float pad, const uint32_t* __restrict__ skip_unless)
+                                    int64_t n_pad, const uint32_t* __restrict__ skip_unless,
+                                    const float* __restrict__ scales, float* __restrict__ out_scales)
 {
     if (skip_unless && *skip_unless == 0u) return;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
-    out[i] = i < n ? src[i * stride] : pad;
+    out[i] = i < n ? src[i * stride] : __int_as_float(0x7f800000);
+    if (out_scales) out_scales[i] = i < n ? scales[i * stride] : 0.f;
 }
 
 // Fused preparation of a row-major matrix in one coalesced read, one warp per
@@ -517,11 +581,12 @@ cudaError_t launch_prep_rows(const float* x, int64_t n, int64_t ld, int D, int d
 }
 
 cudaError_t launch_gather_norms(const float* src, int64_t n, int64_t stride, float* out, int64_t n_pad,
-                                cudaStream_t s, float pad, const uint32_t* skip_unless)
+                                cudaStream_t s, const uint32_t* skip_unless, const float* scales, float* out_scales)
 {
     if (n_pad <= 0) return cudaSuccess;
-    gather_norms_kernel<<<(unsigned)((n_pad + 255) / 256), 256, 0, s>>>(src, n, stride, out, n_pad, pad,
-                                                                         skip_unless);
+    if ((scales == nullptr) != (out_scales == nullptr)) return cudaErrorInvalidValue;
+    gather_norms_kernel<<<(unsigned)((n_pad + 255) / 256), 256, 0, s>>>(src, n, stride, out, n_pad, skip_unless,
+                                                                         scales, out_scales);
     return cudaGetLastError();
 }
 
@@ -535,13 +600,24 @@ cudaError_t launch_norms(const float* x, int64_t n, int64_t ld, int D, float* ou
     return cudaGetLastError();
 }
 
-cudaError_t launch_split(const float* x, int64_t n, int64_t ld, int D, int dp, float* hi, float* lo,
+cudaError_t launch_split_f16(const float* x, int64_t n, int64_t ld, int D, void* hi, void* lo, float* rs, int64_t n_pad,
+                         uint32_t* lo_flags, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    const int64_t tiles = (n + kTileRows - 1) / kTileRows;
+    split_f16_kernel<<<(unsigned)tiles, 256, 0, s>>>(x, n, ld, D, split_pitch(D), static_cast<__half*>(hi),
+                                                       static_cast<__half*>(lo), rs, n_pad, lo_flags, any_lo,
+                                                       skip_unless);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_split_tf32(const float* x, int64_t n, int64_t ld, int D, int dp, float* hi, float* lo,
                          uint32_t* lo_flags, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
     if (dp % 4 != 0 || dp < D) return cudaErrorInvalidValue;  // rows of whole float4s
     const int64_t tiles = (n + 127) / 128;
-    split_tiles_kernel<<<(unsigned)tiles, 256, 0, s>>>(x, n, ld, D, dp, hi, lo, lo_flags, any_lo, skip_unless);
+    split_tf32_kernel<<<(unsigned)tiles, 256, 0, s>>>(x, n, ld, D, dp, hi, lo, lo_flags, any_lo, skip_unless);
     return cudaGetLastError();
 }
 

@@ -286,13 +286,13 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                                 ptx::mma_f8_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db, kIdesc,
                                                (box | kk) != 0);
                             else
-                                ptx::mma_bf16_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db, kIdesc,
+                                ptx::mma_f16_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db, kIdesc,
                                                  (box | kk) != 0);
                         }
                     }
                     // BF16 keys: + ones x norm parts, the norms added inside the tensor core
                     if (kNM && c == slots_per_tile - 1)
-                        ptx::mma_bf16_ss(d_tmem, ptx::desc_sw32_kmajor(ptx::smem_u32(ones)),
+                        ptx::mma_f16_ss(d_tmem, ptx::desc_sw32_kmajor(ptx::smem_u32(ones)),
                                          ptx::desc_sw32_kmajor(ptx::smem_u32(np_ring + (size_t)st * np_bytes(TN))),
                                          kIdesc, 1u);
                     // after the tile's last MMAs the accumulator-ready commit goes first: the

@@ -1,15 +1,9 @@
 // scan_tf32.cu -- tensor-core 3xTF32 threshold scan for FP32 data of any width and
 // shortlists of up to 512 entries.
 //
-// The exact form's distance stage for the shapes the shortlist kernel
-// (fused_tc.cu: queries in tensor memory, D <= 128; shortlists in shared
-// memory, <= 128 entries) cannot take: the reference's pdist_NT SGEMM
-// (include/utils.h:957-985) followed by its selections (bitonic_shared,
-// src/cuknnBitonic.cu:45-254, up to k = 512; the heap of src/cuknnHeap.cu:146-291
-// for large k), restructured as the BF16 threshold scan is (scan_bf16.cu): every
-// key ||c||^2 - 2 q.c strictly below the query's seeded threshold is appended to
-// the query's candidate segment, and select_cand_kernel takes the shortlist from
-// the segments and re-ranks it by exact distance.
+// The scan on split keys (scan_f16.cu) with TF32 operands instead of FP16 ones, at half its rate:
+// it serves the searches whose result depends on the keys' rounding -- shortlists without a margin
+// over k (k close to 512, or to 128 beside the BF16 scan), and rerank = 0, which returns the keys.
 //
 // Keys: with x = hi + lo (hi = tf32(x), lo = tf32(x - hi)), q.c is accumulated in
 // FP32 as qhi.chi + qhi.clo + qlo.chi by tcgen05.mma.kind::tf32; a correction

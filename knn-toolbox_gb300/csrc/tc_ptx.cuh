@@ -130,8 +130,9 @@ __device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, ui
         : "memory");
 }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc]^T, kind::f16 (BF16 operands, FP32 accumulate), cta_group::1
-__device__ __forceinline__ void mma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+// D[tmem] (+)= A[smem desc] * B[smem desc]^T, kind::f16 (BF16 or FP16 operands as named in
+// idesc, both of one type, FP32 accumulate), cta_group::1
+__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate)
 {
     asm volatile(
@@ -142,8 +143,9 @@ __device__ __forceinline__ void mma_bf16_ss(uint32_t d_tmem, uint64_t a_desc, ui
         : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem desc]^T, kind::f16 (BF16 operands, FP32 accumulate), cta_group::1
-__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+// D[tmem] (+)= A[tmem] * B[smem desc]^T, kind::f16 (BF16 or FP16 operands as named in
+// idesc, both of one type, FP32 accumulate), cta_group::1
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
                                             uint32_t accumulate)
 {
     asm volatile(
@@ -318,6 +320,16 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N)
     return (1u << 4)                       // D format f32
            | (1u << 7)                     // A format bf16
            | (1u << 10)                    // B format bf16
+           | ((uint32_t)(N >> 3) << 17)    // N / 8
+           | ((uint32_t)(M >> 4) << 24);   // M / 16
+}
+
+// Instruction descriptor: kind::f16 with FP16 A/B (format code 0), D f32, K-major, M x N.
+__host__ __device__ constexpr uint32_t idesc_f16(int M, int N)
+{
+    return (1u << 4)                       // D format f32
+           | (0u << 7)                     // A format f16
+           | (0u << 10)                    // B format f16
            | ((uint32_t)(N >> 3) << 17)    // N / 8
            | ((uint32_t)(M >> 4) << 24);   // M / 16
 }
