@@ -8,7 +8,7 @@
 // memory, each query carries a threshold T (seeded from samples of the
 // corpus by the engine) and every key strictly below T is appended to the
 // query's candidate segment in global memory.  The final top-kp is chosen
-// from the segments by select_cand_kernel.  Keys are the reference's ranking
+// from the segments by the selection (select.cu).  Keys are the reference's ranking
 // key ||c||^2 - 2 q.c (demo/knn.m:5), formed whole by the tensor core: A = -2 q
 // (exact in BF16) against the corpus rows, then an all-ones A block against the
 // rows' norms split into three BF16 parts (n1 + n2 + n3 = ||c||^2 exactly), one

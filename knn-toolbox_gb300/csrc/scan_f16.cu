@@ -6,7 +6,7 @@
 // selections (bitonic_shared, src/cuknnBitonic.cu:45-254, up to k = 512; the heap of
 // src/cuknnHeap.cu:146-291 for large k), restructured as the BF16 threshold scan is
 // (scan_bf16.cu): every key ||c||^2 - 2 q.c strictly below the query's seeded threshold is
-// appended to the query's candidate segment, and select_cand_kernel takes the shortlist from the
+// appended to the query's candidate segment, and the selection (select.cu) takes the shortlist from the
 // segments and re-ranks it by exact distance.
 //
 // Keys: every row x is scaled by a power of two s that puts max |x| into [2^14, 2^15), then
