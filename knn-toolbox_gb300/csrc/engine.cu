@@ -196,6 +196,21 @@ static int encode_np(CUtensorMap* m, const void* base, int64_t rows, int64_t pit
     return KNNS_OK;
 }
 
+// ---------------------------------------------------------------- flag words of a search
+// E.words: 8 words (see Engine), then the low-part flags of the query tiles and, for a corpus
+// prepared by the search, of its 128-row tiles: cleared by one memset.
+static int flag_words(Engine& E, int64_t Q, int64_t N_own, size_t* count)
+{
+    const size_t nq = (size_t)(Q + kTileRows - 1) / kTileRows + 4;
+    const size_t nc = N_own > 0 ? (size_t)(N_own + kTileRows - 1) / kTileRows + 4 : 0;
+    *count = 8 + nq + nc;
+    const int rc = E.words.ensure(*count * sizeof(uint32_t));
+    if (rc) return rc;
+    E.qlof = (uint32_t*)E.words.p + 8;
+    E.lof = N_own > 0 ? E.qlof + nq : nullptr;
+    return KNNS_OK;
+}
+
 // ---------------------------------------------------------------- planning
 // smallest corpus the threshold scan runs on when asked to (KNNS_SCAN_ON, long shortlists)
 constexpr int64_t kScanMinRowsForced = 16384;
@@ -597,7 +612,6 @@ struct TscanStages {
         int rc = E.qhi.ensure(qb);
         if (!rc) rc = E.qlo.ensure(qb);
         if (!rc) rc = E.qrs.ensure(Q * sizeof(float));
-        if (!rc) rc = E.qlof.ensure(((size_t)cdiv(Q, kTileRows) + 4) * sizeof(uint32_t));
         if (!rc) rc = E.tq.ensure((size_t)2 * Q * sizeof(float));
         if (!rc) rc = E.cand.ensure(sp.cand_words * sizeof(uint64_t));
         if (!rc) rc = E.cnt.ensure(sp.cnt_words * sizeof(uint32_t));
@@ -610,11 +624,20 @@ struct TscanStages {
     }
     size_t workspace() const
     {
-        return E.qhi.cap + E.qlo.cap + E.qrs.cap + E.qlof.cap + E.tq.cap + E.cand.cap + E.cnt.cap + E.cnv.cap +
+        return E.qhi.cap + E.qlo.cap + E.qrs.cap + E.tq.cap + E.cand.cap + E.cnt.cap + E.cnv.cap +
                E.csv.cap + fail.cap + E.part.cap + thr2.cap;
     }
-    // the queries' split and the scan's query operands
-    int split_queries()
+    // The FP16 split of the queries, as outputs of their preparation pass.
+    void prep_outputs(PrepJob* j) const
+    {
+        if (c.tf32) return;
+        j->hi = E.qhi.p;
+        j->lo = E.qlo.p;
+        j->rs = (float*)E.qrs.p;
+        j->lo_flags = E.qlof;
+    }
+    // the scan's query operands (3xTF32 keys: split here)
+    int query_operands()
     {
         if (c.tf32) {
             memset(&a, 0, sizeof(a));
@@ -625,13 +648,13 @@ struct TscanStages {
                 a.ldq = ldq;
                 a.D = D;
             } else {
-                KNN_CUDA(launch_split_tf32(queries, Q, ldq, D, c.dp, (float*)E.qhi.p, (float*)E.qlo.p,
-                                           (uint32_t*)E.qlof.p, q_any_lo, run_if, s));
+                KNN_CUDA(launch_split_tf32(queries, Q, ldq, D, c.dp, (float*)E.qhi.p, (float*)E.qlo.p, E.qlof,
+                                           q_any_lo, run_if, s));
                 ++launches;
                 int rc = encode_rows(&a.tm_qhi, (const float*)E.qhi.p, Q, c.dp, c.dp);
                 if (!rc) rc = encode_rows(&a.tm_qlo, (const float*)E.qlo.p, Q, c.dp, c.dp);
                 if (rc) return rc;
-                a.qlo_flags = (const uint32_t*)E.qlof.p;
+                a.qlo_flags = E.qlof;
             }
             a.cand = (uint64_t*)E.cand.p;
             a.cnt = (uint32_t*)E.cnt.p;
@@ -643,9 +666,6 @@ struct TscanStages {
             return KNNS_OK;
         }
         memset(&f, 0, sizeof(f));
-        KNN_CUDA(launch_split_f16(queries, Q, ldq, D, E.qhi.p, E.qlo.p, (float*)E.qrs.p, Q, (uint32_t*)E.qlof.p,
-                                  q_any_lo, run_if, s));
-        ++launches;
         if (D > kFscanTmemD) {
             int rc = encode_split(&f.tm_qhi, E.qhi.p, Q, D, 1, kTileQ);
             if (!rc) rc = encode_split(&f.tm_qlo, E.qlo.p, Q, D, 1, kTileQ);
@@ -654,7 +674,7 @@ struct TscanStages {
         f.qhi = (const uint16_t*)E.qhi.p;
         f.qlo = (const uint16_t*)E.qlo.p;
         f.qs = (const float*)E.qrs.p;
-        f.qlo_flags = (const uint32_t*)E.qlof.p;
+        f.qlo_flags = E.qlof;
         f.cand = (uint64_t*)E.cand.p;
         f.cnt = (uint32_t*)E.cnt.p;
         f.err = (int*)E.err.p;
@@ -788,8 +808,29 @@ struct TscanStages {
     }
 };
 
-// The corpus's hi / lo copies in this engine's buffers: space, and the split itself (skip_unless: as
-// launch_split_f16); any_lo is a word of the search's flags.
+static PrepJob prep_job(const float* x, int64_t n, int64_t ld, int D, float* norms, int64_t n_pad)
+{
+    PrepJob j;
+    j.x = x;
+    j.n = n;
+    j.ld = ld;
+    j.D = D;
+    j.norms = norms;
+    j.n_pad = n_pad;
+    return j;
+}
+
+// the engine's FP16 corpus copies as outputs of a preparation
+static void split_outputs(Engine& E, PrepJob* j, uint32_t* any_lo)
+{
+    j->hi = E.hi.p;
+    j->lo = E.lo.p;
+    j->rs = (float*)E.rs.p;
+    j->lo_flags = E.lof;
+    j->any_lo = any_lo;
+}
+
+// Space for the corpus's hi / lo copies in this engine's buffers.
 static int ensure_split(Engine& E, const Config& c, int64_t N, int D, int64_t n_pad)
 {
     const size_t b = c.tf32 ? (size_t)N * c.dp * sizeof(float) : (size_t)N * split_pitch(D) * 2;
@@ -799,16 +840,20 @@ static int ensure_split(Engine& E, const Config& c, int64_t N, int D, int64_t n_
     return rc;
 }
 
+// The split of a whole corpus: 3xTF32 copies, or the FP16 side of its preparation (norms too when
+// given).  skip_unless: nothing happens when *skip_unless == 0 at run time.
 static int split_corpus(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, int D, int64_t n_pad,
-                        uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
+                        float* norms, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
 {
-    uint32_t* flags = (uint32_t*)E.loflags.p;
-    if (c.tf32)
-        KNN_CUDA(launch_split_tf32(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, flags, any_lo,
-                                   skip_unless, s));
-    else
-        KNN_CUDA(launch_split_f16(corpus, N, ldc, D, E.hi.p, E.lo.p, (float*)E.rs.p, n_pad, flags, any_lo,
-                                  skip_unless, s));
+    if (c.tf32) {
+        if (norms) KNN_CUDA(launch_row_norms(corpus, N, ldc, D, norms, n_pad, s));
+        KNN_CUDA(launch_split_tf32(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, E.lof, any_lo, skip_unless, s));
+        return KNNS_OK;
+    }
+    PrepJob j = prep_job(corpus, N, ldc, D, norms, n_pad);
+    split_outputs(E, &j, any_lo);
+    j.run_if = skip_unless;
+    KNN_CUDA(launch_prep(j, s));
     return KNNS_OK;
 }
 
@@ -817,9 +862,9 @@ static SplitCopies split_copies(const Engine& E, const Config& c, const Prepared
 {
     if (c.tf32)
         return pc ? SplitCopies{pc->thi.p, pc->tlo.p, nullptr, (const uint32_t*)pc->ttiles.p}
-                  : SplitCopies{E.hi.p, E.lo.p, nullptr, (const uint32_t*)E.loflags.p};
+                  : SplitCopies{E.hi.p, E.lo.p, nullptr, E.lof};
     return pc ? SplitCopies{pc->hi.p, pc->lo.p, (const float*)pc->rs.p, (const uint32_t*)pc->tiles.p}
-              : SplitCopies{E.hi.p, E.lo.p, (const float*)E.rs.p, (const uint32_t*)E.loflags.p};
+              : SplitCopies{E.hi.p, E.lo.p, (const float*)E.rs.p, E.lof};
 }
 
 // The exact form on split keys alone (rows wider than 128, k above 128, corpora below the BF16
@@ -838,17 +883,17 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     if (!pc) {
         rc = E.cn.ensure(n_pad * sizeof(float));
         if (!rc) rc = ensure_split(E, c, N, D, n_pad);
-        if (!rc) rc = E.loflags.ensure(((size_t)cdiv(N, 128) + 4) * sizeof(uint32_t));
         if (rc) return rc;
     }
     rc = E.qn.ensure(Q * sizeof(float));
-    if (!rc) rc = E.words.ensure(8 * sizeof(uint32_t));
+    size_t nwords = 0;
+    if (!rc) rc = flag_words(E, Q, pc ? 0 : N, &nwords);
     if (rc) return rc;
     uint32_t* words = (uint32_t*)E.words.p;
     float* cn = (float*)(pc ? pc->cn.p : E.cn.p);
     TscanStages ts{E, c, sp, corpus, N, ldc, queries, Q, ldq, D, k, cn, split_copies(E, c, pc), (const float*)E.qn.p, dist, idx, idx_f, nullptr, words + 1, E.fail, E.thr2, s};
     if ((rc = ts.ensure())) return rc;
-    const size_t ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap + E.loflags.cap) + E.qn.cap + ts.workspace();
+    const size_t ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qn.cap + ts.workspace();
 
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
     cudaEvent_t tv[Engine::kTimingEvents] = {};
@@ -858,15 +903,16 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
         return KNNS_OK;
     };
     if ((rc = mark(0))) return rc;
-    KNN_CUDA(cudaMemsetAsync(words, 0, 4 * sizeof(uint32_t), s));
+    KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
     if (!pc) {
-        KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, 0, nullptr, cn, n_pad, nullptr, s));
-        if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, words, nullptr, s))) return rc;
-        ts.launches += 2;
+        if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, cn, words, nullptr, s))) return rc;
+        ++ts.launches;
     }
-    KNN_CUDA(launch_prep_rows(queries, Q, ldq, D, 0, nullptr, (float*)E.qn.p, Q, nullptr, s));
+    PrepJob qj = prep_job(queries, Q, ldq, D, (float*)E.qn.p, Q);
+    ts.prep_outputs(&qj);
+    KNN_CUDA(launch_prep(qj, s));
     ++ts.launches;
-    if ((rc = ts.split_queries())) return rc;
+    if ((rc = ts.query_operands())) return rc;
     if ((rc = mark(1))) return rc;
     if ((rc = ts.seed())) return rc;
     if ((rc = mark(2))) return rc;
@@ -942,6 +988,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     // beside the BF16 scan, the exact form's split keys run on the split-key scan; without the scan,
     // on the shortlist kernel
     const bool tf_scan = scan && !bf16_only;
+    // the corpus' BF16 and FP16 copies are written by one pass that follows the data
+    const bool adaptive = tf_scan && !c.tf32 && !pc && host_corpus == nullptr;
     const bool run_old = !scan;
     // the shortlist kernel's split keys are 3xTF32
     if (run_old) c.tf32 = true;
@@ -965,7 +1013,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         if (rc) return rc;
         ws += E.cn.cap;
     }
-    rc = E.words.ensure(8 * sizeof(uint32_t));
+    size_t nwords = 0;
+    rc = flag_words(E, Q, pc ? 0 : N, &nwords);
     if (rc) return rc;
     rc = E.thr.ensure(Q * sizeof(uint32_t));
     if (rc) return rc;
@@ -1012,13 +1061,12 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     if (c.algo == KNNS_ALGO_TC && !pc) {
         if (!bf16_only) {
             rc = ensure_split(E, c, N, D, n_pad);
+            if (!rc && adaptive) rc = E.done.ensure((size_t)prep_batches(N, D));
             if (rc) return rc;
         }
         rc = E.bf.ensure((size_t)N * c.dpb * 2);
         if (rc) return rc;
-        rc = E.loflags.ensure(((size_t)cdiv(N, 128) + 4) * sizeof(uint32_t));
-        if (rc) return rc;
-        ws += E.hi.cap + E.lo.cap + E.rs.cap + E.bf.cap + E.loflags.cap;
+        ws += E.hi.cap + E.lo.cap + E.rs.cap + E.bf.cap + E.words.cap;
         if (f8) {
             rc = E.f8.ensure((size_t)N * c.dpf * 2);
             if (!rc) rc = E.cs.ensure(n_pad * sizeof(float));
@@ -1068,7 +1116,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                    (const uint32_t*)E.words.p + 1, (uint32_t*)E.words.p + 5, E.tfail, E.tthr2, s};
     if (tf_scan) {
         if ((rc = ts.ensure())) return rc;
-        ws += E.qhi.cap + E.qlo.cap + E.qrs.cap + E.qlof.cap + E.tfail.cap + E.tthr2.cap;
+        ws += E.qhi.cap + E.qlo.cap + E.qrs.cap + E.tfail.cap + E.tthr2.cap;
     }
     // Resident corpora (one stream otherwise): the split-key scan runs on a side stream beside the
     // BF16 path, so that the launches of whichever path does not match the data (they return at
@@ -1184,12 +1232,21 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     const uint32_t* flags = c.algo == KNNS_ALGO_TC ? cp.flags : nullptr;
     if (pc) {
         KNN_CUDA(cudaMemcpyAsync(words, pc->words.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-        KNN_CUDA(cudaMemsetAsync(words + 4, 0, 2 * sizeof(uint32_t), s));
+        KNN_CUDA(cudaMemsetAsync(words + 4, 0, (nwords - 4) * sizeof(uint32_t), s));
     } else {
-        KNN_CUDA(cudaMemsetAsync(words, 0, 6 * sizeof(uint32_t), s));
+        KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
     }
     // split keys on request: the data count as not BF16-exact (the preparation only ORs into the word)
     if (o.tf32_only && !bf16_only) KNN_CUDA(cudaMemsetAsync(words + 1, 0x01, 1, s));
+    // BF16 side of a preparation (E4M3 rows beside it in the FP8 form): the copies are the caller's
+    auto bf_job = [&](const float* x, int64_t n, int64_t ld, float* norms, int64_t pad) {
+        PrepJob j = prep_job(x, n, ld, D, norms, pad);
+        j.dpb = c.dpb;
+        j.not_exact = not_exact;
+        j.int_stats = int_stats;
+        j.f8_bytes = 2 * c.dpf;
+        return j;
+    };
     if (blocked) {
         // the corpus blocks, prepared on the preparation stream as they land (their flag words
         // only OR into the words just cleared)
@@ -1201,11 +1258,14 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             int64_t r0, r1;
             blk_rows(b, &r0, &r1);
             if (streamed) KNN_CUDA(cudaStreamWaitEvent(ps, oev(2 + b), 0));
-            KNN_CUDA(launch_prep_rows(corpus + r0 * ld, r1 - r0, ld, D, c.dpb, (char*)E.bf.p + (size_t)r0 * c.dpb * 2,
-                                      cn + r0, b == nblk - 1 ? n_pad - r0 : r1 - r0, not_exact, ps, int_stats,
-                                      f8 ? (char*)E.f8.p + (size_t)r0 * c.dpf * 2 : nullptr, 2 * c.dpf,
-                                      f8 ? (float*)E.cs.p + r0 : nullptr,
-                                      np_keys ? (char*)E.np.p + (size_t)r0 * kNormParts * 2 : nullptr));
+            PrepJob j = bf_job(corpus + r0 * ld, r1 - r0, ld, cn + r0, b == nblk - 1 ? n_pad - r0 : r1 - r0);
+            j.bf = (char*)E.bf.p + (size_t)r0 * c.dpb * 2;
+            if (f8) {
+                j.f8 = (char*)E.f8.p + (size_t)r0 * c.dpf * 2;
+                j.scales = (float*)E.cs.p + r0;
+            }
+            if (np_keys) j.np = (char*)E.np.p + (size_t)r0 * kNormParts * 2;
+            KNN_CUDA(launch_prep(j, ps));
             ++launches;
             KNN_CUDA(cudaEventRecord(oev(2 + nblk + b), ps));
         }
@@ -1214,31 +1274,54 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         // one pass per input: BF16 copy, exactness test, integrality, norms (blocked mode: the
         // corpus block by block, above)
         if (!pc && !blocked) {
-            KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, c.dpb, E.bf.p, cn, n_pad, not_exact, s, int_stats,
-                                      f8 ? E.f8.p : nullptr, 2 * c.dpf, f8 ? (float*)E.cs.p : nullptr,
-                                      np_keys ? E.np.p : nullptr));
+            PrepJob j = bf_job(corpus, N, ldc, cn, n_pad);
+            j.bf = E.bf.p;
+            if (f8) {
+                j.f8 = E.f8.p;
+                j.scales = (float*)E.cs.p;
+            }
+            if (np_keys) j.np = E.np.p;
+            if (adaptive) {
+                split_outputs(E, &j, any_lo);
+                j.done = (uint8_t*)E.done.p;
+            }
+            KNN_CUDA(launch_prep(j, s));
             ++launches;
         }
-        if (f8)
-            KNN_CUDA(launch_prep_rows(queries, Q, ldq, D, c.dpb, nullptr, qn, Q, not_exact, s, int_stats, E.qbf.p,
-                                      2 * c.dpf, (float*)E.qs.p));
-        else
-            KNN_CUDA(launch_prep_rows(queries, Q, ldq, D, c.dpb, scan ? E.qbf.p : nullptr, qn, Q, not_exact, s,
-                                      int_stats));
+        PrepJob qj = bf_job(queries, Q, ldq, qn, Q);
+        if (f8) {
+            qj.f8 = E.qbf.p;
+            qj.scales = (float*)E.qs.p;
+        } else if (scan) {
+            qj.bf = E.qbf.p;
+        }
+        if (tf_scan) ts.prep_outputs(&qj);
+        KNN_CUDA(launch_prep(qj, s));
         ++launches;
         if (!bf16_only && !pc && !blocked) {
-            // the split runs only for data that is not BF16-exact
-            if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, any_lo, not_exact, s))) return rc;
+            // data that are not BF16-exact: the FP16 side of the batches prepared before that was
+            // known (3xTF32 keys: the split of the whole corpus)
+            if (adaptive) {
+                PrepJob j = prep_job(corpus, N, ldc, D, nullptr, n_pad);
+                split_outputs(E, &j, any_lo);
+                j.not_exact = not_exact;
+                j.done = (uint8_t*)E.done.p;
+                j.catch_up = true;
+                j.run_if = not_exact;
+                KNN_CUDA(launch_prep(j, s));
+            } else if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, nullptr, any_lo, not_exact, s))) {
+                return rc;
+            }
             ++launches;
         }
-        if (tf_scan && !blocked && !ts_side && (rc = ts.split_queries())) return rc;
+        if (tf_scan && !blocked && !ts_side && (rc = ts.query_operands())) return rc;
     } else {
         if (!pc) {
-            KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, 0, nullptr, cn, n_pad, nullptr, s));
+            KNN_CUDA(launch_row_norms(corpus, N, ldc, D, cn, n_pad, s));
             ++launches;
         }
         if (qn) {
-            KNN_CUDA(launch_prep_rows(queries, Q, ldq, D, 0, nullptr, qn, Q, nullptr, s));
+            KNN_CUDA(launch_row_norms(queries, Q, ldq, D, qn, Q, s));
             ++launches;
         }
     }
@@ -1407,9 +1490,14 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         int64_t lv_div = 1;
         if (blocked) {
             if (smp_copy) KNN_CUDA(cudaStreamWaitEvent(s, oev(1), 0));
-            KNN_CUDA(launch_prep_rows(smp_src, smp_n, smp_ld, D, c.dpb, E.smp_bf.p, (float*)E.smp_cn.p, smp_pad,
-                                      not_exact, s, int_stats, f8 ? E.smp_f8.p : nullptr, 2 * c.dpf,
-                                      f8 ? (float*)E.smp_cs.p : nullptr, np_keys ? E.smp_np.p : nullptr));
+            PrepJob j = bf_job(smp_src, smp_n, smp_ld, (float*)E.smp_cn.p, smp_pad);
+            j.bf = E.smp_bf.p;
+            if (f8) {
+                j.f8 = E.smp_f8.p;
+                j.scales = (float*)E.smp_cs.p;
+            }
+            if (np_keys) j.np = E.smp_np.p;
+            KNN_CUDA(launch_prep(j, s));
             ++launches;
             key_src = f8 ? E.smp_f8.p : E.smp_bf.p;
             lv_cn = (const float*)E.smp_cn.p;
@@ -1447,7 +1535,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             KNN_CUDA(cudaEventRecord(E.order_event(0), s));
             KNN_CUDA(cudaStreamWaitEvent(ts_stream, E.order_event(0), 0));
             ts.s = ts_stream;
-            if ((rc = ts.split_queries()) || (rc = ts.seed()) || (rc = ts.main_pass()) || (rc = ts.select()) || (rc = ts.fix())) return rc;
+            if ((rc = ts.query_operands()) || (rc = ts.seed()) || (rc = ts.main_pass()) || (rc = ts.select()) || (rc = ts.fix())) return rc;
             KNN_CUDA(cudaEventRecord(E.order_event(1), ts_stream));
         } else if (tf_scan && !blocked && (rc = ts.seed())) {
             return rc;
@@ -1479,10 +1567,10 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             for (int b = 0; b < nblk; ++b) KNN_CUDA(cudaStreamWaitEvent(s, oev(2 + 2 * nblk + b), 0));
             if (tf_scan) {
                 cudaStream_t ps = E.prep_stream();
-                if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, any_lo, not_exact, ps))) return rc;
+                if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, nullptr, any_lo, not_exact, ps))) return rc;
                 ++launches;
                 ts.s = ps;
-                if ((rc = ts.split_queries())) return rc;
+                if ((rc = ts.query_operands())) return rc;
                 for (int b = 0; b < nblk; ++b) KNN_CUDA(cudaStreamWaitEvent(ps, oev(2 + 2 * nblk + b), 0));
                 if ((rc = ts.seed()) || (rc = ts.main_pass()) || (rc = ts.select()) || (rc = ts.fix())) return rc;
                 KNN_CUDA(cudaEventRecord(oev(4 + 3 * nblk), ps));
@@ -1628,11 +1716,26 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     if (rc) return rc;
     uint32_t* w = (uint32_t*)pc->words.p;
     KNN_CUDA(cudaMemsetAsync(w, 0, 8 * sizeof(uint32_t), s));
-    KNN_CUDA(launch_prep_rows(corpus, N, ldc, D, dpb, pc->bf.p, (float*)pc->cn.p, n_pad, w + 1, s, w + 2,
-                              fp8 ? pc->f8.p : nullptr, 2 * dpf, fp8 ? (float*)pc->cs.p : nullptr, pc->np.p));
-    if (f16)
-        KNN_CUDA(launch_split_f16(corpus, N, ldc, D, pc->hi.p, pc->lo.p, (float*)pc->rs.p, n_pad, (uint32_t*)pc->tiles.p,
-                                  w, nullptr, s));
+    PrepJob j = prep_job(corpus, N, ldc, D, (float*)pc->cn.p, n_pad);
+    j.dpb = dpb;
+    j.bf = pc->bf.p;
+    j.not_exact = w + 1;
+    j.int_stats = w + 2;
+    j.np = pc->np.p;
+    if (fp8) {
+        j.f8 = pc->f8.p;
+        j.f8_bytes = 2 * dpf;
+        j.scales = (float*)pc->cs.p;
+    }
+    if (f16) {
+        KNN_CUDA(cudaMemsetAsync(pc->tiles.p, 0, pc->tiles.cap, s));
+        j.hi = pc->hi.p;
+        j.lo = pc->lo.p;
+        j.rs = (float*)pc->rs.p;
+        j.lo_flags = (uint32_t*)pc->tiles.p;
+        j.any_lo = w;
+    }
+    KNN_CUDA(launch_prep(j, s));
     pc->corpus = corpus;
     pc->N = N;
     pc->ldc = ldc;
@@ -2145,7 +2248,7 @@ int knns_debug_prep(const float* x, int64_t n, int64_t ld, int D, float* norms, 
                     uint32_t* words, void* norm_parts)
 {
     clear_error();
-    if (!x || !norms || !bf16 || !f8 || !scales || !words || n <= 0 || D <= 0 || D > kPrepMaxD || ld < D)
+    if (!x || !norms || !bf16 || !f8 || !scales || !words || n <= 0 || D <= 0 || D > 384 || ld < D)
         return set_error(KNNS_ERR_INVALID, "bad args");
     Engine* E = nullptr;
     int rc = get_engine(&E);
@@ -2153,8 +2256,16 @@ int knns_debug_prep(const float* x, int64_t n, int64_t ld, int D, float* norms, 
     std::lock_guard<std::mutex> lk(E->mu);
     cudaStream_t s = E->host_stream();
     KNN_CUDA(cudaMemsetAsync(words, 0, 3 * sizeof(uint32_t), s));
-    KNN_CUDA(launch_prep_rows(x, n, ld, D, (D + 63) & ~63, bf16, norms, n, words, s, words + 1, f8, (D + 127) & ~127,
-                              scales, norm_parts));
+    PrepJob j = prep_job(x, n, ld, D, norms, n);
+    j.dpb = (D + 63) & ~63;
+    j.bf = bf16;
+    j.not_exact = words;
+    j.int_stats = words + 1;
+    j.f8 = f8;
+    j.f8_bytes = (D + 127) & ~127;
+    j.scales = scales;
+    j.np = norm_parts;
+    KNN_CUDA(launch_prep(j, s));
     KNN_CUDA(cudaStreamSynchronize(s));
     return KNNS_OK;
 }
@@ -2214,11 +2325,11 @@ int knns_debug_tc_dot_tile(const float* corpus, int64_t N, const float* queries,
     if ((rc = E->hi.ensure((size_t)n_use * dp * 4))) return rc;
     if ((rc = E->lo.ensure((size_t)n_use * dp * 4))) return rc;
     if ((rc = E->bf.ensure((size_t)n_use * dpb * 2))) return rc;
-    if ((rc = E->loflags.ensure(4 * sizeof(uint32_t)))) return rc;
+    if ((rc = E->words.ensure(8 * sizeof(uint32_t)))) return rc;
     if ((rc = E->part.ensure((size_t)std::min<int64_t>(Q, kTileQ) * 32 * 8))) return rc;
     KNN_CUDA(cudaStreamWaitEvent(s, E->last_done, 0));
     KNN_CUDA(launch_norms(corpus, n_use, D, D, (float*)E->cn.p, n_pad, s));
-    uint32_t* not_exact = (uint32_t*)E->loflags.p;
+    uint32_t* not_exact = (uint32_t*)E->words.p;
     const int64_t q_use = std::min<int64_t>(Q, kTileQ);
     KNN_CUDA(cudaMemsetAsync(not_exact, 0, sizeof(uint32_t), s));
     KNN_CUDA(launch_bf16(corpus, n_use, D, D, dpb, E->bf.p, not_exact, s));

@@ -45,7 +45,7 @@ struct Engine {
     int cc = 0;
     std::mutex mu;
     cudaEvent_t last_done = nullptr;
-    DevBuf cn, qn, part, hi, lo, rs, bf, err, thr, loflags, cn_s, thr2, redo;
+    DevBuf cn, qn, part, hi, lo, rs, bf, err, thr, cn_s, thr2, redo;
     // threshold-scan path: BF16 queries, candidate segments and counts, seeded
     // thresholds, sample norms, failed-query list
     DevBuf qbf, cand, cnt, tq, cnv, fail;
@@ -54,11 +54,16 @@ struct Engine {
     // split-key scan: the queries' hi / lo copies, row scales and the low-part flags of their tiles; the
     // failed-query list and fix-up thresholds of the scan when it runs beside the BF16 scan
     // (exact form)
-    DevBuf qhi, qlo, qrs, qlof, tfail, tthr2;
+    DevBuf qhi, qlo, qrs, tfail, tthr2;
+    // adaptive preparation: one byte per batch of corpus rows (PrepJob::done)
+    DevBuf done;
     // per-search flag words: [0] some corpus tile has a low part, [1] corpus or
     // queries not BF16-exact, [2] some value not an integer, [3] max |x| (float bits), [4] zero,
     // [5] some query tile has a low part
+    // then the low-part flags of the query tiles (qlof) and of the search's own corpus tiles (lof)
     DevBuf words;
+    uint32_t* qlof = nullptr;
+    uint32_t* lof = nullptr;
     DevBuf in_corpus, in_queries, out_dist, out_idx;
     // corpus blocks of host-buffer searches: two running top-k lists (distances, indices)
     DevBuf mrg;

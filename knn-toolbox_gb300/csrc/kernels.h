@@ -27,15 +27,8 @@ enum DeviceError : int {
 
 cudaError_t launch_norms(const float* x, int64_t n, int64_t ld, int D, float* out, int64_t n_pad,
                          cudaStream_t s);
-// FP16 split of every row: hi = fp16(s x), lo = fp16(s x - hi), s the power of two that puts the
-// row's largest |x| into [2^14, 2^15); hi / lo are [n][hp] FP16 (hp = split_pitch(D), zero padded),
-// rs[0..n_pad) the reciprocals 1 / s (0 for n <= i < n_pad).  lo_flags[tile of 128 rows] = any lo
-// != 0 (may be null); *any_lo (zeroed by the caller, may be null) becomes 1 when some tile has a
-// low part.  When skip_unless is given and *skip_unless == 0 at run time, the kernel does nothing.
 constexpr int kTileRows = 128;
 __host__ __device__ constexpr int split_pitch(int D) { return (D + 7) & ~7; }  // rows of whole 16-byte words
-cudaError_t launch_split_f16(const float* x, int64_t n, int64_t ld, int D, void* hi, void* lo, float* rs, int64_t n_pad,
-                         uint32_t* lo_flags, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s);
 // TF32 hi/lo split into [n][dp] arrays; lo_flags[tile of 128 rows] = any lo != 0 (may be null);
 // *any_lo (zeroed by the caller, may be null) becomes 1 when some tile has a low part.  When
 // skip_unless is given and *skip_unless == 0 at run time, the kernel does nothing.
@@ -46,21 +39,50 @@ cudaError_t launch_split_tf32(const float* x, int64_t n, int64_t ld, int D, int 
 cudaError_t launch_bf16(const float* x, int64_t n, int64_t ld, int D, int dpb, void* out, uint32_t* not_exact,
                         cudaStream_t s);
 
-// One pass over a row-major matrix: optional BF16 copy out[n][dpb] (dpb = 0: none)
-// with the exactness flag, optional norms[0..n_pad) (+inf padding), same
-// conventions as launch_norms / launch_bf16.  Rows wider than kPrepMaxD fall
-// back to those two kernels.
-constexpr int kPrepMaxD = 384;
-// int_stats (optional, 2 words, zeroed by the caller): [0] |= 1 when some value is not an
-// integer, [1] = max |x| as float bits.
-// f8 / scales (optional): E4M3 copy [n][f8_bytes] (f8_bytes a multiple of 128, zero padded) with
-// per-row absmax scales (row = scale * codes; scales[n..n_pad) = 0); needs D <= kPrepMaxD.
-// np (optional): norm parts [n][kNormParts] BF16, (n1, n2, n3, 0, ...) with n1 + n2 + n3 equal
-// to the row's FP32 norm; needs D <= kPrepMaxD.
+// One pass over a row-major matrix (prep_rows_kernel); every output is optional.
+constexpr int kPrepMaxD = 2048;
 constexpr int kNormParts = 16;
-cudaError_t launch_prep_rows(const float* x, int64_t n, int64_t ld, int D, int dpb, void* out, float* norms,
-                             int64_t n_pad, uint32_t* not_exact, cudaStream_t s, uint32_t* int_stats = nullptr,
-                             void* f8 = nullptr, int f8_bytes = 0, float* scales = nullptr, void* np = nullptr);
+struct PrepJob {
+    const float* x = nullptr;
+    int64_t n = 0, ld = 0;
+    int D = 0;
+    // norms[0..n_pad): the float rounding of the double sum of squares in column order, +inf padding
+    float* norms = nullptr;
+    int64_t n_pad = 0;
+    // BF16 side: copy [n][dpb]; *not_exact |= 1 when some element is not exactly representable;
+    // int_stats (2 words, zeroed by the caller): [0] |= 1 when some value is not an integer, [1] =
+    // max |x| as float bits; np: norm parts [n][kNormParts] BF16, (n1, n2, n3, 0, ...) with n1 + n2 +
+    // n3 equal to the row's FP32 norm
+    void* bf = nullptr;
+    int dpb = 0;
+    uint32_t* not_exact = nullptr;
+    uint32_t* int_stats = nullptr;
+    void* np = nullptr;
+    // E4M3 copy [n][f8_bytes] (f8_bytes a multiple of 128, zero padded) with per-row absmax scales
+    // (row = scale * codes; scales[n..n_pad) = 0)
+    void* f8 = nullptr;
+    int f8_bytes = 0;
+    float* scales = nullptr;
+    // FP16 side: hi = fp16(s x), lo = fp16(s x - hi), s the power of two that puts the row's largest
+    // |x| into [2^14, 2^15); hi / lo are [n][split_pitch(D)] FP16, zero padded, rs[0..n_pad) the
+    // reciprocals 1 / s (0 for n <= i < n_pad).  lo_flags[tile of 128 rows] and *any_lo (zeroed by
+    // the caller) become 1 when some lo is nonzero
+    void* hi = nullptr;
+    void* lo = nullptr;
+    float* rs = nullptr;
+    uint32_t* lo_flags = nullptr;
+    uint32_t* any_lo = nullptr;
+    // adaptive: the BF16 or the FP16 side per batch of rows, by *not_exact (see prep_rows_kernel);
+    // done: one byte per batch (prep_batches of them), 1 when the FP16 side was written.  catch_up:
+    // the FP16 side of the batches whose done byte is 0, nothing else.
+    uint8_t* done = nullptr;
+    bool catch_up = false;
+    const uint32_t* run_if = nullptr;  // the launch does nothing when *run_if == 0 at run time
+};
+int64_t prep_batches(int64_t n, int D);
+cudaError_t launch_prep(const PrepJob& job, cudaStream_t s);
+// norms of rows of any width
+cudaError_t launch_row_norms(const float* x, int64_t n, int64_t ld, int D, float* norms, int64_t n_pad, cudaStream_t s);
 
 // CUDA-core FP32 fused distance + shortlist.  qpb in {32, 128}.
 size_t simt_smem_bytes(int qpb, int kp);
@@ -196,8 +218,8 @@ cudaError_t launch_tscan(const TscanArgs& a, int splits, cudaStream_t s);
 
 // Tensor-core FP16-split threshold scan (csrc/scan_f16.cu): 128 queries x fscan_tile_rows(D)-row
 // corpus tiles, K in chunks of 64 FP16 columns; the candidate segments are those of the BF16 scan
-// (kScanParts per split, fscan_part_cols(D) columns of every tile each).  Operands as launch_split_f16
-// writes them.
+// (kScanParts per split, fscan_part_cols(D) columns of every tile each).  Operands as launch_prep
+// writes them (FP16 side).
 constexpr int kFscanTmemD = 256;  // widest rows whose queries sit in tensor memory
 struct FscanArgs {
     CUtensorMap tm_qhi, tm_qlo;   // D > kFscanTmemD: queries hi / lo [Q][hp] fp16, box {64, 128}, 128B swizzle

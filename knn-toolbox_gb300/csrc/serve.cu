@@ -95,9 +95,9 @@ struct Slot {
 
 std::vector<void*> workspace_pointers(const Engine& E)
 {
-    return {E.cn.p,   E.qn.p,  E.part.p, E.hi.p,  E.lo.p,  E.rs.p,   E.bf.p,   E.err.p,  E.thr.p,  E.loflags.p, E.cn_s.p,
+    return {E.cn.p,   E.qn.p,  E.part.p, E.hi.p,  E.lo.p,  E.rs.p,   E.bf.p,   E.err.p,  E.thr.p,  E.cn_s.p,
             E.thr2.p, E.redo.p, E.qbf.p, E.cand.p, E.cnt.p, E.tq.p,   E.cnv.p,  E.fail.p, E.words.p, E.qs.p,
-            E.csv.p,  E.qhi.p,  E.qlo.p, E.qrs.p,  E.qlof.p, E.tfail.p, E.tthr2.p};
+            E.csv.p,  E.qhi.p,  E.qlo.p, E.qrs.p,  E.tfail.p, E.tthr2.p};
 }
 
 }  // namespace
@@ -592,8 +592,8 @@ void knns_server_destroy(knns_server* sv)
         cudaFreeHost(sl->h_dist);
         cudaFreeHost(sl->h_idx);
         for (DevBuf* b : {&sl->E.cn, &sl->E.qn, &sl->E.part, &sl->E.hi, &sl->E.lo, &sl->E.bf, &sl->E.err, &sl->E.thr,
-                          &sl->E.loflags, &sl->E.cn_s, &sl->E.thr2, &sl->E.redo, &sl->E.qbf, &sl->E.cand, &sl->E.cnt,
-                          &sl->E.tq, &sl->E.cnv, &sl->E.rs, &sl->E.qs, &sl->E.csv, &sl->E.qhi, &sl->E.qlo, &sl->E.qrs, &sl->E.qlof,
+                          &sl->E.cn_s, &sl->E.thr2, &sl->E.redo, &sl->E.qbf, &sl->E.cand, &sl->E.cnt,
+                          &sl->E.tq, &sl->E.cnv, &sl->E.rs, &sl->E.qs, &sl->E.csv, &sl->E.qhi, &sl->E.qlo, &sl->E.qrs, &sl->E.done,
                           &sl->E.tfail, &sl->E.tthr2, &sl->E.fail, &sl->E.words, &sl->E.in_corpus, &sl->E.in_queries,
                           &sl->E.out_dist, &sl->E.out_idx})
             b->release();

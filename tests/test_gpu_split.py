@@ -81,3 +81,45 @@ def test_index_answers_as_the_search_whichever_keys_serve_it(engine, N, k, reran
         np.testing.assert_array_equal(i.cpu().numpy(), i2.cpu().numpy())
         np.testing.assert_array_equal(d.cpu().numpy(), d2.cpu().numpy())
     ix.close()
+
+
+@pytest.mark.parametrize("where", ["first row", "last row", "scattered", "everywhere", "queries", "nowhere"])
+@pytest.mark.parametrize("D,pad", [(33, 0), (96, 0), (100, 3)])
+def test_adaptive_preparation_by_where_the_data_stop_being_bf16_exact(engine, where, D, pad):
+    # one pass writes the BF16 side of the rows it sees before, the FP16 side of those after the data
+    # turn out not to be BF16-exact; a second one catches up.  Same answers as the split-key scan
+    # alone, which writes the FP16 side of every row.
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(D + pad)
+    N = 200_003
+    X = torch.randint(0, 200, (N, D + pad), generator=g, device="cuda").float()[:, :D]
+    Qs = torch.randint(0, 200, (90, D), generator=g, device="cuda").float()
+    if where == "first row":
+        X[0, 1] += 0.37
+    elif where == "last row":
+        X[N - 1, D - 1] += 0.37
+    elif where == "scattered":
+        X[::4001, 2] += 0.37
+    elif where == "everywhere":
+        X += torch.rand((N, D), generator=g, device="cuda")
+    elif where == "queries":
+        Qs[7, 3] += 0.37
+    d, i = engine.search(X, Qs, 20)
+    assert engine.last_stats()["scan_keys"] == 3
+    d2, i2 = engine.search(X, Qs, 20, scan=engine.SCAN_TF32)
+    assert torch.equal(i, i2) and torch.equal(d, d2)
+
+
+@pytest.mark.parametrize("D", [385, 511, 512, 513, 1000, 1024, 1025, 2047, 2048, 2049])
+def test_norms_of_wide_rows(engine, oracle, D):
+    # rerank = False returns key + ||q||^2 from the CUDA-core keys: bit-exact only with the norms of
+    # the oracle's convention (the float rounding of the double sum in column order)
+    rng = np.random.default_rng(D)
+    X = (rng.standard_normal((300, D)) * 10.0 ** rng.uniform(-6, 6, (300, 1))).astype(np.float32)
+    X[::7] = rng.integers(0, 256, X[::7].shape)
+    X[5] = 0.0
+    Qs = rng.standard_normal((40, D)).astype(np.float32)
+    d, i, st = run(engine, X, Qs, 30, algo=engine.ALGO_SIMT, rerank=False)
+    od, oi = oracle.knn_gemm(X, Qs, 30)
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_array_equal(d, od)
