@@ -417,9 +417,12 @@ struct ScanPlan {
     ScanLevel lv[kMaxSeedLevels];
     int64_t len = 0;
     int S = 1, cap = 0;
+    // seeding starts at level `dense`, whose keys are all kept (densely, ldk a row): the coarser ones
+    // would only bound what it collects
+    int dense = 0, dense_S = 1;
+    int64_t dense_len = 0, ldk = 0;
     int sel_words = 0;  // bound on one query's stored main-pass candidates (selection buffer)
-    int64_t fixA_rows = 0, fixA_len = 0, fixB_rows = 0, fixB_len = 0;
-    int fixA_S = 1, fixB_S = 1;
+    FixGroups fix;  // fix-up of failed queries (their shortlists after one another in E.part)
     bool simt_fix = false;  // the fix-up runs on the CUDA-core kernel (shortlist above kMaxKpTC)
     size_t cand_words = 0, cnt_words = 0, part_words = 0, norm_words = 0;
 };
@@ -451,6 +454,13 @@ static int seg_cap(double per_seg, double sigmas)
 }
 
 static int seed_rank(double m) { return (int)std::ceil(2.0 * m + 4.0 * std::sqrt(m)) + 1; }
+
+// Seeding starts with a dense pass -- every key of a level's rows written out, the threshold taken from
+// them -- over the finest level with at most kDenseRows rows and kDenseKeys keys (Q x rows) in all: each
+// coarser level that it replaces is three launches and 25 to 40 us for any number of queries (65,536 x
+// 128, 1,024 queries: seeding 64 -> 25 us; 32,768 x 1,024: 74 -> 36; 48 queries on 2,000,000 x 128: 74 -> 47),
+// while a dense pass over 20M keys (10,000 x 1,954) costs 94 us, what its two levels did.
+constexpr int64_t kDenseKeys = 24 << 20;
 
 // keys kKeyF16 / kKeyTf32: the plan of the scan on split keys (fix-up on the CUDA-core kernel; dpb
 // only decides its tile: the row width rounded up to 64); otherwise of the BF16 / E4M3 scan of row
@@ -503,6 +513,9 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     for (int l = L - 1; l >= 0; --l) {
         ScanLevel& v = P->lv[l];
         v.j = std::min<int>((int)v.n, seed_rank(m));
+        // short shortlists: rank 7 for an expected 1 left one query in 12,000 short of kp keys, and one
+        // such query costs its search a fix-up over the corpus; two ranks more, one in a million
+        if (l == L - 1 && m < 2.0 && v.n >= 4 * (v.j + 2)) v.j += 2;
         if (l > 0) m = (double)v.j * (double)P->lv[l - 1].n / (double)v.n;
     }
     if (P->lv[L - 1].j > kCandMax / 2 || P->lv[L - 1].n < 4 * P->lv[L - 1].j)
@@ -526,8 +539,19 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
             const double hits = (double)P->lv[l - 1].j * (double)v.n / (double)P->lv[l - 1].n;
             v.cap = std::min<int>((int)(v.len / tn * pc), seg_cap(hits * pc / ((double)tn * v.S), 3.0));
         }
-        P->cand_words = std::max(P->cand_words, (size_t)kScanParts * v.S * Q * v.cap);
-        P->cnt_words = std::max(P->cnt_words, (size_t)kScanParts * v.S * Q);
+        if (l == 0 || (v.n <= kDenseRows && v.n * Q <= kDenseKeys)) {
+            P->dense = l;
+            P->dense_S = seed_splits(qt, tiles, E.sms, kScanMaxSegs / kScanParts);
+            P->dense_len = cdiv(tiles, P->dense_S) * tn;
+            P->dense_S = (int)cdiv(v.n, P->dense_len);
+            P->ldk = tiles * tn;
+            P->cand_words = ((size_t)Q * P->ldk + 1) / 2;
+            P->cnt_words = 0;
+            P->norm_words = 0;
+        } else {
+            P->cand_words = std::max(P->cand_words, (size_t)kScanParts * v.S * Q * v.cap);
+            P->cnt_words = std::max(P->cnt_words, (size_t)kScanParts * v.S * Q);
+        }
         P->norm_words += (size_t)v.n_pad;
     }
     // main pass
@@ -553,15 +577,19 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     const int ft = P->simt_fix ? kSimtTileN : kTileN;
     const int fq = P->simt_fix ? 32 : kTileQ;
     const int64_t tilesF = cdiv(N, ft);
-    P->fixA_rows = std::min<int64_t>(Q, P->simt_fix ? fq : 4 * kTileQ);
-    P->fixA_S = (int)std::max<int64_t>(1, std::min<int64_t>(tilesF, E.sms / cdiv(P->fixA_rows, fq)));
-    P->fixA_len = cdiv(tilesF, P->fixA_S) * ft;
-    P->fixA_S = (int)cdiv(N, P->fixA_len);
-    P->fixB_rows = Q - P->fixA_rows;
-    P->fixB_S = (int)std::min<int64_t>(tilesF, 8);
-    P->fixB_len = cdiv(tilesF, P->fixB_S) * ft;
-    P->fixB_S = (int)cdiv(N, P->fixB_len);
-    P->part_words = std::max((size_t)P->fixA_S * P->fixA_rows * kp, (size_t)P->fixB_S * P->fixB_rows * kp);
+    auto group = [&](int64_t rows, int64_t splits) {
+        FixGroup g;
+        g.rows = rows;
+        g.tiles = (int)cdiv(rows, fq);
+        g.split_len = cdiv(tilesF, std::max<int64_t>(1, std::min(tilesF, splits))) * ft;
+        g.splits = (int)cdiv(N, g.split_len);
+        return g;
+    };
+    const int64_t rowsA = std::min<int64_t>(Q, P->simt_fix ? fq : 4 * kTileQ);
+    P->fix.g[0] = group(rowsA, E.sms / cdiv(rowsA, fq));
+    P->fix.g[1] = group(Q - rowsA, 8);
+    P->part_words = 0;
+    for (const FixGroup& g : P->fix.g) P->part_words += (size_t)g.splits * g.rows * kp;
     return KNNS_OK;
 }
 
@@ -574,6 +602,15 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
 // thresholds, candidates or results returns at once unless *run_if != 0 (the exact form's
 // device-side choice between BF16 and split keys); its failed-query list is its own (fail), so
 // the other path's fix-up never sees it.
+// the plan's fix-up groups with their shortlists in `part`
+static FixGroups fix_groups(const ScanPlan& sp, uint64_t* part, int kp)
+{
+    FixGroups fg = sp.fix;
+    fg.g[0].part = part;
+    fg.g[1].part = part + (size_t)fg.g[0].splits * fg.g[0].rows * kp;
+    return fg;
+}
+
 struct SplitCopies {
     const void* hi;
     const void* lo;
@@ -616,7 +653,6 @@ struct TscanStages {
         if (!rc) rc = E.cand.ensure(sp.cand_words * sizeof(uint64_t));
         if (!rc) rc = E.cnt.ensure(sp.cnt_words * sizeof(uint32_t));
         if (!rc) rc = E.cnv.ensure(sp.norm_words * sizeof(float));
-        if (!rc) rc = E.csv.ensure(sp.norm_words * sizeof(float));
         if (!rc) rc = fail.ensure((size_t)(Q + 1) * sizeof(uint32_t));
         if (!rc) rc = E.part.ensure(sp.part_words * sizeof(uint64_t));
         if (!rc) rc = thr2.ensure(Q * sizeof(uint32_t));
@@ -625,7 +661,7 @@ struct TscanStages {
     size_t workspace() const
     {
         return E.qhi.cap + E.qlo.cap + E.qrs.cap + E.tq.cap + E.cand.cap + E.cnt.cap + E.cnv.cap +
-               E.csv.cap + fail.cap + E.part.cap + thr2.cap;
+               fail.cap + E.part.cap + thr2.cap;
     }
     // The FP16 split of the queries, as outputs of their preparation pass.
     void prep_outputs(PrepJob* j) const
@@ -685,8 +721,10 @@ struct TscanStages {
         return KNNS_OK;
     }
     // one scan over rows 0, stride, 2*stride, ... of the corpus (nview of them)
-    int pass(int64_t nview, int64_t stride, const float* cn_view, const float* cs_view, const float* thr, int splits,
-             int64_t split_len, int cap, const uint32_t* flags)
+    // (3xTF32 keys: cn_view holds the view's norms, gathered; FP16 keys gather them in the kernel);
+    // keys: a dense pass
+    int pass(int64_t nview, int64_t stride, const float* cn_view, const float* thr, int splits, int64_t split_len,
+             int cap, const uint32_t* flags, float* keys = nullptr)
     {
         int r;
         if (c.tf32) {
@@ -699,18 +737,23 @@ struct TscanStages {
             a.split_len = split_len;
             a.cap = cap;
             a.clo_flags = flags;
+            a.keys = keys;
+            a.ldk = sp.ldk;
             KNN_CUDA(launch_tscan(a, splits, s));
         } else {
             r = encode_split(&f.tm_chi, cp.hi, nview, D, stride, fscan_tile_rows(D));
             if (!r) r = encode_split(&f.tm_clo, cp.lo, nview, D, stride, fscan_tile_rows(D));
             if (r) return r;
-            f.cn = cn_view;
-            f.cs = cs_view;
+            f.cn = cn;
+            f.cs = cp.rs;
+            f.stride = stride;
             f.thr = thr;
             f.N = nview;
             f.split_len = split_len;
             f.cap = cap;
             f.clo_flags = flags;
+            f.keys = keys;
+            f.ldk = sp.ldk;
             KNN_CUDA(launch_fscan(f, splits, s));
         }
         ++launches;
@@ -726,38 +769,45 @@ struct TscanStages {
         cs.skip_if_zero = run_if;
         return cs;
     }
-    // seeding, coarse to fine: level l keeps the keys below the previous level's threshold (the
-    // coarsest keeps every key) and yields the key of rank j_l
+    // seeding, coarse to fine: the first level keeps every key, level l those below the previous
+    // level's threshold; each yields the key of rank j_l.  The first also clears the failure count.
     int seed()
     {
         float* Tbuf[2] = {(float*)E.tq.p, (float*)E.tq.p + Q};
         float* cnv = (float*)E.cnv.p;
-        float* csv = (float*)E.csv.p;
         CandSelect cs = cand_select();
         T = nullptr;
-        for (int l = 0; l < sp.levels; ++l) {
+        for (int l = sp.dense; l < sp.levels; ++l) {
             const ScanLevel& v = sp.lv[l];
-            KNN_CUDA(launch_gather_norms(cn, v.n, v.stride, cnv, v.n_pad, s, run_if, cp.rs, cp.rs ? csv : nullptr));
-            int rc = pass(v.n, v.stride, cnv, csv, T, v.S, v.len, v.cap, nullptr);
+            const bool dense = l == sp.dense;
+            if (c.tf32) {
+                KNN_CUDA(launch_gather_norms(cn, v.n, v.stride, cnv, v.n_pad, s, run_if));
+                ++launches;
+            }
+            int rc = pass(v.n, v.stride, cnv, T, dense ? sp.dense_S : v.S, dense ? sp.dense_len : v.len, v.cap, nullptr,
+                          dense ? (float*)E.cand.p : nullptr);
             if (rc) return rc;
-            cs.nseg = kScanParts * v.S;
-            cs.cap = v.cap;
-            cs.thr_out = Tbuf[l & 1];
-            cs.thr_rank = v.j;
-            cs.thr_fallback = T;
-            KNN_CUDA(launch_select_cand(cs, s));
-            launches += 2;
+            if (dense) {
+                KNN_CUDA(launch_dense_threshold((const float*)E.cand.p, sp.ldk, (int)v.n, v.j, Q, Tbuf[l & 1],
+                                                (uint32_t*)fail.p, nullptr, run_if, s));
+            } else {
+                cs.nseg = kScanParts * v.S;
+                cs.cap = v.cap;
+                cs.thr_out = Tbuf[l & 1];
+                cs.thr_rank = v.j;
+                cs.thr_fallback = T;
+                KNN_CUDA(launch_select_cand(cs, s));
+            }
+            ++launches;
             T = Tbuf[l & 1];
             cnv += v.n_pad;
-            csv += v.n_pad;
         }
         return KNNS_OK;
     }
-    int main_pass() { return pass(N, 1, cn, cp.rs, T, sp.S, sp.len, sp.cap, cp.flags); }
+    int main_pass() { return pass(N, 1, cn, T, sp.S, sp.len, sp.cap, cp.flags); }
     int select()
     {
         uint32_t* fail_cnt = (uint32_t*)fail.p;
-        KNN_CUDA(cudaMemsetAsync(fail_cnt, 0, sizeof(uint32_t), s));
         CandSelect cs = cand_select();
         cs.nseg = kScanParts * sp.S;
         cs.cap = sp.cap;
@@ -776,35 +826,28 @@ struct TscanStages {
         cs.out_idx_f = idx_f;
         cs.fail_idx = (int32_t*)fail.p + 1;
         cs.fail_cnt = fail_cnt;
+        cs.fail_thr = (uint32_t*)thr2.p;
         KNN_CUDA(launch_select_cand(cs, s));
         ++launches;
         return KNNS_OK;
     }
     // fix-up: the queries the scan could not answer, on the CUDA-core kernel (exact FP32 keys),
-    // compacted; launches whose rows are all past the failure count return at once
-    int fix_pass(int64_t qbase, int64_t rows, int splits, int64_t split_len)
+    // compacted; blocks whose rows are past the failure count return at once
+    int fix()
     {
-        if (rows <= 0) return KNNS_OK;
-        uint32_t* fail_cnt = (uint32_t*)fail.p;
-        int32_t* fail_idx = (int32_t*)fail.p + 1;
-        uint32_t* t2 = (uint32_t*)thr2.p;
-        KNN_CUDA(cudaMemsetAsync(t2, 0xFF, rows * sizeof(uint32_t), s));
-        KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, rows, ldq, D, c.kp, 32, split_len, splits,
-                             (uint64_t*)E.part.p, t2, s, nullptr, fail_idx, fail_cnt, qbase));
+        const uint32_t* fail_cnt = (const uint32_t*)fail.p;
+        const int32_t* fail_idx = (const int32_t*)fail.p + 1;
+        const FixGroups fg = fix_groups(sp, (uint64_t*)E.part.p, c.kp);
+        KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, 32, 0, 0, nullptr, (uint32_t*)thr2.p, s,
+                             nullptr, fail_idx, fail_cnt, &fg));
         SelectExtra ex;
         ex.qmap = fail_idx;
         ex.qcount = fail_cnt;
-        ex.qbase = qbase;
-        KNN_CUDA(launch_select((const uint64_t*)E.part.p, splits, rows, c.kp, k, corpus, ldc, queries, ldq, D,
-                               c.rerank, c.rerank ? nullptr : qn, dist, idx, idx_f, s, ex));
+        ex.fix = fg;
+        KNN_CUDA(launch_select(nullptr, 0, Q, c.kp, k, corpus, ldc, queries, ldq, D, c.rerank, c.rerank ? nullptr : qn,
+                               dist, idx, idx_f, s, ex));
         launches += 2;
         return KNNS_OK;
-    }
-    int fix()
-    {
-        int rc = fix_pass(0, sp.fixA_rows, sp.fixA_S, sp.fixA_len);
-        if (!rc) rc = fix_pass(sp.fixA_rows, sp.fixB_rows, sp.fixB_S, sp.fixB_len);
-        return rc;
     }
 };
 
@@ -1457,7 +1500,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         // grid rows are the splits split0 .. split0 + splits - 1, launched on stream ls
         auto scan_pass = [&](const void* src, const void* np_src, int64_t nview, int64_t stride, const float* cn_view,
                              const float* cs_view, const float* thr, int splits, int64_t split_len, int cap,
-                             int split0 = 0, cudaStream_t ls = nullptr) -> int {
+                             int split0 = 0, cudaStream_t ls = nullptr, float* keys = nullptr) -> int {
             // the map moves bytes: E4M3 rows are described as rows of 16-bit units
             int r = encode_rows_bf16(&a.tm_c, src, nview, sdp, stride * sdp, scan_box_rows(sdp, sp.accs));
             if (!r && np_keys) r = encode_np(&a.tm_np, np_src, nview, stride * kNormParts, scan_box_rows(sdp, sp.accs));
@@ -1469,6 +1512,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             a.split_len = split_len;
             a.cap = cap;
             a.split0 = split0;
+            a.keys = keys;
+            a.ldk = sp.ldk;
             KNN_CUDA(launch_scan(a, splits, ls ? ls : s));
             ++launches;
             return KNNS_OK;
@@ -1479,8 +1524,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         cs.Q = Q;
         cs.skip_if = scan_gate;
         cs.D = D;
-        // seeding, coarse to fine: level l keeps the keys below the previous level's
-        // threshold (the coarsest keeps every key) and yields the key of rank j_l
+        // seeding, coarse to fine: the first level keeps every key (and clears the failure count),
+        // level l those below the previous level's threshold; each yields the key of rank j_l
         // (blocked mode: the levels read the sample prepared ahead of the corpus, whose row r is
         // corpus row sp.stride0 * r -- the same rows, prepared by the same pass)
         const void* key_src = f8 ? f8_p : bf_p;
@@ -1508,21 +1553,29 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         float* cnv = (float*)E.cnv.p;
         float* csv = f8 ? (float*)E.csv.p : nullptr;
         const float* T = nullptr;
-        for (int l = 0; l < sp.levels; ++l) {
+        for (int l = sp.dense; l < sp.levels; ++l) {
             const ScanLevel& v = sp.lv[l];
+            const bool dense = l == sp.dense;
             if (f8) {
                 // norms and scales of the sample rows: 0 scales for padding, whose +inf norms keep
                 // their keys at +inf (BF16 keys take the norm parts in place)
                 KNN_CUDA(launch_gather_norms(lv_cn, v.n, v.stride / lv_div, cnv, v.n_pad, s, nullptr, lv_cs, csv));
                 ++launches;
             }
-            if ((rc = scan_pass(key_src, lv_np, v.n, v.stride / lv_div, cnv, csv, T, v.S, v.len, v.cap))) return rc;
-            cs.nseg = kScanParts * v.S;
-            cs.cap = v.cap;
-            cs.thr_out = Tbuf[l & 1];
-            cs.thr_rank = v.j;
-            cs.thr_fallback = T;  // a level that fails keeps the previous threshold
-            KNN_CUDA(launch_select_cand(cs, s));
+            if ((rc = scan_pass(key_src, lv_np, v.n, v.stride / lv_div, cnv, csv, T, dense ? sp.dense_S : v.S,
+                                dense ? sp.dense_len : v.len, v.cap, 0, nullptr, dense ? (float*)E.cand.p : nullptr)))
+                return rc;
+            if (dense) {
+                KNN_CUDA(launch_dense_threshold((const float*)E.cand.p, sp.ldk, (int)v.n, v.j, Q, Tbuf[l & 1], fail_cnt,
+                                                scan_gate, nullptr, s));
+            } else {
+                cs.nseg = kScanParts * v.S;
+                cs.cap = v.cap;
+                cs.thr_out = Tbuf[l & 1];
+                cs.thr_rank = v.j;
+                cs.thr_fallback = T;  // a level that fails keeps the previous threshold
+                KNN_CUDA(launch_select_cand(cs, s));
+            }
             ++launches;
             T = Tbuf[l & 1];
             cnv += v.n_pad;
@@ -1577,7 +1630,6 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             }
         }
         if ((rc = mark(3))) return rc;
-        KNN_CUDA(cudaMemsetAsync(fail_cnt, 0, sizeof(uint32_t), s));
         cs.nseg = kScanParts * sp.S;
         cs.cap = sp.cap;
         cs.thr_out = nullptr;
@@ -1600,65 +1652,48 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         cs.out_idx_f = idx_f;
         cs.fail_idx = fail_idx;
         cs.fail_cnt = fail_cnt;
+        cs.fail_thr = (uint32_t*)E.thr2.p;
         KNN_CUDA(launch_select_cand(cs, s));
         ++launches;
         if (tf_scan && !ts_side && !blocked && (rc = ts.select())) return rc;
         if ((rc = mark(4))) return rc;
-        // fix-up: failed queries, compacted, through the shortlist kernel without a threshold
-        // (launches whose rows are all past the failure count return at once)
-        auto fix_pass = [&](int64_t qbase, int64_t rows, int splits, int64_t split_len) -> int {
-            if (rows <= 0) return KNNS_OK;
-            if (sp.simt_fix) {
-                // long shortlists: the CUDA-core kernel with exact FP32 keys, compacted rows
-                uint32_t* thr2 = (uint32_t*)E.thr2.p;
-                KNN_CUDA(cudaMemsetAsync(thr2, 0xFF, rows * sizeof(uint32_t), s));
-                KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, rows, ldq, D, c.kp, 32, split_len, splits, part,
-                                     thr2, s, nullptr, fail_idx, fail_cnt, qbase));
-                SelectExtra ex;
-                ex.qmap = fail_idx;
-                ex.qcount = fail_cnt;
-                ex.qbase = qbase;
-                KNN_CUDA(launch_select(part, splits, rows, c.kp, k, corpus, ldc, queries, ldq, D, c.rerank,
-                                       c.rerank ? nullptr : (const float*)E.qn.p, dist, idx, idx_f, s, ex));
-                launches += 2;
-                return KNNS_OK;
-            }
+        // fix-up: failed queries, compacted, through the shortlist kernel without a threshold (long
+        // shortlists: the CUDA-core kernel with exact FP32 keys); blocks whose rows are past the
+        // failure count return at once
+        const FixGroups fg = fix_groups(sp, part, c.kp);
+        if (sp.simt_fix) {
+            KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, 32, 0, 0, nullptr, (uint32_t*)E.thr2.p, s,
+                                 nullptr, fail_idx, fail_cnt, &fg));
+        } else {
             TcArgs t;
             memset(&t, 0, sizeof(t));
             int r = encode_rows_bf16(&t.tm_bf, bf_p, N, c.dpb, c.dpb);
             if (r) return r;
-            uint32_t* thr2 = (uint32_t*)E.thr2.p;
-            KNN_CUDA(cudaMemsetAsync(thr2, 0xFF, rows * sizeof(uint32_t), s));
             t.not_exact = bf_gate;  // the BF16 variant runs when the data are BF16 (always in the BF16 form)
             t.dpb = c.dpb;
             t.cn = cn;
             t.queries = queries;
-            t.Q = rows;
+            t.Q = Q;
             t.ldq = ldq;
             t.N = N;
-            t.split_len = split_len;
-            t.part = part;
-            t.thr_g = thr2;
+            t.thr_g = (uint32_t*)E.thr2.p;
             t.qmap = fail_idx;
             t.qcount = fail_cnt;
-            t.qbase = qbase;
+            t.fix = fg;
             t.err = (int*)E.err.p;
             t.D = D;
             t.dp = kChunkK;
             t.kp = c.kp;
             t.stages = std::min(4, tc_max_stages(c.kp));
-            KNN_CUDA(launch_tc(t, splits, true, s));
-            SelectExtra ex;
-            ex.qmap = fail_idx;
-            ex.qcount = fail_cnt;
-            ex.qbase = qbase;
-            KNN_CUDA(launch_select(part, splits, rows, c.kp, k, corpus, ldc, queries, ldq, D, c.rerank,
-                                   c.rerank ? nullptr : (const float*)E.qn.p, dist, idx, idx_f, s, ex));
-            launches += 2;
-            return KNNS_OK;
-        };
-        if ((rc = fix_pass(0, sp.fixA_rows, sp.fixA_S, sp.fixA_len))) return rc;
-        if ((rc = fix_pass(sp.fixA_rows, sp.fixB_rows, sp.fixB_S, sp.fixB_len))) return rc;
+            KNN_CUDA(launch_tc(t, 1, true, s));
+        }
+        SelectExtra ex;
+        ex.qmap = fail_idx;
+        ex.qcount = fail_cnt;
+        ex.fix = fg;
+        KNN_CUDA(launch_select(nullptr, 0, Q, c.kp, k, corpus, ldc, queries, ldq, D, c.rerank,
+                               c.rerank ? nullptr : (const float*)E.qn.p, dist, idx, idx_f, s, ex));
+        launches += 2;
         if (tf_scan && !ts_side && !blocked && (rc = ts.fix())) return rc;
         if (ts_side) KNN_CUDA(cudaStreamWaitEvent(s, E.order_event(1), 0));
         if (tf_scan && blocked) KNN_CUDA(cudaStreamWaitEvent(s, oev(4 + 3 * nblk), 0));

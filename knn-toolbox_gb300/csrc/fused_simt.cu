@@ -35,14 +35,22 @@ simt_kernel(const float* __restrict__ corpus, int64_t N, int64_t ldc, const floa
             const float* __restrict__ queries, int64_t Q, int64_t ldq, int D, int kp,
             int64_t split_len, uint64_t* __restrict__ part, uint32_t* __restrict__ thr_g_all,
             const uint32_t* __restrict__ tile_redo, const int32_t* __restrict__ qmap,
-            const uint32_t* __restrict__ qcount, int64_t qbase)
+            const uint32_t* __restrict__ qcount, const FixGroups fix)
 {
     if (tile_redo != nullptr && tile_redo[blockIdx.x] == 0u) return;
-    // compacted rows: row r is query qmap[qbase + r], present while qbase + r < *qcount
-    int64_t qvalid = Q;
+    // fix-up: this block's group, query tile and corpus split
+    int64_t qvalid = Q, qbase = 0;
+    int bx = (int)blockIdx.x, by = (int)blockIdx.y;
     if (qcount != nullptr) {
+        const FixBlock f = fix_block(fix, (int)blockIdx.x);
+        bx = f.tile;
+        by = f.split;
+        Q = f.g.rows;
+        split_len = f.g.split_len;
+        part = f.g.part;
+        qbase = f.row0;
         qvalid = min(Q, (int64_t)*qcount - qbase);
-        if ((int64_t)blockIdx.x * QPB >= qvalid) return;
+        if ((int64_t)bx * QPB >= qvalid) return;
     }
     constexpr int RQ = QPB / 16;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -58,8 +66,8 @@ simt_kernel(const float* __restrict__ corpus, int64_t N, int64_t ldc, const floa
     v.buf = sl + (size_t)QPB * kp;
 
     const int tid = threadIdx.x;
-    const int64_t q0 = (int64_t)blockIdx.x * QPB;
-    const int64_t n_begin = (int64_t)blockIdx.y * split_len;
+    const int64_t q0 = (int64_t)bx * QPB;
+    const int64_t n_begin = (int64_t)by * split_len;
     const int64_t n_end = min(N, n_begin + split_len);
 
     for (int i = tid; i < QPB * kp; i += kThreads) v.list[i] = kSentinel;
@@ -68,7 +76,7 @@ simt_kernel(const float* __restrict__ corpus, int64_t N, int64_t ldc, const floa
     const bool owner = tid < QPB;
     const int64_t q = q0 + tid;
     LaneState st{0, q < qvalid ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000)};
-    uint32_t* thr_g = (owner && q < qvalid) ? thr_g_all : nullptr;
+    uint32_t* thr_g = (owner && q < qvalid) ? thr_g_all + qbase : nullptr;
     const int tx = tid & 15, ty = tid >> 4;
 
     for (int64_t n0 = n_begin; n0 < n_end; n0 += kNT) {
@@ -140,7 +148,7 @@ simt_kernel(const float* __restrict__ corpus, int64_t N, int64_t ldc, const floa
     }
     if (owner) st = flush_all(v, tid, st);
     __syncthreads();
-    uint64_t* out = part + ((size_t)blockIdx.y * Q + q0) * kp;
+    uint64_t* out = part + ((size_t)by * Q + q0) * kp;
     const int64_t nq = min((int64_t)QPB, qvalid - q0);
     for (int64_t i = tid; i < nq * kp; i += kThreads) out[i] = v.list[i];
 }
@@ -153,23 +161,25 @@ size_t simt_smem_bytes(int qpb, int kp)
 cudaError_t launch_simt(const float* corpus, int64_t N, int64_t ldc, const float* cn,
                         const float* queries, int64_t Q, int64_t ldq, int D, int kp, int qpb,
                         int64_t split_len, int splits, uint64_t* part, uint32_t* thr_g, cudaStream_t s,
-                        const uint32_t* tile_redo, const int32_t* qmap, const uint32_t* qcount, int64_t qbase)
+                        const uint32_t* tile_redo, const int32_t* qmap, const uint32_t* qcount, const FixGroups* fix)
 {
-    if ((qmap == nullptr) != (qcount == nullptr) || qbase < 0) return cudaErrorInvalidValue;
+    if ((qmap == nullptr) != (qcount == nullptr) || (qmap == nullptr) != (fix == nullptr)) return cudaErrorInvalidValue;
+    const FixGroups fg = fix ? *fix : FixGroups();
     size_t smem = simt_smem_bytes(qpb, kp);
     dim3 grid((unsigned)((Q + qpb - 1) / qpb), (unsigned)splits);
+    if (fix) grid = dim3((unsigned)fix->blocks());
     if (qpb == 128) {
         cudaError_t e = cudaFuncSetAttribute(simt_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
         simt_kernel<128><<<grid, kThreads, smem, s>>>(corpus, N, ldc, cn, queries, Q, ldq, D, kp,
-                                                      split_len, part, thr_g, tile_redo, qmap, qcount, qbase);
+                                                      split_len, part, thr_g, tile_redo, qmap, qcount, fg);
     } else {
         cudaError_t e = cudaFuncSetAttribute(simt_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
         simt_kernel<32><<<grid, kThreads, smem, s>>>(corpus, N, ldc, cn, queries, Q, ldq, D, kp,
-                                                     split_len, part, thr_g, tile_redo, qmap, qcount, qbase);
+                                                     split_len, part, thr_g, tile_redo, qmap, qcount, fg);
     }
     return cudaGetLastError();
 }

@@ -163,11 +163,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     extern __shared__ __align__(1024) unsigned char sm[];
     // redo pass: only flagged query tiles run
     if (a.tile_redo != nullptr && a.tile_redo[blockIdx.x] == 0u) return;
-    // compacted-query mode: rows past the listed queries accept nothing; empty tiles return
-    int64_t qvalid = a.Q;
+    // fix-up: this block's group, query tile and corpus split; rows past the listed queries accept
+    // nothing, empty tiles return
+    int64_t Q = a.Q, qvalid = a.Q, qbase = 0, split_len = a.split_len;
+    int bx_ = (int)blockIdx.x, by_ = (int)blockIdx.y;
+    uint64_t* part = a.part;
     if (a.qcount != nullptr) {
-        qvalid = min(a.Q, (int64_t)*a.qcount - a.qbase);
-        if ((int64_t)blockIdx.x * kTileQ >= qvalid) return;
+        const FixBlock f = fix_block(a.fix, (int)blockIdx.x);
+        bx_ = f.tile;
+        by_ = f.split;
+        Q = f.g.rows;
+        split_len = f.g.split_len;
+        part = f.g.part;
+        qbase = f.row0;
+        qvalid = min(Q, (int64_t)*a.qcount - qbase);
+        if ((int64_t)bx_ * kTileQ >= qvalid) return;
     }
     // only the variant that matches the data runs
     if (a.not_exact != nullptr) {
@@ -215,9 +225,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     s.keystage = reinterpret_cast<float*>(s.buf + (size_t)kBufCap * kTileQ);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t q0 = (int64_t)blockIdx.x * kTileQ;
-    const int64_t n_begin = (int64_t)blockIdx.y * a.split_len;
-    const int64_t n_end = min(a.N, n_begin + a.split_len);
+    const int64_t q0 = (int64_t)bx_ * kTileQ;
+    const int64_t n_begin = (int64_t)by_ * split_len;
+    const int64_t n_end = min(a.N, n_begin + split_len);
     const int ntiles = (int)((n_end - n_begin + kTileN - 1) / kTileN);
     // K steps: TF32 chunks of 32 elements per 128-byte row; BF16 groups of `bps` boxes of 64
     const int nchunks = kBF16 ? nbox_bf / bps : a.dp / kChunkK;
@@ -376,7 +386,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
 
         // A operand: this thread's query row into TMEM (BF16 pairs, or TF32 hi/lo)
         const bool qok = q < qvalid;
-        const int64_t qsrc = !qok ? 0 : (a.qmap != nullptr ? (int64_t)a.qmap[a.qbase + q] : q);
+        const int64_t qsrc = !qok ? 0 : (a.qmap != nullptr ? (int64_t)a.qmap[qbase + q] : q);
         const float* qrow = a.queries + qsrc * a.ldq;
         uint32_t any_lo = 0;
         if (kBF16) {
@@ -417,7 +427,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
 
         // padding rows of the last query tile accept nothing
         LaneState st{0, qok ? __int_as_float(0x7f800000) : -__int_as_float(0x7f800000)};
-        uint32_t* thr_g = qok ? a.thr_g : nullptr;
+        uint32_t* thr_g = qok && a.thr_g != nullptr ? a.thr_g + qbase : nullptr;
         uint32_t g_pending = thr_g ? __ldcg(thr_g + q) : 0xFFFFFFFFu;
         const bool dump = a.dump != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
         for (int t = 0; t < ntiles; ++t) {
@@ -494,7 +504,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_kernel(const __grid_constant
     }
 
     const int64_t nq = min((int64_t)kTileQ, qvalid - q0);
-    uint64_t* out = a.part + ((size_t)blockIdx.y * a.Q + q0) * a.kp;
+    uint64_t* out = part + ((size_t)by_ * Q + q0) * a.kp;
     for (int64_t i = tid; i < nq * a.kp; i += kTcThreads) out[i] = s.list[i];
 }
 
@@ -505,6 +515,7 @@ cudaError_t launch_tc(const TcArgs& a, int splits, bool bf16, cudaStream_t st)
         return cudaErrorInvalidValue;
     const size_t smem = tc_smem_bytes(a.kp, a.stages);
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);
+    if (a.qcount) grid = dim3((unsigned)a.fix.blocks());
     cudaError_t e;
     if (bf16) {
         e = cudaFuncSetAttribute(tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

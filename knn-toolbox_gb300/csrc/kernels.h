@@ -84,16 +84,44 @@ cudaError_t launch_prep(const PrepJob& job, cudaStream_t s);
 // norms of rows of any width
 cudaError_t launch_row_norms(const float* x, int64_t n, int64_t ld, int D, float* norms, int64_t n_pad, cudaStream_t s);
 
+// Fix-up launches: compacted rows (row r is query qmap[r], present while r < *qcount) in two groups
+// that one 1-D grid covers, the first rows on enough corpus splits to fill the GPU, the rest (rare) on
+// a few.  Blocks of rows past the count return at once.  thr: one word per row, all ones.
+struct FixGroup {
+    int64_t rows = 0, split_len = 0;
+    int tiles = 0, splits = 0;  // query tiles, corpus splits
+    uint64_t* part = nullptr;   // [splits][rows][kp]
+};
+struct FixGroups {
+    FixGroup g[2];
+    int blocks() const { return g[0].tiles * g[0].splits + g[1].tiles * g[1].splits; }
+};
+
+#ifdef __CUDACC__
+struct FixBlock {
+    FixGroup g;
+    int tile, split;  // within the group
+    int64_t row0;     // the group's first compacted row
+};
+__device__ __forceinline__ FixBlock fix_block(const FixGroups& f, int b)
+{
+    const int na = f.g[0].tiles * f.g[0].splits;
+    const bool second = b >= na;
+    const FixGroup g = second ? f.g[1] : f.g[0];
+    const int i = second ? b - na : b;
+    return {g, i / g.splits, i % g.splits, second ? f.g[0].rows : 0};
+}
+#endif
+
 // CUDA-core FP32 fused distance + shortlist.  qpb in {32, 128}.
 size_t simt_smem_bytes(int qpb, int kp);
 // tile_redo (optional): a CTA runs only when tile_redo[blockIdx.x] != 0.
-// qmap / qcount / qbase (optional, together): compacted rows, as for TcArgs -- row r of the
-// launch (r < Q) is query qmap[qbase + r], present only when qbase + r < *qcount.
+// fix (optional, with qmap and qcount): a fix-up launch; Q, split_len, splits and part are the groups'.
 cudaError_t launch_simt(const float* corpus, int64_t N, int64_t ldc, const float* cn,
                         const float* queries, int64_t Q, int64_t ldq, int D, int kp, int qpb,
                         int64_t split_len, int splits, uint64_t* part, uint32_t* thr_g, cudaStream_t s,
                         const uint32_t* tile_redo = nullptr, const int32_t* qmap = nullptr,
-                        const uint32_t* qcount = nullptr, int64_t qbase = 0);
+                        const uint32_t* qcount = nullptr, const FixGroups* fix = nullptr);
 
 // Tensor-core 3xTF32 fused distance + shortlist (tcgen05, TMA, TMEM).
 struct TcArgs {
@@ -112,11 +140,11 @@ struct TcArgs {
     const uint32_t* corpus_any_lo;  // 1 when any corpus tile has a low part (null: assume so)
     const uint32_t* not_exact;      // 0 when corpus and queries are BF16-exact (null: TF32 path only)
     const uint32_t* tile_redo;      // optional: a CTA runs only when tile_redo[blockIdx.x] != 0
-    // optional compacted-query mode: row r of this launch (r < Q) is query qmap[qbase + r],
-    // present only when qbase + r < *qcount; part / thr_g rows are indexed by r
+    // optional (qcount non-null): a fix-up launch of the groups in fix; Q, split_len and part are the
+    // groups', thr_g rows are the compacted ones
     const int32_t* qmap;
     const uint32_t* qcount;
-    int64_t qbase;
+    FixGroups fix;
     float* dump;              // optional: raw dot tile of CTA (0,0), tile 0, [128][128]
     int* err;                 // device error word
     int D;
@@ -158,6 +186,8 @@ struct ScanArgs {
     const uint32_t* skip_if;   // optional: the kernel returns at once when *skip_if != 0
     uint64_t* cand;            // [splits*kScanParts][Q][cap]
     uint32_t* cnt;             // [splits*kScanParts][Q]
+    float* keys;               // dense pass (else null): every key, to keys[q * ldk + row] (rows past the
+    int64_t ldk;               // view: +inf); cand, cnt, cap, thr unused; ldk a multiple of the tile rows
     int* err;                  // device error word
     int64_t Q;
     int64_t N;
@@ -196,6 +226,8 @@ struct TscanArgs {
     const uint32_t* clo_flags;    // [128-row tiles of the view] same for the corpus (null: all)
     uint64_t* cand;               // [splits*kScanParts][Q][cap]
     uint32_t* cnt;                // [splits*kScanParts][Q]
+    float* keys;                  // dense pass, as ScanArgs
+    int64_t ldk;
     int* err;                     // device error word
     int64_t Q;
     int64_t N;
@@ -227,13 +259,16 @@ struct FscanArgs {
     const uint16_t* qhi;          // queries hi / lo [Q][hp] fp16 (D <= kFscanTmemD)
     const uint16_t* qlo;
     const float* qs;              // [Q] query row scales
-    const float* cn;              // [>= N + tile rows] corpus norms of the view, +inf padding
-    const float* cs;              // [>= N + tile rows] corpus row scales of the view, 0 padding
+    const float* cn;              // corpus norms, every stride-th one the view's; stride 1: [>= N + tile
+    const float* cs;              // rows] with +inf padding; row scales likewise, 0 padding
+    int64_t stride;
     const float* thr;             // [Q] thresholds (null: +inf, every key collected)
     const uint32_t* qlo_flags;    // D > kFscanTmemD: [query tiles] 1 when the tile has a low part (null: all)
     const uint32_t* clo_flags;    // [128-row tiles of the view, + 1] same for the corpus (null: all)
     uint64_t* cand;               // [splits*kScanParts][Q][cap]
     uint32_t* cnt;                // [splits*kScanParts][Q]
+    float* keys;                  // dense pass, as ScanArgs
+    int64_t ldk;
     int* err;                     // device error word
     int64_t Q;
     int64_t N;
@@ -257,8 +292,8 @@ cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st);
 //    entries, set redo_out[q / qtile] = 1 and write no result for q;
 //  * redo_in: process only queries whose tile has redo_in[q / qtile] != 0.
 //  * skip_if_zero: the kernel does nothing when *skip_if_zero == 0 (device-side path choice);
-//  * qmap / qcount / qbase: compacted rows, as for TcArgs: part row r is query
-//    qmap[qbase + r], present when qbase + r < *qcount; results go to that query's row.
+//  * qmap / qcount / fix: the rows of a fix-up launch: row r is query qmap[r], present when
+//    r < *qcount; results go to that query's row.
 struct SelectExtra {
     uint32_t* thr_out = nullptr;
     int thr_rank = 0;
@@ -269,13 +304,21 @@ struct SelectExtra {
     const uint32_t* skip_if_zero = nullptr;
     const int32_t* qmap = nullptr;
     const uint32_t* qcount = nullptr;
-    int64_t qbase = 0;
+    FixGroups fix;
 };
 size_t select_smem_bytes(int kp, int D, int rerank);
 cudaError_t launch_select(const uint64_t* part, int splits, int64_t Q, int kp, int k,
                           const float* corpus, int64_t ldc, const float* queries, int64_t ldq,
                           int D, int rerank, const float* qn, float* out_dist, int32_t* out_idx,
                           float* out_idx_f, cudaStream_t s, const SelectExtra& ex = SelectExtra());
+
+// Seeding from a dense pass's keys: thr_out[q] = the next float above the key of rank `rank`
+// (1-based) of keys[q * ldk .. + n), n <= kDenseRows; +inf when fewer keys are finite.  *clear
+// becomes 0 whatever the gates (skip_if / skip_if_zero as CandSelect) say.
+constexpr int kDenseRows = 8192;
+cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int rank, int64_t Q, float* thr_out,
+                                   uint32_t* clear, const uint32_t* skip_if, const uint32_t* skip_if_zero,
+                                   cudaStream_t s);
 
 // Selection over the threshold scan's candidate segments (one warp per query).
 // The candidates of query q are the first min(cnt, cap) words of its nseg
@@ -316,6 +359,7 @@ struct CandSelect {
     float* out_idx_f = nullptr;
     int32_t* fail_idx = nullptr;
     uint32_t* fail_cnt = nullptr;
+    uint32_t* fail_thr = nullptr;  // all ones at every failed query's place (the fix-up's thresholds)
     // exact-key test (optional): keys and distances are exact integers when every corpus and
     // query value is an integer, 2 * D * max|x|^2 < 2^24 and the BF16 copies are exact; the
     // re-rank is then skipped (distance = key + qn[q], the same value it would compute)

@@ -115,7 +115,7 @@ __device__ __forceinline__ bool scan_wait(const ScanArgs& a, const ScanSmem& s, 
     return false;
 }
 
-template <int TN, int kNacc, bool kF8>
+template <int TN, int kNacc, bool kF8, bool kDense>
 __global__ void __launch_bounds__(kScanThreads, 1)
     scan_kernel(const __grid_constant__ ScanArgs a)
 {
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kScanThreads, 1)
             ptx::mbar_init(&s.nfull[b], 1);
             ptx::mbar_init(&s.nempty[b], kEpiWarps);
         }
-        ptx::mbar_init(s.aready, 4);
+        ptx::mbar_init(s.aready, kEpiWarps);
         ptx::mbar_init(s.drain, kIssuers);
         *s.abort = 0;
         ptx::fence_mbar_init();
@@ -315,21 +315,28 @@ __global__ void __launch_bounds__(kScanThreads, 1)
         const int64_t q = q0 + row;
         const bool valid = q < a.Q;
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
-        if (part == 0) {
+        {
             // A operand: this lane's query into TMEM (BF16 pairs or E4M3 quads per 32-bit column,
-            // lower K index in the low bits); BF16 keys take -2 q (exact: a power of two)
-            const uint32_t* qrow = reinterpret_cast<const uint32_t*>(a.qbf) + (valid ? q : 0) * (a.dpb / 2);
-            for (int bx = 0; bx < nbox; ++bx) {
+            // lower K index in the low bits), a box of 32 columns per part in turn; BF16 keys take
+            // -2 q (exact: a power of two)
+            const uint4* qrow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint32_t*>(a.qbf) +
+                                                               (valid ? q : 0) * (a.dpb / 2));
+            for (int bx = part; bx < nbox; bx += kScanParts) {
                 float w[32];
 #pragma unroll
-                for (int u = 0; u < 32; ++u) {
-                    uint32_t x = valid ? __ldg(qrow + bx * 32 + u) : 0u;
-                    if (kNM) {
-                        __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&x);
-                        h = __hmul2(h, __float2bfloat162_rn(-2.f));
-                        x = *reinterpret_cast<const uint32_t*>(&h);
+                for (int u = 0; u < 8; ++u) {
+                    uint4 x4 = make_uint4(0u, 0u, 0u, 0u);
+                    if (valid) x4 = __ldg(qrow + bx * 8 + u);
+                    uint32_t x[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (kNM) {
+                            __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162*>(&x[i]);
+                            h = __hmul2(h, __float2bfloat162_rn(-2.f));
+                            x[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                        w[4 * u + i] = __uint_as_float(x[i]);
                     }
-                    w[u] = __uint_as_float(x);
                 }
                 __syncwarp();
                 ptx::tmem_st32(tmem + lane_base + kACol + (uint32_t)(bx * 32), w);
@@ -343,7 +350,8 @@ __global__ void __launch_bounds__(kScanThreads, 1)
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const float m = kF8 ? -2.0f * (valid ? __ldg(a.qs + q) : 0.f) : -2.0f;
         const size_t seg = (size_t)split * kScanParts + part;
-        uint64_t* out = a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -392,10 +400,19 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 gb = chunk_keys<W2, kF8>(vb, nrm + c2, scl + c2, m, T, vb);
                 if constexpr (W3 > 0) gc = chunk_keys<W3, kF8>(vc, nrm + c3, scl + c3, m, T, vc);
             }
-            if (__any_sync(0xffffffffu, ga != 0u)) chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
-            if (__any_sync(0xffffffffu, (gb | gc) != 0u)) {
-                chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
-                if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
+            if constexpr (kDense) {
+                if (valid) {
+                    float* dst = krow + nb;
+                    chunk_store<W1>(va, dst + c1);
+                    chunk_store<W2>(vb, dst + c2);
+                    if constexpr (W3 > 0) chunk_store<W3>(vc, dst + c3);
+                }
+            } else {
+                if (__any_sync(0xffffffffu, ga != 0u)) chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
+                if (__any_sync(0xffffffffu, (gb | gc) != 0u)) {
+                    chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
+                    if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
+                }
             }
             if constexpr (kF8) {
                 // norm slot ns fully read
@@ -403,7 +420,7 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
             }
         }
-        if (valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
+        if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
 
     ptx::tc_fence_before();
@@ -468,10 +485,10 @@ int scan_plan(int dpb, int want_bps, int* bps, int* ring, bool fp8, int accs)
 template <int TN, int kNacc, bool kF8>
 static cudaError_t launch_scan_t(const ScanArgs& a, dim3 grid, size_t smem, cudaStream_t st)
 {
-    cudaError_t e = cudaFuncSetAttribute(scan_kernel<TN, kNacc, kF8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    auto* kernel = a.keys ? scan_kernel<TN, kNacc, kF8, true> : scan_kernel<TN, kNacc, kF8, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    scan_kernel<TN, kNacc, kF8><<<grid, kScanThreads, smem, st>>>(a);
+    kernel<<<grid, kScanThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -482,7 +499,7 @@ cudaError_t launch_scan(const ScanArgs& a, int splits, cudaStream_t st)
     const int tn = scan_tile_rows(a.dpb, a.accs);
     const bool f8 = a.fp8 != 0;
     if (a.dpb % 64 != 0 || nbox < 1 || nbox > 4 || a.bps < 1 || nbox % a.bps != 0 || a.ring < 2 ||
-        a.ring > kScanMaxRing || a.split_len % tn != 0 || a.cap < 1 || splits < 1 || a.split0 < 0 || a.qbf == nullptr ||
+        a.ring > kScanMaxRing || a.split_len % tn != 0 || (!a.keys && a.cap < 1) || splits < 1 || a.split0 < 0 || a.qbf == nullptr ||
         a.ksteps < 1 || a.ksteps > 4 * nbox || (f8 && (a.cs == nullptr || a.qs == nullptr)))
         return cudaErrorInvalidValue;
     const size_t smem = scan_smem_bytes(a.dpb, a.bps, a.ring, f8, a.accs);

@@ -113,5 +113,14 @@ __device__ __forceinline__ void chunk_append(const float (&key)[W], uint32_t gm,
     }
 }
 
+// W keys of one lane to its row of the dense key matrix (16-byte aligned).
+template <int W>
+__device__ __forceinline__ void chunk_store(const float (&key)[W], float* dst)
+{
+#pragma unroll
+    for (int u = 0; u < W / 4; ++u)
+        reinterpret_cast<float4*>(dst)[u] = make_float4(key[4 * u], key[4 * u + 1], key[4 * u + 2], key[4 * u + 3]);
+}
+
 }  // namespace
 }  // namespace knn

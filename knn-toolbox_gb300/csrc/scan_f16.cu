@@ -24,14 +24,14 @@
 // FP64 relative to ||c||^2 + ||q||^2, rms: uniform D = 128 6.4e-7 against 9.8e-7, D = 1,024 5.9e-6
 // against 8.2e-6, Gaussian D = 96 1.1e-7 against 1.8e-7, mixture D = 96 2.9e-7 against 4.6e-7.
 //
-// Warp roles (608 threads):
+// Warp roles (640 threads):
 //   warp 0      producer: per tile and K chunk of 64 columns (one 128-byte swizzle row) the
-//               corpus boxes (2-D TMA), low parts only where present; per tile the corpus norms
-//               and row scales (1-D bulk copies);
+//               corpus boxes (2-D TMA), low parts only where present;
 //   warps 1, 18 MMA issuers;
 //   warps 2..17 epilogue: thread = query (TMEM lane); warp 2 + 4p + j reads part p of the tile's
 //               columns in lane quarter j, releases the accumulator, forms the keys, appends
-//               those below the threshold.
+//               those below the threshold (dense passes: stores every key in the query's row);
+//   warp 19     per tile the norms and row scales: bulk copies, or a gather for a strided view.
 // Every mbarrier wait is bounded; on timeout the kernel records an error code in the device
 // error word and winds down without hanging the GPU.
 #include <algorithm>
@@ -49,7 +49,7 @@ namespace {
 constexpr int kParts = kScanParts;           // epilogue column parts
 constexpr int kEpi = 4 * kParts;             // epilogue warps
 constexpr int kIss = 2;                      // MMA issuing warps
-constexpr int kThreads = 32 * (1 + kIss + kEpi);
+constexpr int kThreads = 32 * (2 + kIss + kEpi);
 constexpr int kCols = 64;                    // FP16 columns per K chunk (128-byte swizzle rows)
 constexpr uint32_t kBox = 128u * 128u;       // one operand box: 128 rows x 64 FP16
 constexpr uint32_t kCtrl = 512;
@@ -85,6 +85,39 @@ __device__ __forceinline__ bool f_wait(const FscanArgs& a, const FSmem& s, uint6
 // K steps of 16 columns that hold data in chunk c of rows of D columns (the rest are zeros)
 __device__ __forceinline__ int chunk_steps(int D, int c) { return min(4, (D - c * kCols + 15) >> 4); }
 
+// The norm warp: norms and row scales of every tile into their ring (kSlots tiles of kRows, the
+// scales after all norms), +inf and 0 past the view.  Views of the whole corpus are contiguous and
+// padded at least one tile past their end; strided ones (the seeding samples) are gathered.
+template <int kRows, int kSlots>
+__device__ __forceinline__ void load_norms(const FscanArgs& a, const FSmem& s, int64_t n_begin, int ntiles)
+{
+    const int lane = threadIdx.x & 31;
+    for (int t = 0; t < ntiles; ++t) {
+        const int ns = t % kSlots;
+        const int64_t n0 = n_begin + (int64_t)t * kRows;
+        const bool ok = f_wait(a, s, &s.nempty[ns], ((uint32_t)(t / kSlots) & 1u) ^ 1u, kDevTimeoutProducer);
+        if (!__all_sync(0xffffffffu, ok)) return;
+        float* nrm = s.norms + ns * kRows;
+        float* scl = s.norms + (kSlots + ns) * kRows;
+        if (a.stride == 1) {
+            if (lane == 0) {
+                ptx::mbar_arrive_expect_tx(&s.nfull[ns], 2u * kRows * 4u);
+                ptx::bulk_load(nrm, a.cn + n0, kRows * 4u, &s.nfull[ns]);
+                ptx::bulk_load(scl, a.cs + n0, kRows * 4u, &s.nfull[ns]);
+            }
+        } else {
+#pragma unroll
+            for (int i = lane; i < kRows; i += 32) {
+                const bool in = n0 + i < a.N;
+                nrm[i] = in ? __ldg(a.cn + (n0 + i) * a.stride) : __int_as_float(0x7f800000);
+                scl[i] = in ? __ldg(a.cs + (n0 + i) * a.stride) : 0.f;
+            }
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&s.nfull[ns]);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- queries in tensor memory
 // Rows of at most 256 columns.  The query tile's hi and lo parts sit in tensor memory (A from
 // TMEM, two FP16 per column: hi [0, 32 nch), lo [32 nch, 64 nch)), so the ring carries only corpus
@@ -102,6 +135,7 @@ constexpr int kMaxAcc = 3;
 constexpr int kNorm = 8;                     // tiles of corpus norms and scales in flight
 constexpr uint32_t kSlotTA = 2u * kBox;      // corpus hi, corpus lo
 
+template <bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_constant__ FscanArgs a)
 {
     constexpr uint32_t kIdesc = ptx::idesc_f16(kTileQ, kTN);
@@ -192,16 +226,6 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
                 }
                 if (h) it[1] = i;
                 else it[0] = i;
-                if (!ok) break;
-                const int ns = t % kNorm;
-                if (!f_wait(a, s, &s.nempty[ns], ((uint32_t)(t / kNorm) & 1u) ^ 1u, kDevTimeoutProducer)) {
-                    ok = false;
-                    break;
-                }
-                // padded at least one tile past the view (norms with +inf, scales with 0)
-                ptx::mbar_arrive_expect_tx(&s.nfull[ns], 2u * kTN * 4u);
-                ptx::bulk_load(s.norms + ns * kTN, a.cn + n0, kTN * 4u, &s.nfull[ns]);
-                ptx::bulk_load(s.norms + (kNorm + ns) * kTN, a.cs + n0, kTN * 4u, &s.nfull[ns]);
             }
             if (!ok) {
                 // let copies already issued land before the CTA winds down
@@ -212,6 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
                 }
             }
         }
+    } else if (warp == 3 + kEpi) {
+        load_norms<kTN, kNorm>(a, s, n_begin, ntiles);
     } else if (warp == 1 || warp == 2 + kEpi) {
         // ------------------------------------------------------------ MMA issuers
         if (lane == 0) {
@@ -294,7 +320,8 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const float m = valid ? -2.0f * __ldg(a.qs + q) : 0.f;
         const size_t seg = (size_t)split * kParts + part;
-        uint64_t* out = a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -315,12 +342,15 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNorm * kTN, m, T, v);
-            if (__any_sync(0xffffffffu, g != 0u))
+            if constexpr (kDense) {
+                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+            } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+            }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
         }
-        if (valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
+        if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
 
     ptx::tc_fence_before();
@@ -345,6 +375,7 @@ constexpr int kAccW = 2;
 constexpr int kNormW = 4;
 constexpr uint32_t kSlotW = 6u * kBox;       // query hi, query lo, corpus hi (2 boxes), corpus lo
 
+template <bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_constant__ FscanArgs a)
 {
     constexpr uint32_t kIdesc = ptx::idesc_f16(kTileQ, kWN);
@@ -433,15 +464,6 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
                     if (qlo) ptx::tma_load_2d(dst + kBox, &a.tm_qlo, &s.full[st], c * kCols, (int)q0);
                     if (clo) ptx::tma_load_2d(dst + 4 * kBox, &a.tm_clo, &s.full[st], c * kCols, (int)n0);
                 }
-                if (!ok) break;
-                const int ns = t % kNormW;
-                if (!f_wait(a, s, &s.nempty[ns], ((uint32_t)(t / kNormW) & 1u) ^ 1u, kDevTimeoutProducer)) {
-                    ok = false;
-                    break;
-                }
-                ptx::mbar_arrive_expect_tx(&s.nfull[ns], 2u * kWN * 4u);
-                ptx::bulk_load(s.norms + ns * kWN, a.cn + n0, kWN * 4u, &s.nfull[ns]);
-                ptx::bulk_load(s.norms + (kNormW + ns) * kWN, a.cs + n0, kWN * 4u, &s.nfull[ns]);
             }
             if (!ok) {
                 // let copies already issued land before the CTA winds down
@@ -449,6 +471,8 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
                     ptx::mbar_wait(&s.full[j % kRingW], (uint32_t)(j / kRingW) & 1u, kTimeout);
             }
         }
+    } else if (warp == 3 + kEpi) {
+        load_norms<kWN, kNormW>(a, s, n_begin, ntiles);
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
@@ -497,7 +521,8 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const float m = valid ? -2.0f * __ldg(a.qs + q) : 0.f;
         const size_t seg = (size_t)split * kParts + part;
-        uint64_t* out = a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -521,13 +546,21 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
             const float* nrm = s.norms + ns * kWN + 64 * part;
             const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kWN) + (uint32_t)(64 * part);
             const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNormW * kWN, m, T, v);
-            if (__any_sync(0xffffffffu, g != 0u)) chunk_append<32>(v, g, T, base, out, cap, cnt);
+            if constexpr (kDense) {
+                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kWN + 64 * part);
+            } else if (__any_sync(0xffffffffu, g != 0u)) {
+                chunk_append<32>(v, g, T, base, out, cap, cnt);
+            }
             const uint32_t h = chunk_keys<32, true>(w, nrm + 32, nrm + kNormW * kWN + 32, m, T, w);
-            if (__any_sync(0xffffffffu, h != 0u)) chunk_append<32>(w, h, T, base + 32u, out, cap, cnt);
+            if constexpr (kDense) {
+                if (valid) chunk_store<32>(w, krow + n_begin + (int64_t)t * kWN + 64 * part + 32);
+            } else if (__any_sync(0xffffffffu, h != 0u)) {
+                chunk_append<32>(w, h, T, base + 32u, out, cap, cnt);
+            }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
         }
-        if (valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
+        if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
 
     ptx::tc_fence_before();
@@ -552,19 +585,17 @@ cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st)
 {
     const bool ta = a.D <= kFscanTmemD;
     const int tn = fscan_tile_rows(a.D);
-    if (a.D < 1 || a.hp < a.D || a.hp % 8 != 0 || a.split_len % tn != 0 || a.cap < 1 || splits < 1 || a.split0 < 0 ||
+    if (a.D < 1 || a.hp < a.D || a.hp % 8 != 0 || a.split_len % tn != 0 || (!a.keys && a.cap < 1) || a.stride < 1 || splits < 1 || a.split0 < 0 ||
         !a.cn || !a.cs || !a.qs || (ta && (!a.qhi || !a.qlo)))
         return cudaErrorInvalidValue;
     if (a.Q <= 0) return cudaSuccess;
     const size_t smem = ta ? kSmemTA : kSmemW;
-    cudaError_t e = cudaFuncSetAttribute(ta ? fscan_ta_kernel : fscan_wide_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto* kernel = a.keys ? (ta ? fscan_ta_kernel<true> : fscan_wide_kernel<true>)
+                          : (ta ? fscan_ta_kernel<false> : fscan_wide_kernel<false>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);
-    if (ta)
-        fscan_ta_kernel<<<grid, kThreads, smem, st>>>(a);
-    else
-        fscan_wide_kernel<<<grid, kThreads, smem, st>>>(a);
+    kernel<<<grid, kThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -77,6 +77,7 @@ __device__ __forceinline__ bool t_wait(const TscanArgs& a, const TSmem& s, uint6
     return false;
 }
 
+template <bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constant__ TscanArgs a)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -235,7 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const size_t seg = (size_t)split * kParts + part;
-        uint64_t* out = a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -256,12 +258,15 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
-            if (__any_sync(0xffffffffu, g != 0u))
+            if constexpr (kDense) {
+                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+            } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+            }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
         }
-        if (valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
+        if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
 
     ptx::tc_fence_before();
@@ -332,6 +337,7 @@ __device__ __forceinline__ float tf32_round(float x)
     return __uint_as_float(u);
 }
 
+template <bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_constant__ TscanArgs a)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
@@ -516,7 +522,8 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
         }
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const size_t seg = (size_t)split * kParts + part;
-        uint64_t* out = a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
+        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -537,12 +544,15 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
-            if (__any_sync(0xffffffffu, g != 0u))
+            if constexpr (kDense) {
+                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+            } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+            }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
         }
-        if (valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
+        if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
 
     ptx::tc_fence_before();
@@ -570,20 +580,18 @@ int tscan_ring(bool tmem_a)
 cudaError_t launch_tscan(const TscanArgs& a, int splits, cudaStream_t st)
 {
     const bool ta = a.tmem_a != 0;
-    if (a.dp < 32 || a.dp % 32 != 0 || a.split_len % kTN != 0 || a.cap < 1 || splits < 1 || a.split0 < 0 ||
+    if (a.dp < 32 || a.dp % 32 != 0 || a.split_len % kTN != 0 || (!a.keys && a.cap < 1) || splits < 1 || a.split0 < 0 ||
         a.ring < 2 || a.ring > (ta ? kMaxRingTA : kMaxRing) || (ta && (a.dp > 128 || !a.queries || a.D > a.dp)))
         return cudaErrorInvalidValue;
     const size_t smem = tscan_smem_bytes(a.ring, ta);
     if (smem > kScanSmemLimit) return cudaErrorInvalidValue;
     if (a.Q <= 0) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(ta ? tscan_ta_kernel : tscan_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto* kernel = a.keys ? (ta ? tscan_ta_kernel<true> : tscan_kernel<true>)
+                          : (ta ? tscan_ta_kernel<false> : tscan_kernel<false>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);
-    if (ta)
-        tscan_ta_kernel<<<grid, kThreads, smem, st>>>(a);
-    else
-        tscan_kernel<<<grid, kThreads, smem, st>>>(a);
+    kernel<<<grid, kThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -103,15 +103,21 @@ select_kernel(const uint64_t* __restrict__ part, int splits, int64_t Q, int kp, 
     if (q >= Q) return;
     if (ex.redo_in != nullptr && ex.redo_in[q / ex.qtile] == 0u) return;
     int64_t qout = q;  // query whose results this row holds
+    int64_t rows = Q, row = q;
     if (ex.qcount != nullptr) {
-        if (ex.qbase + q >= (int64_t)*ex.qcount) return;
-        qout = ex.qmap[ex.qbase + q];
+        if (q >= (int64_t)*ex.qcount) return;
+        qout = ex.qmap[q];
+        const FixGroup g = q < ex.fix.g[0].rows ? ex.fix.g[0] : ex.fix.g[1];
+        row = q < ex.fix.g[0].rows ? q : q - ex.fix.g[0].rows;
+        rows = g.rows;
+        part = g.part;
+        splits = g.splits;
     }
 
-    for (int j = lane; j < kp; j += 32) cur[j] = part[(size_t)q * kp + j];
+    for (int j = lane; j < kp; j += 32) cur[j] = part[(size_t)row * kp + j];
     __syncwarp();
     for (int s = 1; s < splits; ++s) {
-        const uint64_t* src = part + ((size_t)s * Q + q) * kp;
+        const uint64_t* src = part + ((size_t)s * rows + row) * kp;
         for (int j = lane; j < kp; j += 32) oth[j] = src[j];
         __syncwarp();
         warp_merge_lists(cur, oth, nxt, kp);
@@ -297,6 +303,187 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_threshold_kernel(const 
     }
 }
 
+// ---------------------------------------------------------------- thresholds from dense keys
+// One block per query: the keys, as ordered words, into shared memory.  Ranks up to kDenseRank: the
+// rank-th smallest of 32 group minima (four threads each) bounds the key of that rank from above, so
+// only the few keys up to it are collected and the rank among them counted.  Otherwise the key is
+// found by a byte-wise histogram search from the highest bit in which the finite keys differ.
+// Latency-bound for few queries (48 x 3,907 keys 6.3 us, 11.9 by histogram), by issue slots for many
+// (10,000 x 1,954 keys 35 us against 60).
+constexpr int kDenseT = 128;
+constexpr int kDenseRank = 24;
+constexpr int kDenseList = 256;
+__global__ void __launch_bounds__(kDenseT) dense_threshold_kernel(const float* __restrict__ keys, int64_t ldk, int n,
+                                                                  int rank, float* __restrict__ thr_out,
+                                                                  uint32_t* clear, const uint32_t* skip_if,
+                                                                  const uint32_t* skip_if_zero)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0 && clear != nullptr) *clear = 0u;
+    if (skip_if != nullptr && *skip_if != 0u) return;
+    if (skip_if_zero != nullptr && *skip_if_zero == 0u) return;
+    extern __shared__ __align__(16) uint32_t ord[];  // [n rounded up to 4]
+    __shared__ uint32_t hist[256];
+    __shared__ uint32_t wlo[kDenseT / 32], whi[kDenseT / 32], wcnt[kDenseT / 32], digit_s, rank_s, hit_s;
+    __shared__ uint32_t gmin[32], list_n;
+    __shared__ __align__(16) uint32_t list[kDenseList];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t q = blockIdx.x;
+    if (tid == 0) list_n = 0;
+    constexpr uint32_t kInf = 0xFF800000u;  // f2ord(+inf); NaN keys count as +inf
+    const float* row = keys + q * ldk;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
+    // rows are padded with +inf to whole tiles: the last word of four may lie past n
+    for (int i = 4 * tid; i < n; i += 4 * kDenseT) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(row + i));
+        const float f[4] = {v.x, v.y, v.z, v.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            o[u] = f[u] < __int_as_float(0x7f800000) && i + u < n ? f2ord(f[u]) : kInf;
+            if (o[u] < kInf) {
+                lo = min(lo, o[u]);
+                hi = max(hi, o[u]);
+                ++cnt;
+            }
+        }
+        *reinterpret_cast<uint4*>(ord + i) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    const uint32_t mine = lo;
+    uint32_t g = min(lo, __shfl_xor_sync(0xffffffffu, lo, 1));
+    g = min(g, __shfl_xor_sync(0xffffffffu, g, 2));
+    if ((lane & 3) == 0) gmin[tid >> 2] = g;
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        wlo[warp] = lo;
+        whi[warp] = hi;
+        wcnt[warp] = cnt;
+    }
+    for (int b = tid; b < 256; b += kDenseT) hist[b] = 0;
+    __syncthreads();
+    cnt = 0;
+#pragma unroll
+    for (int w = 0; w < kDenseT / 32; ++w) {
+        lo = min(lo, wlo[w]);
+        hi = max(hi, whi[w]);
+        cnt += wcnt[w];
+    }
+    if (cnt < (uint32_t)rank) {
+        if (tid == 0) thr_out[q] = __int_as_float(0x7f800000);
+        return;
+    }
+    if (rank <= kDenseRank) {
+        // every warp ranks the 32 minima (ties by group), one per lane
+        const uint32_t v = gmin[lane];
+        int less = 0;
+#pragma unroll
+        for (int o = 0; o < 32; ++o) {
+            const uint32_t w = __shfl_sync(0xffffffffu, v, o);
+            less += w < v || (w == v && o < lane) ? 1 : 0;
+        }
+        const uint32_t at = __ballot_sync(0xffffffffu, less == rank - 1);
+        const uint32_t U = __shfl_sync(0xffffffffu, v, __ffs((int)at) - 1);
+        if (U < kInf) {  // at least `rank` keys are not above U
+            if (mine <= U)
+                for (int i = 4 * tid; i < n; i += 4 * kDenseT)
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (ord[i + u] <= U) {
+                            const uint32_t pos = atomicAdd(&list_n, 1u);
+                            if (pos < kDenseList) list[pos] = ord[i + u];
+                        }
+            __syncthreads();
+            const int m = (int)list_n;
+            if (m <= kDenseList) {
+                for (int j = tid; j < m; j += kDenseT) {
+                    const uint32_t w = list[j];
+                    int below = 0, same = 0;
+                    for (int e = 0; e < m; ++e) {
+                        below += list[e] < w ? 1 : 0;
+                        same += list[e] == w ? 1 : 0;
+                    }
+                    // equal keys write the same word
+                    if (below < rank && below + same >= rank) thr_out[q] = nextafterf(ord2f(w), __int_as_float(0x7f800000));
+                }
+                return;
+            }
+        }
+    }
+    int top = 32 - __clz((int)(lo ^ hi));  // bits [0, top) differ
+    uint32_t x = top >= 32 ? 0u : (lo >> top) << top, r = (uint32_t)rank;
+    while (top > 0) {
+        const int sh = max(top - 8, 0);
+        const uint32_t mask = top >= 32 ? 0u : ~((1u << top) - 1u);
+        for (int i = 4 * tid; i < n; i += 4 * kDenseT) {
+            const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+            const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (o[u] < kInf && (o[u] & mask) == x) atomicAdd(&hist[(o[u] >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t b[8], s = 0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                b[u] = hist[8 * lane + u];
+                s += b[u];
+            }
+            uint32_t inc = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += v;
+            }
+            uint32_t run = inc - s;
+            if (run < r && inc >= r) {
+                bool found = false;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (!found && run + b[u] >= r) {
+                        digit_s = (uint32_t)(8 * lane + u);
+                        rank_s = r - run;
+                        hit_s = b[u];
+                        found = true;
+                    }
+                    run += b[u];
+                }
+            }
+        }
+        __syncthreads();
+        x |= digit_s << sh;
+        r = rank_s;
+        top = sh;
+        if (top == 0 || (hit_s == 1u)) break;
+        for (int b = tid; b < 256; b += kDenseT) hist[b] = 0;
+        __syncthreads();
+    }
+    if (top > 0 && hit_s == 1u) {
+        // a single key in the bin: it is the one
+        const uint32_t mask = ~((1u << top) - 1u);
+        for (int i = tid; i < n; i += kDenseT)
+            if (ord[i] < kInf && (ord[i] & mask) == x) {
+                const float key = ord2f(ord[i]);
+                thr_out[q] = nextafterf(key, __int_as_float(0x7f800000));
+            }
+    } else if (tid == 0) {
+        // strictly above the key of that rank: the key itself passes a "< T" test
+        thr_out[q] = nextafterf(ord2f(x), __int_as_float(0x7f800000));
+    }
+}
+
+cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int rank, int64_t Q, float* thr_out,
+                                   uint32_t* clear, const uint32_t* skip_if, const uint32_t* skip_if_zero,
+                                   cudaStream_t s)
+{
+    if (Q <= 0) return cudaSuccess;
+    if (n < 1 || n > kDenseRows || rank < 1 || ldk % 4 != 0 || ldk < n) return cudaErrorInvalidValue;
+    const size_t smem = (size_t)((n + 3) & ~3) * 4;
+    dense_threshold_kernel<<<(unsigned)Q, kDenseT, smem, s>>>(keys, ldk, n, rank, thr_out, clear, skip_if, skip_if_zero);
+    return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- one block per query
 // Result mode of the selection, a whole block on each query.  Bound by the latency of a query's
 // chain of dependent steps (counts, gather, rank search, re-rank, sort) until every SM is full, by
@@ -313,6 +500,7 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_threshold_kernel(const 
 //  * the shortlist is then ordered once, by counting smaller words (up to kRankSortMax) or a
 //    bitonic sort.
 constexpr int kRankSortMax = 128;
+constexpr int64_t kThrBlockQ = 1536;  // threshold mode: a warp per query above
 constexpr int64_t kSelWideQ = 384;  // up to this many queries: 256 threads each, above 128
 
 // Rows of `cur` (m packed words: key or distance above index) in ascending order to the outputs.
@@ -366,7 +554,8 @@ __device__ __forceinline__ void emit_sorted(const CandSelect& c, int64_t q, uint
     for (int j = tid; j < c.k; j += kT) put(j, cur[j]);
 }
 
-template <int kT>
+// kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.
+template <int kT, bool kThr>
 __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
 {
     if (c.skip_if != nullptr && *c.skip_if != 0u) return;
@@ -374,7 +563,7 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
     constexpr int kW = kT / 32;
     extern __shared__ __align__(16) unsigned char smem[];
     uint64_t* cur = reinterpret_cast<uint64_t*>(smem);               // shortlist [pow2_at_least(kp)]
-    uint64_t* buf = cur + pow2_at_least(c.kp);                        // candidates [buf_words]
+    uint64_t* buf = kThr ? cur : cur + pow2_at_least(c.kp);           // candidates [buf_words]
     float* qv = reinterpret_cast<float*>(buf + c.buf_words);         // query [D]
     __shared__ uint32_t hist[256];
     __shared__ uint64_t wmin[kW], wmax[kW];
@@ -382,7 +571,7 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t q = blockIdx.x;
 
-    if (c.rerank)
+    if (!kThr && c.rerank)
         for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
     // segment counts: thread t owns segments t, t + kT, ...
     constexpr int kSeg = kScanMaxSegs / kT;
@@ -411,8 +600,16 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
         if (w < warp) at += t;
         total += t;
     }
-    if (overflow || total < (uint32_t)c.need || total > (uint32_t)c.buf_words) {
-        if (tid == 0) c.fail_idx[atomicAdd(c.fail_cnt, 1u)] = (int32_t)q;
+    if (kThr && (overflow || total < (uint32_t)c.thr_rank || total > (uint32_t)c.buf_words)) {
+        if (tid == 0) c.thr_out[q] = c.thr_fallback ? c.thr_fallback[q] : __int_as_float(0x7f800000);
+        return;
+    }
+    if (!kThr && (overflow || total < (uint32_t)c.need || total > (uint32_t)c.buf_words)) {
+        if (tid == 0) {
+            const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
+            c.fail_idx[pos] = (int32_t)q;
+            c.fail_thr[pos] = 0xFFFFFFFFu;
+        }
         return;
     }
     uint64_t lo = kSentinel, hi = 0;
@@ -434,7 +631,8 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
         }
         at += n[r];
     }
-    const int nn = (int)total, kp = c.kp;
+    const int nn = (int)total, kp = kThr ? c.thr_rank : c.kp;
+    uint64_t W = hi;
     int m = nn;
     uint64_t* list = buf;
     if (nn > kp) {
@@ -505,8 +703,8 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
             for (int b = tid; b < 256; b += kT) hist[b] = 0;
             __syncthreads();
         }
-        const uint64_t W = top > 0 ? x | ((1ull << top) - 1ull) : x;
-        for (int e0 = 0; e0 < nn; e0 += kT) {
+        W = top > 0 ? x | ((1ull << top) - 1ull) : x;
+        for (int e0 = 0; !kThr && e0 < nn; e0 += kT) {
             const int e = e0 + tid;
             const uint64_t w = e < nn ? buf[e] : kSentinel;
             const bool keep = e < nn && w <= W;
@@ -518,6 +716,32 @@ __global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
         }
         m = kp;
         list = cur;
+    }
+    if constexpr (kThr) {
+        // the key of rank thr_rank: the largest word not above W (nn == kp: the largest of all)
+        uint64_t best = 0;
+        if (nn > kp) {
+            for (int e = tid; e < nn; e += kT)
+                if (buf[e] <= W && buf[e] > best) best = buf[e];
+        } else {
+            best = hi;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint64_t b = __shfl_xor_sync(0xffffffffu, best, o);
+            best = b > best ? b : best;
+        }
+        __syncthreads();
+        if (lane == 0) wmax[warp] = best;
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int w = 0; w < kW; ++w) best = wmax[w] > best ? wmax[w] : best;
+            const float key = unpack_key(best);
+            // strictly above the key of rank thr_rank: that key itself passes a "< T" test
+            c.thr_out[q] = key < __int_as_float(0x7f800000) ? nextafterf(key, __int_as_float(0x7f800000)) : key;
+        }
+        return;
     }
     __syncthreads();
 
@@ -661,11 +885,19 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         c.buf_words = c.buf_words > 0 ? std::min(kCandMax, std::max((c.buf_words + 31) / 32 * 32, pow2_at_least(c.kp)))
                                       : kCandMax;
     if (c.nseg < 1 || c.nseg > kScanMaxSegs || c.cap < 1 ||
-        (!thr && (c.kp < 1 || c.kp > kMaxKpScan || c.k > c.kp || c.fail_idx == nullptr || c.fail_cnt == nullptr ||
+        (!thr && (c.kp < 1 || c.kp > kMaxKpScan || c.k > c.kp || c.fail_idx == nullptr || c.fail_cnt == nullptr || c.fail_thr == nullptr ||
                   (!c.rerank && c.qn == nullptr))) ||
         (thr && (c.thr_rank < 1 || c.thr_rank > kCandThrMax)))
         return cudaErrorInvalidValue;
-    if (thr) {
+    if (thr && c.Q <= kThrBlockQ) {
+        // a block per query while warps would leave SMs idle: 62,500-row level of 2,000,000 x 128, 64 /
+        // 777 / 2,048 queries 7.9 (256 threads) / 8.9 (128) / 11.5 against 17.8 / 10.0 / 9.7 us
+        const size_t smem = (size_t)c.buf_words * 8;
+        if (c.Q <= kSelWideQ)
+            select_block_kernel<256, true><<<(unsigned)c.Q, 256, smem, s>>>(c);
+        else
+            select_block_kernel<128, true><<<(unsigned)c.Q, 128, smem, s>>>(c);
+    } else if (thr) {
         const size_t smem = (size_t)kSelWarps * c.buf_words * 8;
         cudaError_t e = cudaFuncSetAttribute(select_threshold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
@@ -676,7 +908,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         // selection of 256 / 777 queries 9.4 / 14.4 against 11.4 / 11.4 us (65,536 x 128, k = 16),
         // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512)
         const size_t smem = ((size_t)pow2_at_least(c.kp) + c.buf_words) * 8 + (size_t)((c.D + 3) & ~3) * 4;
-        auto* kernel = c.Q <= kSelWideQ ? select_block_kernel<256> : select_block_kernel<128>;
+        auto* kernel = c.Q <= kSelWideQ ? select_block_kernel<256, false> : select_block_kernel<128, false>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         kernel<<<(unsigned)c.Q, c.Q <= kSelWideQ ? 256 : 128, smem, s>>>(c);

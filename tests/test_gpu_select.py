@@ -37,3 +37,41 @@ def test_exact_integer_keys_skip_the_rerank(engine, oracle, Q, k):
     od, oi = oracle.knn_gemm(X, Qs, k, kp=st["kp"], rerank=True)
     np.testing.assert_array_equal(i.cpu().numpy(), oi)
     np.testing.assert_array_equal(d.cpu().numpy(), od)
+
+
+@pytest.mark.parametrize("N,Q,k", [(16384, 5, 1), (32768, 300, 16), (131071, 384, 100), (131072, 385, 10),
+                                   (140_000, 1536, 10), (150_000, 1537, 10), (300_000, 20, 512), (40_000, 30, 300),
+                                   (270_000, 100, 100)])
+def test_seeding_sizes(engine, oracle, N, Q, k):
+    # dense seeding passes of few and many rows (rank counted among the keys below a bound, or by
+    # histogram for the long shortlists), the levels after them by warp and by block
+    import torch
+    rng = np.random.default_rng(N + Q)
+    X = rng.integers(0, 256, (N, 32)).astype(np.float32)
+    X[::3, 0] += 0.5 if N < 200_000 else 0.0
+    Qs = rng.integers(0, 256, (Q, 32)).astype(np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
+    st = engine.last_stats()
+    assert st["scan"] == 1 and engine.last_fixups() <= 2
+    sub = rng.choice(Q, min(Q, 40), replace=False)
+    od, oi = oracle.knn_gemm(X, Qs[sub], k, kp=st["kp"], rerank=True)
+    np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
+    np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
+
+
+def test_rows_that_are_not_finite_leave_the_thresholds_open(engine, oracle):
+    # most sample rows are NaN or infinite: too few finite keys for a threshold, every query is
+    # answered all the same
+    import torch
+    rng = np.random.default_rng(2)
+    X = rng.random((20000, 24), dtype=np.float32)
+    keep = np.zeros(20000, bool)
+    keep[5::32] = True
+    X[~keep, 4] = np.where(np.arange(20000)[~keep] % 2, np.nan, np.inf)
+    Qs = rng.random((50, 24), dtype=np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 10)
+    d, i = d.cpu().numpy(), i.cpu().numpy()
+    good = np.flatnonzero(keep)
+    assert keep[i].all()
+    od, oi = oracle.knn_gemm(X[good], Qs, 10, kp=32, rerank=True)
+    oracle.check_parity(X[good], Qs, 10, d, np.searchsorted(good, i), ref_idx=oi, gap_rel=1e-6, dist_rel=1e-5)
