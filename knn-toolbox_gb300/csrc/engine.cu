@@ -258,7 +258,7 @@ int auto_splits(int64_t qtiles, int64_t tiles, int sms, int max_splits)
     return best;
 }
 
-int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const knns_options& o, Config* c)
+static int resolve_keys(const Engine& E, int64_t N, int64_t Q, int D, int k, const knns_options& o, Config* c)
 {
     c->rerank = o.rerank ? 1 : 0;
     c->pilot = o.pilot != 0;
@@ -355,6 +355,48 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
     if (algo == KNNS_ALGO_TC && per % kTileN) per = cdiv(per, kTileN) * kTileN;
     c->split_len = per;
     c->splits = (int)cdiv(N, per);
+    return KNNS_OK;
+}
+
+// Small corpora (below kScanMinRowsForced rows, exact form, nothing asked for by the options).
+//  * Direct: one launch whose blocks each read the whole corpus for one query, while the work of a
+//    block, about N (D + 32), and of all of them stay small.  us per search, shortlist kernel / direct /
+//    dense keys: 1,000 x 32, 16 queries 152 / 13 / 25; 4,000 x 32, 128 queries 277 / 21 / 29; 2,000 x 128,
+//    128 queries 281 / 29 / 33; 1,000 x 32, 1,024 queries 261 / 37 / 33; 8,000 x 32, 128 305 / 33 / 37.
+//  * Dense keys: every key written out by one dense pass of the FP16-split scan and selected from, at
+//    most kSmallKeys of them at a time (8,000 x 300, 128 queries 408 / 155 / 49; 4,000 x 128, 4,096 queries
+//    1,038 / 1,029 / 108; 2,000 x 1,024, 1,024 queries 744 / 1,131 / 74).
+//  * From kSmallScanRows rows, more queries than that go to the FP16-split threshold scan, whose
+//    candidates are a fraction of the keys.
+constexpr int64_t kDirectBlock = 280000;
+constexpr int64_t kDirectTotal = 50000000;
+constexpr int64_t kSmallKeys = 24 << 20;
+constexpr int64_t kSmallScanRows = 8192;
+int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const knns_options& o, Config* c)
+{
+    const int rc = resolve_keys(E, N, Q, D, k, o, c);
+    if (rc || c->tscan || N >= kScanMinRowsForced || N > kSmallRows || E.cc < 100 || o.precision != KNNS_PREC_EXACT ||
+        o.algo != KNNS_ALGO_AUTO || o.scan != KNNS_SCAN_AUTO || o.splits > 0 || !o.pilot || o.tf32_only || !c->rerank ||
+        c->kp < k + kKeyMargin || k > kMaxKpScan)
+        return rc;
+    if (N * (D + 32) <= kDirectBlock && Q * N * (D + 32) <= kDirectTotal) {
+        c->small = 1;
+        c->algo = KNNS_ALGO_SIMT;
+    } else if (D <= kTscanMaxD && c->kp <= kMaxKpScan) {
+        c->algo = KNNS_ALGO_TC;
+        c->tf32 = false;
+        if (Q * N > kSmallKeys && N >= kSmallScanRows && c->kp <= kMaxKpTC) {
+            c->tscan = true;
+            c->dpb = (D + 63) & ~63;
+            c->qtile = kTileQ;
+            c->stages = 0;
+            c->splits = 0;
+            c->split_len = 0;
+        } else {
+            c->small = 2;
+        }
+    }
+    if (c->small) c->splits = 1;
     return KNNS_OK;
 }
 
@@ -971,6 +1013,126 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     return KNNS_OK;
 }
 
+// Searches of small corpora (Config::small).
+static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, const float* queries,
+                     int64_t Q, int64_t ldq, int D, int k, float* dist, int32_t* idx, float* idx_f,
+                     const knns_options& o, cudaStream_t s, knns_stats* st, const PreparedCorpus* pc, bool capture)
+{
+    const bool dense = c.small == 2;
+    const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
+    const int tn = fscan_tile_rows(D);
+    const int64_t tiles = cdiv(N, tn), ldk = tiles * tn;
+    // queries whose keys are held at once: whole query tiles
+    const int64_t chunk = std::max<int64_t>(1, kSmallKeys / N / kTileQ) * kTileQ;
+    size_t ws = 0, nwords = 0;
+    int rc = KNNS_OK, launches = 1;
+    if (dense) {
+        if (!pc) {
+            rc = E.cn.ensure(n_pad * sizeof(float));
+            if (!rc) rc = ensure_split(E, c, N, D, n_pad);
+        }
+        if (!rc) rc = flag_words(E, Q, pc ? 0 : N, &nwords);
+        if (!rc) rc = E.qhi.ensure((size_t)Q * split_pitch(D) * 2);
+        if (!rc) rc = E.qlo.ensure((size_t)Q * split_pitch(D) * 2);
+        if (!rc) rc = E.qrs.ensure(Q * sizeof(float));
+        if (!rc) rc = E.cand.ensure((size_t)std::min(Q, chunk) * ldk * sizeof(float));
+        if (rc) return rc;
+        ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qhi.cap + E.qlo.cap + E.qrs.cap +
+             E.cand.cap;
+    }
+    if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
+    cudaEvent_t tv[Engine::kTimingEvents] = {};
+    if (o.timing && E.timing_slot(tv) != KNNS_OK) return KNNS_ERR_CUDA;
+    auto mark = [&](int i) -> int {
+        if (tv[i]) KNN_CUDA(cudaEventRecord(tv[i], s));
+        return KNNS_OK;
+    };
+    if ((rc = mark(0))) return rc;
+    SmallSelect sel;
+    sel.n = (int)N;
+    sel.need = k;
+    sel.k = k;
+    sel.Q = Q;
+    sel.corpus = corpus;
+    sel.ldc = ldc;
+    sel.queries = queries;
+    sel.ldq = ldq;
+    sel.D = D;
+    sel.out_dist = dist;
+    sel.out_idx = idx;
+    sel.out_idx_f = idx_f;
+    if (dense) {
+        uint32_t* words = (uint32_t*)E.words.p;
+        KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
+        if (!pc) {
+            if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, (float*)E.cn.p, words, nullptr, s))) return rc;
+            ++launches;
+        }
+        PrepJob qj = prep_job(queries, Q, ldq, D, nullptr, Q);
+        qj.hi = E.qhi.p;
+        qj.lo = E.qlo.p;
+        qj.rs = (float*)E.qrs.p;
+        qj.lo_flags = E.qlof;
+        KNN_CUDA(launch_prep(qj, s));
+        if ((rc = mark(1)) || (rc = mark(2))) return rc;
+        const SplitCopies cp = split_copies(E, c, pc);
+        FscanArgs f;
+        memset(&f, 0, sizeof(f));
+        if (D > kFscanTmemD) {
+            rc = encode_split(&f.tm_qhi, E.qhi.p, Q, D, 1, kTileQ);
+            if (!rc) rc = encode_split(&f.tm_qlo, E.qlo.p, Q, D, 1, kTileQ);
+        }
+        if (!rc) rc = encode_split(&f.tm_chi, cp.hi, N, D, 1, tn);
+        if (!rc) rc = encode_split(&f.tm_clo, cp.lo, N, D, 1, tn);
+        if (rc) return rc;
+        f.cn = (const float*)(pc ? pc->cn.p : E.cn.p);
+        f.cs = cp.rs;
+        f.clo_flags = cp.flags;
+        f.keys = (float*)E.cand.p;
+        f.ldk = ldk;
+        f.err = (int*)E.err.p;
+        f.stride = 1;
+        f.N = N;
+        f.D = D;
+        f.hp = split_pitch(D);
+        sel.keys = f.keys;
+        sel.ldk = ldk;
+        sel.need = (int)std::min<int64_t>(c.kp, N);
+        for (int64_t q0 = 0; q0 < Q; q0 += chunk) {
+            const int64_t nq = std::min(chunk, Q - q0);
+            if (q0 > 0 && D > kFscanTmemD) {
+                rc = encode_split(&f.tm_qhi, (const char*)E.qhi.p + q0 * f.hp * 2, nq, D, 1, kTileQ);
+                if (!rc) rc = encode_split(&f.tm_qlo, (const char*)E.qlo.p + q0 * f.hp * 2, nq, D, 1, kTileQ);
+                if (rc) return rc;
+            }
+            f.qhi = (const uint16_t*)E.qhi.p + q0 * f.hp;
+            f.qlo = (const uint16_t*)E.qlo.p + q0 * f.hp;
+            f.qs = (const float*)E.qrs.p + q0;
+            f.qlo_flags = E.qlof + q0 / kTileQ;
+            f.Q = nq;
+            const int S = seed_splits(cdiv(nq, kTileQ), tiles, E.sms, (int)tiles);
+            f.split_len = cdiv(tiles, S) * tn;
+            KNN_CUDA(launch_fscan(f, (int)cdiv(N, f.split_len), s));
+            sel.Q = nq;
+            sel.queries = queries + q0 * ldq;
+            sel.out_dist = dist ? dist + q0 * k : nullptr;
+            sel.out_idx = idx ? idx + q0 * k : nullptr;
+            sel.out_idx_f = idx_f ? idx_f + q0 * k : nullptr;
+            KNN_CUDA(launch_select_small(sel, s));
+            launches += 2;
+        }
+        if ((rc = mark(3))) return rc;
+    } else {
+        for (int i = 1; i <= 3; ++i)
+            if ((rc = mark(i))) return rc;
+        KNN_CUDA(launch_select_small(sel, s));
+    }
+    if ((rc = mark(4)) || (rc = mark(5))) return rc;
+    if (!capture) KNN_CUDA(cudaEventRecord(E.last_done, s));
+    if (st) *st = knns_stats{c.algo, 1, c.kp, 0, launches, 0, (int64_t)ws, 0, 0, 0, 0, 0};
+    return KNNS_OK;
+}
+
 // ---------------------------------------------------------------- search
 int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const float* queries, int64_t Q, int64_t ldq,
                int D, int k, float* dist, int32_t* idx, float* idx_f, const knns_options& o, cudaStream_t s,
@@ -995,7 +1157,12 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     const uint64_t stall_ns = capture ? 0 : g_test_stall_ns.exchange(0);
     if (host_corpus != nullptr && (pc != nullptr || capture || ldc != D))
         return set_error(KNNS_ERR_INVALID, "a corpus streamed from the host needs pitch D and no prepared index");
-    if (c.tscan) {
+    // an index without the exact form's copies is refused below, as ever; the stall hook is the shortlist
+    // kernel's
+    if (c.small && ((pc && !pc->f16) || stall_ns)) {
+        if ((rc = resolve_keys(E, N, Q, D, k, o, &(c = Config())))) return rc;
+    }
+    if (c.tscan || c.small) {
         if (host_corpus != nullptr) {
             // the whole corpus lands before the search starts (no overlap on this path)
             cudaStream_t cs_ = E.copy_stream();
@@ -1009,6 +1176,9 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             KNN_CUDA(cudaEventRecord(e1, cs_));
             KNN_CUDA(cudaStreamWaitEvent(s, e1, 0));
         }
+        if (pc && c.small && (pc->corpus != corpus || pc->N != N || pc->ldc != ldc || pc->D != D))
+            return set_error(KNNS_ERR_INVALID, "prepared corpus does not match the search's corpus");
+        if (c.small) return run_small(E, c, corpus, N, ldc, queries, Q, ldq, D, k, dist, idx, idx_f, o, s, st, pc, capture);
         return run_tscan(E, c, corpus, N, ldc, queries, Q, ldq, D, k, dist, idx, idx_f, o, s, st, pc, capture);
     }
 
@@ -1738,9 +1908,8 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     if (!rc) rc = pc->bf.ensure((size_t)N * dpb * 2);
     if (!rc) rc = pc->words.ensure(8 * sizeof(uint32_t));
     if (!rc) rc = pc->tiles.ensure(((size_t)cdiv(N, 128) + 1) * sizeof(uint32_t));
-    // FP16 hi / lo for corpora that the scans take; smaller ones (and the rare searches that need
-    // 3xTF32 keys, see prepare_tf32) keep TF32 hi / lo
-    const bool f16 = tf32 && N >= kScanMinRowsForced;
+    // FP16 hi / lo; the TF32 copies come with the first search that needs 3xTF32 keys (prepare_tf32)
+    const bool f16 = tf32;
     if (!rc && f16) rc = pc->hi.ensure((size_t)N * split_pitch(D) * 2);
     if (!rc && f16) rc = pc->lo.ensure((size_t)N * split_pitch(D) * 2);
     if (!rc && f16) rc = pc->rs.ensure(n_pad * sizeof(float));
@@ -1780,7 +1949,7 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     pc->fp8 = fp8;
     pc->tf32 = tf32;
     pc->f16 = f16;
-    return tf32 && !f16 ? prepare_tf32(pc, s, false) : KNNS_OK;
+    return KNNS_OK;
 }
 
 int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture)

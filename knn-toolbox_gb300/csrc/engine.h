@@ -37,6 +37,8 @@ struct Config {
     bool tscan = false;
     // split keys are 3xTF32 (shortlists without a margin, rerank = 0, the shortlist kernel), else FP16
     bool tf32 = false;
+    // small corpora: 0 none of these, 1 the exact distances of every row (one launch), 2 every row's key
+    int small = 0;
 };
 
 struct Engine {

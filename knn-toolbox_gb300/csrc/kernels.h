@@ -320,6 +320,28 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
                                    uint32_t* clear, const uint32_t* skip_if, const uint32_t* skip_if_zero,
                                    cudaStream_t s);
 
+// Small corpora, no thresholds: per query, the `need` smallest of n values and the k results.
+//  * keys given: a dense pass's keys (row q at keys + q * ldk); the `need` smallest (key, index) pairs
+//    are re-ranked by exact distance;
+//  * keys null: the exact distances themselves, computed by the kernel (need = k).
+// n <= kSmallRows.  Values that are not finite are never results; missing results are (+inf, -1).
+constexpr int kSmallRows = 16384;
+struct SmallSelect {
+    const float* keys = nullptr;
+    int64_t ldk = 0;
+    int n = 0, need = 0, k = 0;
+    int64_t Q = 0;
+    const float* corpus = nullptr;
+    int64_t ldc = 0;
+    const float* queries = nullptr;
+    int64_t ldq = 0;
+    int D = 0;
+    float* out_dist = nullptr;
+    int32_t* out_idx = nullptr;
+    float* out_idx_f = nullptr;
+};
+cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s);
+
 // Selection over the threshold scan's candidate segments (one warp per query).
 // The candidates of query q are the first min(cnt, cap) words of its nseg
 // segments; total = sum of cnt (the number of keys below the threshold).

@@ -303,6 +303,337 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_threshold_kernel(const 
     }
 }
 
+// ---------------------------------------------------------------- one block per query
+// Result mode of the selection, a whole block on each query.  Bound by the latency of a query's
+// chain of dependent steps (counts, gather, rank search, re-rank, sort) until every SM is full, by
+// issue slots above.  One warp per query took 25 to 150 us for that chain whatever the number of
+// queries (rank search two bits a round, a sort before and one after a re-rank staged through
+// shared memory); measured against it: 32,768 x 1,024, 256 queries 124 -> 19 us, 100,003 x 43, k =
+// 512, 777 queries 157 -> 56, 10,000 queries of 500,000 x 128 integers at k = 100 96 -> 87.  Here
+//  * the kp smallest words are found exactly by a byte-wise histogram search that starts at the
+//    highest bit in which the words differ (two or three rounds), so nothing is sorted before the
+//    re-rank;
+//  * eight lanes compute one candidate's distance, lane u the partial sum over d = u (mod 8) (the
+//    oracle's order), all of a block's rows in flight at once, read from global memory in whole
+//    32-byte sectors, nothing staged;
+//  * the shortlist is then ordered once, by counting smaller words (up to kRankSortMax) or a
+//    bitonic sort.
+constexpr int kRankSortMax = 128;
+constexpr int64_t kThrBlockQ = 1536;  // threshold mode: a warp per query above
+constexpr int64_t kSelWideQ = 384;  // up to this many queries: 256 threads each, above 128
+
+// The first k of `cur` (m packed words: key or distance above index) in ascending order to the
+// outputs, distances plus qq; (+inf, -1) past m.
+template <int kT, typename Args>
+__device__ __forceinline__ void emit_sorted(const Args& c, int64_t q, uint64_t* cur, int m, bool add_qn, float qq)
+{
+    const int tid = threadIdx.x;
+    auto put = [&](int j, uint64_t w) {
+        const bool ok = w != kSentinel;
+        const float dv = !ok ? __int_as_float(0x7f800000) : add_qn ? __fadd_rn(unpack_key(w), qq) : unpack_key(w);
+        const int32_t iv = ok ? (int32_t)unpack_idx(w) : -1;
+        if (c.out_dist) c.out_dist[q * c.k + j] = dv;
+        if (c.out_idx) c.out_idx[q * c.k + j] = iv;
+        if (c.out_idx_f) c.out_idx_f[q * c.k + j] = (float)iv;
+    };
+    if (m <= kRankSortMax) {
+        // words are distinct (indices are): a word's place is the number of smaller words
+        const ulonglong2* p2 = reinterpret_cast<const ulonglong2*>(cur);
+        for (int j = tid; j < m; j += kT) {
+            const uint64_t w = cur[j];
+            int r = 0;
+            for (int e = 0; e < m / 2; ++e) {
+                const ulonglong2 x = p2[e];
+                r += (x.x < w ? 1 : 0) + (x.y < w ? 1 : 0);
+            }
+            if (m & 1) r += cur[m - 1] < w ? 1 : 0;
+            if (r < c.k) put(r, w);
+        }
+        for (int j = m + tid; j < c.k; j += kT) put(j, kSentinel);
+        return;
+    }
+    const int P = pow2_at_least(m);
+    for (int j = m + tid; j < P; j += kT) cur[j] = kSentinel;
+    __syncthreads();
+    for (int size = 2; size <= P; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int i = tid; i < (P >> 1); i += kT) {
+                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
+                const bool up = (lo & size) == 0;
+                const uint64_t x = cur[lo], y = cur[hi];
+                if ((x > y) == up) {
+                    cur[lo] = y;
+                    cur[hi] = x;
+                }
+            }
+            // a warp's pairs stay within its own 64 words while strides are up to 32
+            const int next = stride > 1 ? stride >> 1 : size;
+            if (stride <= 32 && next <= 32) __syncwarp();
+            else __syncthreads();
+        }
+    }
+    for (int j = tid; j < c.k; j += kT) put(j, j < m ? cur[j] : kSentinel);
+}
+
+// Exact distances of the m rows named by list's words (direct difference, the oracle's order: eight
+// partial sums over d mod 8, fixed tree), packed above their indices: eight lanes a row.
+template <int kT>
+__device__ __forceinline__ void rerank_block(uint64_t* list, int m, const float* __restrict__ corpus, int64_t ldc,
+                                             const float* qv, int D)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int u = lane & 7, g = lane >> 3;
+    const int full = D >> 3;  // whole steps of eight columns
+    for (int j0 = 4 * warp; j0 < m; j0 += kT / 8) {
+        const int j = j0 + g;
+        const uint32_t idx = j < m ? unpack_idx(list[j]) : 0u;
+        const float* row = corpus + (int64_t)idx * ldc + u;
+        float p = 0.f;
+        int i = 0;
+        for (; i + 16 <= full; i += 16) {
+            float v[16];
+#pragma unroll
+            for (int t = 0; t < 16; ++t) v[t] = __ldg(row + 8 * (i + t));
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const float x = __fsub_rn(qv[8 * (i + t) + u], v[t]);
+                p = __fmaf_rn(x, x, p);
+            }
+        }
+        for (; i < full; i += 4) {
+            float v[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) v[t] = i + t < full ? __ldg(row + 8 * (i + t)) : 0.f;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (i + t < full) {
+                    const float x = __fsub_rn(qv[8 * (i + t) + u], v[t]);
+                    p = __fmaf_rn(x, x, p);
+                }
+        }
+        if (8 * full + u < D) {
+            const float x = __fsub_rn(qv[8 * full + u], __ldg(row + 8 * full));
+            p = __fmaf_rn(x, x, p);
+        }
+        // ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7))
+        p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 1));
+        p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 2));
+        p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 4));
+        if (u == 0 && j < m) list[j] = pack_key(p, idx);
+    }
+}
+
+// The bin of a 256-bin histogram where the running count reaches rank: its digit, the rank within it
+// and its count, by the calling warp.
+__device__ __forceinline__ void find_bin(const uint32_t* hist, uint32_t rank, uint32_t& digit, uint32_t& within,
+                                         uint32_t& count)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t b[8], s = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        b[u] = hist[8 * lane + u];
+        s += b[u];
+    }
+    uint32_t inc = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    uint32_t run = inc - s;
+    if (run < rank && inc >= rank) {
+        bool found = false;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (!found && run + b[u] >= rank) {
+                digit = (uint32_t)(8 * lane + u);
+                within = rank - run;
+                count = b[u];
+                found = true;
+            }
+            run += b[u];
+        }
+    }
+}
+
+// kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.
+template <int kT, bool kThr>
+__global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
+{
+    if (c.skip_if != nullptr && *c.skip_if != 0u) return;
+    if (c.skip_if_zero != nullptr && *c.skip_if_zero == 0u) return;
+    constexpr int kW = kT / 32;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t* cur = reinterpret_cast<uint64_t*>(smem);               // shortlist [pow2_at_least(kp)]
+    uint64_t* buf = kThr ? cur : cur + pow2_at_least(c.kp);           // candidates [buf_words]
+    float* qv = reinterpret_cast<float*>(buf + c.buf_words);         // query [D]
+    __shared__ uint32_t hist[256];
+    __shared__ uint64_t wmin[kW], wmax[kW];
+    __shared__ uint32_t wtot[kW], digit_s, rank_s, hit_s, m_s;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t q = blockIdx.x;
+
+    if (!kThr && c.rerank)
+        for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
+    // segment counts: thread t owns segments t, t + kT, ...
+    constexpr int kSeg = kScanMaxSegs / kT;
+    uint32_t n[kSeg], mine = 0;
+    bool over = false;
+#pragma unroll
+    for (int r = 0; r < kSeg; ++r) {
+        const int s = tid + kT * r;
+        n[r] = s < c.nseg ? __ldg(c.cnt + (size_t)s * c.Q + q) : 0u;
+        over |= n[r] > (uint32_t)c.cap;
+        mine += n[r];
+    }
+    uint32_t pre = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
+        if (lane >= o) pre += v;
+    }
+    if (lane == 31) wtot[warp] = pre;
+    if (tid == 0) m_s = 0;
+    const bool overflow = __syncthreads_or(over) != 0;
+    uint32_t at = pre - mine, total = 0;
+#pragma unroll
+    for (int w = 0; w < kW; ++w) {
+        const uint32_t t = wtot[w];
+        if (w < warp) at += t;
+        total += t;
+    }
+    if (kThr && (overflow || total < (uint32_t)c.thr_rank || total > (uint32_t)c.buf_words)) {
+        if (tid == 0) c.thr_out[q] = c.thr_fallback ? c.thr_fallback[q] : __int_as_float(0x7f800000);
+        return;
+    }
+    if (!kThr && (overflow || total < (uint32_t)c.need || total > (uint32_t)c.buf_words)) {
+        if (tid == 0) {
+            const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
+            c.fail_idx[pos] = (int32_t)q;
+            c.fail_thr[pos] = 0xFFFFFFFFu;
+        }
+        return;
+    }
+    uint64_t lo = kSentinel, hi = 0;
+#pragma unroll
+    for (int r = 0; r < kSeg; ++r) {
+        const uint64_t* src = c.cand + ((size_t)(tid + kT * r) * c.Q + q) * c.cap;
+        for (uint32_t i0 = 0; i0 < n[r]; i0 += 8) {
+            uint64_t v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = i0 + u < n[r] ? __ldg(src + i0 + u) : 0ull;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (i0 + u < n[r]) {
+                    const uint64_t w = raw_to_ordered(v[u]);
+                    buf[at + i0 + u] = w;
+                    lo = w < lo ? w : lo;
+                    hi = w > hi ? w : hi;
+                }
+        }
+        at += n[r];
+    }
+    const int nn = (int)total, kp = kThr ? c.thr_rank : c.kp;
+    uint64_t W = hi;
+    int m = nn;
+    uint64_t* list = buf;
+    if (nn > kp) {
+        // W: the kp-th smallest word; words share the bits above the highest differing one
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint64_t a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
+            lo = a < lo ? a : lo;
+            hi = b > hi ? b : hi;
+        }
+        if (lane == 0) {
+            wmin[warp] = lo;
+            wmax[warp] = hi;
+        }
+        for (int b = tid; b < 256; b += kT) hist[b] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kW; ++w) {
+            lo = wmin[w] < lo ? wmin[w] : lo;
+            hi = wmax[w] > hi ? wmax[w] : hi;
+        }
+        int top = 64 - __clzll((long long)(lo ^ hi));  // bits [0, top) differ (nn > kp >= 1: words are distinct)
+        uint64_t x = top >= 64 ? 0ull : (lo >> top) << top;
+        uint32_t rank = (uint32_t)kp;                   // among the words that share x's bits [top, 64)
+        for (;;) {
+            const int sh = max(top - 8, 0);
+            const uint64_t mask = top >= 64 ? 0ull : ~((1ull << top) - 1ull);
+            for (int e = tid; e < nn; e += kT) {
+                const uint64_t w = buf[e];
+                if ((w & mask) == x) atomicAdd(&hist[(uint32_t)(w >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+            }
+            __syncthreads();
+            if (warp == 0) find_bin(hist, rank, digit_s, rank_s, hit_s);
+            __syncthreads();
+            x |= (uint64_t)digit_s << sh;
+            rank = rank_s;
+            top = sh;
+            if (rank == hit_s || sh == 0) break;  // the bin ends exactly at rank kp
+            for (int b = tid; b < 256; b += kT) hist[b] = 0;
+            __syncthreads();
+        }
+        W = top > 0 ? x | ((1ull << top) - 1ull) : x;
+        for (int e0 = 0; !kThr && e0 < nn; e0 += kT) {
+            const int e = e0 + tid;
+            const uint64_t w = e < nn ? buf[e] : kSentinel;
+            const bool keep = e < nn && w <= W;
+            const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+            uint32_t base = 0;
+            if (lane == 0 && bal) base = atomicAdd(&m_s, (uint32_t)__popc(bal));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (keep) cur[base + __popc(bal & ((1u << lane) - 1u))] = w;
+        }
+        m = kp;
+        list = cur;
+    }
+    if constexpr (kThr) {
+        // the key of rank thr_rank: the largest word not above W (nn == kp: the largest of all)
+        uint64_t best = 0;
+        if (nn > kp) {
+            for (int e = tid; e < nn; e += kT)
+                if (buf[e] <= W && buf[e] > best) best = buf[e];
+        } else {
+            best = hi;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint64_t b = __shfl_xor_sync(0xffffffffu, best, o);
+            best = b > best ? b : best;
+        }
+        __syncthreads();
+        if (lane == 0) wmax[warp] = best;
+        __syncthreads();
+        if (tid == 0) {
+#pragma unroll
+            for (int w = 0; w < kW; ++w) best = wmax[w] > best ? wmax[w] : best;
+            const float key = unpack_key(best);
+            // strictly above the key of rank thr_rank: that key itself passes a "< T" test
+            c.thr_out[q] = key < __int_as_float(0x7f800000) ? nextafterf(key, __int_as_float(0x7f800000)) : key;
+        }
+        return;
+    }
+    __syncthreads();
+
+    // exact integer keys: the ranking by key is the ranking by distance, distance = key + ||q||^2
+    bool exact = false;
+    if (c.int_stats != nullptr && c.qn != nullptr) {
+        const float mx = __uint_as_float(__ldg(c.int_stats + 1));
+        exact = __ldg(c.int_stats) == 0u && (c.bf16_inexact == nullptr || __ldg(c.bf16_inexact) == 0u) &&
+                2.0 * (double)c.D * (double)mx * (double)mx < 16777216.0;
+    }
+    const bool rr = c.rerank && !exact;
+    if (rr) {
+        rerank_block<kT>(list, m, c.corpus, c.ldc, qv, c.D);
+        __syncthreads();
+    }
+    emit_sorted<kT>(c, q, list, m, !rr, rr ? 0.f : __ldg(c.qn + q));
+}
+
 // ---------------------------------------------------------------- thresholds from dense keys
 // One block per query: the keys, as ordered words, into shared memory.  Ranks up to kDenseRank: the
 // rank-th smallest of 32 group minima (four threads each) bounds the key of that rank from above, so
@@ -423,34 +754,7 @@ __global__ void __launch_bounds__(kDenseT) dense_threshold_kernel(const float* _
                 if (o[u] < kInf && (o[u] & mask) == x) atomicAdd(&hist[(o[u] >> sh) & ((1u << (top - sh)) - 1u)], 1u);
         }
         __syncthreads();
-        if (warp == 0) {
-            uint32_t b[8], s = 0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                b[u] = hist[8 * lane + u];
-                s += b[u];
-            }
-            uint32_t inc = s;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
-            }
-            uint32_t run = inc - s;
-            if (run < r && inc >= r) {
-                bool found = false;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    if (!found && run + b[u] >= r) {
-                        digit_s = (uint32_t)(8 * lane + u);
-                        rank_s = r - run;
-                        hit_s = b[u];
-                        found = true;
-                    }
-                    run += b[u];
-                }
-            }
-        }
+        if (warp == 0) find_bin(hist, r, digit_s, rank_s, hit_s);
         __syncthreads();
         x |= digit_s << sh;
         r = rank_s;
@@ -484,318 +788,203 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
     return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------- one block per query
-// Result mode of the selection, a whole block on each query.  Bound by the latency of a query's
-// chain of dependent steps (counts, gather, rank search, re-rank, sort) until every SM is full, by
-// issue slots above.  One warp per query took 25 to 150 us for that chain whatever the number of
-// queries (rank search two bits a round, a sort before and one after a re-rank staged through
-// shared memory); measured against it: 32,768 x 1,024, 256 queries 124 -> 19 us, 100,003 x 43, k =
-// 512, 777 queries 157 -> 56, 10,000 queries of 500,000 x 128 integers at k = 100 96 -> 87.  Here
-//  * the kp smallest words are found exactly by a byte-wise histogram search that starts at the
-//    highest bit in which the words differ (two or three rounds), so nothing is sorted before the
-//    re-rank;
-//  * eight lanes compute one candidate's distance, lane u the partial sum over d = u (mod 8) (the
-//    oracle's order), all of a block's rows in flight at once, read from global memory in whole
-//    32-byte sectors, nothing staged;
-//  * the shortlist is then ordered once, by counting smaller words (up to kRankSortMax) or a
-//    bitonic sort.
-constexpr int kRankSortMax = 128;
-constexpr int64_t kThrBlockQ = 1536;  // threshold mode: a warp per query above
-constexpr int64_t kSelWideQ = 384;  // up to this many queries: 256 threads each, above 128
-
-// Rows of `cur` (m packed words: key or distance above index) in ascending order to the outputs.
-template <int kT>
-__device__ __forceinline__ void emit_sorted(const CandSelect& c, int64_t q, uint64_t* cur, int m, bool add_qn)
+// ---------------------------------------------------------------- small corpora
+// A block per query over the values of every row (SmallSelect), which sit in shared memory as ordered
+// words: the smallest `need` by a byte-wise histogram search, ties at the end by index.  Direct mode
+// computes the exact distances first, eight lanes a row, four rows a lane in flight: one launch serves
+// the whole search, bound by the reads of the corpus from L2 (each block reads all of it).
+template <int kT, bool kDirect>
+__global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
 {
-    const int tid = threadIdx.x;
-    const float qq = add_qn ? __ldg(c.qn + q) : 0.f;
-    auto put = [&](int j, uint64_t w) {
-        const float dv = add_qn ? __fadd_rn(unpack_key(w), qq) : unpack_key(w);
-        const int32_t iv = (int32_t)unpack_idx(w);
-        if (c.out_dist) c.out_dist[q * c.k + j] = dv;
-        if (c.out_idx) c.out_idx[q * c.k + j] = iv;
-        if (c.out_idx_f) c.out_idx_f[q * c.k + j] = (float)iv;
-    };
-    if (m <= kRankSortMax) {
-        // words are distinct (indices are): a word's place is the number of smaller words
-        const ulonglong2* p2 = reinterpret_cast<const ulonglong2*>(cur);
-        for (int j = tid; j < m; j += kT) {
-            const uint64_t w = cur[j];
-            int r = 0;
-            for (int e = 0; e < m / 2; ++e) {
-                const ulonglong2 x = p2[e];
-                r += (x.x < w ? 1 : 0) + (x.y < w ? 1 : 0);
-            }
-            if (m & 1) r += cur[m - 1] < w ? 1 : 0;
-            if (r < c.k) put(r, w);
-        }
-        return;
-    }
-    const int P = pow2_at_least(m);
-    for (int j = m + tid; j < P; j += kT) cur[j] = kSentinel;
-    __syncthreads();
-    for (int size = 2; size <= P; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = tid; i < (P >> 1); i += kT) {
-                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                const bool up = (lo & size) == 0;
-                const uint64_t x = cur[lo], y = cur[hi];
-                if ((x > y) == up) {
-                    cur[lo] = y;
-                    cur[hi] = x;
-                }
-            }
-            // a warp's pairs stay within its own 64 words while strides are up to 32
-            const int next = stride > 1 ? stride >> 1 : size;
-            if (stride <= 32 && next <= 32) __syncwarp();
-            else __syncthreads();
-        }
-    }
-    for (int j = tid; j < c.k; j += kT) put(j, cur[j]);
-}
-
-// kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.
-template <int kT, bool kThr>
-__global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
-{
-    if (c.skip_if != nullptr && *c.skip_if != 0u) return;
-    if (c.skip_if_zero != nullptr && *c.skip_if_zero == 0u) return;
     constexpr int kW = kT / 32;
+    constexpr uint32_t kInf = 0xFF800000u;  // f2ord(+inf)
     extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t* cur = reinterpret_cast<uint64_t*>(smem);               // shortlist [pow2_at_least(kp)]
-    uint64_t* buf = kThr ? cur : cur + pow2_at_least(c.kp);           // candidates [buf_words]
-    float* qv = reinterpret_cast<float*>(buf + c.buf_words);         // query [D]
+    const int n4 = (c.n + 3) & ~3;
+    uint64_t* cur = reinterpret_cast<uint64_t*>(smem);                             // [pow2_at_least(need)]
+    uint32_t* ord = reinterpret_cast<uint32_t*>(cur + pow2_at_least(c.need));      // [n4]
+    float* qv = reinterpret_cast<float*>(ord + n4);                                // [D]
     __shared__ uint32_t hist[256];
-    __shared__ uint64_t wmin[kW], wmax[kW];
-    __shared__ uint32_t wtot[kW], digit_s, rank_s, hit_s, m_s;
+    __shared__ uint32_t wlo[kW], whi[kW], wcnt[kW], digit_s, rank_s, hit_s, m_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t q = blockIdx.x;
-
-    if (!kThr && c.rerank)
-        for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
-    // segment counts: thread t owns segments t, t + kT, ...
-    constexpr int kSeg = kScanMaxSegs / kT;
-    uint32_t n[kSeg], mine = 0;
-    bool over = false;
-#pragma unroll
-    for (int r = 0; r < kSeg; ++r) {
-        const int s = tid + kT * r;
-        n[r] = s < c.nseg ? __ldg(c.cnt + (size_t)s * c.Q + q) : 0u;
-        over |= n[r] > (uint32_t)c.cap;
-        mine += n[r];
-    }
-    uint32_t pre = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, pre, o);
-        if (lane >= o) pre += v;
-    }
-    if (lane == 31) wtot[warp] = pre;
+    const int n = c.n;
+    for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
+    for (int b = tid; b < 256; b += kT) hist[b] = 0;
     if (tid == 0) m_s = 0;
-    const bool overflow = __syncthreads_or(over) != 0;
-    uint32_t at = pre - mine, total = 0;
-#pragma unroll
-    for (int w = 0; w < kW; ++w) {
-        const uint32_t t = wtot[w];
-        if (w < warp) at += t;
-        total += t;
-    }
-    if (kThr && (overflow || total < (uint32_t)c.thr_rank || total > (uint32_t)c.buf_words)) {
-        if (tid == 0) c.thr_out[q] = c.thr_fallback ? c.thr_fallback[q] : __int_as_float(0x7f800000);
-        return;
-    }
-    if (!kThr && (overflow || total < (uint32_t)c.need || total > (uint32_t)c.buf_words)) {
-        if (tid == 0) {
-            const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
-            c.fail_idx[pos] = (int32_t)q;
-            c.fail_thr[pos] = 0xFFFFFFFFu;
-        }
-        return;
-    }
-    uint64_t lo = kSentinel, hi = 0;
-#pragma unroll
-    for (int r = 0; r < kSeg; ++r) {
-        const uint64_t* src = c.cand + ((size_t)(tid + kT * r) * c.Q + q) * c.cap;
-        for (uint32_t i0 = 0; i0 < n[r]; i0 += 8) {
-            uint64_t v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = i0 + u < n[r] ? __ldg(src + i0 + u) : 0ull;
-#pragma unroll
-            for (int u = 0; u < 8; ++u)
-                if (i0 + u < n[r]) {
-                    const uint64_t w = raw_to_ordered(v[u]);
-                    buf[at + i0 + u] = w;
-                    lo = w < lo ? w : lo;
-                    hi = w > hi ? w : hi;
-                }
-        }
-        at += n[r];
-    }
-    const int nn = (int)total, kp = kThr ? c.thr_rank : c.kp;
-    uint64_t W = hi;
-    int m = nn;
-    uint64_t* list = buf;
-    if (nn > kp) {
-        // W: the kp-th smallest word; words share the bits above the highest differing one
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const uint64_t a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
-            lo = a < lo ? a : lo;
-            hi = b > hi ? b : hi;
-        }
-        if (lane == 0) {
-            wmin[warp] = lo;
-            wmax[warp] = hi;
-        }
-        for (int b = tid; b < 256; b += kT) hist[b] = 0;
+    if constexpr (kDirect) {
         __syncthreads();
+        constexpr int kR = 4;  // rows a lane has in flight
+        const int u = lane & 7, g = lane >> 3, full = c.D >> 3;
+        for (int r0 = 4 * kR * warp; r0 < n; r0 += kT / 8 * kR) {
+            float p[kR];
+            const float* row[kR];
 #pragma unroll
-        for (int w = 0; w < kW; ++w) {
-            lo = wmin[w] < lo ? wmin[w] : lo;
-            hi = wmax[w] > hi ? wmax[w] : hi;
-        }
-        int top = 64 - __clzll((long long)(lo ^ hi));  // bits [0, top) differ (nn > kp >= 1: words are distinct)
-        uint64_t x = top >= 64 ? 0ull : (lo >> top) << top;
-        uint32_t rank = (uint32_t)kp;                   // among the words that share x's bits [top, 64)
-        for (;;) {
-            const int sh = max(top - 8, 0);
-            const uint64_t mask = top >= 64 ? 0ull : ~((1ull << top) - 1ull);
-            for (int e = tid; e < nn; e += kT) {
-                const uint64_t w = buf[e];
-                if ((w & mask) == x) atomicAdd(&hist[(uint32_t)(w >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+            for (int t = 0; t < kR; ++t) {
+                p[t] = 0.f;
+                row[t] = c.corpus + (int64_t)min(r0 + 4 * t + g, n - 1) * c.ldc + u;
             }
-            __syncthreads();
-            if (warp == 0) {
-                // eight bins per lane: the bin where the running count reaches rank
-                uint32_t b[8], s = 0;
+            int i = 0;
+            for (; i + 4 <= full; i += 4) {
+                float v[kR][4];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    b[u] = hist[8 * lane + u];
-                    s += b[u];
-                }
-                uint32_t inc = s;
+                for (int t = 0; t < kR; ++t)
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += v;
-                }
-                const uint32_t exc = inc - s;
-                if (exc < rank && inc >= rank) {
-                    uint32_t run = exc;
-                    bool found = false;
+                    for (int e = 0; e < 4; ++e) v[t][e] = __ldg(row[t] + 8 * (i + e));
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        if (!found && run + b[u] >= rank) {
-                            digit_s = (uint32_t)(8 * lane + u);
-                            rank_s = rank - run;
-                            hit_s = b[u];
-                            found = true;
-                        }
-                        run += b[u];
+                for (int e = 0; e < 4; ++e) {
+                    const float y = qv[8 * (i + e) + u];
+#pragma unroll
+                    for (int t = 0; t < kR; ++t) {
+                        const float x = __fsub_rn(y, v[t][e]);
+                        p[t] = __fmaf_rn(x, x, p[t]);
                     }
                 }
             }
+            for (; 8 * i + u < c.D; ++i) {
+                const float y = qv[8 * i + u];
+#pragma unroll
+                for (int t = 0; t < kR; ++t) {
+                    const float x = __fsub_rn(y, __ldg(row[t] + 8 * i));
+                    p[t] = __fmaf_rn(x, x, p[t]);
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int t = 0; t < kR; ++t) {
+                // ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7))
+                float s = __fadd_rn(p[t], __shfl_xor_sync(0xffffffffu, p[t], 1));
+                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
+                s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
+                const int r = r0 + 4 * t + g;
+                if (u == 0 && r < n) ord[r] = s < __int_as_float(0x7f800000) ? f2ord(s) : kInf;
+            }
+        }
+        for (int i = n + tid; i < n4; i += kT) ord[i] = kInf;
+    } else {
+        const float* row = c.keys + q * c.ldk;
+        for (int i = 4 * tid; i < n; i += 4 * kT) {
+            const float4 v = __ldg(reinterpret_cast<const float4*>(row + i));
+            const float f[4] = {v.x, v.y, v.z, v.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = f[e] < __int_as_float(0x7f800000) && i + e < n ? f2ord(f[e]) : kInf;
+            *reinterpret_cast<uint4*>(ord + i) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+    __syncthreads();
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
+    for (int i = 4 * tid; i < n; i += 4 * kT) {
+        const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+        const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (o[e] < kInf) {
+                lo = min(lo, o[e]);
+                hi = max(hi, o[e]);
+                ++cnt;
+            }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) {
+        wlo[warp] = lo;
+        whi[warp] = hi;
+        wcnt[warp] = cnt;
+    }
+    __syncthreads();
+    cnt = 0;
+#pragma unroll
+    for (int w = 0; w < kW; ++w) {
+        lo = min(lo, wlo[w]);
+        hi = max(hi, whi[w]);
+        cnt += wcnt[w];
+    }
+    // keep the words not above W, and of those equal to W + 1 (when ties > 0) the first `ties`
+    uint32_t W = kInf - 1u, ties = 0;
+    int m = (int)cnt;
+    if (cnt > (uint32_t)c.need) {
+        m = c.need;
+        int top = 32 - __clz((int)(lo ^ hi));  // bits [0, top) differ
+        uint32_t x = top >= 32 ? 0u : (lo >> top) << top, rank = (uint32_t)c.need, hit = cnt;
+        while (top > 0 && rank != hit) {
+            const int sh = max(top - 8, 0);
+            const uint32_t mask = top >= 32 ? 0u : ~((1u << top) - 1u);
+            for (int i = 4 * tid; i < n; i += 4 * kT) {
+                const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+                const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (o[e] < kInf && (o[e] & mask) == x) atomicAdd(&hist[(o[e] >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+            }
             __syncthreads();
-            x |= (uint64_t)digit_s << sh;
+            if (warp == 0) find_bin(hist, rank, digit_s, rank_s, hit_s);
+            __syncthreads();
+            x |= digit_s << sh;
             rank = rank_s;
+            hit = hit_s;
             top = sh;
-            if (rank == hit_s || sh == 0) break;  // the bin ends exactly at rank kp
             for (int b = tid; b < 256; b += kT) hist[b] = 0;
             __syncthreads();
         }
-        W = top > 0 ? x | ((1ull << top) - 1ull) : x;
-        for (int e0 = 0; !kThr && e0 < nn; e0 += kT) {
-            const int e = e0 + tid;
-            const uint64_t w = e < nn ? buf[e] : kSentinel;
-            const bool keep = e < nn && w <= W;
-            const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-            uint32_t base = 0;
-            if (lane == 0 && bal) base = atomicAdd(&m_s, (uint32_t)__popc(bal));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (keep) cur[base + __popc(bal & ((1u << lane) - 1u))] = w;
+        if (rank == hit) {
+            W = top > 0 ? x | ((1u << top) - 1u) : x;
+        } else {  // more words equal to x than are wanted
+            W = x - 1u;
+            ties = rank;
         }
-        m = kp;
-        list = cur;
     }
-    if constexpr (kThr) {
-        // the key of rank thr_rank: the largest word not above W (nn == kp: the largest of all)
-        uint64_t best = 0;
-        if (nn > kp) {
-            for (int e = tid; e < nn; e += kT)
-                if (buf[e] <= W && buf[e] > best) best = buf[e];
-        } else {
-            best = hi;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const uint64_t b = __shfl_xor_sync(0xffffffffu, best, o);
-            best = b > best ? b : best;
-        }
-        __syncthreads();
-        if (lane == 0) wmax[warp] = best;
-        __syncthreads();
-        if (tid == 0) {
-#pragma unroll
-            for (int w = 0; w < kW; ++w) best = wmax[w] > best ? wmax[w] : best;
-            const float key = unpack_key(best);
-            // strictly above the key of rank thr_rank: that key itself passes a "< T" test
-            c.thr_out[q] = key < __int_as_float(0x7f800000) ? nextafterf(key, __int_as_float(0x7f800000)) : key;
-        }
-        return;
+    for (int e0 = 0; e0 < n; e0 += kT) {
+        const int e = e0 + tid;
+        const uint32_t o = e < n ? ord[e] : kInf;
+        const bool keep = o <= W && o < kInf;
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        uint32_t base = 0;
+        if (lane == 0 && bal) base = atomicAdd(&m_s, (uint32_t)__popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (keep) cur[base + __popc(bal & ((1u << lane) - 1u))] = ((uint64_t)o << 32) | (uint32_t)e;
     }
     __syncthreads();
-
-    // exact integer keys: the ranking by key is the ranking by distance, distance = key + ||q||^2
-    bool exact = false;
-    if (c.int_stats != nullptr && c.qn != nullptr) {
-        const float mx = __uint_as_float(__ldg(c.int_stats + 1));
-        exact = __ldg(c.int_stats) == 0u && (c.bf16_inexact == nullptr || __ldg(c.bf16_inexact) == 0u) &&
-                2.0 * (double)c.D * (double)mx * (double)mx < 16777216.0;
-    }
-    const bool rr = c.rerank && !exact;
-    if (rr) {
-        const int u = lane & 7, g = lane >> 3;
-        const int full = c.D >> 3;  // whole steps of eight columns
-        for (int j0 = 4 * warp; j0 < m; j0 += 4 * kW) {
-            const int j = j0 + g;
-            const uint32_t idx = j < m ? unpack_idx(list[j]) : 0u;
-            const float* row = c.corpus + (int64_t)idx * c.ldc + u;
-            float p = 0.f;
-            int i = 0;
-            for (; i + 16 <= full; i += 16) {
-                float v[16];
-#pragma unroll
-                for (int t = 0; t < 16; ++t) v[t] = __ldg(row + 8 * (i + t));
-#pragma unroll
-                for (int t = 0; t < 16; ++t) {
-                    const float x = __fsub_rn(qv[8 * (i + t) + u], v[t]);
-                    p = __fmaf_rn(x, x, p);
-                }
-            }
-            for (; i < full; i += 4) {
-                float v[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) v[t] = i + t < full ? __ldg(row + 8 * (i + t)) : 0.f;
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (i + t < full) {
-                        const float x = __fsub_rn(qv[8 * (i + t) + u], v[t]);
-                        p = __fmaf_rn(x, x, p);
-                    }
-            }
-            if (8 * full + u < c.D) {
-                const float x = __fsub_rn(qv[8 * full + u], __ldg(row + 8 * full));
-                p = __fmaf_rn(x, x, p);
-            }
-            // ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7))
-            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 1));
-            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 2));
-            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 4));
-            if (u == 0 && j < m) list[j] = pack_key(p, idx);
+    if (ties > 0 && warp == 0) {
+        uint32_t at = m_s, left = ties;
+        for (int e0 = 0; e0 < n && left > 0; e0 += 32) {
+            const int e = e0 + lane;
+            const bool tie = e < n && ord[e] == W + 1u;
+            const uint32_t bal = __ballot_sync(0xffffffffu, tie);
+            const uint32_t pos = (uint32_t)__popc(bal & ((1u << lane) - 1u));
+            if (tie && pos < left) cur[at + pos] = ((uint64_t)(W + 1u) << 32) | (uint32_t)e;
+            const uint32_t took = min(left, (uint32_t)__popc(bal));
+            at += took;
+            left -= took;
         }
+    }
+    __syncthreads();
+    if constexpr (!kDirect) {
+        rerank_block<kT>(cur, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
     }
-    emit_sorted<kT>(c, q, list, m, !rr);
+    emit_sorted<kT>(c, q, cur, m, false, 0.f);
+}
+
+template <int kT, bool kDirect>
+static cudaError_t run_select_small(const SmallSelect& c, size_t smem, cudaStream_t s)
+{
+    cudaError_t e = cudaFuncSetAttribute(select_small_kernel<kT, kDirect>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    select_small_kernel<kT, kDirect><<<(unsigned)c.Q, kT, smem, s>>>(c);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s)
+{
+    if (c.Q <= 0) return cudaSuccess;
+    if (c.n < 1 || c.n > kSmallRows || c.k < 1 || c.need < c.k || c.need > kMaxKpScan || c.D < 1 ||
+        (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)))
+        return cudaErrorInvalidValue;
+    const size_t smem = (size_t)pow2_at_least(c.need) * 8 + (size_t)((c.n + 3) & ~3) * 4 + (size_t)((c.D + 3) & ~3) * 4;
+    if (c.keys) return c.Q <= kSelWideQ ? run_select_small<512, false>(c, smem, s) : run_select_small<256, false>(c, smem, s);
+    return c.Q <= 152 ? run_select_small<1024, true>(c, smem, s) : run_select_small<256, true>(c, smem, s);
 }
 
 size_t select_smem_bytes(int kp, int D, int rerank)
