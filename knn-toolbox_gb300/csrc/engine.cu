@@ -82,6 +82,20 @@ void DevBuf::release()
     cap = 0;
 }
 
+int ErrWord::init()
+{
+    KNN_CUDA(cudaHostAlloc((void**)&h, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+    KNN_CUDA(cudaHostGetDevicePointer((void**)&d, h, 0));
+    *h = 0;
+    return KNNS_OK;
+}
+
+void ErrWord::release()
+{
+    if (h) cudaFreeHost(h);
+    h = d = nullptr;
+}
+
 // ---------------------------------------------------------------- engine registry
 static std::mutex g_reg_mu;
 static std::map<int, std::unique_ptr<Engine>> g_engines;
@@ -104,9 +118,8 @@ int get_engine(Engine** out)
     KNN_CUDA(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
     e->cc = major * 10 + minor;
     KNN_CUDA(cudaEventCreateWithFlags(&e->last_done, cudaEventDisableTiming));
-    int rc = e->err.ensure(sizeof(int));
+    int rc = e->err.init();
     if (rc) return rc;
-    KNN_CUDA(cudaMemset(e->err.p, 0, sizeof(int)));
     *out = e.get();
     g_engines[dev] = std::move(e);
     return KNNS_OK;
@@ -736,7 +749,7 @@ struct TscanStages {
             }
             a.cand = (uint64_t*)E.cand.p;
             a.cnt = (uint32_t*)E.cnt.p;
-            a.err = (int*)E.err.p;
+            a.err = E.err.d;
             a.Q = Q;
             a.dp = c.dp;
             a.ring = sp.ring;
@@ -755,7 +768,7 @@ struct TscanStages {
         f.qlo_flags = E.qlof;
         f.cand = (uint64_t*)E.cand.p;
         f.cnt = (uint32_t*)E.cnt.p;
-        f.err = (int*)E.err.p;
+        f.err = E.err.d;
         f.Q = Q;
         f.D = D;
         f.hp = split_pitch(D);
@@ -1090,7 +1103,7 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         f.clo_flags = cp.flags;
         f.keys = (float*)E.cand.p;
         f.ldk = ldk;
-        f.err = (int*)E.err.p;
+        f.err = E.err.d;
         f.stride = 1;
         f.N = N;
         f.D = D;
@@ -1570,7 +1583,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             a.lo_flags = tile_flags ? flags : nullptr;
             a.corpus_any_lo = tile_flags ? any_lo : nullptr;
             a.dump = nullptr;
-            a.err = (int*)E.err.p;
+            a.err = E.err.d;
             a.D = D;
             a.dp = c.dp;
             a.kp = kp;
@@ -1657,7 +1670,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         a.skip_if = scan_gate;
         a.cand = (uint64_t*)E.cand.p;
         a.cnt = (uint32_t*)E.cnt.p;
-        a.err = (int*)E.err.p;
+        a.err = E.err.d;
         a.Q = Q;
         a.dpb = sdp;
         a.ksteps = f8 ? (D + 31) / 32 : (D + 15) / 16;
@@ -1850,7 +1863,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             t.qmap = fail_idx;
             t.qcount = fail_cnt;
             t.fix = fg;
-            t.err = (int*)E.err.p;
+            t.err = E.err.d;
             t.D = D;
             t.dp = kChunkK;
             t.kp = c.kp;
@@ -1974,10 +1987,9 @@ int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture)
 int check_device_error(Engine& E, cudaStream_t s)
 {
     KNN_CUDA(cudaStreamSynchronize(s));
-    int code = 0;
-    KNN_CUDA(cudaMemcpy(&code, E.err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    const int code = *(volatile int*)E.err.h;
     if (code != 0) {
-        KNN_CUDA(cudaMemset(E.err.p, 0, sizeof(int)));
+        *(volatile int*)E.err.h = 0;
         return set_error(KNNS_ERR_DEVICE_TIMEOUT, "kernel gave up a bounded wait (code %d) and wound down", code);
     }
     return KNNS_OK;
@@ -2557,7 +2569,7 @@ int knns_debug_tc_dot_tile(const float* corpus, int64_t N, const float* queries,
     a.lo_flags = nullptr;
     a.corpus_any_lo = nullptr;
     a.dump = dump;
-    a.err = (int*)E->err.p;
+    a.err = E->err.d;
     a.D = D;
     a.dp = dp;
     a.kp = 32;

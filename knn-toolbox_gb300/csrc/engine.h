@@ -18,6 +18,16 @@ struct DevBuf {
     void release();
 };
 
+// The device error word: one int in page-locked host memory that the kernels write through its device
+// address (only when they give up a bounded wait), so that a check after a synchronisation is a load.
+// (Copied from device memory it cost every checked search 6 to 8 us more.)
+struct ErrWord {
+    int* h = nullptr;
+    int* d = nullptr;
+    int init();
+    void release();
+};
+
 struct Config {
     int algo = 0;
     int kp = 0;
@@ -47,7 +57,8 @@ struct Engine {
     int cc = 0;
     std::mutex mu;
     cudaEvent_t last_done = nullptr;
-    DevBuf cn, qn, part, hi, lo, rs, bf, err, thr, cn_s, thr2, redo;
+    DevBuf cn, qn, part, hi, lo, rs, bf, thr, cn_s, thr2, redo;
+    ErrWord err;
     // threshold-scan path: BF16 queries, candidate segments and counts, seeded
     // thresholds, sample norms, failed-query list
     DevBuf qbf, cand, cnt, tq, cnv, fail;

@@ -95,7 +95,7 @@ struct Slot {
 
 std::vector<void*> workspace_pointers(const Engine& E)
 {
-    return {E.cn.p,   E.qn.p,  E.part.p, E.hi.p,  E.lo.p,  E.rs.p,   E.bf.p,   E.err.p,  E.thr.p,  E.cn_s.p,
+    return {E.cn.p,   E.qn.p,  E.part.p, E.hi.p,  E.lo.p,  E.rs.p,   E.bf.p,   E.err.d,  E.thr.p,  E.cn_s.p,
             E.thr2.p, E.redo.p, E.qbf.p, E.cand.p, E.cnt.p, E.tq.p,   E.cnv.p,  E.fail.p, E.words.p, E.qs.p,
             E.csv.p,  E.qhi.p,  E.qlo.p, E.qrs.p,  E.tfail.p, E.tthr2.p};
 }
@@ -160,8 +160,7 @@ int knns_server::setup()
             cudaStreamCreateWithFlags(&sl->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&sl->done_ev, cudaEventDisableTiming) != cudaSuccess)
             return set_error(KNNS_ERR_CUDA, "server slot: stream / event creation failed");
-        if ((rc = sl->E.err.ensure(sizeof(int)))) return rc;
-        if (cudaMemset(sl->E.err.p, 0, sizeof(int)) != cudaSuccess) return set_error(KNNS_ERR_CUDA, "memset");
+        if ((rc = sl->E.err.init())) return rc;
         const size_t qb = (size_t)cfg.max_batch * D * sizeof(float), ob = (size_t)cfg.max_batch * kmax * 4;
         if (cudaMalloc(&sl->d_q, qb) != cudaSuccess || cudaMalloc(&sl->d_dist, ob) != cudaSuccess ||
             cudaMalloc(&sl->d_idx, ob) != cudaSuccess || cudaMallocHost(&sl->h_q, qb) != cudaSuccess ||
@@ -585,13 +584,14 @@ void knns_server_destroy(knns_server* sv)
         if (sl->stream) cudaStreamDestroy(sl->stream);
         if (sl->done_ev) cudaEventDestroy(sl->done_ev);
         if (sl->E.last_done) cudaEventDestroy(sl->E.last_done);
+        sl->E.err.release();
         cudaFree(sl->d_q);
         cudaFree(sl->d_dist);
         cudaFree(sl->d_idx);
         cudaFreeHost(sl->h_q);
         cudaFreeHost(sl->h_dist);
         cudaFreeHost(sl->h_idx);
-        for (DevBuf* b : {&sl->E.cn, &sl->E.qn, &sl->E.part, &sl->E.hi, &sl->E.lo, &sl->E.bf, &sl->E.err, &sl->E.thr,
+        for (DevBuf* b : {&sl->E.cn, &sl->E.qn, &sl->E.part, &sl->E.hi, &sl->E.lo, &sl->E.bf, &sl->E.thr,
                           &sl->E.cn_s, &sl->E.thr2, &sl->E.redo, &sl->E.qbf, &sl->E.cand, &sl->E.cnt,
                           &sl->E.tq, &sl->E.cnv, &sl->E.rs, &sl->E.qs, &sl->E.csv, &sl->E.qhi, &sl->E.qlo, &sl->E.qrs, &sl->E.done,
                           &sl->E.tfail, &sl->E.tthr2, &sl->E.fail, &sl->E.words, &sl->E.in_corpus, &sl->E.in_queries,
