@@ -351,7 +351,9 @@ __global__ void __launch_bounds__(kScanThreads, 1)
         const float m = kF8 ? -2.0f * (valid ? __ldg(a.qs + q) : 0.f) : -2.0f;
         const size_t seg = (size_t)split * kScanParts + part;
         uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
-        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
+        // dense: this warp's rows
+        float* krow = kDense ? a.keys + (q0 + quad * 32) * a.ldk : nullptr;
+        const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -401,12 +403,10 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 if constexpr (W3 > 0) gc = chunk_keys<W3, kF8>(vc, nrm + c3, scl + c3, m, T, vc);
             }
             if constexpr (kDense) {
-                if (valid) {
-                    float* dst = krow + nb;
-                    chunk_store<W1>(va, dst + c1);
-                    chunk_store<W2>(vb, dst + c2);
-                    if constexpr (W3 > 0) chunk_store<W3>(vc, dst + c3);
-                }
+                float* dst = krow + nb;
+                chunk_store<W1>(va, dst + c1, a.ldk, krows);
+                chunk_store<W2>(vb, dst + c2, a.ldk, krows);
+                if constexpr (W3 > 0) chunk_store<W3>(vc, dst + c3, a.ldk, krows);
             } else {
                 if (__any_sync(0xffffffffu, ga != 0u)) chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
                 if (__any_sync(0xffffffffu, (gb | gc) != 0u)) {

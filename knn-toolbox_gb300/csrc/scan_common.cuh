@@ -113,13 +113,37 @@ __device__ __forceinline__ void chunk_append(const float (&key)[W], uint32_t gm,
     }
 }
 
-// W keys of one lane to its row of the dense key matrix (16-byte aligned).
+// The warp's 32 x W keys (lane = row) to 32 rows of the dense key matrix: `base` is row 0's first
+// column (16-byte aligned), `rows` the rows that exist.  Groups of W / 4 lanes first transpose their
+// blocks of 16-byte words, so that a store instruction writes whole 4 W-byte rows: written by lane, its
+// 32 words fell into 32 lines, and the stores of a 128-column tile took about 4,000 cycles of an SM.
 template <int W>
-__device__ __forceinline__ void chunk_store(const float (&key)[W], float* dst)
+__device__ __forceinline__ void chunk_store(float (&key)[W], float* base, int64_t ldk, int rows)
 {
+    constexpr int n = W / 4;
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int u = 0; u < W / 4; ++u)
-        reinterpret_cast<float4*>(dst)[u] = make_float4(key[4 * u], key[4 * u + 1], key[4 * u + 2], key[4 * u + 3]);
+    for (int s = n / 2; s > 0; s >>= 1) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            if (i & s) continue;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float& a = key[4 * i + e];
+                float& b = key[4 * (i | s) + e];
+                const float got = __shfl_xor_sync(0xffffffffu, up ? a : b, s);
+                if (up) a = got;
+                else b = got;
+            }
+        }
+    }
+    const int g = lane & ~(n - 1), l = lane & (n - 1);
+#pragma unroll
+    for (int j = 0; j < n; ++j)
+        if (g + j < rows)
+            *reinterpret_cast<float4*>(base + (g + j) * ldk + 4 * l) =
+                make_float4(key[4 * j], key[4 * j + 1], key[4 * j + 2], key[4 * j + 3]);
 }
 
 }  // namespace

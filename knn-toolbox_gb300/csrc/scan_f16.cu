@@ -321,7 +321,9 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
         const float m = valid ? -2.0f * __ldg(a.qs + q) : 0.f;
         const size_t seg = (size_t)split * kParts + part;
         uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
-        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
+        // dense: this warp's rows
+        float* krow = kDense ? a.keys + (q0 + quad * 32) * a.ldk : nullptr;
+        const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNorm * kTN, m, T, v);
             if constexpr (kDense) {
-                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
             }
@@ -522,7 +524,9 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
         const float m = valid ? -2.0f * __ldg(a.qs + q) : 0.f;
         const size_t seg = (size_t)split * kParts + part;
         uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
-        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
+        // dense: this warp's rows
+        float* krow = kDense ? a.keys + (q0 + quad * 32) * a.ldk : nullptr;
+        const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -547,13 +551,13 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
             const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kWN) + (uint32_t)(64 * part);
             const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNormW * kWN, m, T, v);
             if constexpr (kDense) {
-                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kWN + 64 * part);
+                chunk_store<32>(v, krow + n_begin + (int64_t)t * kWN + 64 * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, base, out, cap, cnt);
             }
             const uint32_t h = chunk_keys<32, true>(w, nrm + 32, nrm + kNormW * kWN + 32, m, T, w);
             if constexpr (kDense) {
-                if (valid) chunk_store<32>(w, krow + n_begin + (int64_t)t * kWN + 64 * part + 32);
+                chunk_store<32>(w, krow + n_begin + (int64_t)t * kWN + 64 * part + 32, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, h != 0u)) {
                 chunk_append<32>(w, h, T, base + 32u, out, cap, cnt);
             }

@@ -237,7 +237,9 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const size_t seg = (size_t)split * kParts + part;
         uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
-        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
+        // dense: this warp's rows
+        float* krow = kDense ? a.keys + (q0 + quad * 32) * a.ldk : nullptr;
+        const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -259,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
             if constexpr (kDense) {
-                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
             }
@@ -523,7 +525,9 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
         const float T = valid ? (a.thr ? __ldg(a.thr + q) : __int_as_float(0x7f800000)) : -__int_as_float(0x7f800000);
         const size_t seg = (size_t)split * kParts + part;
         uint64_t* out = kDense ? nullptr : a.cand + (seg * (size_t)a.Q + (size_t)(valid ? q : 0)) * (size_t)a.cap;
-        float* krow = kDense ? a.keys + (valid ? q : 0) * a.ldk : nullptr;
+        // dense: this warp's rows
+        float* krow = kDense ? a.keys + (q0 + quad * 32) * a.ldk : nullptr;
+        const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
         for (int t = 0; t < ntiles; ++t) {
@@ -545,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
             const float* nrm = s.norms + ns * kTN + 32 * part;
             const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
             if constexpr (kDense) {
-                if (valid) chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part);
+                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
                 chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
             }
