@@ -16,9 +16,10 @@
 //      largest, D32, and an FP64 distance >= D32 - E, where E bounds the error
 //      of an FP32 distance of rounded data, E = (D/8 + 10) * 2^-24 *
 //      (|q| + max|c|)^2 + 1e-5 * D32 (the last term covers the float engine's
-//      own ranking tolerance); accepted when the k-th FP64 distance < D32 - E;
+//      own ranking tolerance) + 1e-44 D (subnormals); accepted when the k-th FP64 distance < D32 - E;
 //   4. any other query is searched again by an FP64 brute-force kernel.
 // Results: the exact FP64 top-k ordered by (distance, index).
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <cstdarg>
@@ -78,7 +79,7 @@ struct Buf {
 
 struct Work {
     std::mutex mu;
-    Buf c32, q32, cand_d, cand_i, qn, cmax, fails, hc, hq, hd, hi;
+    Buf c32, q32, cand_d, cand_i, dd, bound, ncand, cmax, fails, hc, hq, hd, hi;
 };
 
 std::mutex g_mu;
@@ -97,25 +98,48 @@ Work* work_for_device()
 constexpr int kSortMax = 512;    // shortlist entries one warp re-ranks
 constexpr int kBruteBuf = 2048;  // candidate buffer of the brute-force kernel
 
-__global__ void to_f32_kernel(const double* __restrict__ x, int64_t rows, int64_t ld, int D, float* __restrict__ out)
+// FP32 copy of the rows (out[rows][D]) and, when mx is given, an upper bound on the largest row norm
+// (as ordered bits in *mx): one warp a row, coalesced.  The bound comes from an FP32 sum of squares
+// (off by less than 2e-5 of itself for any D the engine takes), or from sqrt(D) max|x| where the squares
+// come near the end of the float range.
+__global__ void __launch_bounds__(256) to_f32_kernel(const double* __restrict__ x, int64_t rows, int64_t ld, int D,
+                                                     float* __restrict__ out, unsigned long long* __restrict__ mx)
 {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rows * D) return;
-    const int64_t r = i / D, c = i % D;
-    out[i] = (float)x[r * ld + c];
-}
-
-// row norms |x| (FP64) and their maximum (as ordered bits in *mx)
-__global__ void norms64_kernel(const double* __restrict__ x, int64_t rows, int64_t ld, int D, double* __restrict__ out,
-                               unsigned long long* __restrict__ mx)
-{
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    double acc = 0.0;
-    for (int d = 0; d < D; ++d) acc = __dadd_rn(acc, __dmul_rn(x[r * ld + d], x[r * ld + d]));
-    const double n = sqrt(acc);
-    if (out) out[r] = n;
-    if (mx) atomicMax(mx, (unsigned long long)__double_as_longlong(n));
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    float best = 0.f;
+    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+        const double* row = x + r * ld;
+        float* dst = out + r * D;
+        float ss = 0.f, big = 0.f;
+        bool lost = false;  // a value that is no float: not even its bound is known
+        for (int c0 = 0; c0 < D; c0 += 256) {
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = c0 + 32 * i + lane < D ? __ldg(row + c0 + 32 * i + lane) : 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int c = c0 + 32 * i + lane;
+                const float f = (float)v[i];
+                if (c < D) dst[c] = f;
+                ss = __fmaf_rn(f, f, ss);
+                big = fmaxf(big, fabsf(f));
+                lost |= !(fabsf(f) < __int_as_float(0x7f800000)) || (f == 0.f && (__double_as_longlong(v[i]) << 1) != 0);
+            }
+        }
+        if (mx == nullptr) continue;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, o));
+        }
+        // in float, rounded up (1e-6 covers the roundings; integer and float work only: a double
+        // comparison a value made this kernel four times slower)
+        float b = ss >= 1e-30f && ss < 1e38f ? sqrtf(ss) * (1.f + 3e-5f) : big * sqrtf((float)D) * (1.f + 1e-5f);
+        if (__any_sync(0xffffffffu, lost)) b = __int_as_float(0x7f800000);
+        best = fmaxf(best, b);
+    }
+    if (mx != nullptr && lane == 0) atomicMax(mx, (unsigned long long)__double_as_longlong((double)best));
 }
 
 __device__ __forceinline__ double dist64(const double* __restrict__ q, const double* __restrict__ c, int D)
@@ -130,73 +154,113 @@ __device__ __forceinline__ double dist64(const double* __restrict__ q, const dou
 
 __device__ __forceinline__ bool pair_less(double a, int ia, double b, int ib) { return a < b || (a == b && ia < ib); }
 
-// Bitonic sort of n (power of two) (distance, index) pairs in shared memory by one warp.
-__device__ void warp_sort_pairs(double* d, int* ix, int n)
+// FP64 distances of the FP32 candidates that can still matter: an FP32 distance is within E of its
+// FP64 one (see the file's head), so the k-th FP64 distance is at most the k-th FP32 one plus E and a
+// candidate more than 2 E past that cannot be among the k.  Block (q, j): candidates 64 j .. 64 j + 63 of
+// query q, a thread each, eight columns in flight; the sum runs in d order.  ncand[q]: how many.
+// Bound by the FP64 pipe (three operations a column, two lanes a cycle an SM) and the rows' latency; as
+// one warp a query over all candidates it took 197 us for 64 queries x 256 x 128.
+constexpr int kDistT = 64;
+__device__ __forceinline__ double err_bound(const double* qv, int D, double d32, unsigned long long cmax_bits)
 {
     const int lane = threadIdx.x & 31;
-    for (int size = 2; size <= n; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = lane; i < (n >> 1); i += 32) {
-                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                const bool up = (lo & size) == 0;
-                if (pair_less(d[hi], ix[hi], d[lo], ix[lo]) == up) {
-                    const double td = d[lo];
-                    d[lo] = d[hi];
-                    d[hi] = td;
-                    const int ti = ix[lo];
-                    ix[lo] = ix[hi];
-                    ix[hi] = ti;
-                }
-            }
-            __syncwarp();
-        }
+    double qq = 0.0;
+    for (int d = lane; d < D; d += 32) qq = __dadd_rn(qq, __dmul_rn(qv[d], qv[d]));
+    for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, o);
+    const double s = sqrt(qq) + __longlong_as_double((long long)cmax_bits);
+    // (the last term: squares and sums rounded in the subnormal range)
+    return ((double)D / 8.0 + 10.0) * 5.9604644775390625e-08 * s * s + 1e-5 * d32 + (double)D * 1e-44;
 }
 
-// One warp per query: FP64 re-rank of the kp FP32 candidates, the acceptance
-// test, the k results or an entry in the failure list.
-__global__ void rerank64_kernel(const double* __restrict__ data, int64_t ldc, const double* __restrict__ queries,
-                                int64_t ldq, int D, int64_t N, const float* __restrict__ cd32,
-                                const int32_t* __restrict__ ci, int kp, int k, int64_t Q,
-                                const unsigned long long* __restrict__ cmax_bits, double* __restrict__ out_d,
-                                int32_t* __restrict__ out_i, uint32_t* __restrict__ fails)
+__global__ void __launch_bounds__(kDistT) dist64_kernel(const double* __restrict__ data, int64_t N, int64_t ldc,
+                                                        const double* __restrict__ queries, int64_t ldq, int D,
+                                                        const float* __restrict__ cd32, const int32_t* __restrict__ ci,
+                                                        int kp, int k, const unsigned long long* __restrict__ cmax_bits,
+                                                        double* __restrict__ dd, int32_t* __restrict__ ncand,
+                                                        double* __restrict__ bound)
 {
-    extern __shared__ unsigned char sm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-    if (q >= Q) return;
-    int P = 32;
-    while (P < kp) P <<= 1;
-    double* dd = reinterpret_cast<double*>(sm) + (size_t)warp * kSortMax;
-    int* ii = reinterpret_cast<int*>(reinterpret_cast<double*>(sm) + (size_t)(blockDim.x >> 5) * kSortMax) +
-              (size_t)warp * kSortMax;
+    const int64_t q = blockIdx.x;
     const double* qv = queries + q * ldq;
-    for (int j = lane; j < P; j += 32) {
-        const int32_t n = j < kp ? ci[q * kp + j] : -1;
-        dd[j] = n >= 0 ? dist64(qv, data + (int64_t)n * ldc, D) : __longlong_as_double(0x7ff0000000000000ll);
-        ii[j] = n >= 0 ? n : 0x7fffffff;
+    const float* d32 = cd32 + q * kp;
+    const double E = err_bound(qv, D, (double)d32[kp - 1], *cmax_bits);
+    const double lim = (double)d32[k - 1] + 2.0 * E;
+    const bool all = kp >= N || !(lim < __longlong_as_double(0x7ff0000000000000ll));
+    const int j = blockIdx.y * kDistT + threadIdx.x;
+    if (blockIdx.y == 0 && threadIdx.x == 0) bound[q] = (double)d32[kp - 1] - E;
+    const bool in = j < kp;
+    const bool want = in && (all || (double)d32[j] <= lim);
+    // candidates come sorted by FP32 distance (missing ones last): the last wanted one counts them
+    if (want && (j == kp - 1 || !(all || (double)d32[j + 1] <= lim))) ncand[q] = j + 1;
+    if (!want) return;
+    const int32_t n = ci[q * kp + j];
+    double acc = 0.0;
+    if (n < 0) {
+        acc = __longlong_as_double(0x7ff0000000000000ll);
+    } else {
+        const double* c = data + (int64_t)n * ldc;
+        int d = 0;
+        for (; d + 8 <= D; d += 8) {
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(c + d + i);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const double t = __dsub_rn(__ldg(qv + d + i), v[i]);
+                acc = __dadd_rn(acc, __dmul_rn(t, t));
+            }
+        }
+        for (; d < D; ++d) {
+            const double t = __dsub_rn(__ldg(qv + d), __ldg(c + d));
+            acc = __dadd_rn(acc, __dmul_rn(t, t));
+        }
     }
-    __syncwarp();
-    warp_sort_pairs(dd, ii, P);
-    // acceptance: the shortlist covers the corpus, or its k-th FP64 distance stays below
-    // the smallest FP64 distance any row outside it can have
-    bool ok = kp >= N;
-    if (!ok) {
-        double qq = 0.0;
-        for (int d = lane; d < D; d += 32) qq = __dadd_rn(qq, __dmul_rn(qv[d], qv[d]));
-        for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, o);
-        const double s = sqrt(qq) + __longlong_as_double((long long)*cmax_bits);
-        const double d32 = (double)cd32[q * kp + kp - 1];
-        const double E = ((double)D / 8.0 + 10.0) * 5.9604644775390625e-08 * s * s + 1e-5 * d32;
-        ok = dd[k - 1] < d32 - E;
+    dd[q * kp + j] = acc;
+}
+
+// One block per query: its candidates in (distance, index) order by counting the smaller ones, the
+// acceptance test, the k results or an entry in the failure list.
+__global__ void __launch_bounds__(256) rerank64_kernel(int64_t N, const double* __restrict__ dd,
+                                                       const int32_t* __restrict__ ci, const int32_t* __restrict__ ncand,
+                                                       const double* __restrict__ bound, int kp, int k,
+                                                       double* __restrict__ out_d, int32_t* __restrict__ out_i,
+                                                       uint32_t* __restrict__ fails)
+{
+    // distances as their bits: not negative, so they order as integers (and a double comparison costs
+    // what 32 integer ones do)
+    __shared__ longlong2 sw[kSortMax];  // {distance bits, index}
+    __shared__ int rank[kSortMax];
+    __shared__ double kth;
+    const int64_t q = blockIdx.x;
+    const int m = ncand[q];
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const int32_t n = ci[q * kp + j];
+        sw[j] = make_longlong2(__double_as_longlong(dd[q * kp + j]), n >= 0 ? n : 0x7fffffff);
     }
-    if (!ok) {
-        if (lane == 0) fails[1 + atomicAdd(fails, 1u)] = (uint32_t)q;
+    if (threadIdx.x == 0) kth = __longlong_as_double(0x7ff0000000000000ll);
+    __syncthreads();
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        int below = 0;
+        const longlong2 w = sw[j];
+        for (int e = 0; e < m; ++e) {
+            const longlong2 x = sw[e];
+            // equal pairs (missing candidates) by place
+            below += x.x < w.x || (x.x == w.x && (x.y < w.y || (x.y == w.y && e < j))) ? 1 : 0;
+        }
+        rank[j] = below;
+        if (below == k - 1) kth = __longlong_as_double(w.x);
+    }
+    __syncthreads();
+    // the shortlist covers the corpus, or its k-th FP64 distance stays below the smallest FP64
+    // distance any row outside it can have
+    if (!(kp >= N || (m >= k && kth < bound[q]))) {
+        if (threadIdx.x == 0) fails[1 + atomicAdd(fails, 1u)] = (uint32_t)q;
         return;
     }
-    for (int j = lane; j < k; j += 32) {
-        out_d[q * k + j] = dd[j];
-        out_i[q * k + j] = ii[j];
-    }
+    for (int j = threadIdx.x; j < m; j += blockDim.x)
+        if (rank[j] < k) {
+            out_d[q * k + rank[j]] = __longlong_as_double(sw[j].x);
+            out_i[q * k + rank[j]] = (int32_t)sw[j].y;
+        }
 }
 
 // One CTA per listed query: FP64 distances to every row, kept in a shared
@@ -286,27 +350,28 @@ int search_device(const double* corpus, int64_t N, int64_t ldc, const double* qu
     if (!rc) rc = W->q32.ensure((size_t)Q * D * 4);
     if (!rc) rc = W->cand_d.ensure((size_t)Q * kp * 4);
     if (!rc) rc = W->cand_i.ensure((size_t)Q * kp * 4);
+    if (!rc) rc = W->dd.ensure((size_t)Q * kp * 8);
+    if (!rc) rc = W->bound.ensure((size_t)Q * 8);
+    if (!rc) rc = W->ncand.ensure((size_t)Q * 4);
     if (!rc) rc = W->cmax.ensure(8);
     if (!rc) rc = W->fails.ensure((size_t)(Q + 1) * 4);
     if (rc) return rc;
-    const int T = 256;
-    to_f32_kernel<<<(unsigned)((N * D + T - 1) / T), T, 0, s>>>(corpus, N, ldc, D, (float*)W->c32.p);
-    to_f32_kernel<<<(unsigned)((Q * D + T - 1) / T), T, 0, s>>>(queries, Q, ldq, D, (float*)W->q32.p);
     F64_CUDA(cudaMemsetAsync(W->cmax.p, 0, 8, s));
     F64_CUDA(cudaMemsetAsync(W->fails.p, 0, 4, s));
-    norms64_kernel<<<(unsigned)((N + T - 1) / T), T, 0, s>>>(corpus, N, ldc, D, nullptr,
-                                                              (unsigned long long*)W->cmax.p);
+    auto blocks = [](int64_t rows) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, 152 * 8)); };
+    to_f32_kernel<<<blocks(N), 256, 0, s>>>(corpus, N, ldc, D, (float*)W->c32.p, (unsigned long long*)W->cmax.p);
+    to_f32_kernel<<<blocks(Q), 256, 0, s>>>(queries, Q, ldq, D, (float*)W->q32.p, nullptr);
     F64_CUDA(cudaGetLastError());
     // FP32 shortlist of kp rows per query, ordered by exact FP32 distance
     rc = knns_search_device((const float*)W->c32.p, N, D, (const float*)W->q32.p, Q, D, D, kp, (float*)W->cand_d.p,
                             (int32_t*)W->cand_i.p, nullptr, s);
     if (rc) return fail(rc, "float shortlist: %s", knns_last_error());
-    const int warps = 4;
-    const size_t smem = (size_t)warps * kSortMax * (8 + 4);
-    F64_CUDA(cudaFuncSetAttribute(rerank64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    rerank64_kernel<<<(unsigned)((Q + warps - 1) / warps), warps * 32, smem, s>>>(
-        corpus, ldc, queries, ldq, D, N, (const float*)W->cand_d.p, (const int32_t*)W->cand_i.p, kp, k, Q,
-        (const unsigned long long*)W->cmax.p, dist, idx, (uint32_t*)W->fails.p);
+    dist64_kernel<<<dim3((unsigned)Q, (unsigned)((kp + kDistT - 1) / kDistT)), kDistT, 0, s>>>(
+        corpus, N, ldc, queries, ldq, D, (const float*)W->cand_d.p, (const int32_t*)W->cand_i.p, kp, k,
+        (const unsigned long long*)W->cmax.p, (double*)W->dd.p, (int32_t*)W->ncand.p, (double*)W->bound.p);
+    rerank64_kernel<<<(unsigned)Q, 256, 0, s>>>(N, (const double*)W->dd.p, (const int32_t*)W->cand_i.p,
+                                                (const int32_t*)W->ncand.p, (const double*)W->bound.p, kp, k, dist, idx,
+                                                (uint32_t*)W->fails.p);
     // queries whose shortlist could not be proven complete (the grid covers every query; the
     // CTAs past the failure count return at once)
     brute64_kernel<<<(unsigned)Q, 256, 0, s>>>(corpus, ldc, N, queries, ldq, D, k, (const uint32_t*)W->fails.p,

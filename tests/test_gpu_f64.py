@@ -83,3 +83,20 @@ def test_file_driver(engine, oracle, tmp_path, double):
     r = subprocess.run([exe, "data.bin", "queries.bin", str(N + 1), str(Q), str(D), str(k)], cwd=tmp_path,
                        capture_output=True, text=True)
     assert r.returncode == 1
+
+
+@pytest.mark.parametrize("N,Q,D,k", [(70, 5, 7, 70), (300, 3, 9, 1), (20000, 64, 33, 256), (20000, 65, 300, 100),
+                                     (600, 10, 8, 512), (30000, 1, 128, 128)])
+@pytest.mark.parametrize("scale", [1.0, 1e-20, 1e15])
+def test_double_library_candidate_bound(engine, oracle, N, Q, D, k, scale):
+    # the FP64 distances are computed for the candidates within the FP32 error bound of the k-th only
+    # (all of them where the shortlist covers the corpus); scales whose squares leave the float range
+    # fall back to the brute force
+    rng = np.random.default_rng(N + D)
+    X = rng.standard_normal((N, D)) * scale
+    X[N // 2:N // 2 + 3] = X[:3]            # ties
+    Qs = rng.standard_normal((Q, D)) * scale
+    d, i = engine.search_host_f64(X, Qs, k)
+    od, oi = oracle.knn_f64d(X, Qs, k)
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_array_equal(d, od)
