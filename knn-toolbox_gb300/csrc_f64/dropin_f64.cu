@@ -98,10 +98,26 @@ Work* work_for_device()
 constexpr int kSortMax = 512;    // shortlist entries one warp re-ranks
 constexpr int kBruteBuf = 2048;  // candidate buffer of the brute-force kernel
 
+// x rounded to FP32 (to nearest, ties to even) in integer arithmetic, for zeros and magnitudes of FP32's
+// normal range (ok): the conversion instruction runs on the FP64 pipe, which it kept the kernel below
+// waiting on (32,768 x 128 values: 34 us, 13 without it, of which the bytes take 7).
+__device__ __forceinline__ float to_f32(double x, bool& ok)
+{
+    const uint64_t u = (uint64_t)__double_as_longlong(x);
+    const uint32_t hi = (uint32_t)(u >> 32), sign = hi & 0x80000000u;
+    const bool zero = (u << 1) == 0ull;
+    ok = zero || ((hi >> 20) & 0x7ffu) - 897u < 254u;
+    // drop 29 fraction bits: half an ulp less one, plus one for an odd last bit; a carry moves into the
+    // exponent (past the largest float: to infinity)
+    const uint64_t r = (u & 0x7fffffffffffffffull) + 0x0fffffffull + ((u >> 29) & 1ull);
+    return __uint_as_float(sign | (zero ? 0u : (uint32_t)(r >> 29) - (896u << 23)));
+}
+
 // FP32 copy of the rows (out[rows][D]) and, when mx is given, an upper bound on the largest row norm
-// (as ordered bits in *mx): one warp a row, coalesced.  The bound comes from an FP32 sum of squares
-// (off by less than 2e-5 of itself for any D the engine takes), or from sqrt(D) max|x| where the squares
-// come near the end of the float range.
+// (as ordered bits in *mx): one warp a row, coalesced, kV values a lane in flight (4 for up to 128
+// columns, 8 above).  The bound comes from an FP32 sum of squares (off by less than 2e-5 of itself for any
+// D the engine takes), or from sqrt(D) max|x| where the squares come near the end of the float range.
+template <int kV>
 __global__ void __launch_bounds__(256) to_f32_kernel(const double* __restrict__ x, int64_t rows, int64_t ld, int D,
                                                      float* __restrict__ out, unsigned long long* __restrict__ mx)
 {
@@ -113,21 +129,35 @@ __global__ void __launch_bounds__(256) to_f32_kernel(const double* __restrict__ 
         float* dst = out + r * D;
         float ss = 0.f, big = 0.f;
         bool lost = false;  // a value that is no float: not even its bound is known
-        for (int c0 = 0; c0 < D; c0 += 256) {
-            double v[8];
+        for (int c0 = 0; c0 < D; c0 += 32 * kV) {
+            double v[kV];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = c0 + 32 * i + lane < D ? __ldg(row + c0 + 32 * i + lane) : 0.0;
+            for (int i = 0; i < kV; ++i) v[i] = c0 + 32 * i + lane < D ? __ldg(row + c0 + 32 * i + lane) : 0.0;
+            float f[kV];
+            bool all = true;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < kV; ++i) {
+                bool ok;
+                f[i] = to_f32(v[i], ok);
+                all &= ok;
+            }
+            // (a vote, so that the compiler leaves the instruction behind a branch)
+            if (!__all_sync(0xffffffffu, all))
+#pragma unroll
+                for (int i = 0; i < kV; ++i) {
+                    f[i] = (float)v[i];
+                    lost |= f[i] != f[i] || (f[i] == 0.f && (__double_as_longlong(v[i]) << 1) != 0);
+                }
+#pragma unroll
+            for (int i = 0; i < kV; ++i) {
                 const int c = c0 + 32 * i + lane;
-                const float f = (float)v[i];
-                if (c < D) dst[c] = f;
-                ss = __fmaf_rn(f, f, ss);
-                big = fmaxf(big, fabsf(f));
-                lost |= !(fabsf(f) < __int_as_float(0x7f800000)) || (f == 0.f && (__double_as_longlong(v[i]) << 1) != 0);
+                if (c < D) dst[c] = f[i];
+                ss = __fmaf_rn(f[i], f[i], ss);
+                big = fmaxf(big, fabsf(f[i]));
             }
         }
         if (mx == nullptr) continue;
+        lost |= !(big < __int_as_float(0x7f800000));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -139,7 +169,16 @@ __global__ void __launch_bounds__(256) to_f32_kernel(const double* __restrict__ 
         if (__any_sync(0xffffffffu, lost)) b = __int_as_float(0x7f800000);
         best = fmaxf(best, b);
     }
-    if (mx != nullptr && lane == 0) atomicMax(mx, (unsigned long long)__double_as_longlong((double)best));
+    if (mx == nullptr) return;
+    // one atomic a block
+    __shared__ float wbest[8];
+    if (lane == 0) wbest[threadIdx.x >> 5] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int w = 1; w < 8; ++w) best = fmaxf(best, wbest[w]);
+        atomicMax(mx, (unsigned long long)__double_as_longlong((double)best));
+    }
 }
 
 __device__ __forceinline__ double dist64(const double* __restrict__ q, const double* __restrict__ c, int D)
@@ -156,11 +195,13 @@ __device__ __forceinline__ bool pair_less(double a, int ia, double b, int ib) { 
 
 // FP64 distances of the FP32 candidates that can still matter: an FP32 distance is within E of its
 // FP64 one (see the file's head), so the k-th FP64 distance is at most the k-th FP32 one plus E and a
-// candidate more than 2 E past that cannot be among the k.  Block (q, j): candidates 64 j .. 64 j + 63 of
-// query q, a thread each, eight columns in flight; the sum runs in d order.  ncand[q]: how many.
-// Bound by the FP64 pipe (three operations a column, two lanes a cycle an SM) and the rows' latency; as
-// one warp a query over all candidates it took 197 us for 64 queries x 256 x 128.
-constexpr int kDistT = 64;
+// candidate more than 2 E past that cannot be among the k.  Block (q, j): candidates 32 j .. 32 j + 31 of
+// query q, a thread each, the next eight columns in flight; the sum runs in d order.  ncand[q]: how many.
+// Bound by the FP64 pipe (three operations a column): a
+// warp's operations take about 90 cycles each whatever runs beside it (blocks of 128 or of 16 threads, or
+// two blocks an SM at most: 22, 25 and 20 us).  64 queries x 256 x 128: 19 us, 24.6 with blocks of two
+// warps and no loads ahead, 197 as one warp a query over all candidates.
+constexpr int kDistT = 32;
 __device__ __forceinline__ double err_bound(const double* qv, int D, double d32, unsigned long long cmax_bits)
 {
     const int lane = threadIdx.x & 31;
@@ -199,14 +240,24 @@ __global__ void __launch_bounds__(kDistT) dist64_kernel(const double* __restrict
     } else {
         const double* c = data + (int64_t)n * ldc;
         int d = 0;
-        for (; d + 8 <= D; d += 8) {
-            double v[8];
+        double v[8];
+        if (D >= 8)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] = __ldg(c + d + i);
+            for (int i = 0; i < 8; ++i) v[i] = __ldg(c + i);
+        for (; d + 8 <= D; d += 8) {
+            double w[8], t[8];
+            const bool more = d + 16 <= D;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[i] = more ? __ldg(c + d + 8 + i) : 0.0;
+            // stage by stage: column by column each operation waited for the one before it
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] = __dsub_rn(__ldg(qv + d + i), v[i]);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] = __dmul_rn(t[i], t[i]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const double t = __dsub_rn(__ldg(qv + d + i), v[i]);
-                acc = __dadd_rn(acc, __dmul_rn(t, t));
+                acc = __dadd_rn(acc, t[i]);
+                v[i] = w[i];
             }
         }
         for (; d < D; ++d) {
@@ -359,14 +410,16 @@ int search_device(const double* corpus, int64_t N, int64_t ldc, const double* qu
     F64_CUDA(cudaMemsetAsync(W->cmax.p, 0, 8, s));
     F64_CUDA(cudaMemsetAsync(W->fails.p, 0, 4, s));
     auto blocks = [](int64_t rows) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, 152 * 8)); };
-    to_f32_kernel<<<blocks(N), 256, 0, s>>>(corpus, N, ldc, D, (float*)W->c32.p, (unsigned long long*)W->cmax.p);
-    to_f32_kernel<<<blocks(Q), 256, 0, s>>>(queries, Q, ldq, D, (float*)W->q32.p, nullptr);
+    auto* to_f32_rows = D <= 128 ? to_f32_kernel<4> : to_f32_kernel<8>;
+    to_f32_rows<<<blocks(N), 256, 0, s>>>(corpus, N, ldc, D, (float*)W->c32.p, (unsigned long long*)W->cmax.p);
+    to_f32_rows<<<blocks(Q), 256, 0, s>>>(queries, Q, ldq, D, (float*)W->q32.p, nullptr);
     F64_CUDA(cudaGetLastError());
     // FP32 shortlist of kp rows per query, ordered by exact FP32 distance
     rc = knns_search_device((const float*)W->c32.p, N, D, (const float*)W->q32.p, Q, D, D, kp, (float*)W->cand_d.p,
                             (int32_t*)W->cand_i.p, nullptr, s);
     if (rc) return fail(rc, "float shortlist: %s", knns_last_error());
-    dist64_kernel<<<dim3((unsigned)Q, (unsigned)((kp + kDistT - 1) / kDistT)), kDistT, 0, s>>>(
+    const dim3 dgrid((unsigned)Q, (unsigned)((kp + kDistT - 1) / kDistT));
+    dist64_kernel<<<dgrid, kDistT, 0, s>>>(
         corpus, N, ldc, queries, ldq, D, (const float*)W->cand_d.p, (const int32_t*)W->cand_i.p, kp, k,
         (const unsigned long long*)W->cmax.p, (double*)W->dd.p, (int32_t*)W->ncand.p, (double*)W->bound.p);
     rerank64_kernel<<<(unsigned)Q, 256, 0, s>>>(N, (const double*)W->dd.p, (const int32_t*)W->cand_i.p,

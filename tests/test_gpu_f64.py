@@ -100,3 +100,18 @@ def test_double_library_candidate_bound(engine, oracle, N, Q, D, k, scale):
     od, oi = oracle.knn_f64d(X, Qs, k)
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_array_equal(d, od)
+
+
+@pytest.mark.parametrize("lo,hi", [(-150, -120), (-30, 20), (110, 130)])
+def test_double_library_rounding_to_float(engine, oracle, lo, hi):
+    # rows halfway between two floats, zeros, and magnitudes below, across and above FP32's normal range
+    rng = np.random.default_rng(abs(hi))
+    X = rng.standard_normal((3000, 12)).astype(np.float32).astype(np.float64)
+    X *= 1.0 + 2.0 ** -24 * rng.integers(-1, 2, X.shape)
+    X *= 2.0 ** rng.integers(lo, hi, (3000, 1))
+    X[rng.random(X.shape) < 0.1] = 0.0
+    Qs = X[::100] * (1.0 + 2.0 ** -30)
+    d, i = engine.search_host_f64(X, Qs, 10)
+    od, oi = oracle.knn_f64d(X, Qs, 10)
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_array_equal(d, od)
