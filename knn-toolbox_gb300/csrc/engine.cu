@@ -521,8 +521,17 @@ constexpr int64_t kDenseKeys = 24 << 20;
 // only decides its tile: the row width rounded up to 64); otherwise of the BF16 / E4M3 scan of row
 // width dpb.
 enum ScanKeys { kKeyBf16, kKeyF8, kKeyF16, kKeyTf32 };
+//
+// blocks: row blocks the main scan is launched in (a corpus that is being copied in), 0 for one launch.
+// A few whole splits of a one-wave plan make a block that leaves most SMs idle when there are few
+// queries: 200,000 x 128, 1,000 queries: 3 of 19 splits, 24 CTAs of 47 tiles, 48 us a block, two of
+// which ran after the last copy.  Such blocks get as many splits as fill the chip, up to kBlockSplits
+// (64 CTAs of 14 tiles, 19 us; the search 697 -> 672 us; with up to 16 splits 13 us a block, but the
+// selection over 512 segments 34 instead of 23).  Blocks that fill it already keep the one-wave plan.
+constexpr int kRowBlocks = 8;
+constexpr int kBlockSplits = 8;
 static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, const knns_options& o, ScanPlan* P,
-                     ScanKeys keys)
+                     ScanKeys keys, int blocks = 0)
 {
     if (o.scan_accs != 0 && o.scan_accs != 2 && o.scan_accs != 4)
         return set_error(KNNS_ERR_INVALID, "threshold scan: %d accumulators (2 or 4)", o.scan_accs);
@@ -614,6 +623,11 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     const int max_splits = kScanMaxSegs / kScanParts;
     P->S = o.splits > 0 ? std::min<int>(std::min(o.splits, max_splits), (int)tiles)
                         : auto_splits(qt, tiles, E.sms, max_splits);
+    if (blocks > 0 && o.splits <= 0) {
+        const int have = (int)cdiv(P->S, std::min(P->S, blocks));  // splits of a block
+        const int fill = seed_splits(qt, cdiv(tiles, blocks), E.sms, kBlockSplits);
+        if (have * qt < E.sms && fill > have) P->S = (int)std::min<int64_t>(tiles, (int64_t)blocks * fill);
+    }
     P->len = cdiv(tiles, P->S) * tn;
     P->S = (int)cdiv(N, P->len);
     const double hm = (double)P->lv[L - 1].j * (double)P->lv[L - 1].stride;
@@ -1204,7 +1218,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     if (c.algo == KNNS_ALGO_TC && o.scan != KNNS_SCAN_OFF && E.cc >= 100 && c.dpb <= 256 && c.rerank) {
         const int64_t min_n = (o.scan == KNNS_SCAN_ON || c.kp > kMaxKpTC) ? kScanMinRowsForced : kScanMinRowsAuto;
         if (N >= min_n) {
-            rc = plan_scan(E, N, Q, c.fp8 ? c.dpf : c.dpb, c.kp, o, &sp, c.fp8 ? kKeyF8 : kKeyBf16);
+            rc = plan_scan(E, N, Q, c.fp8 ? c.dpf : c.dpb, c.kp, o, &sp, c.fp8 ? kKeyF8 : kKeyBf16,
+                           host_corpus != nullptr && !o.single_stream ? kRowBlocks : 0);
             if (rc) return rc;
             scan = true;
         }
@@ -1393,8 +1408,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         if (rc) return rc;
         if (smp_copy) smp_src = (const float*)E.smp.p;
     }
-    constexpr int kBlocks = 8;
-    const int blk_splits = blocked ? (int)cdiv(sp.S, std::min(sp.S, kBlocks)) : 0;  // main-scan splits per block
+    const int blk_splits = blocked ? (int)cdiv(sp.S, std::min(sp.S, kRowBlocks)) : 0;  // main-scan splits per block
     const int nblk = blocked ? (int)cdiv(sp.S, blk_splits) : 0;
     auto blk_rows = [&](int b, int64_t* r0, int64_t* r1) {
         *r0 = (int64_t)b * blk_splits * sp.len;

@@ -98,3 +98,18 @@ def test_corpus_shards_merged_on_device_equal_whole(engine, kind, N, shards, k):
     d0, i0 = engine.search(c, q, k)
     np.testing.assert_array_equal(i1.cpu().numpy(), i0.cpu().numpy())
     np.testing.assert_array_equal(d1.cpu().numpy(), d0.cpu().numpy())
+
+
+@pytest.mark.parametrize("N,Q,k,splits", [(70_001, 1, 16, 64), (200_000, 300, 32, 64), (200_000, 6_000, 10, 24),
+                                          (66_000, 129, 100, 64)])
+def test_host_blocks_fill_the_chip(engine, N, Q, k, splits):
+    # few queries: a copied block's scan takes as many splits as fill the SMs (up to 8), not its share of
+    # a one-wave plan; the answers are the resident search's
+    import torch
+    X, Qs = data("int", N, Q, 96, N + k)
+    Xp = torch.from_numpy(X).pin_memory().numpy()
+    d, i = engine.search_host(Xp, Qs, k)
+    assert engine.last_stats()["scan_splits"] > splits // 2  # whole tiles: at most `splits`
+    dr, ir = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
+    np.testing.assert_array_equal(i, ir.cpu().numpy())
+    np.testing.assert_array_equal(d, dr.cpu().numpy())
