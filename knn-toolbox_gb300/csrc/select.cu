@@ -376,11 +376,60 @@ __device__ __forceinline__ void emit_sorted(const Args& c, int64_t q, uint64_t* 
 }
 
 // Exact distances of the m rows named by list's words (direct difference, the oracle's order: eight
-// partial sums over d mod 8, fixed tree), packed above their indices: eight lanes a row.
+// partial sums over d mod 8, fixed tree), packed above their indices: eight lanes a row.  Bound by the
+// round trips of a group's rows.  Rows of fewer than 128 columns: kB steps of eight columns of kR rows in
+// flight, predicated (the selection of 777 queries, 512 rows of 43 columns each: 56 -> 44 us; 4,096 queries, 48
+// rows of 96: 47.7 -> 42.4); longer ones sixteen steps at a time (predicated batches and batches of 32
+// were slower there, by instructions and by registers: 256 columns 40 against 52 and 51 us).
+template <int kT, int kR, int kB>
+__device__ __forceinline__ void rerank_rows(uint64_t* list, int m, const float* __restrict__ corpus, int64_t ldc,
+                                            const float* qv, int D)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int u = lane & 7, g = lane >> 3;
+    for (int j0 = 4 * kR * warp; j0 < m; j0 += kT / 8 * kR) {
+        uint32_t idx[kR];
+        float p[kR], v[kR][kB];
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            const int j = j0 + 4 * r + g;
+            idx[r] = j < m ? unpack_idx(list[j]) : 0u;
+            const float* row = corpus + (int64_t)idx[r] * ldc + u;
+            p[r] = 0.f;
+#pragma unroll
+            for (int t = 0; t < kB; ++t)
+                if (8 * t + u < D) v[r][t] = __ldg(row + 8 * t);
+        }
+#pragma unroll
+        for (int t = 0; t < kB; ++t)
+            if (8 * t + u < D) {
+                const float y = qv[8 * t + u];
+#pragma unroll
+                for (int r = 0; r < kR; ++r) {
+                    const float x = __fsub_rn(y, v[r][t]);
+                    p[r] = __fmaf_rn(x, x, p[r]);
+                }
+            }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kR; ++r) {
+            // ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7))
+            float s = __fadd_rn(p[r], __shfl_xor_sync(0xffffffffu, p[r], 1));
+            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
+            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
+            const int j = j0 + 4 * r + g;
+            if (u == 0 && j < m) list[j] = pack_key(s, idx[r]);
+        }
+    }
+}
+
 template <int kT>
 __device__ __forceinline__ void rerank_block(uint64_t* list, int m, const float* __restrict__ corpus, int64_t ldc,
                                              const float* qv, int D)
 {
+    if (D <= 32) return rerank_rows<kT, 4, 4>(list, m, corpus, ldc, qv, D);
+    if (D <= 64) return rerank_rows<kT, 2, 8>(list, m, corpus, ldc, qv, D);
+    if (D < 128) return rerank_rows<kT, 1, 16>(list, m, corpus, ldc, qv, D);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int u = lane & 7, g = lane >> 3;
     const int full = D >> 3;  // whole steps of eight columns
@@ -457,9 +506,11 @@ __device__ __forceinline__ void find_bin(const uint32_t* hist, uint32_t rank, ui
     }
 }
 
-// kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.
+// kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.  Blocks an SM:
+// ten of 128 threads (47 registers; at 63 a million rows' 10,000 queries take 97 instead of 88 us), four
+// of 256 (for the re-rank's loads in flight: 256 queries, 32 rows of 1,024 columns 18.9 -> 15.5 us).
 template <int kT, bool kThr>
-__global__ void __launch_bounds__(kT) select_block_kernel(const CandSelect c)
+__global__ void __launch_bounds__(kT, kT == 128 ? 10 : 4) select_block_kernel(const CandSelect c)
 {
     if (c.skip_if != nullptr && *c.skip_if != 0u) return;
     if (c.skip_if_zero != nullptr && *c.skip_if_zero == 0u) return;
@@ -1160,7 +1211,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
     } else {
         // 256 threads shorten one query's chain, 128 fill the chip better once every SM has work:
         // selection of 256 / 777 queries 9.4 / 14.4 against 11.4 / 11.4 us (65,536 x 128, k = 16),
-        // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512)
+        // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512, before the re-rank took two rows at a time)
         const size_t smem = ((size_t)pow2_at_least(c.kp) + c.buf_words) * 8 + (size_t)((c.D + 3) & ~3) * 4;
         auto* kernel = c.Q <= kSelWideQ ? select_block_kernel<256, false> : select_block_kernel<128, false>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -75,3 +75,18 @@ def test_rows_that_are_not_finite_leave_the_thresholds_open(engine, oracle):
     assert keep[i].all()
     od, oi = oracle.knn_gemm(X[good], Qs, 10, kp=32, rerank=True)
     oracle.check_parity(X[good], Qs, 10, d, np.searchsorted(good, i), ref_idx=oi, gap_rel=1e-6, dist_rel=1e-5)
+
+
+@pytest.mark.parametrize("D", [1, 8, 31, 32, 33, 63, 64, 65, 100, 127, 128, 129, 255])
+@pytest.mark.parametrize("Q", [60, 400])
+def test_rerank_row_widths(engine, oracle, Q, D):
+    # the re-rank takes four, two or one rows of a group at a time by the row width; every partial sum
+    # rounds, so the distances show the oracle's order of the sums
+    import torch
+    rng = np.random.default_rng(Q + D)
+    X = (rng.random((17_003, D)) * 1000).astype(np.float32)
+    Qs = (rng.random((Q, D)) * 1000).astype(np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 37)
+    od, oi = oracle.knn_gemm(X, Qs, 37, kp=engine.last_stats()["kp"], rerank=True)
+    np.testing.assert_array_equal(d.cpu().numpy(), od)
+    np.testing.assert_array_equal(i.cpu().numpy(), oi)
