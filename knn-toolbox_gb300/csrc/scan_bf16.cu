@@ -217,13 +217,12 @@ __global__ void __launch_bounds__(kScanThreads, 1)
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         if (lane == 0) {
-            int it = 0;
+            int it = 0, st = 0;
+            uint32_t ph = 0;
             bool ok = true;
             for (int t = 0; t < ntiles && ok; ++t) {
                 const int64_t n0 = n_begin + (int64_t)t * TN;
                 for (int c = 0; c < slots_per_tile; ++c, ++it) {
-                    const int st = it % R;
-                    const uint32_t ph = (uint32_t)(it / R) & 1u;
                     if (!scan_wait(a, s, &s.empty[st], ph ^ 1u, kDevTimeoutProducer)) { ok = false; break; }
                     unsigned char* dst = s.ring + (size_t)st * slot_bytes;
                     // BF16 keys: the tile's norm parts travel with its last slot
@@ -232,6 +231,10 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                     for (int bx = 0; bx < bps; ++bx)
                         ptx::tma_load_2d(dst + (size_t)bx * kBoxB, &a.tm_c, &s.full[st], (c * bps + bx) * 64, (int)n0);
                     if (np_here) ptx::tma_load_2d(np_ring + (size_t)st * np_bytes(TN), &a.tm_np, &s.full[st], 0, (int)n0);
+                    if (++st == R) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
                 }
                 if (!ok) break;
                 if constexpr (kF8) {
@@ -263,44 +266,62 @@ __global__ void __launch_bounds__(kScanThreads, 1)
             bool ok = scan_wait(a, s, s.aready, 0, kDevTimeoutAload);
             ptx::tc_fence_after();
             const uint32_t a_tmem = tmem + kACol;
+            const uint64_t ring_desc = ptx::desc_sw128_kmajor(ptx::smem_u32(s.ring));
+            const uint64_t ones_desc = kNM ? ptx::desc_sw32_kmajor(ptx::smem_u32(ones)) : 0ull;
+            const uint64_t np_desc = kNM ? ptx::desc_sw32_kmajor(ptx::smem_u32(np_ring)) : 0ull;
+            int st = iss * slots_per_tile;
+            uint32_t ph = 0, b = (uint32_t)iss, aph = 1;  // (accumulators start free)
             for (int t = iss; t < ntiles && ok; t += kIssuers) {
-                const int b = t % kNacc;
-                const uint32_t use = (uint32_t)(t / kNacc);
-                if (!scan_wait(a, s, &s.acce[b], (use & 1u) ^ 1u, kDevTimeoutMma)) { ok = false; break; }
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem + (uint32_t)b * TN;
-                int it = t * slots_per_tile;
-                for (int c = 0; c < slots_per_tile; ++c, ++it) {
-                    const int st = it % R;
-                    const uint32_t ph = (uint32_t)(it / R) & 1u;
+                // The accumulator is what a tile waits for, so little may stand between its release and
+                // the first MMA: slots and descriptors advance by additions (by division and anew, 390
+                // cycles of a tile's 1,550; a million rows of 128 columns, 10,000 queries: the pass 1,743 ->
+                // 1,634 us).  It comes before the tile's slots: its release says that the epilogue has
+                // consumed tile t - nacc, so the previous use of every slot of the ring is over and no wait
+                // below can take an older phase of a barrier for the one it waits for.  (Strict turns of
+                // the two issuers, handed over up to five MMAs early, were slower: 1,646 to 2,005 us.)
+                const uint32_t d_tmem = tmem + b * TN;
+                uint64_t db = ring_desc + (uint64_t)((uint32_t)st * slot_bytes >> 4);
+                if (!scan_wait(a, s, &s.acce[b], aph, kDevTimeoutMma)) { ok = false; break; }
+                for (int c = 0; c < slots_per_tile; ++c) {
                     if (!scan_wait(a, s, &s.full[st], ph, kDevTimeoutMma)) { ok = false; break; }
                     ptx::tc_fence_after();
-                    const uint32_t b_base = ptx::smem_u32(s.ring + (size_t)st * slot_bytes);
-                    for (int bx = 0; bx < bps; ++bx) {
+                    // (descriptors count 16-byte units)
+                    if (c > 0) db = ring_desc + (uint64_t)((uint32_t)st * slot_bytes >> 4);
+                    for (int bx = 0; bx < bps; ++bx, db += kBoxB >> 4) {
                         const int box = c * bps + bx;
                         // K steps (32 bytes) past the last data column hold zeros on both sides: skipped
-                        const int kn = min(4, a.ksteps - 4 * box);
-                        for (int kk = 0; kk < kn; ++kk) {
-                            const uint64_t db = ptx::desc_sw128_kmajor(b_base + bx * kBoxB + kk * 32);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk) {
+                            if (4 * box + kk >= a.ksteps) break;
                             if (kF8)
-                                ptx::mma_f8_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db, kIdesc,
+                                ptx::mma_f8_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db + 2 * kk, kIdesc,
                                                (box | kk) != 0);
                             else
-                                ptx::mma_f16_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db, kIdesc,
+                                ptx::mma_f16_ts(d_tmem, a_tmem + (uint32_t)(box * 32 + kk * 8), db + 2 * kk, kIdesc,
                                                  (box | kk) != 0);
                         }
                     }
                     // BF16 keys: + ones x norm parts, the norms added inside the tensor core
                     if (kNM && c == slots_per_tile - 1)
-                        ptx::mma_f16_ss(d_tmem, ptx::desc_sw32_kmajor(ptx::smem_u32(ones)),
-                                         ptx::desc_sw32_kmajor(ptx::smem_u32(np_ring + (size_t)st * np_bytes(TN))),
-                                         kIdesc, 1u);
+                        ptx::mma_f16_ss(d_tmem, ones_desc, np_desc + (uint64_t)((uint32_t)st * np_bytes(TN) >> 4), kIdesc, 1u);
                     // after the tile's last MMAs the accumulator-ready commit goes first: the
                     // epilogue is on the critical path, the producer has the ring's slack
                     if (c == slots_per_tile - 1) ptx::mma_commit(&s.accf[b]);
                     ptx::mma_commit(&s.empty[st]);
+                    if (++st == R) {
+                        st = 0;
+                        ph ^= 1u;
+                    }
                 }
-                if (!ok) break;
+                // the other issuer's tile lies between (a tile's slots are at most half the ring)
+                if ((st += slots_per_tile) >= R) {
+                    st -= R;
+                    ph ^= 1u;
+                }
+                if ((b += kIssuers) >= kNacc) {
+                    b -= kNacc;
+                    aph ^= 1u;
+                }
             }
             // all MMAs issued by this thread retire before TMEM is released
             ptx::mma_commit(s.drain);
@@ -356,24 +377,30 @@ __global__ void __launch_bounds__(kScanThreads, 1)
         const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
-        for (int t = 0; t < ntiles; ++t) {
-            const int b = t % kNacc;
-            const uint32_t use = (uint32_t)(t / kNacc);
-            const int ns = t % kNormSlots;
+        // Every warp takes every tile, so the scan waits for this loop's serial chain: the barriers'
+        // addresses, phases and the tile's row stay in registers, one vote decides whether a tile holds
+        // anything to append, and the tile that reaches past the view is known beforehand (the pass above
+        // 1,811 -> 1,743 us; without any key to append it takes 1,540, its MMAs alone 1,130).
+        const uint32_t accf = ptx::smem_u32(s.accf), acce = ptx::smem_u32(s.acce);
+        const uint32_t nfull = ptx::smem_u32(s.nfull), nempty = ptx::smem_u32(s.nempty);
+        const int c1 = W1 * part, c2 = B2 + W2 * part, c3 = B3 + W3 * part;
+        const int mask_t = n_begin + (int64_t)ntiles * TN > a.N ? ntiles - 1 : -1;
+        uint32_t b = 0, ph = 0, ns = 0, nph = 0, nb = (uint32_t)n_begin;
+        for (int t = 0; t < ntiles; ++t, nb += TN) {
             // warp-uniform outcome: tcgen05.ld below is warp-collective
-            bool ok = scan_wait(a, s, &s.accf[b], use & 1u, kDevTimeoutEpilogue);
-            if (kF8) ok = ok && scan_wait(a, s, &s.nfull[ns], (uint32_t)(t / kNormSlots) & 1u, kDevTimeoutEpilogue);
-            if (!__all_sync(0xffffffffu, ok)) break;
+            bool ok = ptx::mbar_try_wait(accf + 8u * b, ph);
+            if (kF8) ok = ok && ptx::mbar_try_wait(nfull + 8u * ns, nph);
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok = scan_wait(a, s, &s.accf[b], ph, kDevTimeoutEpilogue);
+                if (kF8) ok = ok && scan_wait(a, s, &s.nfull[ns], nph, kDevTimeoutEpilogue);
+                if (!__all_sync(0xffffffffu, ok)) break;
+            }
             ptx::tc_fence_after();
-            // this part's columns (see the chunk layout above)
-            const float* nrm = s.norms + ns * TN;
-            const float* scl = scales + ns * TN;
-            const uint32_t tb = tmem + (uint32_t)b * TN + lane_base;
-            const uint32_t nb = (uint32_t)(n_begin + (int64_t)t * TN);
-            const int c1 = W1 * part, c2 = B2 + W2 * part, c3 = B3 + W3 * part;
-            // all loads in flight together, one wait, then the accumulator is released:
-            // the MMA may overwrite it while the keys are formed (in place) and tested
-            float va[W1], vb[W2], vc[W3 > 0 ? W3 : 4];
+            // this part's columns (see the chunk layout above): all loads in flight together, one
+            // wait, then the accumulator is released -- the MMA may overwrite it while the keys are
+            // formed (in place) and tested
+            const uint32_t tb = tmem + b * TN + lane_base;
+            float va[W1], vb[W2], vc[W3 > 0 ? W3 : 8];
             __syncwarp();
             ptx::tmem_ld<W1>(tb + (uint32_t)c1, va);
             ptx::tmem_ld<W2>(tb + (uint32_t)c2, vb);
@@ -384,23 +411,30 @@ __global__ void __launch_bounds__(kScanThreads, 1)
             if constexpr (W3 > 0) ptx::tie_regs(vc);
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
-            uint32_t ga, gb, gc = 0u;
-            if constexpr (kNM) {
-                // the accumulator holds the keys; the view's last tile masks its rows past the view
-                const int64_t rem = a.N - (n_begin + (int64_t)t * TN);
-                if (rem < TN) {
-                    chunk_mask<W1>(va, c1, (int)rem);
-                    chunk_mask<W2>(vb, c2, (int)rem);
-                    if constexpr (W3 > 0) chunk_mask<W3>(vc, c3, (int)rem);
+            if (lane == 0) ptx::mbar_arrive(acce + 8u * b);
+            if (++b == kNacc) {
+                b = 0;
+                ph ^= 1u;
+            }
+            if constexpr (kF8) {
+                const float* nrm = s.norms + ns * TN;
+                const float* scl = scales + ns * TN;
+                chunk_f8_keys<W1>(va, nrm + c1, scl + c1, m);
+                chunk_f8_keys<W2>(vb, nrm + c2, scl + c2, m);
+                if constexpr (W3 > 0) chunk_f8_keys<W3>(vc, nrm + c3, scl + c3, m);
+                // norm slot ns fully read
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);
+                if (++ns == kNormSlots) {
+                    ns = 0;
+                    nph ^= 1u;
                 }
-                ga = chunk_test<W1>(va, T);
-                gb = chunk_test<W2>(vb, T);
-                if constexpr (W3 > 0) gc = chunk_test<W3>(vc, T);
-            } else {
-                ga = chunk_keys<W1, kF8>(va, nrm + c1, scl + c1, m, T, va);
-                gb = chunk_keys<W2, kF8>(vb, nrm + c2, scl + c2, m, T, vb);
-                if constexpr (W3 > 0) gc = chunk_keys<W3, kF8>(vc, nrm + c3, scl + c3, m, T, vc);
+            } else if (t == mask_t) {
+                // the accumulator holds the keys; the view's last tile masks its rows past the view
+                const int rem = (int)(a.N - (n_begin + (int64_t)t * TN));
+                chunk_mask<W1>(va, c1, rem);
+                chunk_mask<W2>(vb, c2, rem);
+                if constexpr (W3 > 0) chunk_mask<W3>(vc, c3, rem);
             }
             if constexpr (kDense) {
                 float* dst = krow + nb;
@@ -408,16 +442,19 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 chunk_store<W2>(vb, dst + c2, a.ldk, krows);
                 if constexpr (W3 > 0) chunk_store<W3>(vc, dst + c3, a.ldk, krows);
             } else {
-                if (__any_sync(0xffffffffu, ga != 0u)) chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
-                if (__any_sync(0xffffffffu, (gb | gc) != 0u)) {
+                float ga[W1 / 8], gb[W2 / 8], gc[1];
+                chunk_minima<W1>(va, ga);
+                chunk_minima<W2>(vb, gb);
+                float mn = fminf(min_of(ga), min_of(gb));
+                if constexpr (W3 > 0) {
+                    chunk_minima<W3>(vc, gc);
+                    mn = fminf(mn, gc[0]);
+                }
+                if (__any_sync(0xffffffffu, mn < T)) {
+                    chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
                     chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
                     if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
                 }
-            }
-            if constexpr (kF8) {
-                // norm slot ns fully read
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
             }
         }
         if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
@@ -479,6 +516,10 @@ int scan_plan(int dpb, int want_bps, int* bps, int* ring, bool fp8, int accs)
     if (b == 0) return -1;
     *bps = b;
     *ring = slots(b);
+    // four accumulators: an issuer's wait for one says only that tile t - 4 is over, so a slot's previous
+    // use must lie that far back or be the issuer's own (t - 2)
+    const int spt = nbox / b;
+    if (accs == 4 && *ring >= 2 * spt && *ring < 4 * spt) *ring = 2 * spt;
     return 0;
 }
 

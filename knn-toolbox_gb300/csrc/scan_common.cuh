@@ -52,6 +52,23 @@ __device__ __forceinline__ uint32_t chunk_keys(const float (&v)[W], const float*
     return gm;
 }
 
+// E4M3 keys of a W-column chunk, in place: ||c||^2 + m (s_c acc), m = -2 s_q.
+template <int W>
+__device__ __forceinline__ void chunk_f8_keys(float (&v)[W], const float* nrm, const float* scl, float m)
+{
+    const float4* n4 = reinterpret_cast<const float4*>(nrm);
+    const float4* s4 = reinterpret_cast<const float4*>(scl);
+#pragma unroll
+    for (int u = 0; u < W / 4; ++u) {
+        const float4 c = n4[u], sc = s4[u];
+        float t0, t1, t2, t3;
+        ptx::mul2(t0, t1, v[4 * u], v[4 * u + 1], sc.x, sc.y);
+        ptx::mul2(t2, t3, v[4 * u + 2], v[4 * u + 3], sc.z, sc.w);
+        ptx::fma2(v[4 * u], v[4 * u + 1], t0, t1, m, c.x, c.y);
+        ptx::fma2(v[4 * u + 2], v[4 * u + 3], t2, t3, m, c.z, c.w);
+    }
+}
+
 // Mask of the 8-column groups of a W-column chunk of keys that hold a key below T.
 template <int W>
 __device__ __forceinline__ uint32_t chunk_test(const float (&key)[W], float T)
@@ -74,6 +91,55 @@ __device__ __forceinline__ void chunk_mask(float (&key)[W], int c0, int rem)
 #pragma unroll
     for (int j = 0; j < W; ++j)
         if (c0 + j >= rem) key[j] = __int_as_float(0x7f800000);
+}
+
+// Minima of a chunk's 8-column groups.
+template <int W>
+__device__ __forceinline__ void chunk_minima(const float (&key)[W], float (&gm)[W / 8])
+{
+#pragma unroll
+    for (int g = 0; g < W / 8; ++g) gm[g] = min8(key + 8 * g);
+}
+template <int N>
+__device__ __forceinline__ float min_of(const float (&v)[N])
+{
+    float m = v[0];
+#pragma unroll
+    for (int i = 1; i + 1 < N; i += 2) m = ptx::fmin3(m, v[i], v[i + 1]);
+    return N % 2 == 0 ? fminf(m, v[N - 1]) : m;
+}
+
+// Append the keys below T, in increasing corpus index, given the groups' minima.  Words hold the raw
+// key bits above the index; the selection maps them to ordered keys.  A group with a single key below
+// T (the usual case) stores its minimum at the position found from the mask of hits; more hits take
+// the column walk.
+template <int W>
+__device__ __forceinline__ void chunk_append(const float (&key)[W], const float (&gm)[W / 8], float T, uint32_t base,
+                                             uint64_t* out, uint32_t cap, uint32_t& cnt)
+{
+#pragma unroll
+    for (int g = 0; g < W / 8; ++g) {
+        if (gm[g] < T) {
+            const float* kg = key + 8 * g;
+            uint32_t hm = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) hm |= (kg[j] < T ? 1u : 0u) << j;
+            if ((hm & (hm - 1u)) == 0u) {
+                if (cnt < cap)
+                    out[cnt] = ((uint64_t)__float_as_uint(gm[g]) << 32) | (uint64_t)(base + (uint32_t)(8 * g + __ffs((int)hm) - 1));
+                ++cnt;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float k = kg[j];
+                    const bool h = k < T;
+                    if (h && cnt < cap)
+                        out[cnt] = ((uint64_t)__float_as_uint(k) << 32) | (uint64_t)(base + (uint32_t)(8 * g + j));
+                    cnt += h ? 1u : 0u;
+                }
+            }
+        }
+    }
 }
 
 // Append the keys below T of the flagged groups, in increasing corpus index.
