@@ -419,9 +419,9 @@ __global__ void __launch_bounds__(kScanThreads, 1)
             if constexpr (kF8) {
                 const float* nrm = s.norms + ns * TN;
                 const float* scl = scales + ns * TN;
-                chunk_f8_keys<W1>(va, nrm + c1, scl + c1, m);
-                chunk_f8_keys<W2>(vb, nrm + c2, scl + c2, m);
-                if constexpr (W3 > 0) chunk_f8_keys<W3>(vc, nrm + c3, scl + c3, m);
+                chunk_scaled_keys<W1>(va, nrm + c1, scl + c1, m);
+                chunk_scaled_keys<W2>(vb, nrm + c2, scl + c2, m);
+                if constexpr (W3 > 0) chunk_scaled_keys<W3>(vc, nrm + c3, scl + c3, m);
                 // norm slot ns fully read
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);

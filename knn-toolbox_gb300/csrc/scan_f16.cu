@@ -246,35 +246,45 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
             ptx::tc_fence_after();
             const uint32_t alo = *s.alo;
             const uint32_t lo_col = 32u * (uint32_t)nch;
-            int i = 0;
+            // Little may stand between an accumulator's release and the tile's first MMA: slots, phases
+            // and accumulators advance by additions, and the tile's first chunk (a slot of the issuer's
+            // own, long full) is looked at before the accumulator (with divisions by the number of
+            // accumulators here and in the epilogue the pass over 1,000,003 x 96 with 2,000 queries took
+            // 760 us, 726 so, at the card's power limit).
+            const uint64_t ring_desc = ptx::desc_sw128_kmajor(ptx::smem_u32(s.ring));  // (in 16-byte units)
+            int st = iss * kRingHalf;
+            uint32_t ph = 0, b = (uint32_t)iss, aph = 1;  // (accumulators start free)
             for (int t = iss; t < ntiles && ok; t += kIss) {
-                const int b = t % nacc;
-                const uint32_t use = (uint32_t)(t / nacc);
-                if (!f_wait(a, s, &s.acce[b], (use & 1u) ^ 1u, kDevTimeoutMma)) { ok = false; break; }
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem + acc_col + (uint32_t)b * kTN;
-                for (int c = 0; c < nch; ++c, ++i) {
-                    const int st = iss * kRingHalf + i % kRingHalf;
-                    if (!f_wait(a, s, &s.full[st], (uint32_t)(i / kRingHalf) & 1u, kDevTimeoutMma)) { ok = false; break; }
-                    ptx::tc_fence_after();
+                const uint32_t d_tmem = tmem + acc_col + b * kTN;
+                for (int c = 0; c < nch; ++c) {
+                    if (!f_wait(a, s, &s.full[st], ph, kDevTimeoutMma)) { ok = false; break; }
                     const uint32_t clo = s.slot_lo[st];
-                    const uint32_t base = ptx::smem_u32(s.ring + (size_t)st * kSlotTA);
+                    const uint64_t base = ring_desc + (uint64_t)((uint32_t)st * kSlotTA >> 4);
                     const int ks = chunk_steps(a.D, c);
+                    if (c == 0 && !f_wait(a, s, &s.acce[b], aph, kDevTimeoutMma)) { ok = false; break; }
+                    ptx::tc_fence_after();
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
                         if (kk >= ks) break;
                         // K steps of 16 FP16 (32 bytes, 8 TMEM columns)
-                        const uint64_t ch = ptx::desc_sw128_kmajor(base + kk * 32);
+                        const uint64_t ch = base + 2 * kk;
                         const uint32_t ahi = tmem + (uint32_t)(c * 32 + kk * 8);
                         ptx::mma_f16_ts(d_tmem, ahi, ch, kIdesc, (c | kk) != 0);
-                        if (clo) ptx::mma_f16_ts(d_tmem, ahi, ptx::desc_sw128_kmajor(base + kBox + kk * 32), kIdesc, 1u);
+                        if (clo) ptx::mma_f16_ts(d_tmem, ahi, ch + (kBox >> 4), kIdesc, 1u);
                         if (alo) ptx::mma_f16_ts(d_tmem, ahi + lo_col, ch, kIdesc, 1u);
                     }
                     // the tile's last chunk: accumulator-ready first (the epilogue waits on it)
                     if (c == nch - 1) ptx::mma_commit(&s.accf[b]);
                     ptx::mma_commit(&s.empty[st]);
+                    if (++st == (iss + 1) * kRingHalf) {
+                        st = iss * kRingHalf;
+                        ph ^= 1u;
+                    }
                 }
-                if (!ok) break;
+                if ((b += kIss) >= (uint32_t)nacc) {
+                    b -= (uint32_t)nacc;
+                    aph ^= 1u;
+                }
             }
             // all MMAs issued by this thread retire before TMEM is released
             ptx::mma_commit(s.drain);
@@ -326,31 +336,47 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
         const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
-        for (int t = 0; t < ntiles; ++t) {
-            const int b = t % nacc;
-            const uint32_t use = (uint32_t)(t / nacc);
-            const int ns = t % kNorm;
+        // Every warp takes every tile: barrier addresses, phases and the tile's row stay in registers,
+        // and one vote decides whether the tile holds anything to append.
+        const uint32_t accf = ptx::smem_u32(s.accf), acce = ptx::smem_u32(s.acce);
+        const uint32_t nfull = ptx::smem_u32(s.nfull), nempty = ptx::smem_u32(s.nempty);
+        const uint32_t c0 = 32u * (uint32_t)part, tb = tmem + acc_col + lane_base + c0;
+        uint32_t b = 0, ph = 0, ns = 0, nph = 0, nb = (uint32_t)n_begin + c0;
+        for (int t = 0; t < ntiles; ++t, nb += kTN) {
             // warp-uniform outcome: tcgen05.ld below is warp-collective
-            const bool ok = f_wait(a, s, &s.accf[b], use & 1u, kDevTimeoutEpilogue) &&
-                            f_wait(a, s, &s.nfull[ns], (uint32_t)(t / kNorm) & 1u, kDevTimeoutEpilogue);
-            if (!__all_sync(0xffffffffu, ok)) break;
+            bool ok = ptx::mbar_try_wait(accf + 8u * b, ph) && ptx::mbar_try_wait(nfull + 8u * ns, nph);
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok = f_wait(a, s, &s.accf[b], ph, kDevTimeoutEpilogue) && f_wait(a, s, &s.nfull[ns], nph, kDevTimeoutEpilogue);
+                if (!__all_sync(0xffffffffu, ok)) break;
+            }
             ptx::tc_fence_after();
             float v[32];
             __syncwarp();
-            ptx::tmem_ld32(tmem + acc_col + (uint32_t)b * kTN + lane_base + (uint32_t)(32 * part), v);
+            ptx::tmem_ld32(tb + b * kTN, v);
             ptx::tmem_wait_ld_regs(v);
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
-            const float* nrm = s.norms + ns * kTN + 32 * part;
-            const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNorm * kTN, m, T, v);
-            if constexpr (kDense) {
-                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
-            } else if (__any_sync(0xffffffffu, g != 0u)) {
-                chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+            if (lane == 0) ptx::mbar_arrive(acce + 8u * b);
+            if (++b == (uint32_t)nacc) {
+                b = 0;
+                ph ^= 1u;
             }
+            const float* nrm = s.norms + ns * kTN + c0;
+            chunk_scaled_keys<32>(v, nrm, nrm + kNorm * kTN, m);
+            // norm slot ns fully read
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
+            if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);
+            if (++ns == kNorm) {
+                ns = 0;
+                nph ^= 1u;
+            }
+            if constexpr (kDense) {
+                chunk_store<32>(v, krow + nb, a.ldk, krows);
+            } else {
+                float g[4];
+                chunk_minima<32>(v, g);
+                if (__any_sync(0xffffffffu, min_of(g) < T)) chunk_append<32>(v, g, T, nb, out, cap, cnt);
+            }
         }
         if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
@@ -376,6 +402,54 @@ constexpr int kRingW = 2;
 constexpr int kAccW = 2;
 constexpr int kNormW = 4;
 constexpr uint32_t kSlotW = 6u * kBox;       // query hi, query lo, corpus hi (2 boxes), corpus lo
+
+// Append of a chunk by the mask of its 8-column groups that hold a key below T: the two chunks of a
+// 256-row tile leave no registers for the groups' minima (47 us a pass over 32,768 x 1,024 with 256
+// queries; 51 and 49 with them, spilled).
+// Words hold the raw key bits above the index; the selection maps them to
+// ordered keys.  A lane whose group holds a single key below T (the usual case
+// where a warp appends at all) stores the group's minimum at the key's position
+// found from the mask of hits; more hits take the column walk.
+template <int W>
+__device__ __forceinline__ void masked_append(const float (&key)[W], uint32_t gm, float T, uint32_t base,
+                                             uint64_t* out, uint32_t cap, uint32_t& cnt)
+{
+    constexpr int G = 8;
+#pragma unroll
+    for (int g = 0; g < W / G; ++g) {
+        if ((gm >> g) & 1u) {
+            const float* kg = key + G * g;
+            uint32_t hm = 0;
+#pragma unroll
+            for (int j = 0; j < G; ++j) hm |= (kg[j] < T ? 1u : 0u) << j;
+            if ((hm & (hm - 1u)) == 0u) {
+                const float k = min8(kg);
+                if (cnt < cap)
+                    out[cnt] = ((uint64_t)__float_as_uint(k) << 32) |
+                               (uint64_t)(base + (uint32_t)(G * g + __ffs((int)hm) - 1));
+                ++cnt;
+            } else {
+#pragma unroll
+                for (int j = 0; j < G; ++j) {
+                    const float k = kg[j];
+                    const bool h = k < T;
+                    if (h && cnt < cap)
+                        out[cnt] = ((uint64_t)__float_as_uint(k) << 32) | (uint64_t)(base + (uint32_t)(G * g + j));
+                    cnt += h ? 1u : 0u;
+                }
+            }
+        }
+    }
+}
+template <int W>
+__device__ __forceinline__ uint32_t masked_keys(float (&v)[W], const float* nrm, const float* scl, float m, float T)
+{
+    chunk_scaled_keys<W>(v, nrm, scl, m);
+    uint32_t gm = 0;
+#pragma unroll
+    for (int g = 0; g < W / 8; ++g) gm |= (min8(v + 8 * g) < T ? 1u : 0u) << g;
+    return gm;
+}
 
 template <bool kDense>
 __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_constant__ FscanArgs a)
@@ -549,17 +623,17 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
             const float* nrm = s.norms + ns * kWN + 64 * part;
             const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kWN) + (uint32_t)(64 * part);
-            const uint32_t g = chunk_keys<32, true>(v, nrm, nrm + kNormW * kWN, m, T, v);
+            const uint32_t g = masked_keys<32>(v, nrm, nrm + kNormW * kWN, m, T);
             if constexpr (kDense) {
                 chunk_store<32>(v, krow + n_begin + (int64_t)t * kWN + 64 * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
-                chunk_append<32>(v, g, T, base, out, cap, cnt);
+                masked_append<32>(v, g, T, base, out, cap, cnt);
             }
-            const uint32_t h = chunk_keys<32, true>(w, nrm + 32, nrm + kNormW * kWN + 32, m, T, w);
+            const uint32_t h = masked_keys<32>(w, nrm + 32, nrm + kNormW * kWN + 32, m, T);
             if constexpr (kDense) {
                 chunk_store<32>(w, krow + n_begin + (int64_t)t * kWN + 64 * part + 32, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, h != 0u)) {
-                chunk_append<32>(w, h, T, base + 32u, out, cap, cnt);
+                masked_append<32>(w, h, T, base + 32u, out, cap, cnt);
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);

@@ -259,11 +259,14 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
             const float* nrm = s.norms + ns * kTN + 32 * part;
-            const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
+            const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part);
+            chunk_norm_keys<32>(v, nrm);
             if constexpr (kDense) {
-                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
-            } else if (__any_sync(0xffffffffu, g != 0u)) {
-                chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+                chunk_store<32>(v, krow + base, a.ldk, krows);
+            } else {
+                float g[4];
+                chunk_minima<32>(v, g);
+                if (__any_sync(0xffffffffu, min_of(g) < T)) chunk_append<32>(v, g, T, base, out, cap, cnt);
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
@@ -288,15 +291,9 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_kernel(const __grid_constan
 // bandwidth.  Tensor memory: A hi [0, dp), A lo [dp, 2 dp), two 128-column accumulators at
 // 256 and 384.  Two MMA issuers, warps 1 and 18, take the even and the odd tiles, one
 // accumulator each: the tensor pipe queues little work beyond the MMA being issued, so one
-// thread's barrier waits and commits idle it.  A slot wait must not read an older phase of
-// the slot's barrier as complete.  An issuer waits for tile t's accumulator before its slots,
-// after which the epilogue has consumed tile t - 2: every use of the ring up to tile t - 2
-// has landed and been released.  With at most as many chunks per tile as ring slots (4 and
-// 6), a slot's use two rounds back lies in tile t - 2 or earlier, so it is released.  If the
-// slot's previous use was one of this issuer's own, it waited for that fill; if it was the
-// other issuer's, the issuer first waits for that use's release (which follows its fill) and
-// only then for the slot's next fill.  The release wait costs nothing: the producer waits for
-// it before refilling the slot.  Keys, epilogue and segments are those of tscan_kernel, so
+// thread's barrier waits and commits idle it.  Each has its own half of the ring: a slot's uses all
+// belong to one issuer, which waits for each of them in order, so no wait can take an older phase of
+// a slot's barrier for a newer one.  Keys, epilogue and segments are those of tscan_kernel, so
 // the candidates are the same.
 constexpr int kAccTA = 2;
 constexpr uint32_t kAccColTA = 256;
@@ -375,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
     const int64_t n_end = min(a.N, n_begin + a.split_len);
     const int ntiles = n_end > n_begin ? (int)((n_end - n_begin + kTN - 1) / kTN) : 0;
     const int nch = a.dp / 32;
-    const int niss = nch <= R ? 2 : 1;  // MMA issuers (see above; the launcher keeps nch <= R)
+    const int half = R / 2;  // an issuer's ring slots
 
     if (tid == 0) {
         for (int i = 0; i < R; ++i) {
@@ -391,7 +388,7 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
             ptx::mbar_init(&s.nempty[b], kEpi);
         }
         ptx::mbar_init(s.aready, 4);
-        ptx::mbar_init(s.drain, niss);
+        ptx::mbar_init(s.drain, kIss);
         *s.abort = 0;
         *s.alo = 0;
         ptx::fence_mbar_init();
@@ -410,21 +407,32 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
     if (warp == 0) {
         // ------------------------------------------------------------ producer
         if (lane == 0) {
-            int it = 0;
+            // slots and phases of the two halves
+            int st[2] = {0, half};
+            uint32_t ph[2] = {0, 0};
+            int used[2] = {0, 0};
             bool ok = true;
             for (int t = 0; t < ntiles && ok; ++t) {
                 const int64_t n0 = n_begin + (int64_t)t * kTN;
                 const uint32_t clo = a.clo_flags ? __ldg(a.clo_flags + n0 / kTN) : 1u;
-                for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % R;
-                    const uint32_t ph = (uint32_t)(it / R) & 1u;
-                    if (!ta_wait(a, s, &s.empty[st], ph ^ 1u, kDevTimeoutProducer)) { ok = false; break; }
-                    unsigned char* dst = s.ring + (size_t)st * kSlotTA;
-                    s.slot_lo[st] = clo;  // published by the arrive below
-                    ptx::mbar_arrive_expect_tx(&s.full[st], kBox * (clo ? 2u : 1u));
-                    ptx::tma_load_2d(dst, &a.tm_chi, &s.full[st], c * 32, (int)n0);
-                    if (clo) ptx::tma_load_2d(dst + kBox, &a.tm_clo, &s.full[st], c * 32, (int)n0);
+                const int h = t & 1;
+                int x = h ? st[1] : st[0], u = h ? used[1] : used[0];
+                uint32_t p = h ? ph[1] : ph[0];
+                for (int c = 0; c < nch; ++c) {
+                    if (!ta_wait(a, s, &s.empty[x], p ^ 1u, kDevTimeoutProducer)) { ok = false; break; }
+                    unsigned char* dst = s.ring + (size_t)x * kSlotTA;
+                    s.slot_lo[x] = clo;  // published by the arrive below
+                    ptx::mbar_arrive_expect_tx(&s.full[x], kBox * (clo ? 2u : 1u));
+                    ptx::tma_load_2d(dst, &a.tm_chi, &s.full[x], c * 32, (int)n0);
+                    if (clo) ptx::tma_load_2d(dst + kBox, &a.tm_clo, &s.full[x], c * 32, (int)n0);
+                    ++u;
+                    if (++x == (h + 1) * half) {
+                        x = h * half;
+                        p ^= 1u;
+                    }
                 }
+                if (h) st[1] = x, ph[1] = p, used[1] = u;
+                else st[0] = x, ph[0] = p, used[0] = u;
                 if (!ok) break;
                 const int ns = t % kNorm;
                 if (!ta_wait(a, s, &s.nempty[ns], ((uint32_t)(t / kNorm) & 1u) ^ 1u, kDevTimeoutProducer)) {
@@ -437,53 +445,55 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
             }
             if (!ok) {
                 // let copies already issued land before the CTA winds down
-                const int first = it - R > 0 ? it - R : 0;
-                for (int j = first; j < it; ++j) ptx::mbar_wait(&s.full[j % R], (uint32_t)(j / R) & 1u, kTimeout);
+                for (int h = 0; h < 2; ++h) {
+                    const int n = h ? used[1] : used[0];
+                    for (int e = max(0, n - half); e < n; ++e)
+                        ptx::mbar_wait(&s.full[h * half + e % half], (uint32_t)(e / half) & 1u, kTimeout);
+                }
             }
         }
-    } else if (warp == 1 || (warp == 2 + kEpi && niss == 2)) {
+    } else if (warp == 1 || warp == 2 + kEpi) {
         // ------------------------------------------------------------ MMA issuers
-        // issuer i takes the tiles t = i (mod niss); each commit tracks only its own MMAs
+        // issuer i takes the tiles t = i (mod 2), into accumulator i; each commit tracks only its own
+        // MMAs.  Little stands between the accumulator's release and the tile's first MMA: slots and
+        // descriptors advance by additions, and the tile's first chunk is looked at before (with the
+        // K steps past the data left out: 100,003 x 43, 777 queries 60 -> 53 us).
         if (lane == 0) {
             const int iss = warp == 1 ? 0 : 1;
             bool ok = ta_wait(a, s, s.aready, 0, kDevTimeoutAload);
             ptx::tc_fence_after();
             const uint32_t alo = *s.alo;
-            for (int t = iss; t < ntiles && ok; t += niss) {
-                const int b = t % kAccTA;
-                const uint32_t use = (uint32_t)(t / kAccTA);
-                if (!ta_wait(a, s, &s.acce[b], (use & 1u) ^ 1u, kDevTimeoutMma)) { ok = false; break; }
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem + kAccColTA + (uint32_t)b * kTN;
-                int it = t * nch;
-                for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % R;
-                    const uint32_t ph = (uint32_t)(it / R) & 1u;
-                    // the slot's previous use in the other issuer's tile: its release first
-                    const int prev = it - R;
-                    if (niss == 2 && prev >= 0 && (prev / nch) % 2 != iss &&
-                        !ta_wait(a, s, &s.empty[st], ph ^ 1u, kDevTimeoutMma)) {
-                        ok = false;
-                        break;
-                    }
+            const uint64_t ring_desc = ptx::desc_sw128_kmajor(ptx::smem_u32(s.ring));  // (in 16-byte units)
+            const uint32_t d_tmem = tmem + kAccColTA + (uint32_t)iss * kTN;
+            int st = iss * half;
+            uint32_t ph = 0, aph = 1;  // (accumulators start free)
+            for (int t = iss; t < ntiles && ok; t += kIss, aph ^= 1u) {
+                for (int c = 0; c < nch; ++c) {
                     if (!ta_wait(a, s, &s.full[st], ph, kDevTimeoutMma)) { ok = false; break; }
-                    ptx::tc_fence_after();
                     const uint32_t clo = s.slot_lo[st];
-                    const uint32_t base = ptx::smem_u32(s.ring + (size_t)st * kSlotTA);
+                    const uint64_t base = ring_desc + (uint64_t)((uint32_t)st * kSlotTA >> 4);
+                    // K steps of 8 fp32 (32 bytes within the 128-byte swizzle rows); those past the last
+                    // data column hold zeros on both sides: skipped
+                    const int ks = min(4, (a.D - 32 * c + 7) >> 3);
+                    if (c == 0 && !ta_wait(a, s, &s.acce[iss], aph, kDevTimeoutMma)) { ok = false; break; }
+                    ptx::tc_fence_after();
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk) {
-                        // K steps of 8 fp32 (32 bytes) within the 128-byte swizzle rows
-                        const uint64_t ch = ptx::desc_sw128_kmajor(base + kk * 32);
+                        if (kk >= ks) break;
+                        const uint64_t ch = base + 2 * kk;
                         const uint32_t ahi = tmem + (uint32_t)(c * 32 + kk * 8);
                         ptx::mma_tf32_ts(d_tmem, ahi, ch, kIdesc, (c | kk) != 0);
-                        if (clo) ptx::mma_tf32_ts(d_tmem, ahi, ptx::desc_sw128_kmajor(base + kBox + kk * 32), kIdesc, 1u);
+                        if (clo) ptx::mma_tf32_ts(d_tmem, ahi, ch + (kBox >> 4), kIdesc, 1u);
                         if (alo) ptx::mma_tf32_ts(d_tmem, ahi + (uint32_t)a.dp, ch, kIdesc, 1u);
                     }
                     // the tile's last chunk: accumulator-ready first (the epilogue waits on it)
-                    if (c == nch - 1) ptx::mma_commit(&s.accf[b]);
+                    if (c == nch - 1) ptx::mma_commit(&s.accf[iss]);
                     ptx::mma_commit(&s.empty[st]);
+                    if (++st == (iss + 1) * half) {
+                        st = iss * half;
+                        ph ^= 1u;
+                    }
                 }
-                if (!ok) break;
             }
             // all MMAs issued by this thread retire before TMEM is released
             ptx::mma_commit(s.drain);
@@ -530,31 +540,43 @@ __global__ void __launch_bounds__(kThreads, 1) tscan_ta_kernel(const __grid_cons
         const int krows = (int)min((int64_t)32, a.Q - (q0 + quad * 32));
         uint32_t cnt = 0;
         const uint32_t cap = (uint32_t)a.cap;
-        for (int t = 0; t < ntiles; ++t) {
-            const int b = t % kAccTA;
-            const uint32_t use = (uint32_t)(t / kAccTA);
-            const int ns = t % kNorm;
+        const uint32_t accf = ptx::smem_u32(s.accf), acce = ptx::smem_u32(s.acce);
+        const uint32_t nfull = ptx::smem_u32(s.nfull), nempty = ptx::smem_u32(s.nempty);
+        const uint32_t c0 = 32u * (uint32_t)part, tb = tmem + kAccColTA + lane_base + c0;
+        uint32_t b = 0, ph = 0, ns = 0, nph = 0, nb = (uint32_t)n_begin + c0;
+        for (int t = 0; t < ntiles; ++t, nb += kTN) {
             // warp-uniform outcome: tcgen05.ld below is warp-collective
-            const bool ok = ta_wait(a, s, &s.accf[b], use & 1u, kDevTimeoutEpilogue) &&
-                            ta_wait(a, s, &s.nfull[ns], (uint32_t)(t / kNorm) & 1u, kDevTimeoutEpilogue);
-            if (!__all_sync(0xffffffffu, ok)) break;
+            bool ok = ptx::mbar_try_wait(accf + 8u * b, ph) && ptx::mbar_try_wait(nfull + 8u * ns, nph);
+            if (!__all_sync(0xffffffffu, ok)) {
+                ok = ta_wait(a, s, &s.accf[b], ph, kDevTimeoutEpilogue) && ta_wait(a, s, &s.nfull[ns], nph, kDevTimeoutEpilogue);
+                if (!__all_sync(0xffffffffu, ok)) break;
+            }
             ptx::tc_fence_after();
             float v[32];
             __syncwarp();
-            ptx::tmem_ld32(tmem + kAccColTA + (uint32_t)b * kTN + lane_base + (uint32_t)(32 * part), v);
+            ptx::tmem_ld32(tb + b * kTN, v);
             ptx::tmem_wait_ld_regs(v);
             ptx::tc_fence_before();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
-            const float* nrm = s.norms + ns * kTN + 32 * part;
-            const uint32_t g = chunk_keys<32, false>(v, nrm, nrm, -2.0f, T, v);
-            if constexpr (kDense) {
-                chunk_store<32>(v, krow + n_begin + (int64_t)t * kTN + 32 * part, a.ldk, krows);
-            } else if (__any_sync(0xffffffffu, g != 0u)) {
-                chunk_append<32>(v, g, T, (uint32_t)(n_begin + (int64_t)t * kTN) + (uint32_t)(32 * part), out, cap, cnt);
+            if (lane == 0) ptx::mbar_arrive(acce + 8u * b);
+            if (++b == kAccTA) {
+                b = 0;
+                ph ^= 1u;
             }
+            chunk_norm_keys<32>(v, s.norms + ns * kTN + c0);
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
+            if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);
+            if (++ns == kNorm) {
+                ns = 0;
+                nph ^= 1u;
+            }
+            if constexpr (kDense) {
+                chunk_store<32>(v, krow + nb, a.ldk, krows);
+            } else {
+                float g[4];
+                chunk_minima<32>(v, g);
+                if (__any_sync(0xffffffffu, min_of(g) < T)) chunk_append<32>(v, g, T, nb, out, cap, cnt);
+            }
         }
         if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
     }
