@@ -510,6 +510,28 @@ static int seg_cap(double per_seg, double sigmas)
 
 static int seed_rank(double m) { return (int)std::ceil(2.0 * m + 4.0 * std::sqrt(m)) + 1; }
 
+// Rank at the finest of the levels, of n rows, for an expected m keys of the shortlist there.  Short
+// shortlists: rank 7 for an expected 1 left one query in 12,000 short of kp keys, and one such query
+// costs its search a fix-up over the corpus; two ranks more, one in a million (one rank more where a
+// rank is worth five shortlists or more: one in 100,000 of at most 128 queries).
+static int finest_rank(double m, int64_t n)
+{
+    int j = std::min<int>((int)n, seed_rank(m));
+    const int more = m < 0.2 ? 1 : 2;
+    if (m < 2.0 && n >= 4 * (j + more)) j += more;
+    return j;
+}
+
+// Most candidates of a query (mean plus six standard deviations) that the selection's buffer must hold
+static double cand_bound(int j, int64_t stride) { return (double)j * stride + 6.0 * (double)stride * std::sqrt((double)j) + 64.0; }
+
+// Up to one tile of queries on rows of 256 bytes or more the main pass waits for memory, so its
+// epilogue has room for more candidates: the finest sample may be as coarse as the dense pass's own
+// level, and the level between them (a scan and a selection, 20 us for any number of queries) goes.
+// 48 queries on 2,000,000 x 128: stride 256 instead of 32 behind 512, 157 -> 146 us.  (Not coarser: the candidates
+// per query grow with the stride.)
+constexpr int64_t kSeedStrideFew = 256;
+
 // Seeding starts with a dense pass -- every key of a level's rows written out, the threshold taken from
 // them -- over the finest level with at most kDenseRows rows and kDenseKeys keys (Q x rows) in all: each
 // coarser level that it replaces is three launches and 25 to 40 us for any number of queries (65,536 x
@@ -557,6 +579,16 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     // levels, finest first: strides s, kSeedRatio s, ... until the sample is small enough to keep
     // every key (kSeedCoarsest rows)
     P->stride0 = seed_stride(kp, N);
+    int cand_max = kCandMax;
+    if (Q <= kTileQ && dpb >= 128) {
+        int64_t w = P->stride0;
+        while (cdiv(N, w) > kDenseRows) w *= 2;
+        if (w > P->stride0 && w <= kSeedStrideFew &&
+            cand_bound(finest_rank((double)kp / (double)w, cdiv(N, w)), w) <= (double)kCandMaxFew) {
+            P->stride0 = w;
+            cand_max = kCandMaxFew;
+        }
+    }
     int64_t st[kMaxSeedLevels];
     int L = 0;
     for (int64_t stride = P->stride0;; stride *= kSeedRatio) {
@@ -576,10 +608,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     double m = (double)kp / (double)P->stride0;
     for (int l = L - 1; l >= 0; --l) {
         ScanLevel& v = P->lv[l];
-        v.j = std::min<int>((int)v.n, seed_rank(m));
-        // short shortlists: rank 7 for an expected 1 left one query in 12,000 short of kp keys, and one
-        // such query costs its search a fix-up over the corpus; two ranks more, one in a million
-        if (l == L - 1 && m < 2.0 && v.n >= 4 * (v.j + 2)) v.j += 2;
+        v.j = l == L - 1 ? finest_rank(m, v.n) : std::min<int>((int)v.n, seed_rank(m));
         if (l > 0) m = (double)v.j * (double)P->lv[l - 1].n / (double)v.n;
     }
     if (P->lv[L - 1].j > kCandMax / 2 || P->lv[L - 1].n < 4 * P->lv[L - 1].j)
@@ -636,7 +665,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     // bounds it but for queries whose strided sample misrepresents them (those fail over to
     // the fix-up either way); the selection buffer is sized to it, not to its ceiling
     P->sel_words = (int)std::min<double>(
-        (double)kCandMax, std::ceil((hm + 6.0 * (double)P->lv[L - 1].stride * std::sqrt((double)P->lv[L - 1].j) + 64.0) / 32.0) * 32.0);
+        (double)cand_max, std::ceil(cand_bound(P->lv[L - 1].j, P->lv[L - 1].stride) / 32.0) * 32.0);
     P->cand_words = std::max(P->cand_words, (size_t)kScanParts * P->S * Q * P->cap);
     P->cnt_words = std::max(P->cnt_words, (size_t)kScanParts * P->S * Q);
     // fix-up of failed queries: up to 512 on a full wave, the rest (rare) on 8 splits; shortlists

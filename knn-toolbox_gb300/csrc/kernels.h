@@ -347,12 +347,13 @@ cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s);
 // segments; total = sum of cnt (the number of keys below the threshold).
 //  * thr_out (threshold mode): thr_out[q] = the next float above the key of
 //    rank thr_rank (1-based) when total >= thr_rank, no segment overflowed and
-//    total <= kCandMax; otherwise thr_out[q] = thr_fallback[q] (+inf if null);
+//    total <= its buffer; otherwise thr_out[q] = thr_fallback[q] (+inf if null);
 //  * result mode: the kp smallest (key, index) words form the shortlist, then
 //    re-rank / output as launch_select.  A query whose candidates cannot be
-//    trusted (overflow, total < need, total > kCandMax) is appended to
+//    trusted (overflow, total < need, total > buf_words) is appended to
 //    fail_idx (count in *fail_cnt) and gets no result.
 constexpr int kCandMax = 2048;
+constexpr int kCandMaxFew = 6144;  // for a plan's own buffer size, of few queries
 constexpr int kMaxKpScan = 512;  // longest shortlist the threshold scan's selection keeps
 constexpr int kScanMaxSegs = 512;  // candidate segments per query (splits x kScanParts)
 struct CandSelect {

@@ -1187,7 +1187,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
     if (thr)
         c.buf_words = (int)std::min<int64_t>(kCandThrMax, ((int64_t)c.nseg * c.cap + 31) / 32 * 32);
     else if (c.kp >= 1 && c.kp <= kMaxKpScan)
-        c.buf_words = c.buf_words > 0 ? std::min(kCandMax, std::max((c.buf_words + 31) / 32 * 32, pow2_at_least(c.kp)))
+        c.buf_words = c.buf_words > 0 ? std::min(kCandMaxFew, std::max((c.buf_words + 31) / 32 * 32, pow2_at_least(c.kp)))
                                       : kCandMax;
     if (c.nseg < 1 || c.nseg > kScanMaxSegs || c.cap < 1 ||
         (!thr && (c.kp < 1 || c.kp > kMaxKpScan || c.k > c.kp || c.fail_idx == nullptr || c.fail_cnt == nullptr || c.fail_thr == nullptr ||

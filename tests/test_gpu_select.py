@@ -90,3 +90,26 @@ def test_rerank_row_widths(engine, oracle, Q, D):
     od, oi = oracle.knn_gemm(X, Qs, 37, kp=engine.last_stats()["kp"], rerank=True)
     np.testing.assert_array_equal(d.cpu().numpy(), od)
     np.testing.assert_array_equal(i.cpu().numpy(), oi)
+
+
+@pytest.mark.parametrize("kind", ["int", "float"])
+@pytest.mark.parametrize("N,Q,k", [(262_144, 128, 10), (262_145, 128, 10), (270_000, 129, 10), (600_001, 100, 100),
+                                   (1_000_003, 3, 1), (400_000, 40, 512)])
+def test_few_queries_seed_from_one_level(engine, oracle, kind, N, Q, k):
+    # one tile of queries on a large corpus: thresholds from the dense pass alone, with more candidates per
+    # query in the main pass and its selection
+    import torch
+    rng = np.random.default_rng(N + Q)
+    if kind == "int":
+        X = rng.integers(0, 256, (N, 66)).astype(np.float32)
+        Qs = rng.integers(0, 256, (Q, 66)).astype(np.float32)
+    else:
+        X = rng.standard_normal((N, 66), dtype=np.float32)
+        Qs = rng.standard_normal((Q, 66), dtype=np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
+    st = engine.last_stats()
+    assert st["scan"] == 1 and engine.last_fixups() <= 1
+    sub = rng.choice(Q, min(Q, 12), replace=False)
+    od, oi = oracle.knn_gemm(X, Qs[sub], k, kp=st["kp"], rerank=True)
+    np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
+    np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
