@@ -982,19 +982,22 @@ static int ensure_split(Engine& E, const Config& c, int64_t N, int D, int64_t n_
 }
 
 // The split of a whole corpus: 3xTF32 copies, or the FP16 side of its preparation (norms too when
-// given).  skip_unless: nothing happens when *skip_unless == 0 at run time.
+// given).  skip_unless: nothing happens when *skip_unless == 0 at run time.  queries: their
+// preparation, which shares a launch with the corpus's (null: none).
 static int split_corpus(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, int D, int64_t n_pad,
-                        float* norms, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s)
+                        float* norms, uint32_t* any_lo, const uint32_t* skip_unless, cudaStream_t s,
+                        const PrepJob* queries = nullptr)
 {
     if (c.tf32) {
-        if (norms) KNN_CUDA(launch_row_norms(corpus, N, ldc, D, norms, n_pad, s));
+        if (norms && queries) KNN_CUDA(launch_prep(prep_job(corpus, N, ldc, D, norms, n_pad), s, queries));
+        else if (norms) KNN_CUDA(launch_row_norms(corpus, N, ldc, D, norms, n_pad, s));
         KNN_CUDA(launch_split_tf32(corpus, N, ldc, D, c.dp, (float*)E.hi.p, (float*)E.lo.p, E.lof, any_lo, skip_unless, s));
         return KNNS_OK;
     }
     PrepJob j = prep_job(corpus, N, ldc, D, norms, n_pad);
     split_outputs(E, &j, any_lo);
     j.run_if = skip_unless;
-    KNN_CUDA(launch_prep(j, s));
+    KNN_CUDA(launch_prep(j, s, queries));
     return KNNS_OK;
 }
 
@@ -1045,13 +1048,10 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     };
     if ((rc = mark(0))) return rc;
     KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
-    if (!pc) {
-        if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, cn, words, nullptr, s))) return rc;
-        ++ts.launches;
-    }
     PrepJob qj = prep_job(queries, Q, ldq, D, (float*)E.qn.p, Q);
     ts.prep_outputs(&qj);
-    KNN_CUDA(launch_prep(qj, s));
+    if (pc) KNN_CUDA(launch_prep(qj, s));
+    else if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, cn, words, nullptr, s, &qj))) return rc;
     ++ts.launches;
     if ((rc = ts.query_operands())) return rc;
     if ((rc = mark(1))) return rc;
@@ -1120,16 +1120,13 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
     if (dense) {
         uint32_t* words = (uint32_t*)E.words.p;
         KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
-        if (!pc) {
-            if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, (float*)E.cn.p, words, nullptr, s))) return rc;
-            ++launches;
-        }
         PrepJob qj = prep_job(queries, Q, ldq, D, nullptr, Q);
         qj.hi = E.qhi.p;
         qj.lo = E.qlo.p;
         qj.rs = (float*)E.qrs.p;
         qj.lo_flags = E.qlof;
-        KNN_CUDA(launch_prep(qj, s));
+        if (pc) KNN_CUDA(launch_prep(qj, s));
+        else if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, (float*)E.cn.p, words, nullptr, s, &qj))) return rc;
         if ((rc = mark(1)) || (rc = mark(2))) return rc;
         const SplitCopies cp = split_copies(E, c, pc);
         FscanArgs f;
@@ -1540,8 +1537,16 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         }
     }
     if (c.algo == KNNS_ALGO_TC) {
-        // one pass per input: BF16 copy, exactness test, integrality, norms (blocked mode: the
-        // corpus block by block, above)
+        // one pass over the inputs: BF16 copy, exactness test, integrality, norms (blocked mode: the
+        // corpus block by block, above).  Corpus and queries share a launch (4 us of a search).
+        PrepJob qj = bf_job(queries, Q, ldq, qn, Q);
+        if (f8) {
+            qj.f8 = E.qbf.p;
+            qj.scales = (float*)E.qs.p;
+        } else if (scan) {
+            qj.bf = E.qbf.p;
+        }
+        if (tf_scan) ts.prep_outputs(&qj);
         if (!pc && !blocked) {
             PrepJob j = bf_job(corpus, N, ldc, cn, n_pad);
             j.bf = E.bf.p;
@@ -1554,18 +1559,10 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                 split_outputs(E, &j, any_lo);
                 j.done = (uint8_t*)E.done.p;
             }
-            KNN_CUDA(launch_prep(j, s));
-            ++launches;
+            KNN_CUDA(launch_prep(j, s, &qj));
+        } else {
+            KNN_CUDA(launch_prep(qj, s));
         }
-        PrepJob qj = bf_job(queries, Q, ldq, qn, Q);
-        if (f8) {
-            qj.f8 = E.qbf.p;
-            qj.scales = (float*)E.qs.p;
-        } else if (scan) {
-            qj.bf = E.qbf.p;
-        }
-        if (tf_scan) ts.prep_outputs(&qj);
-        KNN_CUDA(launch_prep(qj, s));
         ++launches;
         if (!bf16_only && !pc && !blocked) {
             // data that are not BF16-exact: the FP16 side of the batches prepared before that was

@@ -80,7 +80,8 @@ struct PrepJob {
     const uint32_t* run_if = nullptr;  // the launch does nothing when *run_if == 0 at run time
 };
 int64_t prep_batches(int64_t n, int D);
-cudaError_t launch_prep(const PrepJob& job, cudaStream_t s);
+// second: a job of the same kind and row width to share the launch with (its own launch otherwise)
+cudaError_t launch_prep(const PrepJob& job, cudaStream_t s, const PrepJob* second = nullptr);
 // norms of rows of any width
 cudaError_t launch_row_norms(const float* x, int64_t n, int64_t ld, int D, float* norms, int64_t n_pad, cudaStream_t s);
 

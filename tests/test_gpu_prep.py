@@ -88,3 +88,25 @@ def test_prep_outputs_bit_exact(engine, oracle, D, pad):
     assert w[0] == int((xb.float().numpy() != x).any())
     assert w[1] == int((x != np.rint(x)).any())
     assert w[2] == np.float32(mx.max()).view(np.uint32)
+
+
+@pytest.mark.parametrize("N,Q,D", [(17_001, 1, 64), (140_000, 700, 64), (17_001, 5, 300), (17_001, 3000, 300),
+                                   (140_000, 40_000, 32)])
+@pytest.mark.parametrize("kind", ["int", "float"])
+def test_corpus_and_queries_share_a_launch(engine, N, Q, D, kind):
+    # corpus and queries are prepared by one launch where they load alike, by two where only one of them
+    # starts 16-byte aligned; few, many and more query batches than a wave's blocks: the same answers
+    import torch
+    rng = np.random.default_rng(N + Q + D)
+    hi = 200 if kind == "int" else 1
+    X = rng.random((N, D)).astype(np.float32) * hi
+    W = rng.random((Q, D + 1)).astype(np.float32) * hi
+    if kind == "int":
+        X, W = np.floor(X), np.floor(W)
+    c, w = torch.from_numpy(X).cuda(), torch.from_numpy(W).cuda()
+    d0, i0 = engine.search(c, w[:, 1:].contiguous(), 9)
+    d1, i1 = engine.search(c, w[:, 1:], 9)
+    assert torch.equal(d0, d1) and torch.equal(i0, i1)
+    # each query alone in its launch's share: the answers of the first and the last
+    d2, i2 = engine.search(c, w[-1:, 1:].contiguous(), 9)
+    assert torch.equal(d0[-1:], d2) and torch.equal(i0[-1:], i2)
