@@ -839,8 +839,15 @@ struct TscanStages {
             a.ldk = sp.ldk;
             KNN_CUDA(launch_tscan(a, splits, s));
         } else {
-            r = encode_split(&f.tm_chi, cp.hi, nview, D, stride, fscan_tile_rows(D));
-            if (!r) r = encode_split(&f.tm_clo, cp.lo, nview, D, stride, fscan_tile_rows(D));
+            const int tn = keys ? fscan_dense_rows(D, Q, nview, E.sms) : fscan_tile_rows(D);
+            if (tn < fscan_tile_rows(D)) {
+                // (narrower tiles: one a CTA)
+                split_len = tn;
+                splits = (int)cdiv(nview, tn);
+            }
+            f.dense_rows = tn;
+            r = encode_split(&f.tm_chi, cp.hi, nview, D, stride, tn);
+            if (!r) r = encode_split(&f.tm_clo, cp.lo, nview, D, stride, tn);
             if (r) return r;
             f.cn = cn;
             f.cs = cp.rs;
@@ -1142,6 +1149,7 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         f.cs = cp.rs;
         f.clo_flags = cp.flags;
         f.keys = (float*)E.cand.p;
+        f.dense_rows = tn;
         f.ldk = ldk;
         f.err = E.err.d;
         f.stride = 1;

@@ -277,10 +277,13 @@ struct FscanArgs {
     int cap;
     int D;
     int hp;                       // row pitch of the queries' copies
+    int dense_rows;               // dense pass: corpus rows per tile (fscan_dense_rows)
     int split0;                   // first split of this launch
     const uint32_t* run_if;       // optional: the kernel returns at once when *run_if == 0
 };
 int fscan_tile_rows(int D);
+// tile rows of a dense pass over n rows
+int fscan_dense_rows(int D, int64_t Q, int64_t n, int sms);
 int fscan_part_cols(int D);
 int fscan_ring(int D);
 cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st);

@@ -397,11 +397,16 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
 // read 12 KB and its slot fills 96 KB, 160 bytes of shared memory per MMA cycle against 217 for
 // 128-row tiles.  One issuer takes every tile in order (slots are refilled within a tile); its
 // waits hide behind the 128-cycle MMAs already issued.
+// Dense passes whose tiles would leave more than half of the SMs idle take tiles of 128 rows (256 queries on
+// 8,192 of 32,768 x 1,024 rows: 64 CTAs of one tile 24 us, 128 CTAs 16).
 constexpr int kWN = 256;
-constexpr int kRingW = 2;
+constexpr int kWNarrow = 128;
+constexpr int kRingW = 2;                    // tiles of 256 rows; 3 of 128
+constexpr int kMaxRingW = 3;
 constexpr int kAccW = 2;
 constexpr int kNormW = 4;
-constexpr uint32_t kSlotW = 6u * kBox;       // query hi, query lo, corpus hi (2 boxes), corpus lo
+// query hi, query lo, corpus hi (2 boxes, or 1), corpus lo
+constexpr uint32_t slot_w(int rows) { return (2u + 2u * (uint32_t)(rows / 128)) * kBox; }
 
 // Append of a chunk by the mask of its 8-column groups that hold a key below T: the two chunks of a
 // 256-row tile leave no registers for the groups' minima (47 us a pass over 32,768 x 1,024 with 256
@@ -451,10 +456,14 @@ __device__ __forceinline__ uint32_t masked_keys(float (&v)[W], const float* nrm,
     return gm;
 }
 
-template <bool kDense>
+template <bool kDense, int kW>
 __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_constant__ FscanArgs a)
 {
-    constexpr uint32_t kIdesc = ptx::idesc_f16(kTileQ, kWN);
+    constexpr uint32_t kIdesc = ptx::idesc_f16(kTileQ, kW);
+    constexpr int kBoxes = kW / 128;         // 128-row boxes of a corpus operand
+    constexpr int kRing = kW == kWN ? kRingW : kMaxRingW;
+    constexpr uint32_t kSlotW = slot_w(kW);
+    constexpr int kPart = kW / kParts;       // columns of a tile an epilogue warp takes
     extern __shared__ __align__(1024) unsigned char sm[];
     if (a.run_if != nullptr && *a.run_if == 0u) return;
     if ((ptx::smem_u32(sm) & 1023u) != 0u) {
@@ -463,11 +472,11 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
     }
     FSmem s;
     s.ring = sm;
-    s.norms = reinterpret_cast<float*>(sm + (size_t)kRingW * kSlotW);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(s.norms + 2 * kNormW * kWN);
+    s.norms = reinterpret_cast<float*>(sm + (size_t)kRing * kSlotW);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(s.norms + 2 * kNormW * kW);
     s.full = bars;
-    s.empty = s.full + kRingW;
-    s.accf = s.empty + kRingW;
+    s.empty = s.full + kRing;
+    s.accf = s.empty + kRing;
     s.acce = s.accf + kAccW;
     s.nfull = s.acce + kAccW;
     s.nempty = s.nfull + kNormW;
@@ -484,11 +493,11 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
     const int split = a.split0 + (int)blockIdx.y;
     const int64_t n_begin = (int64_t)split * a.split_len;
     const int64_t n_end = min(a.N, n_begin + a.split_len);
-    const int ntiles = n_end > n_begin ? (int)((n_end - n_begin + kWN - 1) / kWN) : 0;
+    const int ntiles = n_end > n_begin ? (int)((n_end - n_begin + kW - 1) / kW) : 0;
     const int nch = (a.D + kCols - 1) / kCols;
 
     if (tid == 0) {
-        for (int i = 0; i < kRingW; ++i) {
+        for (int i = 0; i < kRing; ++i) {
             ptx::mbar_init(&s.full[i], 1);
             ptx::mbar_init(&s.empty[i], 1);
         }
@@ -524,31 +533,31 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
             int it = 0;
             bool ok = true;
             for (int t = 0; t < ntiles && ok; ++t) {
-                const int64_t n0 = n_begin + (int64_t)t * kWN;
-                // flags of the tile's two 128-row halves (allocated past the last row's tile)
+                const int64_t n0 = n_begin + (int64_t)t * kW;
+                // flags of the tile's 128-row boxes (allocated past the last row's tile)
                 const uint32_t clo =
-                    a.clo_flags ? __ldg(a.clo_flags + n0 / 128) | __ldg(a.clo_flags + n0 / 128 + 1) : 1u;
+                    a.clo_flags ? __ldg(a.clo_flags + n0 / 128) | __ldg(a.clo_flags + n0 / 128 + kBoxes - 1) : 1u;
                 for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % kRingW;
-                    const uint32_t ph = (uint32_t)(it / kRingW) & 1u;
+                    const int st = it % kRing;
+                    const uint32_t ph = (uint32_t)(it / kRing) & 1u;
                     if (!f_wait(a, s, &s.empty[st], ph ^ 1u, kDevTimeoutProducer)) { ok = false; break; }
                     unsigned char* dst = s.ring + (size_t)st * kSlotW;
                     s.slot_lo[st] = (clo ? 1u : 0u) | (qlo ? 2u : 0u);  // published by the arrive below
-                    ptx::mbar_arrive_expect_tx(&s.full[st], kBox * (3u + (qlo ? 1u : 0u) + (clo ? 2u : 0u)));
+                    ptx::mbar_arrive_expect_tx(&s.full[st], kBox * (1u + kBoxes + (qlo ? 1u : 0u) + (clo ? (uint32_t)kBoxes : 0u)));
                     ptx::tma_load_2d(dst, &a.tm_qhi, &s.full[st], c * kCols, (int)q0);
                     ptx::tma_load_2d(dst + 2 * kBox, &a.tm_chi, &s.full[st], c * kCols, (int)n0);
                     if (qlo) ptx::tma_load_2d(dst + kBox, &a.tm_qlo, &s.full[st], c * kCols, (int)q0);
-                    if (clo) ptx::tma_load_2d(dst + 4 * kBox, &a.tm_clo, &s.full[st], c * kCols, (int)n0);
+                    if (clo) ptx::tma_load_2d(dst + (2 + kBoxes) * kBox, &a.tm_clo, &s.full[st], c * kCols, (int)n0);
                 }
             }
             if (!ok) {
                 // let copies already issued land before the CTA winds down
-                for (int j = max(0, it - kRingW); j < it; ++j)
-                    ptx::mbar_wait(&s.full[j % kRingW], (uint32_t)(j / kRingW) & 1u, kTimeout);
+                for (int j = max(0, it - kRing); j < it; ++j)
+                    ptx::mbar_wait(&s.full[j % kRing], (uint32_t)(j / kRing) & 1u, kTimeout);
             }
         }
     } else if (warp == 3 + kEpi) {
-        load_norms<kWN, kNormW>(a, s, n_begin, ntiles);
+        load_norms<kW, kNormW>(a, s, n_begin, ntiles);
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
@@ -559,10 +568,10 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
                 const uint32_t use = (uint32_t)(t / kAccW);
                 if (!f_wait(a, s, &s.acce[b], (use & 1u) ^ 1u, kDevTimeoutMma)) { ok = false; break; }
                 ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem + (uint32_t)b * kWN;
+                const uint32_t d_tmem = tmem + (uint32_t)b * kW;
                 for (int c = 0; c < nch; ++c, ++it) {
-                    const int st = it % kRingW;
-                    if (!f_wait(a, s, &s.full[st], (uint32_t)(it / kRingW) & 1u, kDevTimeoutMma)) { ok = false; break; }
+                    const int st = it % kRing;
+                    if (!f_wait(a, s, &s.full[st], (uint32_t)(it / kRing) & 1u, kDevTimeoutMma)) { ok = false; break; }
                     ptx::tc_fence_after();
                     const uint32_t lo = s.slot_lo[st];
                     const uint32_t base = ptx::smem_u32(s.ring + (size_t)st * kSlotW);
@@ -573,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
                         const uint64_t qh = ptx::desc_sw128_kmajor(base + kk * 32);
                         const uint64_t ch = ptx::desc_sw128_kmajor(base + 2 * kBox + kk * 32);
                         ptx::mma_f16_ss(d_tmem, qh, ch, kIdesc, (c | kk) != 0);
-                        if (lo & 1u) ptx::mma_f16_ss(d_tmem, qh, ptx::desc_sw128_kmajor(base + 4 * kBox + kk * 32), kIdesc, 1u);
+                        if (lo & 1u) ptx::mma_f16_ss(d_tmem, qh, ptx::desc_sw128_kmajor(base + (2 + kBoxes) * kBox + kk * 32), kIdesc, 1u);
                         if (lo & 2u) ptx::mma_f16_ss(d_tmem, ptx::desc_sw128_kmajor(base + kBox + kk * 32), ch, kIdesc, 1u);
                     }
                     if (c == nch - 1) ptx::mma_commit(&s.accf[b]);
@@ -589,7 +598,7 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
         // ------------------------------------------------------------ epilogue
         const int ew = warp - 2;
         const int quad = warp & 3;
-        const int part = ew >> 2;   // columns [64 part, 64 part + 64) of every tile
+        const int part = ew >> 2;   // columns [kPart part, kPart part + kPart) of every tile
         const int row = quad * 32 + lane;
         const int64_t q = q0 + row;
         const bool valid = q < a.Q;
@@ -611,29 +620,31 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
                             f_wait(a, s, &s.nfull[ns], (uint32_t)(t / kNormW) & 1u, kDevTimeoutEpilogue);
             if (!__all_sync(0xffffffffu, ok)) break;
             ptx::tc_fence_after();
-            const uint32_t tb = tmem + (uint32_t)b * kWN + lane_base + (uint32_t)(64 * part);
+            const uint32_t tb = tmem + (uint32_t)b * kW + lane_base + (uint32_t)(kPart * part);
             float v[32], w[32];
             __syncwarp();
             ptx::tmem_ld32(tb, v);
-            ptx::tmem_ld32(tb + 32, w);
+            if constexpr (kPart == 64) ptx::tmem_ld32(tb + 32, w);
             ptx::tmem_wait_ld_regs(v);
-            ptx::tie_regs(w);
+            if constexpr (kPart == 64) ptx::tie_regs(w);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.acce[b]);
-            const float* nrm = s.norms + ns * kWN + 64 * part;
-            const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kWN) + (uint32_t)(64 * part);
-            const uint32_t g = masked_keys<32>(v, nrm, nrm + kNormW * kWN, m, T);
+            const float* nrm = s.norms + ns * kW + kPart * part;
+            const uint32_t base = (uint32_t)(n_begin + (int64_t)t * kW) + (uint32_t)(kPart * part);
+            const uint32_t g = masked_keys<32>(v, nrm, nrm + kNormW * kW, m, T);
             if constexpr (kDense) {
-                chunk_store<32>(v, krow + n_begin + (int64_t)t * kWN + 64 * part, a.ldk, krows);
+                chunk_store<32>(v, krow + n_begin + (int64_t)t * kW + kPart * part, a.ldk, krows);
             } else if (__any_sync(0xffffffffu, g != 0u)) {
                 masked_append<32>(v, g, T, base, out, cap, cnt);
             }
-            const uint32_t h = masked_keys<32>(w, nrm + 32, nrm + kNormW * kWN + 32, m, T);
-            if constexpr (kDense) {
-                chunk_store<32>(w, krow + n_begin + (int64_t)t * kWN + 64 * part + 32, a.ldk, krows);
-            } else if (__any_sync(0xffffffffu, h != 0u)) {
-                masked_append<32>(w, h, T, base + 32u, out, cap, cnt);
+            if constexpr (kPart == 64) {
+                const uint32_t h = masked_keys<32>(w, nrm + 32, nrm + kNormW * kW + 32, m, T);
+                if constexpr (kDense) {
+                    chunk_store<32>(w, krow + n_begin + (int64_t)t * kW + kPart * part + 32, a.ldk, krows);
+                } else if (__any_sync(0xffffffffu, h != 0u)) {
+                    masked_append<32>(w, h, T, base + 32u, out, cap, cnt);
+                }
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&s.nempty[ns]);
@@ -651,25 +662,36 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_wide_kernel(const __grid_co
 }
 
 constexpr size_t kSmemTA = (size_t)kRingTA * kSlotTA + 2 * kNorm * kTN * 4 + kCtrl;
-constexpr size_t kSmemW = (size_t)kRingW * kSlotW + 2 * kNormW * kWN * 4 + kCtrl;
-static_assert(kSmemTA <= kScanSmemLimit && kSmemW <= kScanSmemLimit, "shared memory of the FP16-split scan");
+constexpr size_t smem_w(int rows)
+{
+    return (size_t)(rows == kWN ? kRingW : kMaxRingW) * slot_w(rows) + 2 * kNormW * rows * 4 + kCtrl;
+}
+static_assert(kSmemTA <= kScanSmemLimit && smem_w(kWN) <= kScanSmemLimit && smem_w(kWNarrow) <= kScanSmemLimit,
+              "shared memory of the FP16-split scan");
 }  // namespace
 
 int fscan_tile_rows(int D) { return D <= kFscanTmemD ? kTN : kWN; }
+int fscan_dense_rows(int D, int64_t Q, int64_t n, int sms)
+{
+    if (D <= kFscanTmemD) return kTN;
+    return 2 * ((Q + kTileQ - 1) / kTileQ) * ((n + kWN - 1) / kWN) <= sms ? kWNarrow : kWN;
+}
 int fscan_part_cols(int D) { return fscan_tile_rows(D) / kParts; }
 int fscan_ring(int D) { return D <= kFscanTmemD ? kRingTA : kRingW; }
 
 cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st)
 {
     const bool ta = a.D <= kFscanTmemD;
-    const int tn = fscan_tile_rows(a.D);
+    const int tn = a.keys ? a.dense_rows : fscan_tile_rows(a.D);
+    if (a.keys && (ta ? tn != kTN : tn != kWN && tn != kWNarrow)) return cudaErrorInvalidValue;
     if (a.D < 1 || a.hp < a.D || a.hp % 8 != 0 || a.split_len % tn != 0 || (!a.keys && a.cap < 1) || a.stride < 1 || splits < 1 || a.split0 < 0 ||
         !a.cn || !a.cs || !a.qs || (ta && (!a.qhi || !a.qlo)))
         return cudaErrorInvalidValue;
     if (a.Q <= 0) return cudaSuccess;
-    const size_t smem = ta ? kSmemTA : kSmemW;
-    auto* kernel = a.keys ? (ta ? fscan_ta_kernel<true> : fscan_wide_kernel<true>)
-                          : (ta ? fscan_ta_kernel<false> : fscan_wide_kernel<false>);
+    const size_t smem = ta ? kSmemTA : smem_w(tn);
+    auto* kernel = !a.keys ? (ta ? fscan_ta_kernel<false> : fscan_wide_kernel<false, kWN>)
+                   : ta    ? fscan_ta_kernel<true>
+                   : tn == kWN ? fscan_wide_kernel<true, kWN> : fscan_wide_kernel<true, kWNarrow>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);

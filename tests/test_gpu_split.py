@@ -123,3 +123,20 @@ def test_norms_of_wide_rows(engine, oracle, D):
     od, oi = oracle.knn_gemm(X, Qs, 30)
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_array_equal(d, od)
+
+
+@pytest.mark.parametrize("Q", [1, 129, 256, 300])
+@pytest.mark.parametrize("N,D", [(16_385, 257), (33_000, 300), (40_001, 700)])
+def test_wide_rows_narrow_dense_tiles(engine, oracle, N, D, Q):
+    # rows wider than 256 columns: a seeding pass of few tiles takes 128-row tiles, of more 256-row ones
+    import torch
+    rng = np.random.default_rng(N + Q)
+    X = rng.standard_normal((N, D), dtype=np.float32)
+    Qs = rng.standard_normal((Q, D), dtype=np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 20)
+    st = engine.last_stats()
+    assert st["scan"] == 1 and engine.last_fixups() <= 1
+    sub = rng.choice(Q, min(Q, 20), replace=False)
+    od, oi = oracle.knn_gemm(X, Qs[sub], 20, kp=st["kp"], rerank=True)
+    np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
+    np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
