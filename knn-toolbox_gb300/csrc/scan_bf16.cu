@@ -445,15 +445,21 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 float ga[W1 / 8], gb[W2 / 8], gc[1];
                 chunk_minima<W1>(va, ga);
                 chunk_minima<W2>(vb, gb);
-                float mn = fminf(min_of(ga), min_of(gb));
+                const float ma = min_of(ga);
+                float mb = min_of(gb);
                 if constexpr (W3 > 0) {
                     chunk_minima<W3>(vc, gc);
-                    mn = fminf(mn, gc[0]);
+                    mb = fminf(mb, gc[0]);
                 }
-                if (__any_sync(0xffffffffu, mn < T)) {
-                    chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
-                    chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
-                    if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
+                if (__any_sync(0xffffffffu, fminf(ma, mb) < T)) {
+                    // (E4M3 keys, whose loop is longer: a second vote per half, 811 -> 801 us for 2,000,000 x 256;
+                    // BF16 keys 1,634 -> 1,669 with it)
+                    if (!kF8 || __any_sync(0xffffffffu, ma < T))
+                        chunk_append<W1>(va, ga, T, nb + (uint32_t)c1, out, cap, cnt);
+                    if (!kF8 || __any_sync(0xffffffffu, mb < T)) {
+                        chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
+                        if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
+                    }
                 }
             }
         }

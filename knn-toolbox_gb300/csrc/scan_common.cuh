@@ -86,7 +86,8 @@ __device__ __forceinline__ void chunk_append(const float (&key)[W], const float 
             const float* kg = key + 8 * g;
             uint32_t hm = 0;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) hm |= (kg[j] < T ? 1u : 0u) << j;
+            for (int j = 0; j < 8; ++j)
+                if (kg[j] < T) hm |= 1u << j;
             if ((hm & (hm - 1u)) == 0u) {
                 if (cnt < cap)
                     out[cnt] = ((uint64_t)__float_as_uint(gm[g]) << 32) | (uint64_t)(base + (uint32_t)(8 * g + __ffs((int)hm) - 1));
