@@ -320,6 +320,9 @@ __global__ void __launch_bounds__(kSelWarps * 32) select_threshold_kernel(const 
 //    bitonic sort.
 constexpr int kRankSortMax = 128;
 constexpr int64_t kThrBlockQ = 1536;  // threshold mode: a warp per query above
+// Up to a query an SM: 512 threads each, which shorten one query's chain of round trips (48 queries on
+// 2,000,000 x 128: threshold from 7,813 keys 7.5 -> 4.9 us, selection 12.9 -> 11.8, the search 150 -> 145).
+constexpr int64_t kSelFewQ = 152;
 constexpr int64_t kSelWideQ = 384;  // up to this many queries: 256 threads each, above 128
 
 // The first k of `cur` (m packed words: key or distance above index) in ascending order to the
@@ -510,7 +513,7 @@ __device__ __forceinline__ void find_bin(const uint32_t* hist, uint32_t rank, ui
 // ten of 128 threads (47 registers; at 63 a million rows' 10,000 queries take 97 instead of 88 us), four
 // of 256 (for the re-rank's loads in flight: 256 queries, 32 rows of 1,024 columns 18.9 -> 15.5 us).
 template <int kT, bool kThr>
-__global__ void __launch_bounds__(kT, kT == 128 ? 10 : 4) select_block_kernel(const CandSelect c)
+__global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_kernel(const CandSelect c)
 {
     if (c.skip_if != nullptr && *c.skip_if != 0u) return;
     if (c.skip_if_zero != nullptr && *c.skip_if_zero == 0u) return;
@@ -722,14 +725,14 @@ __device__ __forceinline__ void load_ordered(const float* __restrict__ row, int 
 
 // ---------------------------------------------------------------- thresholds from dense keys
 // One block per query: the keys, as ordered words, into shared memory.  Ranks up to kDenseRank: the
-// rank-th smallest of 32 group minima (four threads each) bounds the key of that rank from above, so
+// rank-th smallest of 32 group minima (four threads each, or sixteen) bounds the key of that rank from above, so
 // only the few keys up to it are collected and the rank among them counted.  Otherwise the key is
 // found by a byte-wise histogram search from the highest bit in which the finite keys differ.
 // Latency-bound for few queries (48 x 3,907 keys 6.3 us, 11.9 by histogram), by issue slots for many
 // (10,000 x 1,954 keys 35 us against 60).
-constexpr int kDenseT = 128;
 constexpr int kDenseRank = 24;
 constexpr int kDenseList = 256;
+template <int kDenseT>
 __global__ void __launch_bounds__(kDenseT) dense_threshold_kernel(const float* __restrict__ keys, int64_t ldk, int n,
                                                                   int rank, float* __restrict__ thr_out,
                                                                   uint32_t* clear, const uint32_t* skip_if,
@@ -751,9 +754,11 @@ __global__ void __launch_bounds__(kDenseT) dense_threshold_kernel(const float* _
     uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
     load_ordered<kDenseT>(row, n, ord, lo, hi, cnt);
     const uint32_t mine = lo;
-    uint32_t g = min(lo, __shfl_xor_sync(0xffffffffu, lo, 1));
-    g = min(g, __shfl_xor_sync(0xffffffffu, g, 2));
-    if ((lane & 3) == 0) gmin[tid >> 2] = g;
+    constexpr int kGroup = kDenseT / 32;  // threads a group
+    uint32_t g = lo;
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1) g = min(g, __shfl_xor_sync(0xffffffffu, g, o));
+    if ((lane & (kGroup - 1)) == 0) gmin[tid / kGroup] = g;
     lo = __reduce_min_sync(0xffffffffu, lo);
     hi = __reduce_max_sync(0xffffffffu, hi);
     cnt = __reduce_add_sync(0xffffffffu, cnt);
@@ -855,7 +860,10 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
     if (Q <= 0) return cudaSuccess;
     if (n < 1 || n > kDenseRows || rank < 1 || ldk % 4 != 0 || ldk < n) return cudaErrorInvalidValue;
     const size_t smem = (size_t)((n + 3) & ~3) * 4;
-    dense_threshold_kernel<<<(unsigned)Q, kDenseT, smem, s>>>(keys, ldk, n, rank, thr_out, clear, skip_if, skip_if_zero);
+    if (Q <= kSelFewQ)
+        dense_threshold_kernel<512><<<(unsigned)Q, 512, smem, s>>>(keys, ldk, n, rank, thr_out, clear, skip_if, skip_if_zero);
+    else
+        dense_threshold_kernel<128><<<(unsigned)Q, 128, smem, s>>>(keys, ldk, n, rank, thr_out, clear, skip_if, skip_if_zero);
     return cudaGetLastError();
 }
 
@@ -1198,7 +1206,9 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         // a block per query while warps would leave SMs idle: 62,500-row level of 2,000,000 x 128, 64 /
         // 777 / 2,048 queries 7.9 (256 threads) / 8.9 (128) / 11.5 against 17.8 / 10.0 / 9.7 us
         const size_t smem = (size_t)c.buf_words * 8;
-        if (c.Q <= kSelWideQ)
+        if (c.Q <= kSelFewQ)
+            select_block_kernel<512, true><<<(unsigned)c.Q, 512, smem, s>>>(c);
+        else if (c.Q <= kSelWideQ)
             select_block_kernel<256, true><<<(unsigned)c.Q, 256, smem, s>>>(c);
         else
             select_block_kernel<128, true><<<(unsigned)c.Q, 128, smem, s>>>(c);
@@ -1213,10 +1223,13 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         // selection of 256 / 777 queries 9.4 / 14.4 against 11.4 / 11.4 us (65,536 x 128, k = 16),
         // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512, before the re-rank took two rows at a time)
         const size_t smem = ((size_t)pow2_at_least(c.kp) + c.buf_words) * 8 + (size_t)((c.D + 3) & ~3) * 4;
-        auto* kernel = c.Q <= kSelWideQ ? select_block_kernel<256, false> : select_block_kernel<128, false>;
+        const int t = c.Q <= kSelFewQ ? 512 : c.Q <= kSelWideQ ? 256 : 128;
+        auto* kernel = t == 512   ? select_block_kernel<512, false>
+                       : t == 256 ? select_block_kernel<256, false>
+                                  : select_block_kernel<128, false>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kernel<<<(unsigned)c.Q, c.Q <= kSelWideQ ? 256 : 128, smem, s>>>(c);
+        kernel<<<(unsigned)c.Q, t, smem, s>>>(c);
     }
     return cudaGetLastError();
 }

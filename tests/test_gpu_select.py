@@ -113,3 +113,19 @@ def test_few_queries_seed_from_one_level(engine, oracle, kind, N, Q, k):
     od, oi = oracle.knn_gemm(X, Qs[sub], k, kp=st["kp"], rerank=True)
     np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
     np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
+
+
+@pytest.mark.parametrize("Q", [152, 153])
+@pytest.mark.parametrize("N,k", [(20_000, 10), (140_000, 100), (300_000, 300)])
+def test_block_sizes_by_queries(engine, oracle, Q, N, k):
+    # 512 threads a query up to a query an SM, 256 above: thresholds and selections, shortlists counted and sorted
+    import torch
+    rng = np.random.default_rng(N + Q)
+    X = rng.integers(0, 64, (N, 20)).astype(np.float32)
+    Qs = rng.integers(0, 64, (Q, 20)).astype(np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
+    st = engine.last_stats()
+    sub = rng.choice(Q, 20, replace=False)
+    od, oi = oracle.knn_gemm(X, Qs[sub], k, kp=st["kp"], rerank=True)
+    np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
+    np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
