@@ -995,6 +995,7 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
             if (tid == 0) hit_s = 0;
             __syncthreads();
             if (warp == 0) find_bin(hist, r, digit_s, rank_s, hit_s);
+            __syncthreads();
             for (int b = tid; b < 256; b += kT) hist[b] = 0;
             __syncthreads();
             h = hit_s;
