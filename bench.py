@@ -21,7 +21,7 @@ step budget allows (the default run times the full 10,000-query batch).
 The plain-form line also carries `accuracy` (recall@k and the largest relative
 distance error against the FP64 oracle on a query sample, outside the timed
 region) and `forms`: the same workload through the BF16 shortlist form (c from
-the autotuner) and through the plain form on 3xTF32 keys (`tf32_only`), each
+the autotuner) and through the plain form on split keys (`tf32_only`), each
 timed like the headline and checked against the same FP64 sample.
 """
 import argparse
@@ -48,12 +48,12 @@ WORKLOADS = {
     "mix4m": dict(desc="Gaussian mixture corpus 4,000,000 x 96 (1,024 centres N(0,1), sigma 0.15, rows "
                        "L2-normalised), 10,000 queries, k=10, seed 2",
                   gen="gauss_mixture", N=4_000_000, D=96, Q=10_000, k=10, seed=2),
-    # profiling-sized cut of mix4m for ncu captures of the 3xTF32 scan (corpus still larger than L2)
+    # profiling-sized cut of mix4m for ncu captures of the split-key scan (corpus still larger than L2)
     "mix1m": dict(desc="Gaussian mixture corpus 1,000,000 x 96 (1,024 centres N(0,1), sigma 0.15, rows "
                        "L2-normalised), 2,500 queries, k=10, seed 2",
                   gen="gauss_mixture", N=1_000_000, D=96, Q=2_500, k=10, seed=2),
     # serving form: resident corpus, Poisson arrivals of requests of uneven size and k
-    "serve2m": dict(desc="serving: int-descriptor corpus 2,000,000 x 128 resident (FP32 + BF16 + TF32 copies), "
+    "serve2m": dict(desc="serving: int-descriptor corpus 2,000,000 x 128 resident (FP32 + BF16 + FP16 hi / lo copies), "
                          "Poisson arrivals, request sizes log-uniform on [1,512], k in {1,10,100}, seed 1",
                     gen="int_descriptor", N=2_000_000, D=128, Q=0, k=0, seed=1, serve=True),
     # precision form with E4M3 keys: anisotropic Gaussian N(0, diag(1/sqrt(1+j)))
@@ -107,8 +107,6 @@ def measured_peaks():
 NCU_TRAFFIC = {
     ("scan_kernel", "int1m"): 398.3e6,
     ("scan_kernel", "aniso8m"): 2537.0e6,
-    ("tscan_kernel", "uniform64k"): 69.9e6,
-    ("tscan_kernel", "mix4m"): 3405.0e6,
 }
 
 
@@ -220,14 +218,17 @@ class ClockSampler:
                 "reasons": reasons, "samples": len(rows)}
 
 
-def path_of(st, bf16_keys):
+def path_of(st, bf16_keys, k):
     """(path, dominant kernel) of a search from its statistics: bf16_keys when its keys are BF16 /
-    E4M3 (a precision form, or BF16-exact data in the exact form)."""
+    E4M3 (a precision form, or BF16-exact data in the exact form).  Other FP32 data take FP16-split
+    keys, or 3xTF32 keys where the shortlist has no margin over k."""
     import cuknns
     keys = st.get("scan_keys", 0)
     if keys & 1 and (bf16_keys or not keys & 2):
         return "threshold scan (BF16 / E4M3 keys)", "scan_kernel"
     if keys & 2:
+        if st["kp"] >= k + 8:
+            return "threshold scan (FP16-split keys)", "fscan_kernel"
         return "threshold scan (3xTF32 keys)", "tscan_kernel"
     if st["algo"] == cuknns.ALGO_TC:
         return "shortlist kernel (tcgen05)", "tc_kernel"
@@ -235,9 +236,10 @@ def path_of(st, bf16_keys):
 
 
 def lo_tile_fraction(x, rows=128):
-    """Fraction of 128-row tiles whose TF32 low part (x - tf32(x), rounded to TF32) is nonzero.
+    """Fraction of 128-row tiles whose low part (x - tf32(x), rounded to TF32) is nonzero: values of
+    more than 11 significant bits, which is also what the FP16 split's high part holds.
 
-    The tensor-core kernel runs the two correction products of 3xTF32 only on
+    The tensor-core kernels run the two correction products of split keys only on
     such tiles, so this sets the executed tensor work.
     """
     def tf32(a):
@@ -447,11 +449,11 @@ def run_gb300(args, w):
     with ClockSampler(local) as clk:
         el_ms, hl_stages, st = timed(search_step(prec, args.shortlist, single_stream=args.single_stream),
                                      args.steps)
-    # the path that ran: the exact form decides between BF16 and 3xTF32 keys on the device (BF16
+    # the path that ran: the exact form decides between BF16 and split keys on the device (BF16
     # keys when every corpus and query value is exact in BF16); the data tell which
     bf16_exact = bool(((corpus_np.view(np.uint32) & 0xFFFF) == 0).all() and
                       ((queries_np.view(np.uint32) & 0xFFFF) == 0).all())
-    path, kern = path_of(st, args.precision != "exact" or bf16_exact)
+    path, kern = path_of(st, args.precision != "exact" or bf16_exact, k)
     # whole-job throughput: replicas search world x Q queries; a corpus split searches Q
     value = Q * args.steps * (1 if split_corpus else world) / (el_ms / 1e3)
     # stage times and the dominant kernel's launch time: the same search with every kernel on the
@@ -488,7 +490,7 @@ def run_gb300(args, w):
 
     accuracy = accuracy_now()
 
-    # ---- the other forms on the same workload (plain form only): BF16 shortlist, 3xTF32 keys
+    # ---- the other forms on the same workload (plain form only): BF16 shortlist, split keys
     forms = None
     if prec == cuknns.PREC_EXACT and not args.no_forms and not split_corpus:
         forms = {"exact": {"queries_per_s": value, "accuracy": accuracy, "path": path}}
@@ -500,21 +502,21 @@ def run_gb300(args, w):
         t_steps = max(3, min(args.steps, 20))
         t_ms, t_stages, t_st = timed(search_step(cuknns.PREC_EXACT, 0, tf32_only=True, single_stream=True), t_steps)
         f_c, f_q = lo_tile_fraction(corpus_np), lo_tile_fraction(queries_np)
-        t_path, t_kern = path_of(t_st, False)
-        t_scan = t_kern == "tscan_kernel"
-        # the TF32 scan's main pass is its own stage; the shortlist kernel's stage includes its pilot
+        t_path, t_kern = path_of(t_st, False, k)
+        t_scan = t_kern in ("fscan_kernel", "tscan_kernel")
+        # the split-key scan's main pass is its own stage; the shortlist kernel's stage includes its pilot
         t_fused = (t_stages[2] if t_scan else t_stages[1] + t_stages[2]) / max(1, t_stages[5])
         products = 1.0 + f_c + f_q
         t_flops = products * 2.0 * N * Q * D * (1.0 + (1.0 / 16.0 if t_st["pilot"] and not t_scan else 0.0))
-        tf32_peak = tf32_peak_live()
+        split_peak = measured_peaks()[0]["bf16_tflops"] if t_kern == "fscan_kernel" else tf32_peak_live()
         forms["tf32_plain"] = {"queries_per_s": Q * t_steps * world / (t_ms / 1e3), "ms_per_step": t_ms / t_steps,
-                               "steps": t_steps, "kernel": f"{t_kern} (3xTF32)", "path": t_path,
+                               "steps": t_steps, "kernel": t_kern, "path": t_path,
                                "products_per_useful_product": products,
-                               "note": "3xTF32 keys; a correction product is skipped where the TF32 low part of the "
+                               "note": "split keys forced; a correction product is skipped where the low part of the "
                                        "corpus tile or query tile is zero (exact zeros), as on integer data",
                                "fused_ms": t_fused,
-                               "tf32_tflops_executed": t_flops / (t_fused / 1e3) / 1e12,
-                               "tf32_peak_measured": tf32_peak,
+                               "split_tflops_executed": t_flops / (t_fused / 1e3) / 1e12,
+                               "split_peak_measured": split_peak,
                                "accuracy": accuracy_now()}
         forms["bf16_over_tf32"] = forms["bf16_shortlist"]["queries_per_s"] / forms["tf32_plain"]["queries_per_s"]
         # leave the headline's answers in the output buffers
@@ -532,7 +534,7 @@ def run_gb300(args, w):
     on_scan = kern == "scan_kernel"
     # shortlist kernels: the fused stage includes their pilot pass; the scans' seeding passes are
     # their own stage
-    fused_avg_ms = (fused_ms if kern in ("scan_kernel", "tscan_kernel") else seed_ms + fused_ms) / max(1, nt)
+    fused_avg_ms = (fused_ms if kern in ("scan_kernel", "fscan_kernel", "tscan_kernel") else seed_ms + fused_ms) / max(1, nt)
     if on_scan:
         # the main pass alone is timed (seeding passes are their own stage); one product per pair
         flops = 2.0 * N * Q * D
@@ -554,19 +556,21 @@ def run_gb300(args, w):
                 "flops_per_launch": flops, "padded_k": int(padded_k)}
     elif st["algo"] == cuknns.ALGO_TC:
         # executed tensor work of the fused stage (main pass + the 1/16-sample pilot pass of the
-        # shortlist kernel; the TF32 scan's main pass alone)
+        # shortlist kernel; the split-key scan's main pass alone)
         pilot_f = 1.0 + (1.0 / 16.0 if st["pilot"] and kern == "tc_kernel" else 0.0)
         if args.precision != "exact" or bf16_exact:
             kind, products, peak = ("bf16 shortlist" if args.precision != "exact" else "bf16 (data BF16-exact)",
                                     1.0, peaks["bf16_tflops"])
             peak_src = f"{peak_kind} bf16 dense burst"
         else:
-            # 3xTF32 issues hi.hi always and the two correction products only for
-            # tiles whose TF32 low part is nonzero (corpus tile / query tile)
+            # split keys issue hi.hi always and the two correction products only for
+            # tiles whose low part is nonzero (corpus tile / query tile)
             f_c, f_q = lo_tile_fraction(corpus_np), lo_tile_fraction(queries_np)
-            kind, products = "3xTF32", 1.0 + f_c + f_q
-            live = tf32_peak_live()
-            if live is not None:
+            kind, products = "FP16 split" if kern == "fscan_kernel" else "3xTF32", 1.0 + f_c + f_q
+            live = None if kern == "fscan_kernel" else tf32_peak_live()
+            if kern == "fscan_kernel":
+                peak, peak_src = peaks["bf16_tflops"], f"{peak_kind} bf16 dense burst (kind::f16)"
+            elif live is not None:
                 peak, peak_src = live, "cuBLAS TF32 8192^3 GEMM burst, measured in this run"
             else:
                 peak, peak_src = peaks["bf16_tflops"] / 2.0, f"{peak_kind} bf16 dense burst / 2 (nominal TF32 rate)"
@@ -721,8 +725,8 @@ def main():
     ap.add_argument("--shortlist", type=int, default=0,
                     help="bf16 / fp8: shortlist factor c (0 = chosen by the autotuner)")
     ap.add_argument("--scan", default="auto", choices=["auto", "on", "off", "tf32"],
-                    help="threshold scan (auto: BF16 keys for BF16-exact data and 3xTF32 keys otherwise from "
-                         "131,072 rows, 3xTF32 keys from 16,384; on: the pair from 16,384; tf32: 3xTF32 alone)")
+                    help="threshold scan (auto: BF16 keys for BF16-exact data and split keys otherwise from "
+                         "131,072 rows, split keys from 16,384; on: the pair from 16,384; tf32: split keys alone)")
     ap.add_argument("--scan-boxes", type=int, default=0, help="threshold scan: K boxes per ring slot (0 = auto)")
     ap.add_argument("--single-stream", action="store_true",
                     help="the headline search with every kernel on one stream (a fixed launch order for "
@@ -735,7 +739,7 @@ def main():
     ap.add_argument("--recall-queries", type=int, default=0,
                     help="queries of the FP64-oracle accuracy sample (0 = 100)")
     ap.add_argument("--no-forms", action="store_true",
-                    help="plain form: skip the BF16-shortlist and 3xTF32 comparison runs")
+                    help="plain form: skip the BF16-shortlist and split-key comparison runs")
     ap.add_argument("--split", default="queries", choices=["queries", "corpus"],
                     help="N > 1 GPUs: replicas with their own queries (weak scaling), or one query batch "
                          "against a corpus split across the GPUs (strong scaling: all-gather + merge)")
