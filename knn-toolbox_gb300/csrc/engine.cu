@@ -522,8 +522,17 @@ static int finest_rank(double m, int64_t n)
     return j;
 }
 
-// Most candidates of a query (mean plus six standard deviations) that the selection's buffer must hold
-static double cand_bound(int j, int64_t stride) { return (double)j * stride + 6.0 * (double)stride * std::sqrt((double)j) + 64.0; }
+// Most candidates of a query that the selection's buffer must hold: its main-pass count is about stride x
+// (a Gamma(j) variable), whose upper tail is long.  Six standard deviations leave one query in 200,000 over (5 %
+// of searches with 10,000 queries, which then pay a fix-up over the corpus: 4.1 ms on the 4,000,000 x 96
+// mixture, where one query of 10,000 was over), eight one in five million or fewer; the buffer's share
+// of shared memory costs the selection 0 to 1 us of 40 to 90.
+static double cand_bound(int j, int64_t stride, double sigmas)
+{
+    return (double)j * stride + sigmas * (double)stride * std::sqrt((double)j) + 64.0;
+}
+constexpr double kCandSigmas = 8.0;
+constexpr double kCandSigmasFew = 6.0;  // at most 128 queries
 
 // Up to one tile of queries on rows of 256 bytes or more the main pass waits for memory, so its
 // epilogue has room for more candidates: the finest sample may be as coarse as the dense pass's own
@@ -584,7 +593,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
         int64_t w = P->stride0;
         while (cdiv(N, w) > kDenseRows) w *= 2;
         if (w > P->stride0 && w <= kSeedStrideFew &&
-            cand_bound(finest_rank((double)kp / (double)w, cdiv(N, w)), w) <= (double)kCandMaxFew) {
+            cand_bound(finest_rank((double)kp / (double)w, cdiv(N, w)), w, kCandSigmasFew) <= (double)kCandMaxFew) {
             P->stride0 = w;
             cand_max = kCandMaxFew;
         }
@@ -661,11 +670,10 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     P->S = (int)cdiv(N, P->len);
     const double hm = (double)P->lv[L - 1].j * (double)P->lv[L - 1].stride;
     P->cap = std::min<int>((int)(P->len / tn * pc), seg_cap(hm * pc / ((double)tn * P->S), 2.0));
-    // a query's main-pass count is about stride x (a Gamma(j) variable): hm + 6 stride sqrt(j)
-    // bounds it but for queries whose strided sample misrepresents them (those fail over to
-    // the fix-up either way); the selection buffer is sized to it, not to its ceiling
+    // (a query above the bound fails over to the fix-up, as an overflowing segment does)
     P->sel_words = (int)std::min<double>(
-        (double)cand_max, std::ceil(cand_bound(P->lv[L - 1].j, P->lv[L - 1].stride) / 32.0) * 32.0);
+        (double)cand_max, std::ceil(cand_bound(P->lv[L - 1].j, P->lv[L - 1].stride,
+                                                  cand_max > kCandMax ? kCandSigmasFew : kCandSigmas) / 32.0) * 32.0);
     P->cand_words = std::max(P->cand_words, (size_t)kScanParts * P->S * Q * P->cap);
     P->cnt_words = std::max(P->cnt_words, (size_t)kScanParts * P->S * Q);
     // fix-up of failed queries: up to 512 on a full wave, the rest (rare) on 8 splits; shortlists
