@@ -19,8 +19,8 @@
 // corpus tile (or query tile) is skipped -- it would add exact zeros.
 //
 // Both kernels are bound by the tensor pipe (3 x 2 N Q D FLOPs).  Main pass against the 3xTF32 one
-// (same box): 1,000,003 x 96, 2,000 queries 755 us against 1,356 (1,528 TFLOP/s executed); 65,536 x
-// 128, 1,024 queries 40 against 74; 32,768 x 1,024, 256 queries 48 against 92.  Key error against
+// (same box): 1,000,003 x 96, 2,000 queries 726 us against 1,356 (1,620 TFLOP/s executed, at the card's
+// power limit); 65,536 x 128, 1,024 queries 39 against 74; 32,768 x 1,024, 256 queries 48 against 92.  Key error against
 // FP64 relative to ||c||^2 + ||q||^2, rms: uniform D = 128 6.4e-7 against 9.8e-7, D = 1,024 5.9e-6
 // against 8.2e-6, Gaussian D = 96 1.1e-7 against 1.8e-7, mixture D = 96 2.9e-7 against 4.6e-7.
 //

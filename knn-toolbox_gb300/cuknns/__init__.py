@@ -462,7 +462,7 @@ INDEX_FP8 = 2
 
 
 class Index:
-    """A device corpus prepared once (BF16 copy, norms, flags, TF32 copies, E4M3 codes): searches skip its preparation.
+    """A device corpus prepared once (BF16 copy, norms, flags, FP16 hi / lo copies, E4M3 codes): searches skip its preparation.
 
     The torch tensor is kept referenced: the engine reads it on every search.
     """
