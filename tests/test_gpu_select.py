@@ -129,3 +129,20 @@ def test_block_sizes_by_queries(engine, oracle, Q, N, k):
     od, oi = oracle.knn_gemm(X, Qs[sub], k, kp=st["kp"], rerank=True)
     np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
     np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
+
+
+@pytest.mark.parametrize("Q", [1536, 1537, 3000])
+@pytest.mark.parametrize("N,hi", [(16_384, 2), (20_001, 3), (33_333, 2), (140_000, 4)])
+def test_dense_thresholds_with_ties(engine, oracle, Q, N, hi):
+    # thresholds from dense keys by a block (1,536 queries) and by a warp: few distinct keys, so that more
+    # words reach the bound than the warp's list holds
+    import torch
+    rng = np.random.default_rng(N + Q)
+    X = rng.integers(0, hi, (N, 9)).astype(np.float32)
+    Qs = rng.integers(0, hi, (Q, 9)).astype(np.float32)
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 10)
+    st = engine.last_stats()
+    sub = rng.choice(Q, 30, replace=False)
+    od, oi = oracle.knn_gemm(X, Qs[sub], 10, kp=st["kp"], rerank=True)
+    np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
+    np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
