@@ -16,7 +16,8 @@
 //      largest, D32, and an FP64 distance >= D32 - E, where E bounds the error
 //      of an FP32 distance of rounded data, E = (D/8 + 10) * 2^-24 *
 //      (|q| + max|c|)^2 + 1e-5 * D32 (the last term covers the float engine's
-//      own ranking tolerance) + 1e-44 D (subnormals); accepted when the k-th FP64 distance < D32 - E;
+//      own ranking tolerance) + 1e-44 D (subnormals); accepted when the k-th FP64 distance < D32 - E,
+//      or when the shortlist holds every row;
 //   4. any other query is searched again by an FP64 brute-force kernel.
 // Results: the exact FP64 top-k ordered by (distance, index).
 #include <algorithm>
@@ -283,12 +284,14 @@ __global__ void __launch_bounds__(256) rerank64_kernel(int64_t N, const double* 
     __shared__ double kth;
     const int64_t q = blockIdx.x;
     const int m = ncand[q];
+    bool gap = false;
     for (int j = threadIdx.x; j < m; j += blockDim.x) {
         const int32_t n = ci[q * kp + j];
+        gap |= n < 0;
         sw[j] = make_longlong2(__double_as_longlong(dd[q * kp + j]), n >= 0 ? n : 0x7fffffff);
     }
     if (threadIdx.x == 0) kth = __longlong_as_double(0x7ff0000000000000ll);
-    __syncthreads();
+    const bool missing = __syncthreads_or(gap) != 0;
     for (int j = threadIdx.x; j < m; j += blockDim.x) {
         int below = 0;
         const longlong2 w = sw[j];
@@ -301,9 +304,9 @@ __global__ void __launch_bounds__(256) rerank64_kernel(int64_t N, const double* 
         if (below == k - 1) kth = __longlong_as_double(w.x);
     }
     __syncthreads();
-    // the shortlist covers the corpus, or its k-th FP64 distance stays below the smallest FP64
-    // distance any row outside it can have
-    if (!(kp >= N || (m >= k && kth < bound[q]))) {
+    // the shortlist covers the corpus (a row whose norm or key overflowed FP32 is missing from it), or its
+    // k-th FP64 distance stays below the smallest FP64 distance any row outside it can have
+    if (!(kp >= N ? !missing : m >= k && kth < bound[q])) {
         if (threadIdx.x == 0) fails[1 + atomicAdd(fails, 1u)] = (uint32_t)q;
         return;
     }

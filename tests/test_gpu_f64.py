@@ -115,3 +115,14 @@ def test_double_library_rounding_to_float(engine, oracle, lo, hi):
     od, oi = oracle.knn_f64d(X, Qs, 10)
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_array_equal(d, od)
+
+
+@pytest.mark.parametrize("N,D,k,scale", [(40, 6, 10, 1e20), (70, 9, 70, 1e20), (5, 3, 5, 1e25), (42, 300, 10, 1e20)])
+def test_double_library_distances_past_the_float_range(engine, oracle, N, D, k, scale):
+    # the FP32 shortlist could hold every row (N <= max(k + 32, 2 k)), but holds none of these
+    rng = np.random.default_rng(N)
+    X, Qs = rng.standard_normal((N, D)) * scale, rng.standard_normal((7, D)) * scale
+    d, i = engine.search_host_f64(X, Qs, k)
+    od, oi = oracle.knn_f64d(X, Qs, k)
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_array_equal(d, od)
