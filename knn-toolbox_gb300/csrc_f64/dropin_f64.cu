@@ -16,8 +16,8 @@
 //      largest, D32, and an FP64 distance >= D32 - E, where E bounds the error
 //      of an FP32 distance of rounded data, E = (D/8 + 10) * 2^-24 *
 //      (|q| + max|c|)^2 + 1e-5 * D32 (the last term covers the float engine's
-//      own ranking tolerance) + 1e-44 D (subnormals); accepted when the k-th FP64 distance < D32 - E,
-//      or when the shortlist holds every row;
+//      own ranking tolerance) + 1e-44 D (subnormals), unbounded where norms can leave the float range;
+//      accepted when the k-th FP64 distance < D32 - E, or when the shortlist holds every row;
 //   4. any other query is searched again by an FP64 brute-force kernel.
 // Results: the exact FP64 top-k ordered by (distance, index).
 #include <algorithm>
@@ -210,6 +210,9 @@ __device__ __forceinline__ double err_bound(const double* qv, int D, double d32,
     for (int d = lane; d < D; d += 32) qq = __dadd_rn(qq, __dmul_rn(qv[d], qv[d]));
     for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, o);
     const double s = sqrt(qq) + __longlong_as_double((long long)cmax_bits);
+    // norms and products that can leave the float range: rows without an FP32 key are in no shortlist,
+    // however near they are, so none proves anything
+    if (!(s * s < 1e38)) return __longlong_as_double(0x7ff0000000000000ll);
     // (the last term: squares and sums rounded in the subnormal range)
     return ((double)D / 8.0 + 10.0) * 5.9604644775390625e-08 * s * s + 1e-5 * d32 + (double)D * 1e-44;
 }

@@ -126,3 +126,15 @@ def test_double_library_distances_past_the_float_range(engine, oracle, N, D, k, 
     od, oi = oracle.knn_f64d(X, Qs, k)
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_array_equal(d, od)
+
+
+@pytest.mark.parametrize("N", [100, 20000])
+def test_double_library_norms_past_the_float_range(engine, oracle, N):
+    # the nearest rows have squared norms above 3.4e38, so no FP32 key, but small distances; every other
+    # row has both
+    X = np.concatenate([np.linspace(1.5e19, 1.8e19, N - 10), np.linspace(1.846e19, 1.86e19, 10)])[:, None]
+    Qs = np.array([[1.84e19], [-1e19]])
+    d, i = engine.search_host_f64(X, Qs, 10)
+    od, oi = oracle.knn_f64d(X, Qs, 10)
+    np.testing.assert_array_equal(i, oi)
+    np.testing.assert_array_equal(d, od)
