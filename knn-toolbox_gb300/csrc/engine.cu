@@ -392,6 +392,7 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
         o.algo != KNNS_ALGO_AUTO || o.scan != KNNS_SCAN_AUTO || o.splits > 0 || !o.pilot || o.tf32_only || !c->rerank ||
         c->kp < k + kKeyMargin || k > kMaxKpScan)
         return rc;
+    c->fp32 = c->algo == KNNS_ALGO_SIMT;
     if (N * (D + 32) <= kDirectBlock && Q * N * (D + 32) <= kDirectTotal) {
         c->small = 1;
         c->algo = KNNS_ALGO_SIMT;
@@ -1123,6 +1124,8 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
     sel.n = (int)N;
     sel.need = k;
     sel.k = k;
+    sel.kp = dense ? 0 : c.kp;
+    sel.fp32_keys = c.fp32;
     sel.Q = Q;
     sel.corpus = corpus;
     sel.ldc = ldc;

@@ -49,6 +49,8 @@ struct Config {
     bool tf32 = false;
     // small corpora: 0 none of these, 1 the exact distances of every row (one launch), 2 every row's key
     int small = 0;
+    // ... of shapes whose keys are FP32 ones without these (the CUDA-core kernel's)
+    bool fp32 = false;
 };
 
 struct Engine {

@@ -327,13 +327,16 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
 // Small corpora, no thresholds: per query, the `need` smallest of n values and the k results.
 //  * keys given: a dense pass's keys (row q at keys + q * ldk); the `need` smallest (key, index) pairs
 //    are re-ranked by exact distance;
-//  * keys null: the exact distances themselves, computed by the kernel (need = k).
-// n <= kSmallRows.  Values that are not finite are never results; missing results are (+inf, -1).
+//  * keys null: the exact distances themselves, computed by the kernel (need = k).  Where squares leave the
+//    float range: the kp smallest (key, index) pairs re-ranked as above, the keys in FP32 arithmetic, by the
+//    kernel too (of a query that is not finite: only with fp32_keys).
+// n <= kSmallRows.  Rows whose key is not below +inf are never results; missing results are (+inf, -1).
 constexpr int kSmallRows = 16384;
 struct SmallSelect {
     const float* keys = nullptr;
     int64_t ldk = 0;
-    int n = 0, need = 0, k = 0;
+    int n = 0, need = 0, k = 0, kp = 0;
+    bool fp32_keys = false;
     int64_t Q = 0;
     const float* corpus = nullptr;
     int64_t ldc = 0;

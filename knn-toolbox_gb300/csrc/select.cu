@@ -975,19 +975,59 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
 // index (10,000 keys, 500 queries, shortlist 32: 21.5 us that way).  Direct mode
 // computes the exact distances first, eight lanes a row, four rows a lane in flight: one launch serves
 // the whole search, bound by the reads of the corpus from L2 (each block reads all of it).
+// Direct mode's distances alone decide while every squared norm and distance stays below kDirectMost: then no
+// norm and no key ||c||^2 - 2 q.c leaves the float range.  Otherwise the rows are ranked by their FP32 keys as
+// everywhere else (small_keys), so that a row whose norm or key overflows is no result and one whose distance
+// alone does is (+inf, its index).
 constexpr int kSmallList = 256;
+constexpr float kDirectMost = 1e37f;
+
+// Every row's key as an ordered word (+inf where it is not below +inf), a thread a row: in the arithmetic of the
+// CUDA-core kernel where the shape's keys are FP32 ones; otherwise from the product q.c rounded once, as a tensor-core
+// step adds its products (partial sums do not overflow).  Keys of a query that is not finite: FP32 keys have
+// them, split keys do not.
+static __device__ __noinline__ void small_keys(const SmallSelect& c, const float* qv, bool finite, uint32_t* ord)
+{
+    constexpr uint32_t kInf = 0xFF800000u;
+    for (int i = threadIdx.x; i < c.n; i += blockDim.x) {
+        const float* row = c.corpus + (int64_t)i * c.ldc;
+        float dot = 0.f;
+        double wide = 0.0, norm = 0.0;
+        for (int d = 0; d < c.D; ++d) {
+            const float x = __ldg(row + d);
+            dot = __fmaf_rn(qv[d], x, dot);
+            wide = __fma_rn((double)qv[d], (double)x, wide);
+            norm = __fma_rn((double)x, (double)x, norm);
+        }
+        if (!c.fp32_keys) dot = __double2float_rn(wide);
+        const float key = __fmaf_rn(-2.0f, dot, __double2float_rn(norm));
+        ord[i] = (finite || c.fp32_keys) && key < __int_as_float(0x7f800000) ? f2ord(key) : kInf;
+    }
+}
+
+// The exact distances of cur[0..m) (a thread a row) over their keys.
+static __device__ __noinline__ void small_rerank(const SmallSelect& c, const float* qv, uint64_t* cur, int m)
+{
+    for (int j = threadIdx.x; j < m; j += blockDim.x) {
+        const uint32_t i = unpack_idx(cur[j]);
+        cur[j] = pack_key(exact_dist_row(qv, c.corpus + (int64_t)i * c.ldc, c.D), i);
+    }
+}
+
 template <int kT, bool kDirect>
-__global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
+__global__ void __launch_bounds__(kT) select_small_kernel(const __grid_constant__ SmallSelect c)
 {
     constexpr int kW = kT / 32;
     constexpr uint32_t kInf = 0xFF800000u;  // f2ord(+inf)
     extern __shared__ __align__(16) unsigned char smem[];
     const int n4 = (c.n + 3) & ~3;
-    uint64_t* cur = reinterpret_cast<uint64_t*>(smem);                             // [pow2_at_least(need)]
-    uint32_t* ord = reinterpret_cast<uint32_t*>(cur + pow2_at_least(c.need));      // [n4]
+    uint64_t* cur = reinterpret_cast<uint64_t*>(smem);                             // [pow2_at_least(need, kp)]
+    uint32_t* ord = reinterpret_cast<uint32_t*>(cur + pow2_at_least(max(c.need, c.kp)));  // [n4]
     float* qv = reinterpret_cast<float*>(ord + n4);                                // [D]
     __shared__ uint32_t hist[256];
     __shared__ uint32_t wlo[kW], whi[kW], wcnt[kW], digit_s, rank_s, hit_s, m_s;
+    __shared__ float qq_s;     // direct mode: ||q||^2, and whether q is finite
+    __shared__ bool finite_s;
     __shared__ __align__(16) uint64_t list[kSmallList];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t q = blockIdx.x;
@@ -995,9 +1035,61 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
     for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
     for (int b = tid; b < 256; b += kT) hist[b] = 0;
     if (tid == 0) m_s = 0;
-    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0, mine = 0;
+    // the extent of the words below +inf and their number: the thread's ...
+    auto extent = [&]() {
+        lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
+        for (int i = 4 * tid; i < n; i += 4 * kT) {
+            const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+            const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (o[e] < kInf) {
+                    lo = min(lo, o[e]);
+                    hi = max(hi, o[e]);
+                    ++cnt;
+                }
+        }
+    };
+    // ... and the block's (mine: the thread's smallest word, all ones when it has none)
+    auto join = [&]() {
+        mine = lo;
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane == 0) {
+            wlo[warp] = lo;
+            whi[warp] = hi;
+            wcnt[warp] = cnt;
+        }
+        __syncthreads();
+        cnt = 0;
+#pragma unroll
+        for (int w = 0; w < kW; ++w) {
+            lo = min(lo, wlo[w]);
+            hi = max(hi, whi[w]);
+            cnt += wcnt[w];
+        }
+    };
+    int need = c.need;
+    bool keyed = false;  // direct mode: ranked by keys after all
     if constexpr (kDirect) {
         __syncthreads();
+        if (warp == 0) {
+            float s = 0.f;
+            bool bad = false;
+            for (int d = lane; d < c.D; d += 32) {
+                s = __fmaf_rn(qv[d], qv[d], s);
+                bad |= !(fabsf(qv[d]) < __int_as_float(0x7f800000));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            bad = __any_sync(0xffffffffu, bad);
+            if (lane == 0) {
+                qq_s = s;
+                finite_s = !bad;
+            }
+        }
         constexpr int kR = 4;  // rows a lane has in flight
         const int u = lane & 7, g = lane >> 3, full = c.D >> 3;
         for (int r0 = 4 * kR * warp; r0 < n; r0 += kT / 8 * kR) {
@@ -1046,44 +1138,29 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
         }
         for (int i = n + tid; i < n4; i += kT) ord[i] = kInf;
         __syncthreads();
-        for (int i = 4 * tid; i < n; i += 4 * kT) {
-            const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
-            const uint32_t o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (o[e] < kInf) {
-                    lo = min(lo, o[e]);
-                    hi = max(hi, o[e]);
-                    ++cnt;
-                }
-        }
+        extent();
     } else {
         load_ordered<kT>(c.keys + q * c.ldk, n, ord, lo, hi, cnt);
     }
-    const uint32_t mine = lo;  // the thread's smallest word (all ones when none is finite)
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    if (lane == 0) {
-        wlo[warp] = lo;
-        whi[warp] = hi;
-        wcnt[warp] = cnt;
-    }
-    __syncthreads();
-    cnt = 0;
-#pragma unroll
-    for (int w = 0; w < kW; ++w) {
-        lo = min(lo, wlo[w]);
-        hi = max(hi, whi[w]);
-        cnt += wcnt[w];
+    join();
+    if constexpr (kDirect) {
+        if (cnt < (uint32_t)n || hi >= f2ord(kDirectMost) || !(qq_s < kDirectMost)) {
+            keyed = true;
+            need = min(c.kp, n);
+            __syncthreads();
+            small_keys(c, qv, finite_s, ord);
+            __syncthreads();
+            extent();
+            join();
+        }
     }
     // keep the words not above W, and of those equal to W + 1 (when ties > 0) the first `ties`
     uint32_t W = kInf - 1u, ties = 0;
-    int m = (int)min(cnt, (uint32_t)c.need);
+    int m = (int)min(cnt, (uint32_t)need);
     bool done = false;
     int top = 32 - __clz((int)(lo ^ hi));  // bits [0, top) differ
-    uint32_t x = top >= 32 ? 0u : (lo >> top) << top, rank = (uint32_t)c.need, hit = cnt;
-    if (cnt > (uint32_t)c.need && c.need <= kT / 2 && n >= 4 * kT) {
+    uint32_t x = top >= 32 ? 0u : (lo >> top) << top, rank = (uint32_t)need, hit = cnt;
+    if (cnt > (uint32_t)need && need <= kT / 2 && n >= 4 * kT) {
         // the need-th smallest thread minimum, or a bound on it at the end of a small bin
         int tp = top;
         uint32_t y = x, r = rank, h = kT;
@@ -1131,7 +1208,7 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
         }
         __syncthreads();
     }
-    if (!done && cnt > (uint32_t)c.need) {
+    if (!done && cnt > (uint32_t)need) {
         while (top > 0 && rank != hit) {
             const int sh = max(top - 8, 0);
             const uint32_t mask = top >= 32 ? 0u : ~((1u << top) - 1u);
@@ -1187,6 +1264,9 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const SmallSelect c)
     if constexpr (!kDirect) {
         rerank_block<kT>(cur, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
+    } else if (keyed) {
+        small_rerank(c, qv, cur, m);
+        __syncthreads();
     }
     emit_sorted<kT>(c, q, cur, m, false, 0.f);
 }
@@ -1205,9 +1285,9 @@ cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s)
 {
     if (c.Q <= 0) return cudaSuccess;
     if (c.n < 1 || c.n > kSmallRows || c.k < 1 || c.need < c.k || c.need > kMaxKpScan || c.D < 1 ||
-        (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)))
+        (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)) || (!c.keys && (c.kp < c.k || c.kp > kMaxKpScan)))
         return cudaErrorInvalidValue;
-    const size_t smem = (size_t)pow2_at_least(c.need) * 8 + (size_t)((c.n + 3) & ~3) * 4 + (size_t)((c.D + 3) & ~3) * 4;
+    const size_t smem = (size_t)pow2_at_least(std::max(c.need, c.kp)) * 8 + (size_t)((c.n + 3) & ~3) * 4 + (size_t)((c.D + 3) & ~3) * 4;
     if (c.keys) return c.Q <= kSelWideQ ? run_select_small<512, false>(c, smem, s) : run_select_small<256, false>(c, smem, s);
     return c.Q <= 152 ? run_select_small<1024, true>(c, smem, s) : run_select_small<256, true>(c, smem, s);
 }
