@@ -479,7 +479,8 @@ struct ScanPlan {
     int64_t dense_len = 0, ldk = 0;
     int sel_words = 0;  // bound on one query's stored main-pass candidates (selection buffer)
     FixGroups fix;  // fix-up of failed queries (their shortlists after one another in E.part)
-    bool simt_fix = false;  // the fix-up runs on the CUDA-core kernel (shortlist above kMaxKpTC)
+    bool simt_fix = false;  // the fix-up runs on the CUDA-core kernel (shortlist above kMaxKpTC), ...
+    int fix_qpb = 32;       // ... in tiles of so many queries
     size_t cand_words = 0, cnt_words = 0, part_words = 0, norm_words = 0;
 };
 
@@ -562,8 +563,11 @@ enum ScanKeys { kKeyBf16, kKeyF8, kKeyF16, kKeyTf32 };
 // selection over 512 segments 34 instead of 23).  Blocks that fill it already keep the one-wave plan.
 constexpr int kRowBlocks = 8;
 constexpr int kBlockSplits = 8;
+// certify: many queries may fail (CandSelect::certify), and their shortlists are at most kMaxKpTC long: the fix-up
+// runs as the CUDA-core kernel does for all of them, in tiles of 128 queries (2,600 queries of 12,000 x 130, every
+// one failing: 2,197 us a search with tiles of 32 and 8 splits, 1,863 so).
 static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, const knns_options& o, ScanPlan* P,
-                     ScanKeys keys, int blocks = 0)
+                     ScanKeys keys, int blocks = 0, bool certify = false)
 {
     if (o.scan_accs != 0 && o.scan_accs != 2 && o.scan_accs != 4)
         return set_error(KNNS_ERR_INVALID, "threshold scan: %d accumulators (2 or 4)", o.scan_accs);
@@ -682,7 +686,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     // (exact FP32 keys): the first 32 failed queries on a wave of splits, the rest on 8
     P->simt_fix = kp > kMaxKpTC || split;
     const int ft = P->simt_fix ? kSimtTileN : kTileN;
-    const int fq = P->simt_fix ? 32 : kTileQ;
+    const int fq = P->fix_qpb = certify ? 128 : P->simt_fix ? 32 : kTileQ;
     const int64_t tilesF = cdiv(N, ft);
     auto group = [&](int64_t rows, int64_t splits) {
         FixGroup g;
@@ -694,7 +698,7 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
     };
     const int64_t rowsA = std::min<int64_t>(Q, P->simt_fix ? fq : 4 * kTileQ);
     P->fix.g[0] = group(rowsA, E.sms / cdiv(rowsA, fq));
-    P->fix.g[1] = group(Q - rowsA, 8);
+    P->fix.g[1] = group(Q - rowsA, certify ? auto_splits(std::max<int64_t>(1, cdiv(Q - rowsA, fq)), tilesF, E.sms, 256) : 8);
     P->part_words = 0;
     for (const FixGroup& g : P->fix.g) P->part_words += (size_t)g.splits * g.rows * kp;
     return KNNS_OK;
@@ -941,6 +945,7 @@ struct TscanStages {
         cs.fail_idx = (int32_t*)fail.p + 1;
         cs.fail_cnt = fail_cnt;
         cs.fail_thr = (uint32_t*)thr2.p;
+        cs.certify = c.fp32;
         KNN_CUDA(launch_select_cand(cs, s));
         ++launches;
         return KNNS_OK;
@@ -952,7 +957,7 @@ struct TscanStages {
         const uint32_t* fail_cnt = (const uint32_t*)fail.p;
         const int32_t* fail_idx = (const int32_t*)fail.p + 1;
         const FixGroups fg = fix_groups(sp, (uint64_t*)E.part.p, c.kp);
-        KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, 32, 0, 0, nullptr, (uint32_t*)thr2.p, s,
+        KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, sp.fix_qpb, 0, 0, nullptr, (uint32_t*)thr2.p, s,
                              nullptr, fail_idx, fail_cnt, &fg));
         SelectExtra ex;
         ex.qmap = fail_idx;
@@ -1034,7 +1039,7 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
                      const knns_options& o, cudaStream_t s, knns_stats* st, const PreparedCorpus* pc, bool capture)
 {
     ScanPlan sp;
-    int rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp, c.tf32 ? kKeyTf32 : kKeyF16);
+    int rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp, c.tf32 ? kKeyTf32 : kKeyF16, 0, c.fp32);
     if (rc) return rc;
     if (pc && !pc->tf32)
         return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies of this width");

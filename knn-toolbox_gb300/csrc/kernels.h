@@ -326,7 +326,9 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
 
 // Small corpora, no thresholds: per query, the `need` smallest of n values and the k results.
 //  * keys given: a dense pass's keys (row q at keys + q * ldk); the `need` smallest (key, index) pairs
-//    are re-ranked by exact distance;
+//    are re-ranked by exact distance.  With fp32_keys (shapes whose keys are FP32 ones but for this path) a
+//    shortlist that may miss one of the k nearest, the split keys' errors considered, is replaced by every row
+//    that they do not rule out;
 //  * keys null: the exact distances themselves, computed by the kernel (need = k).  Where squares leave the
 //    float range: the kp smallest (key, index) pairs re-ranked as above, the keys in FP32 arithmetic, by the
 //    kernel too (of a query that is not finite: only with fp32_keys).
@@ -390,6 +392,7 @@ struct CandSelect {
     int32_t* fail_idx = nullptr;
     uint32_t* fail_cnt = nullptr;
     uint32_t* fail_thr = nullptr;  // all ones at every failed query's place (the fix-up's thresholds)
+    bool certify = false;          // a query also fails when its shortlist may miss a row (as SmallSelect::fp32_keys)
     // exact-key test (optional): keys and distances are exact integers when every corpus and
     // query value is an integer, 2 * D * max|x|^2 < 2^24 and the BF16 copies are exact; the
     // re-rank is then skipped (distance = key + qn[q], the same value it would compute)

@@ -509,10 +509,51 @@ __device__ __forceinline__ void find_bin(const uint32_t* hist, uint32_t rank, ui
     }
 }
 
+// Shortlists by split-FP16 keys where the shape's keys are FP32 ones otherwise (corpora below 16,384 rows, more than
+// 128 columns or entries): the split's products are coarser than FP32's, so such a shortlist counts only if no row
+// outside it can be nearer than its k-th (else: widen, or the CUDA-core fix-up).  split_key_error: what the key of a row
+// within C of the origin can err by against a query of squared norm qq, both as FP32 sums,
+//   2 |q| C (3 n + 4) 2^-22   products: n = D / 16 steps of three MMAs, two ulps of the accumulator a step (measured:
+//                             half an ulp, by truncation; 1,024 uniform columns 5.9e-6 |q| |c| in all against
+//                             4.7e-5 here); split residues
+//   (C^2 + |q| C) 2^-22       the norm's and the key's own roundings
+//   |q|^2 2^-17               ||q||^2 as summed here
+//   D 1e-44                   squares in the subnormal range
+// 10,000 x 300 uniform rows: 3e-3 in all, the 10th and 32nd neighbours 0.7 apart.
+__device__ __forceinline__ float split_key_error(float qq, float C, int D)
+{
+    const float R = sqrtf(qq);
+    return 2.f * R * C * (float)(3 * ((D + 15) / 16) + 4) * 0x1p-22f + (C * C + R * C) * 0x1p-22f + qq * 0x1p-17f +
+           (float)D * 1e-44f;
+}
+// relative error of a re-ranked distance
+__device__ __forceinline__ float dist_error(int D) { return (float)(D / 8 + 8) * 0x1p-24f; }
+
+// Lower bound on the re-ranked distance of rows whose keys are `key` or more: one at a squared distance below S = key +
+// ||q||^2 has |c| <= |q| + sqrt(S).  -inf when nothing is sure.
+__device__ __forceinline__ float outside_bound(float key, float qq, int D)
+{
+    const float S = key + qq;
+    const float b = (S - split_key_error(qq, sqrtf(qq) + sqrtf(fmaxf(S, 0.f)), D)) * (1.f - dist_error(D));
+    return b > 0.f ? b : -__int_as_float(0x7f800000);  // (NaN: -inf)
+}
+
+// Whether k of the re-ranked list's distances lie below the bound.
+template <int kT>
+__device__ __forceinline__ bool list_holds(const uint64_t* list, int m, int k, float bound)
+{
+    int n = 0;
+    for (int j0 = 0; j0 < m; j0 += kT) {
+        const int j = j0 + (int)threadIdx.x;
+        n += __syncthreads_count(j < m && unpack_key(list[j]) < bound);
+    }
+    return n >= k;
+}
+
 // kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.  Blocks an SM:
 // ten of 128 threads (47 registers; at 63 a million rows' 10,000 queries take 97 instead of 88 us), four
 // of 256 (for the re-rank's loads in flight: 256 queries, 32 rows of 1,024 columns 18.9 -> 15.5 us).
-template <int kT, bool kThr>
+template <int kT, bool kThr, bool kCertify = false>
 __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_kernel(const CandSelect c)
 {
     if (c.skip_if != nullptr && *c.skip_if != 0u) return;
@@ -681,9 +722,44 @@ __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_k
                 2.0 * (double)c.D * (double)mx * (double)mx < 16777216.0;
     }
     const bool rr = c.rerank && !exact;
+    float bound = 0.f;
+    if constexpr (kCertify) {
+        // the largest key of the shortlist, and ||q||^2
+        __shared__ uint32_t wkey[kW];
+        __shared__ float wqq[kW];
+        uint32_t key = 0;
+        float qq = 0.f;
+        for (int j = tid; j < m; j += kT) key = max(key, (uint32_t)(list[j] >> 32));
+        for (int d = tid; d < c.D; d += kT) qq = __fmaf_rn(qv[d], qv[d], qq);
+        key = __reduce_max_sync(0xffffffffu, key);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        if (lane == 0) {
+            wkey[warp] = key;
+            wqq[warp] = qq;
+        }
+        __syncthreads();
+        qq = 0.f;
+#pragma unroll
+        for (int w = 0; w < kW; ++w) {
+            key = max(key, wkey[w]);
+            qq += wqq[w];
+        }
+        bound = outside_bound(ord2f(key), qq, c.D);
+    }
     if (rr) {
         rerank_block<kT>(list, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
+    }
+    if constexpr (kCertify) {
+        if (!list_holds<kT>(list, m, c.k, bound)) {
+            if (tid == 0) {
+                const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
+                c.fail_idx[pos] = (int32_t)q;
+                c.fail_thr[pos] = 0xFFFFFFFFu;
+            }
+            return;
+        }
     }
     emit_sorted<kT>(c, q, list, m, !rr, rr ? 0.f : __ldg(c.qn + q));
 }
@@ -1001,7 +1077,7 @@ static __device__ __noinline__ void small_keys(const SmallSelect& c, const float
         }
         if (!c.fp32_keys) dot = __double2float_rn(wide);
         const float key = __fmaf_rn(-2.0f, dot, __double2float_rn(norm));
-        ord[i] = (finite || c.fp32_keys) && key < __int_as_float(0x7f800000) ? f2ord(key) : kInf;
+        ord[i] = (c.fp32_keys || finite) && key < __int_as_float(0x7f800000) ? f2ord(key) : kInf;
     }
 }
 
@@ -1014,66 +1090,295 @@ static __device__ __noinline__ void small_rerank(const SmallSelect& c, const flo
     }
 }
 
-template <int kT, bool kDirect>
-__global__ void __launch_bounds__(kT) select_small_kernel(const __grid_constant__ SmallSelect c)
+// A shortlist of split keys that is not certain to hold the k nearest (its re-ranked words cur[0..m), qq: ||q||^2):
+// the exact distances of every row that its key does not rule out, as words over the keys, +inf for the others.
+// A row at the k-th distance of the shortlist or nearer has |c| <= |q| + that distance, so its key lies below U.
+// Eight lanes a row, each warp 32 rows in turn.  False (nothing written) where squares may leave the float range.
+// (10,000 x 300, 500 queries, every column offset by 20: a tenth of the rows; by 80: all of them.)
+template <int kT>
+static __device__ __noinline__ bool widen(const SmallSelect& c, const float* qv, float qq, const uint64_t* cur, int m,
+                                          uint32_t* ord)
 {
-    constexpr int kW = kT / 32;
+    constexpr uint32_t kInf = 0xFF800000u;
+    constexpr int kB = 16;  // steps of eight columns in flight
+    __shared__ float kth_s;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, u = lane & 7, g = lane >> 3;
+    for (int j = threadIdx.x; j < m; j += kT) {
+        const uint64_t w = cur[j];
+        int below = 0;
+        for (int e = 0; e < m; ++e) below += cur[e] < w ? 1 : 0;
+        if (below == c.k - 1) kth_s = unpack_key(w);
+    }
+    __syncthreads();
+    const float kth = kth_s;
+    if (!(qq < kDirectMost) || !(kth < kDirectMost)) return false;
+    const float S = kth * (1.f + 2.f * dist_error(c.D)) + (float)c.D * 1e-44f;
+    const uint32_t U = f2ord(S - qq + split_key_error(qq, sqrtf(qq) + sqrtf(S), c.D));
+    for (int r0 = 32 * warp; r0 < c.n; r0 += kT) {
+        const uint32_t o = r0 + lane < c.n ? ord[r0 + lane] : kInf;
+        uint32_t todo = __ballot_sync(0xffffffffu, o <= U && o < kInf);
+        if (r0 + lane < c.n && !((todo >> lane) & 1u)) ord[r0 + lane] = kInf;
+        while (todo) {
+            uint32_t t = todo;
+            for (int i = 0; i < g; ++i) t &= t - 1u;
+            const bool in = t != 0u;
+            const int r = r0 + (in ? __ffs((int)t) - 1 : 0);
+            const float* row = c.corpus + (int64_t)r * c.ldc + u;
+            float p = 0.f;
+            for (int d0 = 0; d0 < c.D; d0 += 8 * kB) {
+                float v[kB];
+#pragma unroll
+                for (int i = 0; i < kB; ++i)
+                    if (in && d0 + 8 * i + u < c.D) v[i] = __ldg(row + d0 + 8 * i);
+#pragma unroll
+                for (int i = 0; i < kB; ++i)
+                    if (in && d0 + 8 * i + u < c.D) {
+                        const float x = __fsub_rn(qv[d0 + 8 * i + u], v[i]);
+                        p = __fmaf_rn(x, x, p);
+                    }
+            }
+            __syncwarp();
+            // ((p0 + p1) + (p2 + p3)) + ((p4 + p5) + (p6 + p7))
+            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 1));
+            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 2));
+            p = __fadd_rn(p, __shfl_xor_sync(0xffffffffu, p, 4));
+            if (u == 0 && in) ord[r] = p < __int_as_float(0x7f800000) ? f2ord(p) : kInf;
+            for (int i = 0; i < 4; ++i) todo &= todo - 1u;
+        }
+    }
+    return true;
+}
+
+// What the block shares while it picks words.
+template <int kT>
+struct SmallShared {
+    uint32_t hist[256];
+    uint32_t wlo[kT / 32], whi[kT / 32], wcnt[kT / 32], digit, rank, hit, m;
+    float wqq[kT / 32];
+    __align__(16) uint64_t list[kSmallList];
+    float qq;     // direct mode: ||q||^2 ...
+    bool finite;  // ... and whether q is finite
+};
+
+// The extent of the words below +inf and their number: a thread's ...
+struct WordExtent {
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0, mine = 0;  // mine: the thread's smallest, all ones when it has none
+};
+template <int kT>
+__device__ __forceinline__ WordExtent thread_extent(const uint32_t* ord, int n)
+{
+    constexpr uint32_t kInf = 0xFF800000u;
+    WordExtent x;
+    for (int i = 4 * (int)threadIdx.x; i < n; i += 4 * kT) {
+        const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+        const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (o[e] < kInf) {
+                x.lo = min(x.lo, o[e]);
+                x.hi = max(x.hi, o[e]);
+                ++x.cnt;
+            }
+    }
+    return x;
+}
+// ... and the block's (the words are visible to it afterwards).
+template <int kT>
+__device__ __forceinline__ void block_extent(SmallShared<kT>& S, WordExtent& x)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    x.mine = x.lo;
+    x.lo = __reduce_min_sync(0xffffffffu, x.lo);
+    x.hi = __reduce_max_sync(0xffffffffu, x.hi);
+    x.cnt = __reduce_add_sync(0xffffffffu, x.cnt);
+    if (lane == 0) {
+        S.wlo[warp] = x.lo;
+        S.whi[warp] = x.hi;
+        S.wcnt[warp] = x.cnt;
+    }
+    __syncthreads();
+    x.cnt = 0;
+#pragma unroll
+    for (int w = 0; w < kT / 32; ++w) {
+        x.lo = min(x.lo, S.wlo[w]);
+        x.hi = max(x.hi, S.whi[w]);
+        x.cnt += S.wcnt[w];
+    }
+}
+
+// The `need` smallest (word, index) pairs of ord[0..n) into cur, in no order; how many.  edge: no other word is smaller.
+// S.hist and S.m are zero before and (S.hist) after.
+template <int kT>
+__device__ __forceinline__ int pick_words(SmallShared<kT>& S, const uint32_t* ord, int n, int need, const WordExtent& xt,
+                                          uint64_t* cur, uint32_t& edge)
+{
+    constexpr uint32_t kInf = 0xFF800000u;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t lo = xt.lo, hi = xt.hi, cnt = xt.cnt, mine = xt.mine;
+    // keep the words not above W, and of those equal to W + 1 (when ties > 0) the first `ties`
+    uint32_t W = kInf - 1u, ties = 0;
+    edge = kInf;
+    const int m = (int)min(cnt, (uint32_t)need);
+    bool done = false;
+    int top = 32 - __clz((int)(lo ^ hi));  // bits [0, top) differ
+    uint32_t x = top >= 32 ? 0u : (lo >> top) << top, rank = (uint32_t)need, hit = cnt;
+    if (cnt > (uint32_t)need && need <= kT / 2 && n >= 4 * kT) {
+        // the need-th smallest thread minimum, or a bound on it at the end of a small bin
+        int tp = top;
+        uint32_t y = x, r = rank, h = kT;
+        while (tp > 0 && h - r > 8u) {
+            const int sh = max(tp - 8, 0);
+            const uint32_t mask = tp >= 32 ? 0u : ~((1u << tp) - 1u);
+            if (mine < kInf && (mine & mask) == y) atomicAdd(&S.hist[(mine >> sh) & ((1u << (tp - sh)) - 1u)], 1u);
+            __syncthreads();
+            if (tid == 0) S.hit = 0;
+            __syncthreads();
+            if (warp == 0) find_bin(S.hist, r, S.digit, S.rank, S.hit);
+            __syncthreads();
+            for (int b = tid; b < 256; b += kT) S.hist[b] = 0;
+            __syncthreads();
+            h = S.hit;
+            if (h == 0) break;  // fewer than need threads hold finite words
+            y |= S.digit << sh;
+            r = S.rank;
+            tp = sh;
+        }
+        if (h != 0) {
+            const uint32_t U = tp > 0 ? y | ((1u << tp) - 1u) : y;
+            if (mine <= U)
+                for (int i = 4 * tid; i < n; i += 4 * kT)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (ord[i + e] <= U) {
+                            const uint32_t pos = atomicAdd(&S.m, 1u);
+                            if (pos < kSmallList) S.list[pos] = ((uint64_t)ord[i + e] << 32) | (uint32_t)(i + e);
+                        }
+            __syncthreads();
+            const int found = (int)S.m;
+            if (found <= kSmallList) {
+                // words are distinct: a word's place is the number of smaller ones
+                for (int j = tid; j < found; j += kT) {
+                    const uint64_t w = S.list[j];
+                    int below = 0;
+                    for (int e = 0; e < found; ++e) below += S.list[e] < w ? 1 : 0;
+                    if (below < m) cur[below] = w;
+                }
+                done = true;
+            }
+            __syncthreads();
+            if (done) edge = (uint32_t)(cur[m - 1] >> 32);
+            if (tid == 0) S.m = 0;
+        }
+        __syncthreads();
+    }
+    if (!done && cnt > (uint32_t)need) {
+        while (top > 0 && rank != hit) {
+            const int sh = max(top - 8, 0);
+            const uint32_t mask = top >= 32 ? 0u : ~((1u << top) - 1u);
+            for (int i = 4 * tid; i < n; i += 4 * kT) {
+                const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
+                const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (o[e] < kInf && (o[e] & mask) == x) atomicAdd(&S.hist[(o[e] >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+            }
+            __syncthreads();
+            if (warp == 0) find_bin(S.hist, rank, S.digit, S.rank, S.hit);
+            __syncthreads();
+            x |= S.digit << sh;
+            rank = S.rank;
+            hit = S.hit;
+            top = sh;
+            for (int b = tid; b < 256; b += kT) S.hist[b] = 0;
+            __syncthreads();
+        }
+        if (rank == hit) {
+            W = top > 0 ? x | ((1u << top) - 1u) : x;
+        } else {  // more words equal to x than are wanted
+            W = x - 1u;
+            ties = rank;
+        }
+        edge = W + 1u;
+    }
+    for (int e0 = 0; !done && e0 < n; e0 += kT) {
+        const int e = e0 + tid;
+        const uint32_t o = e < n ? ord[e] : kInf;
+        const bool keep = o <= W && o < kInf;
+        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
+        uint32_t base = 0;
+        if (lane == 0 && bal) base = atomicAdd(&S.m, (uint32_t)__popc(bal));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (keep) cur[base + __popc(bal & ((1u << lane) - 1u))] = ((uint64_t)o << 32) | (uint32_t)e;
+    }
+    __syncthreads();
+    if (ties > 0 && warp == 0) {
+        uint32_t at = S.m, left = ties;
+        for (int e0 = 0; e0 < n && left > 0; e0 += 32) {
+            const int e = e0 + lane;
+            const bool tie = e < n && ord[e] == W + 1u;
+            const uint32_t bal = __ballot_sync(0xffffffffu, tie);
+            const uint32_t pos = (uint32_t)__popc(bal & ((1u << lane) - 1u));
+            if (tie && pos < left) cur[at + pos] = ((uint64_t)(W + 1u) << 32) | (uint32_t)e;
+            const uint32_t took = min(left, (uint32_t)__popc(bal));
+            at += took;
+            left -= took;
+        }
+    }
+    __syncthreads();
+    return m;
+}
+
+// A second way to the results, for queries that the first is not certain of: `ord` becomes the exact distances of
+// the rows that the shortlist cur[0..m) does not rule out (wide), or every row's FP32 key.
+template <int kT>
+static __device__ __noinline__ void pick_again(const SmallSelect& c, int64_t q, const float* qv, float qq, bool wide, int m,
+                                               uint64_t* cur, uint32_t* ord, SmallShared<kT>& S)
+{
+    wide = wide && widen<kT>(c, qv, qq, cur, m, ord);
+    if (!wide) {
+        __syncthreads();
+        small_keys(c, qv, S.finite, ord);
+    }
+    if (threadIdx.x == 0) S.m = 0;
+    __syncthreads();
+    WordExtent x = thread_extent<kT>(ord, c.n);
+    block_extent<kT>(S, x);
+    uint32_t edge;
+    m = pick_words<kT>(S, ord, c.n, wide ? c.k : min(max(c.need, c.kp), c.n), x, cur, edge);
+    if (!wide) {
+        small_rerank(c, qv, cur, m);
+        __syncthreads();
+    }
+    emit_sorted<kT>(c, q, cur, m, false, 0.f);
+}
+
+enum SmallMode { kSmallDense, kSmallCertified, kSmallDirect };
+template <int kT, int kMode>
+__global__ void __launch_bounds__(kT, kMode == kSmallCertified ? 1024 / kT : 0) select_small_kernel(const __grid_constant__ SmallSelect c)
+{
     constexpr uint32_t kInf = 0xFF800000u;  // f2ord(+inf)
     extern __shared__ __align__(16) unsigned char smem[];
     const int n4 = (c.n + 3) & ~3;
     uint64_t* cur = reinterpret_cast<uint64_t*>(smem);                             // [pow2_at_least(need, kp)]
     uint32_t* ord = reinterpret_cast<uint32_t*>(cur + pow2_at_least(max(c.need, c.kp)));  // [n4]
     float* qv = reinterpret_cast<float*>(ord + n4);                                // [D]
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t wlo[kW], whi[kW], wcnt[kW], digit_s, rank_s, hit_s, m_s;
-    __shared__ float qq_s;     // direct mode: ||q||^2, and whether q is finite
-    __shared__ bool finite_s;
-    __shared__ __align__(16) uint64_t list[kSmallList];
+    __shared__ SmallShared<kT> S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int64_t q = blockIdx.x;
     const int n = c.n;
-    for (int d = tid; d < c.D; d += kT) qv[d] = __ldg(c.queries + q * c.ldq + d);
-    for (int b = tid; b < 256; b += kT) hist[b] = 0;
-    if (tid == 0) m_s = 0;
-    uint32_t lo = 0xFFFFFFFFu, hi = 0u, cnt = 0, mine = 0;
-    // the extent of the words below +inf and their number: the thread's ...
-    auto extent = [&]() {
-        lo = 0xFFFFFFFFu, hi = 0u, cnt = 0;
-        for (int i = 4 * tid; i < n; i += 4 * kT) {
-            const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
-            const uint32_t o[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (o[e] < kInf) {
-                    lo = min(lo, o[e]);
-                    hi = max(hi, o[e]);
-                    ++cnt;
-                }
-        }
-    };
-    // ... and the block's (mine: the thread's smallest word, all ones when it has none)
-    auto join = [&]() {
-        mine = lo;
-        lo = __reduce_min_sync(0xffffffffu, lo);
-        hi = __reduce_max_sync(0xffffffffu, hi);
-        cnt = __reduce_add_sync(0xffffffffu, cnt);
-        if (lane == 0) {
-            wlo[warp] = lo;
-            whi[warp] = hi;
-            wcnt[warp] = cnt;
-        }
-        __syncthreads();
-        cnt = 0;
-#pragma unroll
-        for (int w = 0; w < kW; ++w) {
-            lo = min(lo, wlo[w]);
-            hi = max(hi, whi[w]);
-            cnt += wcnt[w];
-        }
-    };
-    int need = c.need;
-    bool keyed = false;  // direct mode: ranked by keys after all
-    if constexpr (kDirect) {
+    float qq = 0.f;  // the thread's share of ||q||^2, then all of it (certified mode)
+    for (int d = tid; d < c.D; d += kT) {
+        const float y = __ldg(c.queries + q * c.ldq + d);
+        qv[d] = y;
+        qq = __fmaf_rn(y, y, qq);
+    }
+    for (int b = tid; b < 256; b += kT) S.hist[b] = 0;
+    if (tid == 0) {
+        S.m = 0;
+        S.finite = true;
+    }
+    WordExtent x;
+    if constexpr (kMode == kSmallDirect) {
         __syncthreads();
         if (warp == 0) {
             float s = 0.f;
@@ -1086,8 +1391,8 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const __grid_constant_
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             bad = __any_sync(0xffffffffu, bad);
             if (lane == 0) {
-                qq_s = s;
-                finite_s = !bad;
+                S.qq = s;
+                S.finite = !bad;
             }
         }
         constexpr int kR = 4;  // rows a lane has in flight
@@ -1138,146 +1443,46 @@ __global__ void __launch_bounds__(kT) select_small_kernel(const __grid_constant_
         }
         for (int i = n + tid; i < n4; i += kT) ord[i] = kInf;
         __syncthreads();
-        extent();
+        x = thread_extent<kT>(ord, n);
     } else {
-        load_ordered<kT>(c.keys + q * c.ldk, n, ord, lo, hi, cnt);
+        load_ordered<kT>(c.keys + q * c.ldk, n, ord, x.lo, x.hi, x.cnt);
     }
-    join();
-    if constexpr (kDirect) {
-        if (cnt < (uint32_t)n || hi >= f2ord(kDirectMost) || !(qq_s < kDirectMost)) {
-            keyed = true;
-            need = min(c.kp, n);
-            __syncthreads();
-            small_keys(c, qv, finite_s, ord);
-            __syncthreads();
-            extent();
-            join();
-        }
-    }
-    // keep the words not above W, and of those equal to W + 1 (when ties > 0) the first `ties`
-    uint32_t W = kInf - 1u, ties = 0;
-    int m = (int)min(cnt, (uint32_t)need);
-    bool done = false;
-    int top = 32 - __clz((int)(lo ^ hi));  // bits [0, top) differ
-    uint32_t x = top >= 32 ? 0u : (lo >> top) << top, rank = (uint32_t)need, hit = cnt;
-    if (cnt > (uint32_t)need && need <= kT / 2 && n >= 4 * kT) {
-        // the need-th smallest thread minimum, or a bound on it at the end of a small bin
-        int tp = top;
-        uint32_t y = x, r = rank, h = kT;
-        while (tp > 0 && h - r > 8u) {
-            const int sh = max(tp - 8, 0);
-            const uint32_t mask = tp >= 32 ? 0u : ~((1u << tp) - 1u);
-            if (mine < kInf && (mine & mask) == y) atomicAdd(&hist[(mine >> sh) & ((1u << (tp - sh)) - 1u)], 1u);
-            __syncthreads();
-            if (tid == 0) hit_s = 0;
-            __syncthreads();
-            if (warp == 0) find_bin(hist, r, digit_s, rank_s, hit_s);
-            __syncthreads();
-            for (int b = tid; b < 256; b += kT) hist[b] = 0;
-            __syncthreads();
-            h = hit_s;
-            if (h == 0) break;  // fewer than need threads hold finite words
-            y |= digit_s << sh;
-            r = rank_s;
-            tp = sh;
-        }
-        if (h != 0) {
-            const uint32_t U = tp > 0 ? y | ((1u << tp) - 1u) : y;
-            if (mine <= U)
-                for (int i = 4 * tid; i < n; i += 4 * kT)
+    if constexpr (kMode == kSmallCertified) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (ord[i + e] <= U) {
-                            const uint32_t pos = atomicAdd(&m_s, 1u);
-                            if (pos < kSmallList) list[pos] = ((uint64_t)ord[i + e] << 32) | (uint32_t)(i + e);
-                        }
-            __syncthreads();
-            const int found = (int)m_s;
-            if (found <= kSmallList) {
-                // words are distinct: a word's place is the number of smaller ones
-                for (int j = tid; j < found; j += kT) {
-                    const uint64_t w = list[j];
-                    int below = 0;
-                    for (int e = 0; e < found; ++e) below += list[e] < w ? 1 : 0;
-                    if (below < m) cur[below] = w;
-                }
-                done = true;
-            }
-            __syncthreads();
-            if (tid == 0) m_s = 0;
-        }
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) qq += __shfl_xor_sync(0xffffffffu, qq, o);
+        if (lane == 0) S.wqq[warp] = qq;
     }
-    if (!done && cnt > (uint32_t)need) {
-        while (top > 0 && rank != hit) {
-            const int sh = max(top - 8, 0);
-            const uint32_t mask = top >= 32 ? 0u : ~((1u << top) - 1u);
-            for (int i = 4 * tid; i < n; i += 4 * kT) {
-                const uint4 v = *reinterpret_cast<const uint4*>(ord + i);
-                const uint32_t o[4] = {v.x, v.y, v.z, v.w};
+    block_extent<kT>(S, x);
+    if constexpr (kMode == kSmallDirect) {
+        if (x.cnt < (uint32_t)n || x.hi >= f2ord(kDirectMost) || !(S.qq < kDirectMost))
+            return pick_again<kT>(c, q, qv, 0.f, false, 0, cur, ord, S);
+    }
+    uint32_t edge;
+    const int m = pick_words<kT>(S, ord, n, c.need, x, cur, edge);
+    if constexpr (kMode == kSmallCertified) {
+        qq = 0.f;
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (o[e] < kInf && (o[e] & mask) == x) atomicAdd(&hist[(o[e] >> sh) & ((1u << (top - sh)) - 1u)], 1u);
-            }
-            __syncthreads();
-            if (warp == 0) find_bin(hist, rank, digit_s, rank_s, hit_s);
-            __syncthreads();
-            x |= digit_s << sh;
-            rank = rank_s;
-            hit = hit_s;
-            top = sh;
-            for (int b = tid; b < 256; b += kT) hist[b] = 0;
-            __syncthreads();
-        }
-        if (rank == hit) {
-            W = top > 0 ? x | ((1u << top) - 1u) : x;
-        } else {  // more words equal to x than are wanted
-            W = x - 1u;
-            ties = rank;
-        }
-    }
-    for (int e0 = 0; !done && e0 < n; e0 += kT) {
-        const int e = e0 + tid;
-        const uint32_t o = e < n ? ord[e] : kInf;
-        const bool keep = o <= W && o < kInf;
-        const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-        uint32_t base = 0;
-        if (lane == 0 && bal) base = atomicAdd(&m_s, (uint32_t)__popc(bal));
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (keep) cur[base + __popc(bal & ((1u << lane) - 1u))] = ((uint64_t)o << 32) | (uint32_t)e;
-    }
-    __syncthreads();
-    if (ties > 0 && warp == 0) {
-        uint32_t at = m_s, left = ties;
-        for (int e0 = 0; e0 < n && left > 0; e0 += 32) {
-            const int e = e0 + lane;
-            const bool tie = e < n && ord[e] == W + 1u;
-            const uint32_t bal = __ballot_sync(0xffffffffu, tie);
-            const uint32_t pos = (uint32_t)__popc(bal & ((1u << lane) - 1u));
-            if (tie && pos < left) cur[at + pos] = ((uint64_t)(W + 1u) << 32) | (uint32_t)e;
-            const uint32_t took = min(left, (uint32_t)__popc(bal));
-            at += took;
-            left -= took;
-        }
-    }
-    __syncthreads();
-    if constexpr (!kDirect) {
+        for (int w = 0; w < kT / 32; ++w) qq += S.wqq[w];
         rerank_block<kT>(cur, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
-    } else if (keyed) {
-        small_rerank(c, qv, cur, m);
+        // every row with a key, or k results that no other row can precede
+        const bool every = x.cnt <= (uint32_t)c.need;
+        if (!(every ? qq < __int_as_float(0x7f800000) : list_holds<kT>(cur, m, c.k, outside_bound(ord2f(edge), qq, c.D))))
+            return pick_again<kT>(c, q, qv, qq, !every, m, cur, ord, S);
+    } else if constexpr (kMode == kSmallDense) {
+        rerank_block<kT>(cur, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
     }
     emit_sorted<kT>(c, q, cur, m, false, 0.f);
 }
 
-template <int kT, bool kDirect>
+template <int kT, int kMode>
 static cudaError_t run_select_small(const SmallSelect& c, size_t smem, cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(select_small_kernel<kT, kDirect>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(select_small_kernel<kT, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    select_small_kernel<kT, kDirect><<<(unsigned)c.Q, kT, smem, s>>>(c);
+    select_small_kernel<kT, kMode><<<(unsigned)c.Q, kT, smem, s>>>(c);
     return cudaGetLastError();
 }
 
@@ -1288,8 +1493,13 @@ cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s)
         (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)) || (!c.keys && (c.kp < c.k || c.kp > kMaxKpScan)))
         return cudaErrorInvalidValue;
     const size_t smem = (size_t)pow2_at_least(std::max(c.need, c.kp)) * 8 + (size_t)((c.n + 3) & ~3) * 4 + (size_t)((c.D + 3) & ~3) * 4;
-    if (c.keys) return c.Q <= kSelWideQ ? run_select_small<512, false>(c, smem, s) : run_select_small<256, false>(c, smem, s);
-    return c.Q <= 152 ? run_select_small<1024, true>(c, smem, s) : run_select_small<256, true>(c, smem, s);
+    if (c.keys && c.fp32_keys)
+        return c.Q <= kSelWideQ ? run_select_small<512, kSmallCertified>(c, smem, s)
+                                : run_select_small<256, kSmallCertified>(c, smem, s);
+    if (c.keys)
+        return c.Q <= kSelWideQ ? run_select_small<512, kSmallDense>(c, smem, s)
+                                : run_select_small<256, kSmallDense>(c, smem, s);
+    return c.Q <= 152 ? run_select_small<1024, kSmallDirect>(c, smem, s) : run_select_small<256, kSmallDirect>(c, smem, s);
 }
 
 size_t select_smem_bytes(int kp, int D, int rerank)
@@ -1380,7 +1590,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
                                       : kCandMax;
     if (c.nseg < 1 || c.nseg > kScanMaxSegs || c.cap < 1 ||
         (!thr && (c.kp < 1 || c.kp > kMaxKpScan || c.k > c.kp || c.fail_idx == nullptr || c.fail_cnt == nullptr || c.fail_thr == nullptr ||
-                  (!c.rerank && c.qn == nullptr))) ||
+                  (!c.rerank && c.qn == nullptr) || (c.certify && (!c.rerank || c.int_stats != nullptr)))) ||
         (thr && (c.thr_rank < 1 || c.thr_rank > kCandThrMax)))
         return cudaErrorInvalidValue;
     if (thr && c.Q <= kThrBlockQ) {
@@ -1405,7 +1615,10 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512, before the re-rank took two rows at a time)
         const size_t smem = ((size_t)pow2_at_least(c.kp) + c.buf_words) * 8 + (size_t)((c.D + 3) & ~3) * 4;
         const int t = c.Q <= kSelFewQ ? 512 : c.Q <= kSelWideQ ? 256 : 128;
-        auto* kernel = t == 512   ? select_block_kernel<512, false>
+        auto* kernel = c.certify  ? (t == 512   ? select_block_kernel<512, false, true>
+                                     : t == 256 ? select_block_kernel<256, false, true>
+                                                : select_block_kernel<128, false, true>)
+                       : t == 512 ? select_block_kernel<512, false>
                        : t == 256 ? select_block_kernel<256, false>
                                   : select_block_kernel<128, false>;
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

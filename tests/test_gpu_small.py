@@ -96,3 +96,46 @@ def test_index_host_and_dropin_agree(engine, N, D, Q, k):
     with pytest.raises(engine.KnnsError):
         bare.search(q, k)
     bare.close()
+
+
+@pytest.mark.parametrize("N,Q,D,k", [(10000, 100, 300, 10), (12000, 2600, 130, 10), (8000, 100, 64, 200), (3000, 60, 1024, 5),
+                                     (16000, 40, 2048, 64), (5000, 40, 200, 493)])
+@pytest.mark.parametrize("offset", [0, 20, 80])
+def test_split_keys_are_no_further_off_than_fp32_keys(engine, N, Q, D, k, offset):
+    # wide rows and long shortlists: FP32 keys without the split-key paths.  A common offset costs the keys
+    # their low bits: a shortlist that is not certain to hold the neighbours is replaced by that of FP32 keys
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N + D)
+    c = torch.rand((N, D), generator=g, device="cuda") + offset
+    q = torch.rand((Q, D), generator=g, device="cuda") + offset
+    d, i, d0, i0, st = both(engine, c, q, k)
+    n = min(Q, 60)
+    ex = torch.stack([torch.topk(((x - c.double()) ** 2).sum(1), k, largest=False).values for x in q[:n].double()])
+    far, far0 = ((t[:n].double() / ex).max().item() for t in (d, d0))
+    assert far <= max(far0, 1 + DIST_REL)
+    if offset == 0:
+        # distances in FP32 and FP64 may order near-ties differently, nothing else
+        assert far < 1 + DIST_REL
+
+
+@pytest.mark.parametrize("N,Q,D,k", [(9000, 70, 200, 10), (5000, 3000, 600, 4), (4000, 400, 40, 150)])
+def test_ties_across_the_end_of_a_split_key_shortlist(engine, N, Q, D, k):
+    # equal distances inside and outside the shortlist: the lowest indices, as from FP32 keys
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c = torch.rand((N, D), generator=g, device="cuda")
+    c[N // 3:N // 3 + 700] = c[5]
+    q = torch.rand((Q, D), generator=g, device="cuda")
+    q[::7] = c[5]
+    d, i, d0, i0, st = both(engine, c, q, k)
+    assert torch.equal(i, i0) and torch.equal(d, d0)
+
+
+@pytest.mark.parametrize("N,Q,D", [(9000, 20, 200), (40, 20, 9000)])
+def test_infinite_queries_of_wide_rows(engine, N, Q, D):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c, q = torch.randn((N, D), generator=g, device="cuda"), torch.randn((Q, D), generator=g, device="cuda")
+    q[3, 1], q[4, 2], q[5, 0], q[6, 7] = float("inf"), float("-inf"), float("nan"), 3e38
+    d, i, d0, i0, st = both(engine, c, q, 9)
+    assert torch.equal(i, i0) and torch.equal(d, d0)
