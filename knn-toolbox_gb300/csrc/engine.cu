@@ -550,6 +550,33 @@ constexpr int64_t kSeedStrideFew = 256;
 // while a dense pass over 20M keys (10,000 x 1,954) costs 94 us, what its two levels did.
 constexpr int64_t kDenseKeys = 24 << 20;
 
+// Fix-up of failed queries: up to 512 on a full wave, the rest (rare) on 8 splits; shortlists above the
+// tensor-core kernel's kMaxKpTC, and the split-key scan's, go to the CUDA-core kernel (exact FP32 keys) in tiles of
+// qpb queries: the first tile on a wave of splits, the rest on 8.  Where all may fail together (certified
+// shortlists), the rest get the splits of a search of their own (2,600 queries of 12,000 x 130, every one failing:
+// 2,197 us a search with tiles of 32 and 8 splits, 1,863 with tiles of 128 and these).  Returns the words of the
+// groups' shortlists.
+static size_t plan_fix(const Engine& E, int64_t N, int64_t Q, int kp, int qpb, bool many, FixGroups* f)
+{
+    const int ft = qpb > 0 ? kSimtTileN : kTileN;
+    const int fq = qpb > 0 ? qpb : kTileQ;
+    const int64_t tiles = cdiv(N, ft);
+    auto group = [&](int64_t rows, int64_t splits) {
+        FixGroup g;
+        g.rows = rows;
+        g.tiles = (int)cdiv(rows, fq);
+        g.split_len = cdiv(tiles, std::max<int64_t>(1, std::min(tiles, splits))) * ft;
+        g.splits = (int)cdiv(N, g.split_len);
+        return g;
+    };
+    const int64_t rowsA = std::min<int64_t>(Q, qpb > 0 ? fq : 4 * kTileQ), rest = Q - rowsA;
+    f->g[0] = group(rowsA, E.sms / cdiv(rowsA, fq));
+    f->g[1] = group(rest, many && rest > 0 ? auto_splits(cdiv(rest, fq), tiles, E.sms, 64) : 8);
+    size_t words = 0;
+    for (const FixGroup& g : f->g) words += (size_t)g.splits * g.rows * kp;
+    return words;
+}
+
 // keys kKeyF16 / kKeyTf32: the plan of the scan on split keys (fix-up on the CUDA-core kernel; dpb
 // only decides its tile: the row width rounded up to 64); otherwise of the BF16 / E4M3 scan of row
 // width dpb.
@@ -563,9 +590,7 @@ enum ScanKeys { kKeyBf16, kKeyF8, kKeyF16, kKeyTf32 };
 // selection over 512 segments 34 instead of 23).  Blocks that fill it already keep the one-wave plan.
 constexpr int kRowBlocks = 8;
 constexpr int kBlockSplits = 8;
-// certify: many queries may fail (CandSelect::certify), and their shortlists are at most kMaxKpTC long: the fix-up
-// runs as the CUDA-core kernel does for all of them, in tiles of 128 queries (2,600 queries of 12,000 x 130, every
-// one failing: 2,197 us a search with tiles of 32 and 8 splits, 1,863 so).
+// certify: the queries' shortlists are checked (CandSelect::certify).
 static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, const knns_options& o, ScanPlan* P,
                      ScanKeys keys, int blocks = 0, bool certify = false)
 {
@@ -681,26 +706,9 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
                                                   cand_max > kCandMax ? kCandSigmasFew : kCandSigmas) / 32.0) * 32.0);
     P->cand_words = std::max(P->cand_words, (size_t)kScanParts * P->S * Q * P->cap);
     P->cnt_words = std::max(P->cnt_words, (size_t)kScanParts * P->S * Q);
-    // fix-up of failed queries: up to 512 on a full wave, the rest (rare) on 8 splits; shortlists
-    // above the tensor-core kernel's kMaxKpTC go to the CUDA-core kernel in tiles of 32 queries
-    // (exact FP32 keys): the first 32 failed queries on a wave of splits, the rest on 8
     P->simt_fix = kp > kMaxKpTC || split;
-    const int ft = P->simt_fix ? kSimtTileN : kTileN;
-    const int fq = P->fix_qpb = certify ? 128 : P->simt_fix ? 32 : kTileQ;
-    const int64_t tilesF = cdiv(N, ft);
-    auto group = [&](int64_t rows, int64_t splits) {
-        FixGroup g;
-        g.rows = rows;
-        g.tiles = (int)cdiv(rows, fq);
-        g.split_len = cdiv(tilesF, std::max<int64_t>(1, std::min(tilesF, splits))) * ft;
-        g.splits = (int)cdiv(N, g.split_len);
-        return g;
-    };
-    const int64_t rowsA = std::min<int64_t>(Q, P->simt_fix ? fq : 4 * kTileQ);
-    P->fix.g[0] = group(rowsA, E.sms / cdiv(rowsA, fq));
-    P->fix.g[1] = group(Q - rowsA, certify ? auto_splits(std::max<int64_t>(1, cdiv(Q - rowsA, fq)), tilesF, E.sms, 256) : 8);
-    P->part_words = 0;
-    for (const FixGroup& g : P->fix.g) P->part_words += (size_t)g.splits * g.rows * kp;
+    P->fix_qpb = certify ? 128 : 32;
+    P->part_words = plan_fix(E, N, Q, kp, P->simt_fix ? P->fix_qpb : 0, certify, &P->fix);
     return KNNS_OK;
 }
 
@@ -714,9 +722,8 @@ static int plan_scan(const Engine& E, int64_t N, int64_t Q, int dpb, int kp, con
 // device-side choice between BF16 and split keys); its failed-query list is its own (fail), so
 // the other path's fix-up never sees it.
 // the plan's fix-up groups with their shortlists in `part`
-static FixGroups fix_groups(const ScanPlan& sp, uint64_t* part, int kp)
+static FixGroups fix_groups(FixGroups fg, uint64_t* part, int kp)
 {
-    FixGroups fg = sp.fix;
     fg.g[0].part = part;
     fg.g[1].part = part + (size_t)fg.g[0].splits * fg.g[0].rows * kp;
     return fg;
@@ -956,7 +963,7 @@ struct TscanStages {
     {
         const uint32_t* fail_cnt = (const uint32_t*)fail.p;
         const int32_t* fail_idx = (const int32_t*)fail.p + 1;
-        const FixGroups fg = fix_groups(sp, (uint64_t*)E.part.p, c.kp);
+        const FixGroups fg = fix_groups(sp.fix, (uint64_t*)E.part.p, c.kp);
         KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, sp.fix_qpb, 0, 0, nullptr, (uint32_t*)thr2.p, s,
                              nullptr, fail_idx, fail_cnt, &fg));
         SelectExtra ex;
@@ -1090,6 +1097,12 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     return KNNS_OK;
 }
 
+// Certified shortlists of corpora of kFixWork values and more: a query that most rows remain possible for goes to the
+// CUDA-core kernel, whose tiles share the corpus, instead of reading all of it (1,400 queries of 16,000 x 2,048, every
+// column offset by 20: 38 ms read so, 11.5 there).  Its two launches cost 6 us where none fails, which smaller
+// searches would notice (10,000 x 300, 500 queries: 91 us, 1.4 ms with every row read, 0.7 by FP32 keys).
+constexpr int64_t kFixWork = 8 << 20;
+
 // Searches of small corpora (Config::small).
 static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N, int64_t ldc, const float* queries,
                      int64_t Q, int64_t ldq, int D, int k, float* dist, int32_t* idx, float* idx_f,
@@ -1103,6 +1116,18 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
     const int64_t chunk = std::max<int64_t>(1, kSmallKeys / N / kTileQ) * kTileQ;
     size_t ws = 0, nwords = 0;
     int rc = KNNS_OK, launches = 1;
+    const bool with_fix = dense && c.fp32 && N * D >= kFixWork;
+    const int fix_qpb = c.kp <= kMaxKpTC ? 128 : 32;
+    FixGroups fix;
+    if (with_fix) {
+        const int64_t rows = std::min(Q, chunk);
+        rc = E.part.ensure(plan_fix(E, N, rows, c.kp, fix_qpb, true, &fix) * sizeof(uint64_t));
+        if (!rc) rc = E.fail.ensure(rows * sizeof(int32_t));
+        if (!rc) rc = E.thr2.ensure(rows * sizeof(uint32_t));
+        if (rc) return rc;
+        fix = fix_groups(fix, (uint64_t*)E.part.p, c.kp);
+        ws = E.part.cap + E.fail.cap + E.thr2.cap;
+    }
     if (dense) {
         if (!pc) {
             rc = E.cn.ensure(n_pad * sizeof(float));
@@ -1114,7 +1139,7 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         if (!rc) rc = E.qrs.ensure(Q * sizeof(float));
         if (!rc) rc = E.cand.ensure((size_t)std::min(Q, chunk) * ldk * sizeof(float));
         if (rc) return rc;
-        ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qhi.cap + E.qlo.cap + E.qrs.cap +
+        ws += (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qhi.cap + E.qlo.cap + E.qrs.cap +
              E.cand.cap;
     }
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
@@ -1175,6 +1200,11 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         sel.keys = f.keys;
         sel.ldk = ldk;
         sel.need = (int)std::min<int64_t>(c.kp, N);
+        if (with_fix) {
+            sel.fail_idx = (int32_t*)E.fail.p;
+            sel.fail_cnt = words + 6;
+            sel.fail_thr = (uint32_t*)E.thr2.p;
+        }
         for (int64_t q0 = 0; q0 < Q; q0 += chunk) {
             const int64_t nq = std::min(chunk, Q - q0);
             if (q0 > 0 && D > kFscanTmemD) {
@@ -1195,8 +1225,20 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
             sel.out_dist = dist ? dist + q0 * k : nullptr;
             sel.out_idx = idx ? idx + q0 * k : nullptr;
             sel.out_idx_f = idx_f ? idx_f + q0 * k : nullptr;
+            if (with_fix && q0 > 0) KNN_CUDA(cudaMemsetAsync(sel.fail_cnt, 0, sizeof(uint32_t), s));
             KNN_CUDA(launch_select_small(sel, s));
             launches += 2;
+            if (with_fix) {
+                KNN_CUDA(launch_simt(corpus, N, ldc, f.cn, sel.queries, nq, ldq, D, c.kp, fix_qpb, 0, 0, nullptr,
+                                     sel.fail_thr, s, nullptr, sel.fail_idx, sel.fail_cnt, &fix));
+                SelectExtra ex;
+                ex.qmap = sel.fail_idx;
+                ex.qcount = sel.fail_cnt;
+                ex.fix = fix;
+                KNN_CUDA(launch_select(nullptr, 0, nq, c.kp, k, corpus, ldc, sel.queries, ldq, D, 1, nullptr,
+                                       sel.out_dist, sel.out_idx, sel.out_idx_f, s, ex));
+                launches += 2;
+            }
         }
         if ((rc = mark(3))) return rc;
     } else {
@@ -1907,7 +1949,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         // fix-up: failed queries, compacted, through the shortlist kernel without a threshold (long
         // shortlists: the CUDA-core kernel with exact FP32 keys); blocks whose rows are past the
         // failure count return at once
-        const FixGroups fg = fix_groups(sp, part, c.kp);
+        const FixGroups fg = fix_groups(sp.fix, part, c.kp);
         if (sp.simt_fix) {
             KNN_CUDA(launch_simt(corpus, N, ldc, cn, queries, Q, ldq, D, c.kp, 32, 0, 0, nullptr, (uint32_t*)E.thr2.p, s,
                                  nullptr, fail_idx, fail_cnt, &fg));

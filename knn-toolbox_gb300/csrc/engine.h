@@ -74,7 +74,7 @@ struct Engine {
     DevBuf done;
     // per-search flag words: [0] some corpus tile has a low part, [1] corpus or
     // queries not BF16-exact, [2] some value not an integer, [3] max |x| (float bits), [4] zero,
-    // [5] some query tile has a low part
+    // [5] some query tile has a low part, [6] failed queries of a small corpus;
     // then the low-part flags of the query tiles (qlof) and of the search's own corpus tiles (lof)
     DevBuf words;
     uint32_t* qlof = nullptr;

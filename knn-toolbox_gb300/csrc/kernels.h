@@ -328,7 +328,8 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
 //  * keys given: a dense pass's keys (row q at keys + q * ldk); the `need` smallest (key, index) pairs
 //    are re-ranked by exact distance.  With fp32_keys (shapes whose keys are FP32 ones but for this path) a
 //    shortlist that may miss one of the k nearest, the split keys' errors considered, is replaced by every row
-//    that they do not rule out;
+//    that they do not rule out -- or, where fail_idx is given and those are most rows, the query gets no result but
+//    a place there (count in *fail_cnt; fail_thr as CandSelect);
 //  * keys null: the exact distances themselves, computed by the kernel (need = k).  Where squares leave the
 //    float range: the kp smallest (key, index) pairs re-ranked as above, the keys in FP32 arithmetic, by the
 //    kernel too (of a query that is not finite: only with fp32_keys).
@@ -339,6 +340,9 @@ struct SmallSelect {
     int64_t ldk = 0;
     int n = 0, need = 0, k = 0, kp = 0;
     bool fp32_keys = false;
+    int32_t* fail_idx = nullptr;
+    uint32_t* fail_cnt = nullptr;
+    uint32_t* fail_thr = nullptr;
     int64_t Q = 0;
     const float* corpus = nullptr;
     int64_t ldc = 0;

@@ -1093,11 +1093,13 @@ static __device__ __noinline__ void small_rerank(const SmallSelect& c, const flo
 // A shortlist of split keys that is not certain to hold the k nearest (its re-ranked words cur[0..m), qq: ||q||^2):
 // the exact distances of every row that its key does not rule out, as words over the keys, +inf for the others.
 // A row at the k-th distance of the shortlist or nearer has |c| <= |q| + that distance, so its key lies below U.
-// Eight lanes a row, each warp 32 rows in turn.  False (nothing written) where squares may leave the float range.
-// (10,000 x 300, 500 queries, every column offset by 20: a tenth of the rows; by 80: all of them.)
+// Eight lanes a row, each warp 32 rows in turn (10,000 x 300, 500 queries, every column offset by 20, which leaves a
+// tenth of the rows: 245 us a search; by 80, which leaves all, 1,364.  Two rows a group, eight steps each: 253 and
+// 1,201, but 1,549 instead of 1,273 for 1,400 queries of 16,000 x 2,048 that few rows remain possible for).  False,
+// and nothing written, where squares may leave the float range or (give_up) a quarter of the rows and more remain.
 template <int kT>
 static __device__ __noinline__ bool widen(const SmallSelect& c, const float* qv, float qq, const uint64_t* cur, int m,
-                                          uint32_t* ord)
+                                          bool give_up, uint32_t* ord)
 {
     constexpr uint32_t kInf = 0xFF800000u;
     constexpr int kB = 16;  // steps of eight columns in flight
@@ -1114,12 +1116,20 @@ static __device__ __noinline__ bool widen(const SmallSelect& c, const float* qv,
     if (!(qq < kDirectMost) || !(kth < kDirectMost)) return false;
     const float S = kth * (1.f + 2.f * dist_error(c.D)) + (float)c.D * 1e-44f;
     const uint32_t U = f2ord(S - qq + split_key_error(qq, sqrtf(qq) + sqrtf(S), c.D));
+    if (give_up) {
+        int rows = 0;
+        for (int r0 = 0; r0 < c.n; r0 += kT) {
+            const int r = r0 + (int)threadIdx.x;
+            rows += __syncthreads_count(r < c.n && ord[r] <= U && ord[r] < kInf);
+        }
+        if (rows >= c.n / 4) return false;
+    }
     for (int r0 = 32 * warp; r0 < c.n; r0 += kT) {
         const uint32_t o = r0 + lane < c.n ? ord[r0 + lane] : kInf;
         uint32_t todo = __ballot_sync(0xffffffffu, o <= U && o < kInf);
         if (r0 + lane < c.n && !((todo >> lane) & 1u)) ord[r0 + lane] = kInf;
         while (todo) {
-            uint32_t t = todo;
+            uint32_t t = todo;  // the group takes the g-th row left
             for (int i = 0; i < g; ++i) t &= t - 1u;
             const bool in = t != 0u;
             const int r = r0 + (in ? __ffs((int)t) - 1 : 0);
@@ -1334,7 +1344,15 @@ template <int kT>
 static __device__ __noinline__ void pick_again(const SmallSelect& c, int64_t q, const float* qv, float qq, bool wide, int m,
                                                uint64_t* cur, uint32_t* ord, SmallShared<kT>& S)
 {
-    wide = wide && widen<kT>(c, qv, qq, cur, m, ord);
+    wide = wide && widen<kT>(c, qv, qq, cur, m, c.fail_idx != nullptr, ord);
+    if (!wide && c.fail_idx != nullptr) {
+        if (threadIdx.x == 0) {
+            const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
+            c.fail_idx[pos] = (int32_t)q;
+            c.fail_thr[pos] = 0xFFFFFFFFu;
+        }
+        return;
+    }
     if (!wide) {
         __syncthreads();
         small_keys(c, qv, S.finite, ord);
@@ -1490,7 +1508,8 @@ cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s)
 {
     if (c.Q <= 0) return cudaSuccess;
     if (c.n < 1 || c.n > kSmallRows || c.k < 1 || c.need < c.k || c.need > kMaxKpScan || c.D < 1 ||
-        (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)) || (!c.keys && (c.kp < c.k || c.kp > kMaxKpScan)))
+        (c.keys && (c.ldk % 4 != 0 || c.ldk < c.n)) || (!c.keys && (c.kp < c.k || c.kp > kMaxKpScan)) ||
+        (c.fail_idx && (!c.keys || !c.fp32_keys || !c.fail_cnt || !c.fail_thr)))
         return cudaErrorInvalidValue;
     const size_t smem = (size_t)pow2_at_least(std::max(c.need, c.kp)) * 8 + (size_t)((c.n + 3) & ~3) * 4 + (size_t)((c.D + 3) & ~3) * 4;
     if (c.keys && c.fp32_keys)

@@ -99,7 +99,7 @@ def test_index_host_and_dropin_agree(engine, N, D, Q, k):
 
 
 @pytest.mark.parametrize("N,Q,D,k", [(10000, 100, 300, 10), (12000, 2600, 130, 10), (8000, 100, 64, 200), (3000, 60, 1024, 5),
-                                     (16000, 40, 2048, 64), (5000, 40, 200, 493)])
+                                     (16000, 40, 2048, 64), (5000, 40, 200, 493), (16000, 600, 530, 300)])
 @pytest.mark.parametrize("offset", [0, 20, 80])
 def test_split_keys_are_no_further_off_than_fp32_keys(engine, N, Q, D, k, offset):
     # wide rows and long shortlists: FP32 keys without the split-key paths.  A common offset costs the keys
@@ -131,7 +131,7 @@ def test_ties_across_the_end_of_a_split_key_shortlist(engine, N, Q, D, k):
     assert torch.equal(i, i0) and torch.equal(d, d0)
 
 
-@pytest.mark.parametrize("N,Q,D", [(9000, 20, 200), (40, 20, 9000)])
+@pytest.mark.parametrize("N,Q,D", [(9000, 20, 200), (40, 20, 9000), (9000, 300, 1000)])
 def test_infinite_queries_of_wide_rows(engine, N, Q, D):
     import torch
     g = torch.Generator(device="cuda").manual_seed(N)
