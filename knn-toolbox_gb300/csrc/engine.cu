@@ -1276,9 +1276,10 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     const uint64_t stall_ns = capture ? 0 : g_test_stall_ns.exchange(0);
     if (host_corpus != nullptr && (pc != nullptr || capture || ldc != D))
         return set_error(KNNS_ERR_INVALID, "a corpus streamed from the host needs pitch D and no prepared index");
-    // an index without the exact form's copies is refused below, as ever; the stall hook is the shortlist
-    // kernel's
-    if (c.small && ((pc && !pc->f16) || stall_ns)) {
+    // (what a small corpus's own paths -- these, or the threshold scan below its usual size -- cannot serve takes the
+    // route it has without them: an index without the exact form's copies, refused below or searched on the CUDA
+    // cores; the stall hook, which is the shortlist kernel's)
+    if ((c.small || (c.tscan && N < kScanMinRowsForced)) && ((pc && !pc->f16) || stall_ns)) {
         if ((rc = resolve_keys(E, N, Q, D, k, o, &(c = Config())))) return rc;
     }
     if (c.tscan || c.small) {

@@ -139,3 +139,20 @@ def test_infinite_queries_of_wide_rows(engine, N, Q, D):
     q[3, 1], q[4, 2], q[5, 0], q[6, 7] = float("inf"), float("-inf"), float("nan"), 3e38
     d, i, d0, i0, st = both(engine, c, q, 9)
     assert torch.equal(i, i0) and torch.equal(d, d0)
+
+
+@pytest.mark.parametrize("N,Q,D", [(9000, 3000, 200), (9000, 30, 200), (3000, 9, 20)])
+def test_index_without_copies(engine, N, Q, D):
+    # wide rows are searched on the CUDA cores, which need no copies; others are refused
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N + Q)
+    c, q = torch.rand((N, D), generator=g, device="cuda"), torch.rand((Q, D), generator=g, device="cuda")
+    ix = engine.Index(c, tf32=False)
+    if D > 128:
+        d, i = ix.search(q, 10)
+        d0, i0 = engine.search(c, q, 10, pilot=False)
+        assert torch.equal(i, i0) and torch.equal(d, d0)
+    else:
+        with pytest.raises(engine.KnnsError):
+            ix.search(q, 10)
+    ix.close()
