@@ -1050,7 +1050,6 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     if (rc) return rc;
     if (pc && !pc->tf32)
         return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies of this width");
-    if (pc && c.tf32 && (rc = prepare_tf32(pc, s, capture))) return rc;
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     if (!pc) {
         rc = E.cn.ensure(n_pad * sizeof(float));
@@ -1282,6 +1281,8 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     if ((c.small || (c.tscan && N < kScanMinRowsForced)) && ((pc && !pc->f16) || stall_ns)) {
         if ((rc = resolve_keys(E, N, Q, D, k, o, &(c = Config())))) return rc;
     }
+    // an index without room for FP16 copies: 3xTF32 keys
+    if (pc && pc->tf32 && !pc->f16) c.tf32 = true;
     if (c.tscan || c.small) {
         if (host_corpus != nullptr) {
             // the whole corpus lands before the search starts (no overlap on this path)
@@ -1336,7 +1337,6 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
         if (f8 && !pc->fp8) return set_error(KNNS_ERR_INVALID, "the FP8 form needs an index prepared with E4M3 copies");
         if (c.algo == KNNS_ALGO_TC && !bf16_only && !pc->tf32)
             return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies");
-        if (c.algo == KNNS_ALGO_TC && !bf16_only && c.tf32 && (rc = prepare_tf32(pc, s, capture))) return rc;
     }
 
     // norms padded with +inf at least one tile (of any kernel) past the corpus
@@ -2021,23 +2021,35 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     if (!pc || !corpus || N <= 0 || D <= 0 || ldc < D) return set_error(KNNS_ERR_INVALID, "invalid corpus");
     if (N > 0x7fffffffLL) return set_error(KNNS_ERR_UNSUPPORTED, "corpus larger than 2^31-1 rows");
     if (E.cc < 100) return set_error(KNNS_ERR_UNSUPPORTED, "a prepared corpus needs sm_100+");
-    const int dpb = (D + 63) & ~63;
+    const int dpb = (D + 63) & ~63, dp = round32(D);
     if (dpb > 256) return set_error(KNNS_ERR_UNSUPPORTED, "a prepared corpus needs D <= 256");
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     int rc = pc->cn.ensure(n_pad * sizeof(float));
     if (!rc) rc = pc->bf.ensure((size_t)N * dpb * 2);
     if (!rc) rc = pc->words.ensure(8 * sizeof(uint32_t));
     if (!rc) rc = pc->tiles.ensure(((size_t)cdiv(N, 128) + 1) * sizeof(uint32_t));
-    // FP16 hi / lo; the TF32 copies come with the first search that needs 3xTF32 keys (prepare_tf32)
-    const bool f16 = tf32;
-    if (!rc && f16) rc = pc->hi.ensure((size_t)N * split_pitch(D) * 2);
-    if (!rc && f16) rc = pc->lo.ensure((size_t)N * split_pitch(D) * 2);
-    if (!rc && f16) rc = pc->rs.ensure(n_pad * sizeof(float));
+    // the exact form's copies: TF32 hi / lo, for shortlists without a margin, distances read off the keys and the
+    // shortlist kernel
+    if (!rc && tf32) rc = pc->thi.ensure((size_t)N * dp * sizeof(float));
+    if (!rc && tf32) rc = pc->tlo.ensure((size_t)N * dp * sizeof(float));
+    if (!rc && tf32) rc = pc->ttiles.ensure(((size_t)cdiv(N, kTileRows) + 1) * sizeof(uint32_t));
     const int dpf = ((D + 127) & ~127) / 2;
     if (!rc && fp8) rc = pc->f8.ensure((size_t)N * dpf * 2);
     if (!rc && fp8) rc = pc->cs.ensure(n_pad * sizeof(float));
     if (!rc) rc = pc->np.ensure((size_t)N * kNormParts * 2);
     if (rc) return rc;
+    // ... and FP16 hi / lo with row scales, keys at twice the rate where the shortlist has a margin: made while
+    // as much memory again and 2 GB stay free, else such searches take the TF32 copies too
+    const size_t half = (size_t)N * split_pitch(D) * 2;
+    size_t fr = 0, tot = 0;
+    bool f16 = tf32 && cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr >= 4 * half + ((size_t)2 << 30);
+    if (f16 && (pc->hi.ensure(half) || pc->lo.ensure(half) || pc->rs.ensure(n_pad * sizeof(float)))) {
+        f16 = false;
+        pc->hi.release();
+        pc->lo.release();
+        pc->rs.release();
+        clear_error();
+    }
     uint32_t* w = (uint32_t*)pc->words.p;
     KNN_CUDA(cudaMemsetAsync(w, 0, 8 * sizeof(uint32_t), s));
     PrepJob j = prep_job(corpus, N, ldc, D, (float*)pc->cn.p, n_pad);
@@ -2057,9 +2069,11 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
         j.lo = pc->lo.p;
         j.rs = (float*)pc->rs.p;
         j.lo_flags = (uint32_t*)pc->tiles.p;
-        j.any_lo = w;
     }
     KNN_CUDA(launch_prep(j, s));
+    if (tf32)
+        KNN_CUDA(launch_split_tf32(corpus, N, ldc, D, dp, (float*)pc->thi.p, (float*)pc->tlo.p, (uint32_t*)pc->ttiles.p, w,
+                                   nullptr, s));
     pc->corpus = corpus;
     pc->N = N;
     pc->ldc = ldc;
@@ -2069,25 +2083,6 @@ int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N
     pc->fp8 = fp8;
     pc->tf32 = tf32;
     pc->f16 = f16;
-    return KNNS_OK;
-}
-
-int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture)
-{
-    std::lock_guard<std::mutex> lk(pc->tmu);
-    if (pc->thi_ready) return KNNS_OK;
-    if (capture) return set_error(KNNS_ERR_INVALID, "the index's TF32 copies have to exist before a capture");
-    const int dp = round32(pc->D);
-    const size_t b = (size_t)pc->N * dp * sizeof(float);
-    int rc = pc->thi.ensure(b);
-    if (!rc) rc = pc->tlo.ensure(b);
-    if (!rc) rc = pc->ttiles.ensure(((size_t)cdiv(pc->N, kTileRows) + 1) * sizeof(uint32_t));
-    if (rc) return rc;
-    KNN_CUDA(launch_split_tf32(pc->corpus, pc->N, pc->ldc, pc->D, dp, (float*)pc->thi.p, (float*)pc->tlo.p,
-                               (uint32_t*)pc->ttiles.p, pc->f16 ? nullptr : (uint32_t*)pc->words.p, nullptr, s));
-    // once per index: later searches on any stream see the copies
-    KNN_CUDA(cudaStreamSynchronize(s));
-    pc->thi_ready = true;
     return KNNS_OK;
 }
 

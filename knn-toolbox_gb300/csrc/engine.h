@@ -113,9 +113,9 @@ struct Engine {
 };
 
 // A corpus prepared once and kept resident (the serving index): BF16 copy,
-// norms, optional FP16 hi/lo copies with row scales and per-tile low-part flags,
-// optional E4M3 codes with per-row scales, and the corpus half of the flag words ([0] low part, [1] not BF16-exact,
-// [2] not integer, [3] max |x| bits).  The caller keeps the FP32 corpus alive
+// norms, optional TF32 hi/lo and FP16 hi/lo copies (these with row scales) with per-tile low-part flags,
+// optional E4M3 codes with per-row scales, and the corpus half of the flag words ([0] TF32 low part, [1] not
+// BF16-exact, [2] not integer, [3] max |x| bits).  The caller keeps the FP32 corpus alive
 // and unchanged while the index is used.
 struct PreparedCorpus {
     const float* corpus = nullptr;
@@ -123,12 +123,10 @@ struct PreparedCorpus {
     int D = 0, dpb = 0, dpf = 0;
     bool tf32 = false, fp8 = false;
     DevBuf cn, bf, hi, lo, rs, tiles, words, f8, cs, np;
-    // FP16 copies present (hi, lo, rs, tiles); TF32 copies, made by the first search that needs them
-    // (prepare_tf32)
+    // the exact form's copies (tf32): TF32 hi / lo and their tile flags (thi, tlo, ttiles), and FP16 ones (hi, lo,
+    // rs, tiles) where memory allowed (f16)
     bool f16 = false;
-    mutable std::mutex tmu;
-    mutable bool thi_ready = false;
-    mutable DevBuf thi, tlo, ttiles;
+    DevBuf thi, tlo, ttiles;
     void release();
 };
 
@@ -152,9 +150,6 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
                const float* host_corpus = nullptr);
 int prepare_corpus(Engine& E, PreparedCorpus* pc, const float* corpus, int64_t N, int64_t ldc, int D, bool tf32,
                    cudaStream_t s, bool fp8 = false);
-// TF32 hi / lo copies of a prepared corpus (nothing when they exist; an error while capturing).
-// Synchronises s when it makes them.
-int prepare_tf32(const PreparedCorpus* pc, cudaStream_t s, bool capture);
 int check_device_error(Engine& E, cudaStream_t s);
 int search_host(const float* corpus, int64_t N, const float* queries, int64_t Q, int D, int k, float* dist,
                 int32_t* idx, float* idx_f_host, const knns_options& o, double* seconds, knns_stats* st);

@@ -159,3 +159,44 @@ def test_shortlist_autotuner(engine):
         hit = sum(len(set(ex[r]) & set(lo[r])) for r in range(len(ex)))
         assert hit / ex.size < 0.999
     ix.close()
+
+
+@pytest.mark.parametrize("kw,k", [({"rerank": False}, 10), ({}, 512), ({}, 125), ({"scan": 2}, 10), ({"algo": 1}, 10)])
+def test_index_is_complete_when_created(engine, kw, k):
+    # the copies of every kind of key exist then: no search on the index allocates any
+    import torch
+    assert engine.SCAN_OFF == 2 and engine.ALGO_TC == 1
+    g = torch.Generator(device="cuda").manual_seed(k)
+    c, q = torch.rand((200_000, 96), generator=g, device="cuda"), torch.rand((64, 96), generator=g, device="cuda")
+    warm = engine.Index(c)
+    d0, i0 = warm.search(q, k, **kw)
+    ix = engine.Index(c)
+    d, i = torch.empty_like(d0), torch.empty_like(i0)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ix.search(q, k, dist=d, idx=i, **kw)
+    assert torch.cuda.mem_get_info()[0] == free
+    assert torch.equal(d, d0) and torch.equal(i, i0)
+    warm.close()
+    ix.close()
+
+
+@pytest.mark.parametrize("N,k,rerank", [(9_000, 10, True), (60_000, 10, True), (200_000, 10, True), (60_000, 12, False)])
+def test_index_with_little_memory_left(engine, N, k, rerank):
+    # no FP16 copies are made when they would leave too little: 3xTF32 keys serve every search, same answers
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c, q = torch.rand((N, 96), generator=g, device="cuda"), torch.rand((70, 96), generator=g, device="cuda")
+    ix = engine.Index(c)
+    d0, i0 = ix.search(q, k, rerank=rerank)
+    ix.search(q, k, rerank=False)  # (the engine's buffers have their sizes)
+    ix.close()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (3 << 29), dtype=torch.uint8, device="cuda")
+    try:
+        ix = engine.Index(c)
+        d, i = ix.search(q, k, rerank=rerank)
+        assert torch.equal(i, i0) and torch.equal(d, d0)
+        ix.close()
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
