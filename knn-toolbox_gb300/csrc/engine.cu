@@ -1511,7 +1511,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
     // ordering events: [0] start, [1] sample landed, [2 + b] block b landed, [2 + nblk + b]
     // block b prepared, [2 + 2 nblk + b] block b scanned, [2 + 3 nblk] flag words cleared,
-    // [3 + 3 nblk] thresholds seeded, [4 + 3 nblk] the split-key scan done
+    // [3 + 3 nblk] thresholds seeded, [4 + 3 nblk] the split-key scan done, [5 + 3 nblk] queries prepared
     auto oev = [&](int i) -> cudaEvent_t { return E.order_event(i); };
     if (host_corpus != nullptr || blocked) {
         if (!oev(5 + 3 * nblk) || !E.copy_stream() || (blocked && (!E.prep_stream() || !E.worker_stream(0) ||
@@ -1629,6 +1629,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             KNN_CUDA(launch_prep(j, s, &qj));
         } else {
             KNN_CUDA(launch_prep(qj, s));
+            if (blocked) KNN_CUDA(cudaEventRecord(oev(5 + 3 * nblk), s));
         }
         ++launches;
         if (!bf16_only && !pc && !blocked) {
@@ -1903,13 +1904,14 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             }
             // What needs the whole corpus, the split copies and the split-key scan (gated on the data's
             // BF16-exactness in the exact form), runs on the preparation stream: the copies (their own
-            // buffers) once the last block is prepared, the flag then final; the scan, which writes
+            // buffers) once the last block and the queries are prepared, the flag then final; the scan, which writes
             // the thresholds and candidate segments the BF16 path also uses, once every block is
             // scanned (a block scanned before a later block cleared the flag ran its BF16 scan), beside
             // the BF16 selection and fix-up on the search's stream: one of the two paths returns at once.
             for (int b = 0; b < nblk; ++b) KNN_CUDA(cudaStreamWaitEvent(s, oev(2 + 2 * nblk + b), 0));
             if (tf_scan) {
                 cudaStream_t ps = E.prep_stream();
+                KNN_CUDA(cudaStreamWaitEvent(ps, oev(5 + 3 * nblk), 0));
                 if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, nullptr, any_lo, not_exact, ps))) return rc;
                 ++launches;
                 ts.s = ps;

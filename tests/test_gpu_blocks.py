@@ -113,3 +113,21 @@ def test_host_blocks_fill_the_chip(engine, N, Q, k, splits):
     dr, ir = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
     np.testing.assert_array_equal(i, ir.cpu().numpy())
     np.testing.assert_array_equal(d, dr.cpu().numpy())
+
+
+@pytest.mark.parametrize("N,Q,D", [(131_072, 40, 32), (200_000, 3_000, 64), (140_001, 129, 96)])
+def test_host_blocks_of_an_exact_corpus_and_inexact_queries(engine, N, Q, D):
+    # the corpus alone is BF16-exact, one query is not: the split copies, made once the last block has
+    # landed, must see what the queries' preparation found out
+    import torch
+    X, Qs = data("int", N, Q, D, N + Q)
+    Y = data("int", N, Q, D, N)[0]
+    Qs[Q - 1, D - 1] += 0.37
+    hx, hy = torch.from_numpy(X).pin_memory().numpy(), torch.from_numpy(Y).pin_memory().numpy()
+    dr, ir = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 20)
+    for _ in range(3):
+        engine.search_host(hy, Qs, 20)  # leaves the copies of another corpus
+        d, i = engine.search_host(hx, Qs, 20)
+        assert engine.last_stats()["scan_keys"] == 3
+        np.testing.assert_array_equal(i, ir.cpu().numpy())
+        np.testing.assert_array_equal(d, dr.cpu().numpy())
