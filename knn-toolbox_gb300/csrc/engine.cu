@@ -96,6 +96,21 @@ void ErrWord::release()
     h = d = nullptr;
 }
 
+cudaError_t reserve_smem(const void* kernel, size_t bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> limit;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& have = limit[{dev, kernel}];
+    if (bytes <= have) return cudaSuccess;
+    const cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (r == cudaSuccess) have = bytes;
+    return r;
+}
+
 // ---------------------------------------------------------------- engine registry
 static std::mutex g_reg_mu;
 static std::map<int, std::unique_ptr<Engine>> g_engines;

@@ -169,14 +169,12 @@ cudaError_t launch_simt(const float* corpus, int64_t N, int64_t ldc, const float
     dim3 grid((unsigned)((Q + qpb - 1) / qpb), (unsigned)splits);
     if (fix) grid = dim3((unsigned)fix->blocks());
     if (qpb == 128) {
-        cudaError_t e = cudaFuncSetAttribute(simt_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = reserve_smem((const void*)simt_kernel<128>, smem);
         if (e != cudaSuccess) return e;
         simt_kernel<128><<<grid, kThreads, smem, s>>>(corpus, N, ldc, cn, queries, Q, ldq, D, kp,
                                                       split_len, part, thr_g, tile_redo, qmap, qcount, fg);
     } else {
-        cudaError_t e = cudaFuncSetAttribute(simt_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = reserve_smem((const void*)simt_kernel<32>, smem);
         if (e != cudaSuccess) return e;
         simt_kernel<32><<<grid, kThreads, smem, s>>>(corpus, N, ldc, cn, queries, Q, ldq, D, kp,
                                                      split_len, part, thr_g, tile_redo, qmap, qcount, fg);

@@ -518,11 +518,11 @@ cudaError_t launch_tc(const TcArgs& a, int splits, bool bf16, cudaStream_t st)
     if (a.qcount) grid = dim3((unsigned)a.fix.blocks());
     cudaError_t e;
     if (bf16) {
-        e = cudaFuncSetAttribute(tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = reserve_smem((const void*)tc_kernel<true>, smem);
         if (e != cudaSuccess) return e;
         tc_kernel<true><<<grid, kTcThreads, smem, st>>>(a);
     } else {
-        e = cudaFuncSetAttribute(tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = reserve_smem((const void*)tc_kernel<false>, smem);
         if (e != cudaSuccess) return e;
         tc_kernel<false><<<grid, kTcThreads, smem, st>>>(a);
     }

@@ -25,6 +25,11 @@ enum DeviceError : int {
     kDevMisaligned = 5,
 };
 
+// Raises a kernel's dynamic shared memory limit on the current device to `bytes`.  It is never lowered: engines of
+// other threads (a server's slots) launch the same kernels, and a search with a smaller size set the limit between
+// another's setting it and its launch.
+cudaError_t reserve_smem(const void* kernel, size_t bytes);
+
 cudaError_t launch_norms(const float* x, int64_t n, int64_t ld, int D, float* out, int64_t n_pad,
                          cudaStream_t s);
 constexpr int kTileRows = 128;

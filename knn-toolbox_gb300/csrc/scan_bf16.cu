@@ -533,7 +533,7 @@ template <int TN, int kNacc, bool kF8>
 static cudaError_t launch_scan_t(const ScanArgs& a, dim3 grid, size_t smem, cudaStream_t st)
 {
     auto* kernel = a.keys ? scan_kernel<TN, kNacc, kF8, true> : scan_kernel<TN, kNacc, kF8, false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = reserve_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
     kernel<<<grid, kScanThreads, smem, st>>>(a);
     return cudaGetLastError();

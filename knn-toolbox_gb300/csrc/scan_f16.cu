@@ -692,7 +692,7 @@ cudaError_t launch_fscan(const FscanArgs& a, int splits, cudaStream_t st)
     auto* kernel = !a.keys ? (ta ? fscan_ta_kernel<false> : fscan_wide_kernel<false, kWN>)
                    : ta    ? fscan_ta_kernel<true>
                    : tn == kWN ? fscan_wide_kernel<true, kWN> : fscan_wide_kernel<true, kWNarrow>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = reserve_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);
     kernel<<<grid, kThreads, smem, st>>>(a);

@@ -614,7 +614,7 @@ cudaError_t launch_tscan(const TscanArgs& a, int splits, cudaStream_t st)
     if (a.Q <= 0) return cudaSuccess;
     auto* kernel = a.keys ? (ta ? tscan_ta_kernel<true> : tscan_kernel<true>)
                           : (ta ? tscan_ta_kernel<false> : tscan_kernel<false>);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = reserve_smem((const void*)kernel, smem);
     if (e != cudaSuccess) return e;
     dim3 grid((unsigned)((a.Q + kTileQ - 1) / kTileQ), (unsigned)splits);
     kernel<<<grid, kThreads, smem, st>>>(a);

@@ -1497,8 +1497,7 @@ __global__ void __launch_bounds__(kT, kMode == kSmallCertified ? 1024 / kT : 0) 
 template <int kT, int kMode>
 static cudaError_t run_select_small(const SmallSelect& c, size_t smem, cudaStream_t s)
 {
-    cudaError_t e = cudaFuncSetAttribute(select_small_kernel<kT, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
+    cudaError_t e = reserve_smem((const void*)select_small_kernel<kT, kMode>, smem);
     if (e != cudaSuccess) return e;
     select_small_kernel<kT, kMode><<<(unsigned)c.Q, kT, smem, s>>>(c);
     return cudaGetLastError();
@@ -1534,7 +1533,7 @@ cudaError_t launch_select(const uint64_t* part, int splits, int64_t Q, int kp, i
 {
     if (Q <= 0) return cudaSuccess;
     size_t smem = select_smem_bytes(kp, D, rerank);
-    cudaError_t e = cudaFuncSetAttribute(select_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = reserve_smem((const void*)select_kernel, smem);
     if (e != cudaSuccess) return e;
     unsigned blocks = (unsigned)((Q + kSelWarps - 1) / kSelWarps);
     select_kernel<<<blocks, kSelWarps * 32, smem, s>>>(part, splits, Q, kp, k, corpus, ldc, queries, ldq, D,
@@ -1624,8 +1623,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
             select_block_kernel<128, true><<<(unsigned)c.Q, 128, smem, s>>>(c);
     } else if (thr) {
         const size_t smem = (size_t)kSelWarps * c.buf_words * 8;
-        cudaError_t e = cudaFuncSetAttribute(select_threshold_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+        cudaError_t e = reserve_smem((const void*)select_threshold_kernel, smem);
         if (e != cudaSuccess) return e;
         select_threshold_kernel<<<(unsigned)((c.Q + kSelWarps - 1) / kSelWarps), kSelWarps * 32, smem, s>>>(c);
     } else {
@@ -1640,7 +1638,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
                        : t == 512 ? select_block_kernel<512, false>
                        : t == 256 ? select_block_kernel<256, false>
                                   : select_block_kernel<128, false>;
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = reserve_smem((const void*)kernel, smem);
         if (e != cudaSuccess) return e;
         kernel<<<(unsigned)c.Q, t, smem, s>>>(c);
     }

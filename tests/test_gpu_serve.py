@@ -200,3 +200,42 @@ def test_index_with_little_memory_left(engine, N, k, rerank):
     finally:
         del ballast
         torch.cuda.empty_cache()
+
+
+def test_server_beside_searches_of_other_sizes(engine):
+    # a slot's first search per (batch, k) launches the kernels that the application's searches launch, with
+    # other amounts of shared memory, from another thread
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(1)
+    c = torch.rand((9000, 64), generator=g, device="cuda")
+    big = torch.rand((16000, 64), generator=g, device="cuda")
+    q = torch.rand((40, 64), generator=g, device="cuda")
+    d0, i0 = engine.search(big, q, 100)
+    ix = engine.Index(c)
+    srv = engine.Server(ix, slots=4, max_batch=256)
+    stop, bad = threading.Event(), []
+
+    def app():
+        s = torch.cuda.Stream()
+        while not stop.is_set():
+            try:
+                with torch.cuda.stream(s):
+                    _, i = engine.search(big, q, 100)
+                    if not torch.equal(i, i0):
+                        bad.append("indices differ")
+            except engine.KnnsError as e:
+                bad.append(str(e))
+
+    th = threading.Thread(target=app)
+    th.start()
+    rng = np.random.default_rng(0)
+    try:
+        for k in range(1, 60):
+            for rid in [srv.submit(rng.random((m, 64), dtype=np.float32), k) for m in (3, 100)]:
+                srv.wait(rid)
+    finally:
+        stop.set()
+        th.join()
+        srv.close()
+        ix.close()
+    assert not bad
