@@ -131,3 +131,33 @@ def test_host_blocks_of_an_exact_corpus_and_inexact_queries(engine, N, Q, D):
         assert engine.last_stats()["scan_keys"] == 3
         np.testing.assert_array_equal(i, ir.cpu().numpy())
         np.testing.assert_array_equal(d, dr.cpu().numpy())
+
+
+def block_splits(N, Q, tn, sms=152):
+    """Main-scan splits of a corpus that is copied in: a one-wave plan, or 8 blocks of as many splits as fill the SMs."""
+    up = lambda a, b: -(-a // b)
+    qt, tiles = up(Q, 128), up(N, tn)
+
+    def fewest(cost, lim):
+        return min(range(1, lim + 1), key=lambda s: (round(cost(s), 6), s))
+    S = fewest(lambda s: up(qt * s, sms) * up(tiles, s) * (1 + 0.004 * s), min(tiles, 128))
+    have = up(S, min(S, 8))
+    fill = fewest(lambda s: up(qt * s, sms) * (up(up(tiles, 8), s) + 8), min(up(tiles, 8), 8))
+    if have * qt < sms and fill > have:
+        S = min(tiles, 8 * fill)
+    return up(N, up(tiles, S) * tn)
+
+
+@pytest.mark.parametrize("N,Q,k", [(131_072, 1, 16), (200_000, 300, 32), (200_000, 6_000, 10), (150_001, 129, 100)])
+@pytest.mark.parametrize("kind", ["int", "uniform"])
+def test_host_block_splits(engine, kind, N, Q, k):
+    import torch
+    X, Qs = data(kind, N, Q, 96, N + k)
+    Xp = torch.from_numpy(X).pin_memory().numpy()
+    d, i = engine.search_host(Xp, Qs, k)
+    plan = engine.scan_plan(N, Q, 96, k)
+    assert engine.last_stats()["scan_splits"] == block_splits(N, Q, plan["tile_rows"])
+    dr, ir = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), k)
+    assert engine.last_stats()["scan_splits"] == plan["splits"]
+    np.testing.assert_array_equal(i, ir.cpu().numpy())
+    np.testing.assert_array_equal(d, dr.cpu().numpy())
