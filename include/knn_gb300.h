@@ -330,6 +330,9 @@ typedef struct knns_scan_plan_info {
     int sel_words;                               /* bound on one query's stored main-pass candidates */
 } knns_scan_plan_info;
 int knns_debug_scan_plan(int64_t N, int64_t Q, int D, int k, int sms, int tf32, knns_scan_plan_info *out);
+/* Device bytes a corpus row takes in a host-buffer search (the split of a corpus into device blocks
+ * counts with them); computed on the host alone.  0 for invalid arguments. */
+double knns_debug_host_row_bytes(int64_t N, int64_t Q, int D, int k, const knns_options *opt);
 
 #ifdef __cplusplus
 }

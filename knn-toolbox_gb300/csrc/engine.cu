@@ -2114,19 +2114,40 @@ int check_device_error(Engine& E, cudaStream_t s)
     return KNNS_OK;
 }
 
+// Device bytes of a row of a host-buffer search's corpus: its FP32 values and the copies that a search of these
+// options (or one of a smaller block) makes of it, in the widths they are padded to.
+static double host_row_bytes(const Engine& E, int64_t N, int64_t Q, int D, int k, const knns_options& o)
+{
+    Config c;
+    const bool known = resolve_config(E, N, Q, D, k, o, &c) == KNNS_OK;
+    clear_error();
+    const double dp = round32(D), dpb = (D + 63) & ~63;
+    double b = 4.0 * D + 4 + 4;  // values, norm, flags and the preparation's marks
+    if (known && c.algo == KNNS_ALGO_SIMT) return b;
+    b += 2 * dpb + 2 * kNormParts;
+    const bool bf16_only = known && c.precision != KNNS_PREC_EXACT;
+    // FP16 hi / lo and row scales, or TF32 hi / lo: shortlists without a margin, and what the shortlist kernel serves
+    const bool scan = o.scan != KNNS_SCAN_OFF && c.rerank && N >= (o.scan == KNNS_SCAN_ON ? kScanMinRowsForced : kScanMinRowsAuto);
+    const bool f16 = known && !c.tf32 && (c.tscan || c.small || scan);
+    if (!bf16_only) b += f16 ? 4.0 * split_pitch(D) + 4 : 8 * dp;
+    if (c.fp8) b += 2.0 * c.dpf + 4;
+    return b;
+}
+
 // Corpus rows per device block of a host-buffer search: the requested count, or
 // (requested 0) the whole corpus when its copies fit in about 60 % of the free
 // device memory (the engine's own cached corpus buffers counted as free), else as
 // many rows as do, rounded down to 4096.  0 when not even k rows fit.
-static int64_t host_block_rows(Engine& E, int64_t N, int64_t Q, int D, int k, int requested)
+static int64_t host_block_rows(Engine& E, int64_t N, int64_t Q, int D, int k, const knns_options& o)
 {
+    const int requested = o.block_rows;
     if (requested > 0) return std::max<int64_t>(std::min<int64_t>(requested, N), std::min<int64_t>(k, N));
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return N;
     const double avail = 0.6 * (double)(fr + E.in_corpus.cap + E.bf.cap + E.hi.cap + E.lo.cap + E.cn.cap);
-    // FP32 input, BF16 copy, FP16 hi / lo, norms, scales and flags per row; query-side workspace
-    const double per_row = (double)D * (4 + 2 + 4) + 96;
-    const double fixed = (double)Q * ((double)D * 8 + 8192) + 256.0 * (1 << 20);
+    const double per_row = host_row_bytes(E, N, Q, D, k, o);
+    // query-side workspace (candidate segments: up to 160 MB of the fixed share, see kBlockSplits)
+    const double fixed = (double)Q * ((double)D * 8 + 8192) + 416.0 * (1 << 20);
     const double rows = (avail - fixed) / per_row;
     if (rows >= (double)N) return N;
     const int64_t r = (int64_t)rows / 4096 * 4096;
@@ -2198,7 +2219,7 @@ int search_host(const float* corpus, int64_t N, const float* queries, int64_t Q,
     if (!s) return set_error(KNNS_ERR_CUDA, "stream creation failed");
     if (k > N) return set_error(KNNS_ERR_INVALID, "k=%d exceeds the corpus size N=%lld", k, (long long)N);
     if (o.block_rows < 0) return set_error(KNNS_ERR_INVALID, "negative block_rows");
-    const int64_t br = host_block_rows(*E, N, Q, D, k, o.block_rows);
+    const int64_t br = host_block_rows(*E, N, Q, D, k, o);
     if (br <= 0) return set_error(KNNS_ERR_NOMEM, "no corpus block of at least %d rows fits in device memory", k);
     if (br < N) return search_host_blocked(*E, s, corpus, N, queries, Q, D, k, dist, idx, idx_f_host, o, br, seconds, st);
     const size_t cb = (size_t)N * D * sizeof(float), qb = (size_t)Q * D * sizeof(float);
@@ -2603,6 +2624,16 @@ int knns_debug_prep(const float* x, int64_t n, int64_t ld, int D, float* norms, 
     KNN_CUDA(launch_prep(j, s));
     KNN_CUDA(cudaStreamSynchronize(s));
     return KNNS_OK;
+}
+
+double knns_debug_host_row_bytes(int64_t N, int64_t Q, int D, int k, const knns_options* opt)
+{
+    clear_error();
+    if (!opt || N < 1 || Q < 1 || D < 1 || k < 1) return 0.0;
+    Engine E;  // (reads the device properties alone, as below)
+    E.sms = 152;
+    E.cc = 103;
+    return host_row_bytes(E, N, Q, D, k, *opt);
 }
 
 int knns_debug_scan_plan(int64_t N, int64_t Q, int D, int k, int sms, int tf32, knns_scan_plan_info* out)

@@ -36,7 +36,7 @@ OK, ERR_INVALID, ERR_CUDA, ERR_UNSUPPORTED, ERR_DEVICE_TIMEOUT, ERR_NOMEM = rang
 EXPORTED = ["knns_default_options", "knns_search_device", "knns_search_host", "knns_check_device", "knns_merge_topk",
             "knns_last_error", "knns_last_stats", "knns_last_fixups", "knns_version", "knns_debug_tc_dot_tile",
             "knns_debug_stall_next_search",
-            "knns_debug_prep", "knns_debug_scan_plan",
+            "knns_debug_prep", "knns_debug_scan_plan", "knns_debug_host_row_bytes",
             "knns_timing_collect", "knns_timing_collect5", "knns_search_device_noalloc", "knns_noalloc_prepare",
             "knns_index_create", "knns_index_search", "knns_index_destroy", "knns_autotune_shortlist",
             "knns_server_default_config", "knns_server_create", "knns_server_submit", "knns_server_wait",
@@ -118,6 +118,8 @@ def lib():
     L.knns_debug_stall_next_search.argtypes = [i64]
     L.knns_debug_prep.argtypes = [vp, i64, i64, ci, vp, vp, vp, vp, vp, vp]
     L.knns_debug_scan_plan.argtypes = [i64, i64, ci, ci, ci, ci, ctypes.POINTER(ScanPlanInfo)]
+    L.knns_debug_host_row_bytes.argtypes = [i64, i64, ci, ci, ctypes.POINTER(Options)]
+    L.knns_debug_host_row_bytes.restype = ctypes.c_double
     L.knns_timing_collect.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int)]
     L.knns_timing_collect5.argtypes = [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int)]
     L.knns_search_device_noalloc.argtypes = [vp, i64, i64, vp, i64, i64, ci, ci, vp, vp, vp]
@@ -287,6 +289,11 @@ def scan_plan(N, Q, D, k, sms=152, tf32=False) -> dict:
             "level_rank": list(p.level_rank[:L]), "level_splits": list(p.level_splits[:L]),
             "level_cap": list(p.level_cap[:L]), "splits": p.splits, "split_len": p.split_len, "cap": p.cap,
             "sel_words": p.sel_words}
+
+
+def host_row_bytes(N, Q, D, k, **opts) -> float:
+    """Device bytes a corpus row takes in a host-buffer search of these options (no GPU)."""
+    return lib().knns_debug_host_row_bytes(N, Q, D, k, ctypes.byref(options(**opts)))
 
 
 def debug_prep(x, norm_parts=False):

@@ -77,3 +77,30 @@ def test_plan_rejects_bad_arguments(cuknns):
     # a successful call clears the library's last error (other tests read it)
     cuknns.scan_plan(1000, 10, 128, 10)
     assert cuknns.last_error() == ""
+
+
+@pytest.mark.parametrize("N", [1_000_000, 100_000, 20_000, 9_000])
+@pytest.mark.parametrize("D", [1, 33, 64, 96, 128, 129, 200, 300, 1000])
+@pytest.mark.parametrize("k,opts", [(10, {}), (128, {}), (512, {}), (10, {"rerank": False}), (10, {"scan": 2}),
+                                    (10, {"precision": 1, "shortlist": 4}), (10, {"precision": 2, "shortlist": 2})])
+def test_host_row_bytes_cover_the_copies(cuknns, N, D, k, opts):
+    # a corpus is split into device blocks by what a row takes there: its values and the copies a search
+    # may make of it, in their padded widths
+    assert (cuknns.SCAN_OFF, cuknns.PREC_BF16, cuknns.PREC_FP8) == (2, 1, 2)
+    dp, dpb, hp, dpf = -(-D // 32) * 32, -(-D // 64) * 64, -(-D // 8) * 8, -(-D // 128) * 128
+    got = cuknns.host_row_bytes(N, 1000, D, k, **opts)
+    prec = opts.get("precision", 0)
+    if prec and D > 256:
+        return  # refused
+    need = 4 * D + 4
+    split_off = "scan" in opts or not opts.get("rerank", True)
+    if prec:
+        need += 2 * dpb + (dpf + 4 if prec == 2 else 0)
+    elif D <= 128 and split_off or k in (128, 512) and (k == 512 or (N >= 131_072 and D <= 128)):
+        # 3xTF32 copies: shortlists without a margin, distances read off the keys, the shortlist kernel
+        if not (N < 16_384 and k == 512) and not (D > 128 and "scan" in opts):
+            need += 8 * dp + (2 * dpb if D <= 128 else 0)
+    elif not split_off:
+        need += 4 * hp + 4
+    assert got >= need
+    assert got <= 4 * D + 8 * dp + 2 * dpb + 2 * dpf + 64
