@@ -1126,8 +1126,8 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     const int tn = fscan_tile_rows(D);
     const int64_t tiles = cdiv(N, tn), ldk = tiles * tn;
-    // queries whose keys are held at once: whole query tiles
-    const int64_t chunk = std::max<int64_t>(1, kSmallKeys / N / kTileQ) * kTileQ;
+    // queries whose keys (rows padded to whole tiles) and split copies are held at once: whole query tiles
+    const int64_t chunk = std::max<int64_t>(1, kSmallKeys / ldk / kTileQ) * kTileQ;
     size_t ws = 0, nwords = 0;
     int rc = KNNS_OK, launches = 1;
     const bool with_fix = dense && c.fp32 && N * D >= kFixWork;
@@ -1148,10 +1148,11 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
             if (!rc) rc = ensure_split(E, c, N, D, n_pad);
         }
         if (!rc) rc = flag_words(E, Q, pc ? 0 : N, &nwords);
-        if (!rc) rc = E.qhi.ensure((size_t)Q * split_pitch(D) * 2);
-        if (!rc) rc = E.qlo.ensure((size_t)Q * split_pitch(D) * 2);
-        if (!rc) rc = E.qrs.ensure(Q * sizeof(float));
-        if (!rc) rc = E.cand.ensure((size_t)std::min(Q, chunk) * ldk * sizeof(float));
+        const size_t rows = std::min(Q, chunk);
+        if (!rc) rc = E.qhi.ensure(rows * split_pitch(D) * 2);
+        if (!rc) rc = E.qlo.ensure(rows * split_pitch(D) * 2);
+        if (!rc) rc = E.qrs.ensure(rows * sizeof(float));
+        if (!rc) rc = E.cand.ensure(rows * ldk * sizeof(float));
         if (rc) return rc;
         ws += (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qhi.cap + E.qlo.cap + E.qrs.cap +
              E.cand.cap;
@@ -1182,22 +1183,23 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
     if (dense) {
         uint32_t* words = (uint32_t*)E.words.p;
         KNN_CUDA(cudaMemsetAsync(words, 0, nwords * sizeof(uint32_t), s));
-        PrepJob qj = prep_job(queries, Q, ldq, D, nullptr, Q);
-        qj.hi = E.qhi.p;
-        qj.lo = E.qlo.p;
-        qj.rs = (float*)E.qrs.p;
-        qj.lo_flags = E.qlof;
+        // a chunk's queries, prepared (the first ones with the corpus)
+        auto query_job = [&](int64_t q0, int64_t nq) {
+            PrepJob j = prep_job(queries + q0 * ldq, nq, ldq, D, nullptr, nq);
+            j.hi = E.qhi.p;
+            j.lo = E.qlo.p;
+            j.rs = (float*)E.qrs.p;
+            j.lo_flags = E.qlof + q0 / kTileQ;
+            return j;
+        };
+        const PrepJob qj = query_job(0, std::min(Q, chunk));
         if (pc) KNN_CUDA(launch_prep(qj, s));
         else if ((rc = split_corpus(E, c, corpus, N, ldc, D, n_pad, (float*)E.cn.p, words, nullptr, s, &qj))) return rc;
         if ((rc = mark(1)) || (rc = mark(2))) return rc;
         const SplitCopies cp = split_copies(E, c, pc);
         FscanArgs f;
         memset(&f, 0, sizeof(f));
-        if (D > kFscanTmemD) {
-            rc = encode_split(&f.tm_qhi, E.qhi.p, Q, D, 1, kTileQ);
-            if (!rc) rc = encode_split(&f.tm_qlo, E.qlo.p, Q, D, 1, kTileQ);
-        }
-        if (!rc) rc = encode_split(&f.tm_chi, cp.hi, N, D, 1, tn);
+        rc = encode_split(&f.tm_chi, cp.hi, N, D, 1, tn);
         if (!rc) rc = encode_split(&f.tm_clo, cp.lo, N, D, 1, tn);
         if (rc) return rc;
         f.cn = (const float*)(pc ? pc->cn.p : E.cn.p);
@@ -1211,6 +1213,9 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         f.N = N;
         f.D = D;
         f.hp = split_pitch(D);
+        f.qhi = (const uint16_t*)E.qhi.p;
+        f.qlo = (const uint16_t*)E.qlo.p;
+        f.qs = (const float*)E.qrs.p;
         sel.keys = f.keys;
         sel.ldk = ldk;
         sel.need = (int)std::min<int64_t>(c.kp, N);
@@ -1221,14 +1226,15 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         }
         for (int64_t q0 = 0; q0 < Q; q0 += chunk) {
             const int64_t nq = std::min(chunk, Q - q0);
-            if (q0 > 0 && D > kFscanTmemD) {
-                rc = encode_split(&f.tm_qhi, (const char*)E.qhi.p + q0 * f.hp * 2, nq, D, 1, kTileQ);
-                if (!rc) rc = encode_split(&f.tm_qlo, (const char*)E.qlo.p + q0 * f.hp * 2, nq, D, 1, kTileQ);
+            if (q0 > 0) {
+                KNN_CUDA(launch_prep(query_job(q0, nq), s));
+                ++launches;
+            }
+            if (D > kFscanTmemD) {
+                rc = encode_split(&f.tm_qhi, E.qhi.p, nq, D, 1, kTileQ);
+                if (!rc) rc = encode_split(&f.tm_qlo, E.qlo.p, nq, D, 1, kTileQ);
                 if (rc) return rc;
             }
-            f.qhi = (const uint16_t*)E.qhi.p + q0 * f.hp;
-            f.qlo = (const uint16_t*)E.qlo.p + q0 * f.hp;
-            f.qs = (const float*)E.qrs.p + q0;
             f.qlo_flags = E.qlof + q0 / kTileQ;
             f.Q = nq;
             const int S = seed_splits(cdiv(nq, kTileQ), tiles, E.sms, (int)tiles);

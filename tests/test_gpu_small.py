@@ -156,3 +156,19 @@ def test_index_without_copies(engine, N, Q, D):
         with pytest.raises(engine.KnnsError):
             ix.search(q, 10)
     ix.close()
+
+
+@pytest.mark.parametrize("N,Q,D,most", [(2, 400_000, 300, 400e6), (40, 300_000, 200, 400e6)])
+def test_workspace_of_many_queries(engine, N, Q, D, most):
+    # rows of keys are padded to whole tiles: a handful of corpus rows must not cost a million queries half a
+    # kilobyte each (a fresh process: the engine's buffers only grow)
+    import subprocess
+    import sys
+    code = ("import sys; sys.path.insert(0, 'knn-toolbox_gb300')\nimport torch, cuknns\n"
+            "g = torch.Generator(device='cuda').manual_seed(3)\n"
+            f"c, q = torch.rand(({N}, {D}), generator=g, device='cuda'), torch.rand(({Q}, {D}), generator=g, device='cuda')\n"
+            "d, i = cuknns.search(c, q, 2)\nn = cuknns.last_stats()['workspace_bytes']\n"
+            "d0, i0 = cuknns.search(c, q, 2, pilot=False)\nassert torch.equal(i, i0) and torch.equal(d, d0)\nprint(n)")
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    assert int(r.stdout.split()[-1]) < most
