@@ -151,9 +151,10 @@ const char *knns_last_error(void);
 /* Statistics of the calling thread's last successful search. */
 int knns_last_stats(knns_stats *out);
 
-/* Queries of the calling thread's last threshold-scan search that overflowed
- * their candidate segments and were answered by the fix-up pass (0 when the
- * scan did not run).  Diagnostic: synchronises the device. */
+/* Queries of the last search on the current device that the fix-up pass answered:
+ * those whose candidates overflowed in the threshold scan, whichever keys it ran on,
+ * and those whose split-key shortlists were not certain (0 when neither applies).
+ * Diagnostic: synchronises the device. */
 int knns_last_fixups(int64_t *out);
 
 /*

@@ -1079,6 +1079,7 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     float* cn = (float*)(pc ? pc->cn.p : E.cn.p);
     TscanStages ts{E, c, sp, corpus, N, ldc, queries, Q, ldq, D, k, cn, split_copies(E, c, pc), (const float*)E.qn.p, dist, idx, idx_f, nullptr, words + 1, E.fail, E.thr2, s};
     if ((rc = ts.ensure())) return rc;
+    E.fix_counts[0] = E.fail.p;
     const size_t ws = (pc ? 0 : E.cn.cap + E.hi.cap + E.lo.cap + E.rs.cap) + E.words.cap + E.qn.cap + ts.workspace();
 
     if (!capture) KNN_CUDA(cudaStreamWaitEvent(s, E.last_done, 0));
@@ -1222,6 +1223,7 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         if (with_fix) {
             sel.fail_idx = (int32_t*)E.fail.p;
             sel.fail_cnt = words + 6;
+            E.fix_counts[0] = sel.fail_cnt;
             sel.fail_thr = (uint32_t*)E.thr2.p;
         }
         for (int64_t q0 = 0; q0 < Q; q0 += chunk) {
@@ -1304,6 +1306,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     }
     // an index without room for FP16 copies: 3xTF32 keys
     if (pc && pc->tf32 && !pc->f16) c.tf32 = true;
+    E.fix_counts[0] = E.fix_counts[1] = nullptr;
     if (c.tscan || c.small) {
         if (host_corpus != nullptr) {
             // the whole corpus lands before the search starts (no overlap on this path)
@@ -1469,8 +1472,11 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
     const float* cn_ts = (const float*)(pc ? pc->cn.p : E.cn.p);
     TscanStages ts{E, c, sp_tf, corpus, N, ldc, queries, Q, ldq, D, k, cn_ts, cp, (const float*)E.qn.p, dist, idx, idx_f,
                    (const uint32_t*)E.words.p + 1, (uint32_t*)E.words.p + 5, E.tfail, E.tthr2, s};
+    // (the path that does not run leaves no failed query)
+    if (scan) E.fix_counts[0] = E.fail.p;
     if (tf_scan) {
         if ((rc = ts.ensure())) return rc;
+        E.fix_counts[1] = E.tfail.p;
         ws += E.qhi.cap + E.qlo.cap + E.qrs.cap + E.tfail.cap + E.tthr2.cap;
     }
     // Resident corpora (one stream otherwise): the split-key scan runs on a side stream beside the
@@ -2404,16 +2410,16 @@ int knns_last_fixups(int64_t* out)
     if (!out) return KNNS_ERR_INVALID;
     if (!g_have_stats) return set_error(KNNS_ERR_INVALID, "no search has completed on this thread");
     *out = 0;
-    if (!g_last_stats.scan) return KNNS_OK;
     Engine* E = nullptr;
     int rc = get_engine(&E);
     if (rc) return rc;
     std::lock_guard<std::mutex> lk(E->mu);
-    if (!E->fail.p) return KNNS_OK;
-    uint32_t n = 0;
     KNN_CUDA(cudaDeviceSynchronize());
-    KNN_CUDA(cudaMemcpy(&n, E->fail.p, sizeof n, cudaMemcpyDeviceToHost));
-    *out = (int64_t)n;
+    for (const void* count : E->fix_counts) {
+        uint32_t n = 0;
+        if (count) KNN_CUDA(cudaMemcpy(&n, count, sizeof n, cudaMemcpyDeviceToHost));
+        *out += (int64_t)n;
+    }
     return KNNS_OK;
 }
 

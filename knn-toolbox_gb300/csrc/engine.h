@@ -72,6 +72,8 @@ struct Engine {
     DevBuf qhi, qlo, qrs, tfail, tthr2;
     // adaptive preparation: one byte per batch of corpus rows (PrepJob::done)
     DevBuf done;
+    // counts of failed queries of the last search (null: none of that kind)
+    const void* fix_counts[2] = {};
     // per-search flag words: [0] some corpus tile has a low part, [1] corpus or
     // queries not BF16-exact, [2] some value not an integer, [3] max |x| (float bits), [4] zero,
     // [5] some query tile has a low part, [6] failed queries of a small corpus;

@@ -195,7 +195,7 @@ def timing_collect5():
 
 
 def last_fixups() -> int:
-    """Queries of the last threshold-scan search that the fix-up pass answered (synchronises)."""
+    """Queries of the last search that the fix-up pass answered (synchronises)."""
     n = ctypes.c_int64(0)
     _check(lib().knns_last_fixups(ctypes.byref(n)))
     return n.value

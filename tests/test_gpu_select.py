@@ -146,3 +146,33 @@ def test_dense_thresholds_with_ties(engine, oracle, Q, N, hi):
     od, oi = oracle.knn_gemm(X, Qs[sub], 10, kp=st["kp"], rerank=True)
     np.testing.assert_array_equal(i.cpu().numpy()[sub], oi)
     np.testing.assert_array_equal(d.cpu().numpy()[sub], od)
+
+
+@pytest.mark.parametrize("N,D,kind", [(140_000, 64, "float"), (140_000, 64, "int"), (60_000, 64, "float"), (60_000, 300, "float")])
+def test_fixups_are_counted_whichever_keys_run(engine, N, D, kind):
+    # a query at a row that half of the corpus repeats: its candidates overflow, every other query's do not
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N + D)
+    rows = lambda n: (torch.rand((n, D), generator=g, device="cuda") if kind == "float" else
+                      torch.randint(0, 100, (n, D), generator=g, device="cuda").float())
+    c, q = rows(N), rows(30)
+    c[:N // 2] = c[0]  # (every other row would be every row of the seeding sample)
+    q[3] = c[0]
+    engine.search(c, q, 10)
+    assert engine.last_stats()["scan"] == 1 and 1 <= engine.last_fixups() <= 3
+    engine.search(rows(N), q, 10)
+    assert engine.last_fixups() <= 2
+    engine.search(rows(1000), q, 10)
+    assert engine.last_fixups() == 0
+
+
+@pytest.mark.parametrize("N,Q,D,k", [(9000, 300, 1000, 10), (16000, 200, 600, 300), (12000, 2600, 130, 10)])
+def test_certified_shortlists_of_ordinary_data_hold(engine, N, Q, D, k):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N + D)
+    c, q = torch.rand((N, D), generator=g, device="cuda"), torch.rand((Q, D), generator=g, device="cuda")
+    engine.search(c, q, k)
+    assert engine.last_fixups() == 0
+    # a common offset leaves the split keys too few bits: FP32 keys answer
+    engine.search(c + 500, q + 500, k)
+    assert engine.last_fixups() == Q
