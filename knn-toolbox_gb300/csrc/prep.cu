@@ -467,13 +467,20 @@ static __device__ __noinline__ float double_norm(const float* row, int D)
 {
     const int lane = threadIdx.x & 31;
     double t = 0.0;
+    bool grid = true;  // multiples of 2^-10
     for (int d = lane; d < D; d += 32) {
-        const double x = (double)__ldg(row + d);
+        const float v = __ldg(row + d);
+        const double x = (double)v;
         t = __fma_rn(x, x, t);
+        grid &= rintf(v * 1024.f) == v * 1024.f;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (!(t < __longlong_as_double(0x7ff0000000000000ll))) return (float)t;  // inf or nan in any order
+    // multiples of 2^-20 that sum below 2^33: exact in any order (integers, whose norms lie halfway between two
+    // floats every other time from 2^24 on, else all took the serial loop: 42,649 x 1,400 values 0..199, a host
+    // search 2.3 -> 5.5 ms)
+    if (__all_sync(0xffffffffu, grid) && t < 0x1p33) return __double2float_rn(t);
     // both sums err by their additions' roundings: (D + D / 32 + 6) 2^-53 of the sum in all
     const double B = (double)(2 * D + 8) * 1.01 * 0x1p-53 * t;
     const float a = __double2float_rn(t - B), b = __double2float_rn(t + B);
@@ -574,7 +581,7 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
             rmx[u] = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mx)));
             mx_all = fmaxf(mx_all, rmx[u]);
         }
-        bool all_int = false;
+        bool all_int = false, exact = false;
         if (bf) {
             // integrality, by (x + 1.5 2^23) - 1.5 2^23 == x (integers of 2^22 and more count as
             // fractions: no use of the flag goes that far), and exactness in BF16: the low 16
@@ -610,6 +617,7 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
             const uint32_t w2 = __reduce_or_sync(0xffffffffu, f2);
             frac |= w2 & 1u;
             all_int = (w2 & 1u) == 0u && (float)D * mx * mx < 16777216.f;
+            exact = (w2 & 1u) == 0u && mx <= 4096.f;
             if (check && (w2 & 2u)) {
                 if (p.done != nullptr) {
                     // the other warps' next batches should know
@@ -722,6 +730,9 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
                     ff_reduce_rows<kU>(hi, lo, lane, h, l);
                     ok = certified_norm<kChunks>(h, l, D, f);
                 }
+                // integers up to 2^12: squares, high parts and low parts (below 2^24) are exact integers, so f is
+                // the sum's rounding even where that is a tie
+                ok |= exact;
                 const uint32_t open = __ballot_sync(0xffffffffu, !ok);
                 if (open != 0u) {
 #pragma unroll

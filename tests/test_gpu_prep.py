@@ -110,3 +110,40 @@ def test_corpus_and_queries_share_a_launch(engine, N, Q, D, kind):
     # each query alone in its launch's share: the answers of the first and the last
     d2, i2 = engine.search(c, w[-1:, 1:].contiguous(), 9)
     assert torch.equal(d0[-1:], d2) and torch.equal(i0[-1:], i2)
+
+
+@pytest.mark.parametrize("D", [1, 3, 128, 130, 255, 256, 257, 384])
+@pytest.mark.parametrize("kind", ["int", "int256", "tenths of 2^-10", "mixed"])
+def test_norms_halfway_between_floats(engine, D, kind):
+    # integers and multiples of 2^-10 whose squares sum past 2^24 of their unit: every other norm is a tie,
+    # which only the exact sum settles (rows of 4,096 and more, and a row that is no integer in a batch, too)
+    import torch
+    rng = np.random.default_rng(D)
+    hi = {"int": 4097, "int256": 257, "tenths of 2^-10": 40000, "mixed": 6000}[kind]
+    X = rng.integers(-hi + 1, hi, (2001, D)).astype(np.float64)
+    X[3] = 0
+    X[5] = hi - 1
+    if kind == "tenths of 2^-10":
+        X /= 1024.0
+    if kind == "mixed":
+        X[::5, 0] += 0.25
+    S = (X * X).sum(1)  # exact
+    norms = engine.debug_prep(torch.from_numpy(X.astype(np.float32)).cuda())[0].cpu().numpy()
+    np.testing.assert_array_equal(norms, S.astype(np.float32))
+
+
+@pytest.mark.parametrize("D", [385, 700, 1024, 1400, 2048])
+def test_norms_halfway_between_floats_wide_rows(engine, oracle, D):
+    # read off the CUDA-core keys: rerank = False returns key + ||q||^2
+    import torch
+    rng = np.random.default_rng(D)
+    X = rng.integers(0, 4097, (300, D)).astype(np.float32)
+    X[::3] = rng.integers(0, 200, X[::3].shape)
+    X[7, 3] += 0.5
+    Qs = np.zeros((4, D), np.float32)
+    Qs[1, 0] = 1.0
+    d, i = engine.search(torch.from_numpy(X).cuda(), torch.from_numpy(Qs).cuda(), 300, algo=engine.ALGO_SIMT, rerank=False)
+    S = (X.astype(np.float64) ** 2).sum(1).astype(np.float32)
+    o = np.lexsort((np.arange(300), S))
+    np.testing.assert_array_equal(i[0].cpu().numpy(), o)
+    np.testing.assert_array_equal(d[0].cpu().numpy(), S[o])
