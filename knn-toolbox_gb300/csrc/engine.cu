@@ -1219,6 +1219,7 @@ static int run_small(Engine& E, const Config& c, const float* corpus, int64_t N,
         f.qs = (const float*)E.qrs.p;
         sel.keys = f.keys;
         sel.ldk = ldk;
+        sel.cn = f.cn;
         sel.need = (int)std::min<int64_t>(c.kp, N);
         if (with_fix) {
             sel.fail_idx = (int32_t*)E.fail.p;

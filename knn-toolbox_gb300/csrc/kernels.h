@@ -348,6 +348,7 @@ struct SmallSelect {
     int64_t ldk = 0;
     int n = 0, need = 0, k = 0, kp = 0;
     bool fp32_keys = false;
+    const float* cn = nullptr;  // [n] row norms (optional)
     int32_t* fail_idx = nullptr;
     uint32_t* fail_cnt = nullptr;
     uint32_t* fail_thr = nullptr;

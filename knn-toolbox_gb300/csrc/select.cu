@@ -1058,26 +1058,46 @@ cudaError_t launch_dense_threshold(const float* keys, int64_t ldk, int n, int ra
 constexpr int kSmallList = 256;
 constexpr float kDirectMost = 1e37f;
 
-// Every row's key as an ordered word (+inf where it is not below +inf), a thread a row: in the arithmetic of the
-// CUDA-core kernel where the shape's keys are FP32 ones; otherwise from the product q.c rounded once, as a tensor-core
-// step adds its products (partial sums do not overflow).  Keys of a query that is not finite: FP32 keys have
-// them, split keys do not.
+// Every row's key as an ordered word (+inf where it is not below +inf), a thread a row, sixteen columns in flight: in
+// the arithmetic of the CUDA-core kernel where the shape's keys are FP32 ones; otherwise from a product q.c whose
+// partial sums do not overflow, as a tensor-core step adds its products.  Norms: the search's (cn), or here a
+// compensated float sum (the FP64 pipe took ten times as long as the rest).  A query with infinite values has FP32
+// keys, which those values decide, but no split keys.
 static __device__ __noinline__ void small_keys(const SmallSelect& c, const float* qv, bool finite, uint32_t* ord)
 {
     constexpr uint32_t kInf = 0xFF800000u;
+    constexpr int kB = 16;
+    const float inf = __int_as_float(0x7f800000);
+    float big = 0.f;
+    if (!c.fp32_keys)
+        for (int d = 0; d < c.D; ++d) big = fmaxf(big, fabsf(qv[d]));
+    // (a row with a norm lies below 2^64)
+    const float down = big >= 0x1p32f ? 0x1p-80f : 1.f, up = big >= 0x1p32f ? 0x1p80f : 1.f;
     for (int i = threadIdx.x; i < c.n; i += blockDim.x) {
         const float* row = c.corpus + (int64_t)i * c.ldc;
-        float dot = 0.f;
-        double wide = 0.0, norm = 0.0;
-        for (int d = 0; d < c.D; ++d) {
-            const float x = __ldg(row + d);
-            dot = __fmaf_rn(qv[d], x, dot);
-            wide = __fma_rn((double)qv[d], (double)x, wide);
-            norm = __fma_rn((double)x, (double)x, norm);
+        float dot = 0.f, n0 = 0.f, n1 = 0.f;
+        if (!finite && c.cn != nullptr)
+            for (int d = 0; d < c.D; ++d)
+                if (!(fabsf(qv[d]) < inf)) dot = __fmaf_rn(qv[d], __ldg(row + d), dot);
+        for (int d0 = 0; d0 < c.D && (finite || c.cn == nullptr); d0 += kB) {
+            float v[kB];
+#pragma unroll
+            for (int e = 0; e < kB; ++e) v[e] = d0 + e < c.D ? __ldg(row + d0 + e) : 0.f;
+#pragma unroll
+            for (int e = 0; e < kB; ++e)
+                if (d0 + e < c.D) {
+                    dot = __fmaf_rn(qv[d0 + e] * down, v[e], dot);
+                    if (c.cn == nullptr) {
+                        // n0 + n1 += v^2: the square's residual and the sum's (TwoSum)
+                        const float sq = __fmul_rn(v[e], v[e]), s = __fadd_rn(n0, sq), b = __fsub_rn(s, n0);
+                        n1 += __fmaf_rn(v[e], v[e], -sq) + (__fsub_rn(n0, __fsub_rn(s, b)) + __fsub_rn(sq, b));
+                        n0 = s;
+                    }
+                }
         }
-        if (!c.fp32_keys) dot = __double2float_rn(wide);
-        const float key = __fmaf_rn(-2.0f, dot, __double2float_rn(norm));
-        ord[i] = (c.fp32_keys || finite) && key < __int_as_float(0x7f800000) ? f2ord(key) : kInf;
+        const float norm = c.cn != nullptr ? __ldg(c.cn + i) : n0 < inf ? __fadd_rn(n0, n1) : n0;
+        const float key = __fmaf_rn(-2.0f, dot * up, norm);
+        ord[i] = (c.fp32_keys || finite) && key < inf ? f2ord(key) : kInf;
     }
 }
 
@@ -1166,8 +1186,7 @@ struct SmallShared {
     uint32_t wlo[kT / 32], whi[kT / 32], wcnt[kT / 32], digit, rank, hit, m;
     float wqq[kT / 32];
     __align__(16) uint64_t list[kSmallList];
-    float qq;     // direct mode: ||q||^2 ...
-    bool finite;  // ... and whether q is finite
+    float qq;  // direct mode: ||q||^2
 };
 
 // The extent of the words below +inf and their number: a thread's ...
@@ -1344,6 +1363,14 @@ template <int kT>
 static __device__ __noinline__ void pick_again(const SmallSelect& c, int64_t q, const float* qv, float qq, bool wide, int m,
                                                uint64_t* cur, uint32_t* ord, SmallShared<kT>& S)
 {
+    const float inf = __int_as_float(0x7f800000);
+    bool odd = false;
+    for (int d = threadIdx.x; d < c.D; d += kT) odd |= !(fabsf(qv[d]) < inf);
+    const bool finite = __syncthreads_or(odd) == 0;
+    if (qq != qq) {  // some value is NaN, and so is every key
+        emit_sorted<kT>(c, q, cur, 0, false, 0.f);
+        return;
+    }
     wide = wide && widen<kT>(c, qv, qq, cur, m, c.fail_idx != nullptr, ord);
     if (!wide && c.fail_idx != nullptr) {
         if (threadIdx.x == 0) {
@@ -1355,7 +1382,7 @@ static __device__ __noinline__ void pick_again(const SmallSelect& c, int64_t q, 
     }
     if (!wide) {
         __syncthreads();
-        small_keys(c, qv, S.finite, ord);
+        small_keys(c, qv, finite, ord);
     }
     if (threadIdx.x == 0) S.m = 0;
     __syncthreads();
@@ -1391,27 +1418,17 @@ __global__ void __launch_bounds__(kT, kMode == kSmallCertified ? 1024 / kT : 0) 
         qq = __fmaf_rn(y, y, qq);
     }
     for (int b = tid; b < 256; b += kT) S.hist[b] = 0;
-    if (tid == 0) {
-        S.m = 0;
-        S.finite = true;
-    }
+    if (tid == 0) S.m = 0;
     WordExtent x;
+    bool over = false;  // direct mode: some distance overflows (one that is NaN has a row without a key)
     if constexpr (kMode == kSmallDirect) {
         __syncthreads();
         if (warp == 0) {
             float s = 0.f;
-            bool bad = false;
-            for (int d = lane; d < c.D; d += 32) {
-                s = __fmaf_rn(qv[d], qv[d], s);
-                bad |= !(fabsf(qv[d]) < __int_as_float(0x7f800000));
-            }
+            for (int d = lane; d < c.D; d += 32) s = __fmaf_rn(qv[d], qv[d], s);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            bad = __any_sync(0xffffffffu, bad);
-            if (lane == 0) {
-                S.qq = s;
-                S.finite = !bad;
-            }
+            if (lane == 0) S.qq = s;
         }
         constexpr int kR = 4;  // rows a lane has in flight
         const int u = lane & 7, g = lane >> 3, full = c.D >> 3;
@@ -1456,11 +1473,12 @@ __global__ void __launch_bounds__(kT, kMode == kSmallCertified ? 1024 / kT : 0) 
                 s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 2));
                 s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
                 const int r = r0 + 4 * t + g;
+                over |= s == __int_as_float(0x7f800000);
                 if (u == 0 && r < n) ord[r] = s < __int_as_float(0x7f800000) ? f2ord(s) : kInf;
             }
         }
         for (int i = n + tid; i < n4; i += kT) ord[i] = kInf;
-        __syncthreads();
+        over = __syncthreads_or(over) != 0;
         x = thread_extent<kT>(ord, n);
     } else {
         load_ordered<kT>(c.keys + q * c.ldk, n, ord, x.lo, x.hi, x.cnt);
@@ -1472,8 +1490,8 @@ __global__ void __launch_bounds__(kT, kMode == kSmallCertified ? 1024 / kT : 0) 
     }
     block_extent<kT>(S, x);
     if constexpr (kMode == kSmallDirect) {
-        if (x.cnt < (uint32_t)n || x.hi >= f2ord(kDirectMost) || !(S.qq < kDirectMost))
-            return pick_again<kT>(c, q, qv, 0.f, false, 0, cur, ord, S);
+        if (over || x.hi >= f2ord(kDirectMost) || !(S.qq < kDirectMost))
+            return pick_again<kT>(c, q, qv, S.qq, false, 0, cur, ord, S);
     }
     uint32_t edge;
     const int m = pick_words<kT>(S, ord, n, c.need, x, cur, edge);
