@@ -277,6 +277,7 @@ __global__ void __launch_bounds__(kDistT) dist64_kernel(const double* __restrict
 __global__ void __launch_bounds__(256) rerank64_kernel(int64_t N, const double* __restrict__ dd,
                                                        const int32_t* __restrict__ ci, const int32_t* __restrict__ ncand,
                                                        const double* __restrict__ bound, int kp, int k,
+                                                       const double* __restrict__ queries, int64_t ldq, int D,
                                                        double* __restrict__ out_d, int32_t* __restrict__ out_i,
                                                        uint32_t* __restrict__ fails)
 {
@@ -294,7 +295,14 @@ __global__ void __launch_bounds__(256) rerank64_kernel(int64_t N, const double* 
         sw[j] = make_longlong2(__double_as_longlong(dd[q * kp + j]), n >= 0 ? n : 0x7fffffff);
     }
     if (threadIdx.x == 0) kth = __longlong_as_double(0x7ff0000000000000ll);
-    const bool missing = __syncthreads_or(gap) != 0;
+    bool missing = __syncthreads_or(gap) != 0;
+    if (missing && kp >= N) {
+        // (a query that is not finite has no finite distance to look for)
+        bool inf = false;
+        for (int d = threadIdx.x; d < D; d += blockDim.x)
+            inf |= !(fabs(queries[q * ldq + d]) < __longlong_as_double(0x7ff0000000000000ll));
+        missing = __syncthreads_or(inf) == 0;
+    }
     for (int j = threadIdx.x; j < m; j += blockDim.x) {
         int below = 0;
         const longlong2 w = sw[j];
@@ -429,7 +437,7 @@ int search_device(const double* corpus, int64_t N, int64_t ldc, const double* qu
         corpus, N, ldc, queries, ldq, D, (const float*)W->cand_d.p, (const int32_t*)W->cand_i.p, kp, k,
         (const unsigned long long*)W->cmax.p, (double*)W->dd.p, (int32_t*)W->ncand.p, (double*)W->bound.p);
     rerank64_kernel<<<(unsigned)Q, 256, 0, s>>>(N, (const double*)W->dd.p, (const int32_t*)W->cand_i.p,
-                                                (const int32_t*)W->ncand.p, (const double*)W->bound.p, kp, k, dist, idx,
+                                                (const int32_t*)W->ncand.p, (const double*)W->bound.p, kp, k, queries, ldq, D, dist, idx,
                                                 (uint32_t*)W->fails.p);
     // queries whose shortlist could not be proven complete (the grid covers every query; the
     // CTAs past the failure count return at once)

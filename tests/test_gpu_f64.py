@@ -138,3 +138,16 @@ def test_double_library_norms_past_the_float_range(engine, oracle, N):
     od, oi = oracle.knn_f64d(X, Qs, 10)
     np.testing.assert_array_equal(i, oi)
     np.testing.assert_array_equal(d, od)
+
+
+@pytest.mark.parametrize("N", [11, 36])  # k + 32 rows and fewer
+def test_double_library_infinite_query_of_a_covered_corpus(engine, N):
+    # no distance is finite; the rows that the FP32 shortlist holds come back by index
+    rng = np.random.default_rng(N)
+    X, Qs = rng.random((N, 412)) + 0.1, rng.random((3, 412))
+    X[N - 1, 5] = np.inf
+    Qs[1, 3] = np.inf
+    d, i = engine.search_host_f64(X, Qs, 4)
+    assert np.isinf(d[1]).all()
+    np.testing.assert_array_equal(i[1], np.arange(4))
+    assert np.isfinite(d[[0, 2]]).all()
