@@ -967,6 +967,7 @@ struct TscanStages {
         cs.fail_idx = (int32_t*)fail.p + 1;
         cs.fail_cnt = fail_cnt;
         cs.fail_thr = (uint32_t*)thr2.p;
+        cs.small = N < kScanMinRowsForced;
         cs.certify = c.fp32;
         KNN_CUDA(launch_select_cand(cs, s));
         ++launches;

@@ -405,7 +405,9 @@ struct CandSelect {
     int32_t* fail_idx = nullptr;
     uint32_t* fail_cnt = nullptr;
     uint32_t* fail_thr = nullptr;  // all ones at every failed query's place (the fix-up's thresholds)
-    bool certify = false;          // a query also fails when its shortlist may miss a row (as SmallSelect::fp32_keys)
+    // corpora below 16,384 rows, re-ranked: certify -- a query also fails when its shortlist may miss a row (as
+    // SmallSelect::fp32_keys); else a query that is not finite does not fail but has no results
+    bool small = false, certify = false;
     // exact-key test (optional): keys and distances are exact integers when every corpus and
     // query value is an integer, 2 * D * max|x|^2 < 2^24 and the BF16 copies are exact; the
     // re-rank is then skipped (distance = key + qn[q], the same value it would compute)

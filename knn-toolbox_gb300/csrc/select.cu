@@ -553,7 +553,7 @@ __device__ __forceinline__ bool list_holds(const uint64_t* list, int m, int k, f
 // kThr: threshold mode -- the next float above the key of rank thr_rank, or the fallback.  Blocks an SM:
 // ten of 128 threads (47 registers; at 63 a million rows' 10,000 queries take 97 instead of 88 us), four
 // of 256 (for the re-rank's loads in flight: 256 queries, 32 rows of 1,024 columns 18.9 -> 15.5 us).
-template <int kT, bool kThr, bool kCertify = false>
+template <int kT, bool kThr, bool kSmall = false>
 __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_kernel(const CandSelect c)
 {
     if (c.skip_if != nullptr && *c.skip_if != 0u) return;
@@ -603,6 +603,15 @@ __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_k
         return;
     }
     if (!kThr && (overflow || total < (uint32_t)c.need || total > (uint32_t)c.buf_words)) {
+        if constexpr (kSmall) {
+            // a query that is not finite has no split keys, and with them no results
+            bool odd = false;
+            for (int d = tid; d < c.D; d += kT) odd |= !(fabsf(__ldg(c.queries + q * c.ldq + d)) < __int_as_float(0x7f800000));
+            if (!c.certify && __syncthreads_or(odd)) {
+                emit_sorted<kT>(c, q, cur, 0, false, 0.f);
+                return;
+            }
+        }
         if (tid == 0) {
             const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
             c.fail_idx[pos] = (int32_t)q;
@@ -723,7 +732,7 @@ __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_k
     }
     const bool rr = c.rerank && !exact;
     float bound = 0.f;
-    if constexpr (kCertify) {
+    if (kSmall && c.certify) {
         // the largest key of the shortlist, and ||q||^2
         __shared__ uint32_t wkey[kW];
         __shared__ float wqq[kW];
@@ -751,7 +760,7 @@ __global__ void __launch_bounds__(kT, kT == 128 ? 10 : 1024 / kT) select_block_k
         rerank_block<kT>(list, m, c.corpus, c.ldc, qv, c.D);
         __syncthreads();
     }
-    if constexpr (kCertify) {
+    if (kSmall && c.certify) {
         if (!list_holds<kT>(list, m, c.k, bound)) {
             if (tid == 0) {
                 const uint32_t pos = atomicAdd(c.fail_cnt, 1u);
@@ -1626,7 +1635,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
                                       : kCandMax;
     if (c.nseg < 1 || c.nseg > kScanMaxSegs || c.cap < 1 ||
         (!thr && (c.kp < 1 || c.kp > kMaxKpScan || c.k > c.kp || c.fail_idx == nullptr || c.fail_cnt == nullptr || c.fail_thr == nullptr ||
-                  (!c.rerank && c.qn == nullptr) || (c.certify && (!c.rerank || c.int_stats != nullptr)))) ||
+                  (!c.rerank && c.qn == nullptr) || (c.certify && !c.small) || (c.small && (!c.rerank || c.int_stats != nullptr)))) ||
         (thr && (c.thr_rank < 1 || c.thr_rank > kCandThrMax)))
         return cudaErrorInvalidValue;
     if (thr && c.Q <= kThrBlockQ) {
@@ -1650,7 +1659,7 @@ cudaError_t launch_select_cand(const CandSelect& c_in, cudaStream_t s)
         // 31.9 / 64.0 against 50.0 / 55.5 us (100,003 x 43, k = 512, before the re-rank took two rows at a time)
         const size_t smem = ((size_t)pow2_at_least(c.kp) + c.buf_words) * 8 + (size_t)((c.D + 3) & ~3) * 4;
         const int t = c.Q <= kSelFewQ ? 512 : c.Q <= kSelWideQ ? 256 : 128;
-        auto* kernel = c.certify  ? (t == 512   ? select_block_kernel<512, false, true>
+        auto* kernel = c.small    ? (t == 512   ? select_block_kernel<512, false, true>
                                      : t == 256 ? select_block_kernel<256, false, true>
                                                 : select_block_kernel<128, false, true>)
                        : t == 512 ? select_block_kernel<512, false>

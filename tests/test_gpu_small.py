@@ -172,3 +172,15 @@ def test_workspace_of_many_queries(engine, N, Q, D, most):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     assert int(r.stdout.split()[-1]) < most
+
+
+@pytest.mark.parametrize("N,Q,D", [(9000, 3000, 40), (3000, 200, 90), (500, 20, 7)])
+def test_infinite_queries_of_narrow_rows(engine, N, Q, D):
+    # split keys of such a query are NaN: no results, whichever path the number of queries takes
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c, q = torch.randn((N, D), generator=g, device="cuda"), torch.randn((Q, D), generator=g, device="cuda")
+    q[3, 1], q[4, 2], q[5, 0] = float("inf"), float("-inf"), float("nan")
+    d, i, d0, i0, st = both(engine, c, q, 9)
+    assert (i[3:6] == -1).all() and torch.isinf(d[3:6]).all()
+    assert torch.equal(i, i0) and torch.equal(d, d0)
