@@ -396,6 +396,11 @@ static int resolve_keys(const Engine& E, int64_t N, int64_t Q, int D, int k, con
 //    1,038 / 1,029 / 108; 2,000 x 1,024, 1,024 queries 744 / 1,131 / 74).
 //  * From kSmallScanRows rows, more queries than that go to the FP16-split threshold scan, whose
 //    candidates are a fraction of the keys.
+//  * A handful of short rows and more than kFewValuesQ queries: the shortlist kernel, which takes 128 queries a block where
+//    these take one (1,000,000 queries of 30 x 3 rows 4,027 us against 4,827, of 8 x 3 3,956 against 4,420; of 8 x 32
+//    4,658 against 4,643, of 30 x 32 7,050 against 5,109).
+constexpr int64_t kFewValues = 128;
+constexpr int64_t kFewValuesQ = 131072;
 constexpr int64_t kDirectBlock = 280000;
 constexpr int64_t kDirectTotal = 50000000;
 constexpr int64_t kSmallKeys = 24 << 20;
@@ -405,7 +410,7 @@ int resolve_config(const Engine& E, int64_t N, int64_t Q, int D, int k, const kn
     const int rc = resolve_keys(E, N, Q, D, k, o, c);
     if (rc || c->tscan || N >= kScanMinRowsForced || N > kSmallRows || E.cc < 100 || o.precision != KNNS_PREC_EXACT ||
         o.algo != KNNS_ALGO_AUTO || o.scan != KNNS_SCAN_AUTO || o.splits > 0 || !o.pilot || o.tf32_only || !c->rerank ||
-        c->kp < k + kKeyMargin || k > kMaxKpScan)
+        c->kp < k + kKeyMargin || k > kMaxKpScan || (Q > kFewValuesQ && N * D <= kFewValues))
         return rc;
     c->fp32 = c->algo == KNNS_ALGO_SIMT;
     if (N * (D + 32) <= kDirectBlock && Q * N * (D + 32) <= kDirectTotal) {

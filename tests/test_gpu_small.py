@@ -184,3 +184,12 @@ def test_infinite_queries_of_narrow_rows(engine, N, Q, D):
     d, i, d0, i0, st = both(engine, c, q, 9)
     assert (i[3:6] == -1).all() and torch.isinf(d[3:6]).all()
     assert torch.equal(i, i0) and torch.equal(d, d0)
+
+
+@pytest.mark.parametrize("N,Q,D,k", [(30, 140_000, 3, 10), (128, 131_073, 1, 5), (129, 131_073, 1, 5), (1, 300_000, 9, 1)])
+def test_a_handful_of_values_and_very_many_queries(engine, N, Q, D, k):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(N)
+    c, q = torch.rand((N, D), generator=g, device="cuda"), torch.rand((Q, D), generator=g, device="cuda")
+    d, i, d0, i0, st = both(engine, c, q, k)
+    assert torch.equal(i, i0) and torch.equal(d, d0)
