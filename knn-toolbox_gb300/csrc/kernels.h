@@ -208,6 +208,7 @@ struct ScanArgs {
     int ring;                  // ring slots
     int fp8;                   // keys from E4M3 operands with per-row scales
     int split0;                // first split of this launch (grid row y is split split0 + y)
+    uint32_t zero;             // 0 (release_norms)
     int accs;                  // TMEM accumulators: 2 (tiles of 224 / 192 rows) or 4 (tiles of 96)
 };
 // corpus rows per tile (MMA N): with 2 accumulators 224 for dpb <= 128, 192 for dpb <= 256;
@@ -248,6 +249,7 @@ struct TscanArgs {
     const uint32_t* run_if;       // optional: the kernel returns at once when *run_if == 0
     // dp <= 128: the queries' TF32 hi / lo parts in tensor memory, split by the kernel from the
     // FP32 queries (tm_qhi, tm_qlo, qlo_flags unused); the ring carries corpus chunks only
+    uint32_t zero;                // 0 (release_norms)
     int tmem_a;
     const float* queries;         // [Q][ldq] fp32 (tmem_a)
     int64_t ldq;
@@ -287,6 +289,7 @@ struct FscanArgs {
     int hp;                       // row pitch of the queries' copies
     int dense_rows;               // dense pass: corpus rows per tile (fscan_dense_rows)
     int split0;                   // first split of this launch
+    uint32_t zero;                // 0 (release_norms)
     const uint32_t* run_if;       // optional: the kernel returns at once when *run_if == 0
 };
 int fscan_tile_rows(int D);

@@ -422,13 +422,6 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                 chunk_scaled_keys<W1>(va, nrm + c1, scl + c1, m);
                 chunk_scaled_keys<W2>(vb, nrm + c2, scl + c2, m);
                 if constexpr (W3 > 0) chunk_scaled_keys<W3>(vc, nrm + c3, scl + c3, m);
-                // norm slot ns fully read
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);
-                if (++ns == kNormSlots) {
-                    ns = 0;
-                    nph ^= 1u;
-                }
             } else if (t == mask_t) {
                 // the accumulator holds the keys; the view's last tile masks its rows past the view
                 const int rem = (int)(a.N - (n_begin + (int64_t)t * TN));
@@ -451,7 +444,9 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                     chunk_minima<W3>(vc, gc);
                     mb = fminf(mb, gc[0]);
                 }
-                if (__any_sync(0xffffffffu, fminf(ma, mb) < T)) {
+                const uint32_t hot = __ballot_sync(0xffffffffu, fminf(ma, mb) < T);
+                if constexpr (kF8) release_norms(nempty + 8u * ns, hot, a.zero);
+                if (hot) {
                     // (E4M3 keys, whose loop is longer: a second vote per half, 811 -> 801 us for 2,000,000 x 256;
                     // BF16 keys 1,634 -> 1,669 with it)
                     if (!kF8 || __any_sync(0xffffffffu, ma < T))
@@ -460,6 +455,13 @@ __global__ void __launch_bounds__(kScanThreads, 1)
                         chunk_append<W2>(vb, gb, T, nb + (uint32_t)c2, out, cap, cnt);
                         if constexpr (W3 > 0) chunk_append<W3>(vc, gc, T, nb + (uint32_t)c3, out, cap, cnt);
                     }
+                }
+            }
+            if constexpr (kF8) {
+                if constexpr (kDense) release_norms(nempty + 8u * ns);
+                if (++ns == kNormSlots) {
+                    ns = 0;
+                    nph ^= 1u;
                 }
             }
         }

@@ -47,6 +47,21 @@ __device__ __forceinline__ void chunk_norm_keys(float (&v)[W], const float* nrm)
     }
 }
 
+// Release of a norm slot by an epilogue warp, once its loads have returned.  Right after the loads in program order
+// the arrival could overtake them, queued behind the appends of earlier tiles, and the slot be filled anew: beside
+// queries that append whole tiles rows were lost (9,000 x 5 rows, nine tenths of the values zero: 20 of 3,000 queries).
+// So the arrival's address depends on the vote over all lanes' keys (zero: 0, which the compiler does not know).
+__device__ __forceinline__ void release_norms(uint32_t bar, uint32_t vote, uint32_t zero)
+{
+    if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(bar + (vote & zero));
+}
+// ... of a dense pass, after the shuffles of its stores have used the keys.
+__device__ __forceinline__ void release_norms(uint32_t bar)
+{
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(bar);
+}
+
 // Keys of the columns at or past `rem` (rows past the corpus view in its last tile) set to +inf.
 template <int W>
 __device__ __forceinline__ void chunk_mask(float (&key)[W], int c0, int rem)

@@ -363,19 +363,19 @@ __global__ void __launch_bounds__(kThreads, 1) fscan_ta_kernel(const __grid_cons
             }
             const float* nrm = s.norms + ns * kTN + c0;
             chunk_scaled_keys<32>(v, nrm, nrm + kNorm * kTN, m);
-            // norm slot ns fully read
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(nempty + 8u * ns);
-            if (++ns == kNorm) {
-                ns = 0;
-                nph ^= 1u;
-            }
             if constexpr (kDense) {
                 chunk_store<32>(v, krow + nb, a.ldk, krows);
+                release_norms(nempty + 8u * ns);
             } else {
                 float g[4];
                 chunk_minima<32>(v, g);
-                if (__any_sync(0xffffffffu, min_of(g) < T)) chunk_append<32>(v, g, T, nb, out, cap, cnt);
+                const uint32_t hot = __ballot_sync(0xffffffffu, min_of(g) < T);
+                release_norms(nempty + 8u * ns, hot, a.zero);
+                if (hot) chunk_append<32>(v, g, T, nb, out, cap, cnt);
+            }
+            if (++ns == kNorm) {
+                ns = 0;
+                nph ^= 1u;
             }
         }
         if (!kDense && valid) a.cnt[seg * (size_t)a.Q + (size_t)q] = cnt;
