@@ -186,7 +186,7 @@ def test_infinite_queries_of_narrow_rows(engine, N, Q, D):
     assert torch.equal(i, i0) and torch.equal(d, d0)
 
 
-@pytest.mark.parametrize("N,Q,D,k", [(30, 140_000, 3, 10), (128, 131_073, 1, 5), (129, 131_073, 1, 5), (1, 300_000, 9, 1)])
+@pytest.mark.parametrize("N,Q,D,k", [(30, 140_000, 3, 10), (128, 131_073, 1, 5), (129, 131_073, 1, 5), (1, 300_000, 9, 1), (20, 32_769, 6, 3), (20, 32_768, 6, 3)])
 def test_a_handful_of_values_and_very_many_queries(engine, N, Q, D, k):
     import torch
     g = torch.Generator(device="cuda").manual_seed(N)
