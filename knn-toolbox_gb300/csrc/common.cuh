@@ -81,18 +81,6 @@ __device__ __forceinline__ float row_scale(float mx, float& inv)
     return __uint_as_float((uint32_t)b << 23);
 }
 
-// s x0, s x1 as hi + lo FP16 pairs; returns whether a low part is nonzero.  A value that is not
-// finite leaves NaN in lo (inf - inf), so its keys are NaN and enter no segment.
-__device__ __forceinline__ uint32_t split_pair(float x0, float x1, float sc, uint32_t& hi, uint32_t& lo)
-{
-    const float y0 = __fmul_rn(x0, sc), y1 = __fmul_rn(x1, sc);
-    const __half2 h = __floats2half2_rn(y0, y1);
-    const __half2 l = __floats2half2_rn(__fsub_rn(y0, __low2float(h)), __fsub_rn(y1, __high2float(h)));
-    hi = *reinterpret_cast<const uint32_t*>(&h);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-    return lo & 0x7fff7fffu;
-}
-
 // ---------------------------------------------------------------------------
 // Warp-level primitives
 // ---------------------------------------------------------------------------

@@ -247,9 +247,8 @@ constexpr int64_t kScanMinRowsForced = 16384;
 constexpr int64_t kScanMinRowsAuto = 131072;
 // accumulators of the threshold scan when the options leave it open
 constexpr int kScanAccsAuto = 2;
-// widest rows the FP16-split scan takes: its K loop has no limit, the selection's re-rank stages
-// candidate rows in shared memory (four rows of 2048 values per warp)
-constexpr int kTscanMaxD = 2048;
+// widest rows the split-key scan takes: what the preparation kernel covers (kPrepMaxD)
+constexpr int kTscanMaxD = kPrepMaxD;
 static inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int round32(int x) { return (x + 31) & ~31; }
 static inline int round16(int x) { return (x + 15) & ~15; }
@@ -258,7 +257,8 @@ static inline int round16(int x) { return (x + 15) & ~15; }
 // rounding differs from the 3xTF32 keys' (it is smaller: rms over row norms 0.5 to 0.8 of it at
 // every width measured), so a shortlist without a margin, whose last entries decide the result,
 // could end in another row; results there, and distances read off the keys (rerank = 0), stay those of
-// the 3xTF32 keys.  With 8 entries to spare no result depends on the keys' rounding.
+// the 3xTF32 keys.  Eight entries to spare make up for differences in rounding unless more rows than
+// that lie within it of the k-th distance, when either kind of key may miss one.
 constexpr int kKeyMargin = 8;
 
 // Shortlist length: k plus a re-rank margin of max(8, k/8), in multiples of 16.
@@ -1012,13 +1012,12 @@ static PrepJob prep_job(const float* x, int64_t n, int64_t ld, int D, float* nor
 }
 
 // the engine's FP16 corpus copies as outputs of a preparation
-static void split_outputs(Engine& E, PrepJob* j, uint32_t* any_lo)
+static void split_outputs(Engine& E, PrepJob* j)
 {
     j->hi = E.hi.p;
     j->lo = E.lo.p;
     j->rs = (float*)E.rs.p;
     j->lo_flags = E.lof;
-    j->any_lo = any_lo;
 }
 
 // Space for the corpus's hi / lo copies in this engine's buffers.
@@ -1045,7 +1044,7 @@ static int split_corpus(Engine& E, const Config& c, const float* corpus, int64_t
         return KNNS_OK;
     }
     PrepJob j = prep_job(corpus, N, ldc, D, norms, n_pad);
-    split_outputs(E, &j, any_lo);
+    split_outputs(E, &j);
     j.run_if = skip_unless;
     KNN_CUDA(launch_prep(j, s, queries));
     return KNNS_OK;
@@ -1071,7 +1070,7 @@ static int run_tscan(Engine& E, const Config& c, const float* corpus, int64_t N,
     int rc = plan_scan(E, N, Q, c.dpb, c.kp, o, &sp, c.tf32 ? kKeyTf32 : kKeyF16, 0, c.fp32);
     if (rc) return rc;
     if (pc && !pc->tf32)
-        return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies of this width");
+        return set_error(KNNS_ERR_INVALID, "the exact form needs an index with its hi / lo copies (KNNS_INDEX_TF32)");
     const int64_t n_pad = cdiv(N, kScanTileN) * kScanTileN + kScanTileN;
     if (!pc) {
         rc = E.cn.ensure(n_pad * sizeof(float));
@@ -1368,7 +1367,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             return set_error(KNNS_ERR_INVALID, "prepared corpus does not match the search's corpus");
         if (f8 && !pc->fp8) return set_error(KNNS_ERR_INVALID, "the FP8 form needs an index prepared with E4M3 copies");
         if (c.algo == KNNS_ALGO_TC && !bf16_only && !pc->tf32)
-            return set_error(KNNS_ERR_INVALID, "the exact form needs an index prepared with TF32 copies");
+            return set_error(KNNS_ERR_INVALID, "the exact form needs an index with its hi / lo copies (KNNS_INDEX_TF32)");
     }
 
     // norms padded with +inf at least one tile (of any kernel) past the corpus
@@ -1658,7 +1657,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             }
             if (np_keys) j.np = E.np.p;
             if (adaptive) {
-                split_outputs(E, &j, any_lo);
+                split_outputs(E, &j);
                 j.done = (uint8_t*)E.done.p;
             }
             KNN_CUDA(launch_prep(j, s, &qj));
@@ -1672,7 +1671,7 @@ int run_search(Engine& E, const float* corpus, int64_t N, int64_t ldc, const flo
             // known (3xTF32 keys: the split of the whole corpus)
             if (adaptive) {
                 PrepJob j = prep_job(corpus, N, ldc, D, nullptr, n_pad);
-                split_outputs(E, &j, any_lo);
+                split_outputs(E, &j);
                 j.not_exact = not_exact;
                 j.done = (uint8_t*)E.done.p;
                 j.catch_up = true;
@@ -2576,7 +2575,7 @@ int knns_autotune_shortlist(knns_index* ix, const float* queries, int64_t Q, int
             return set_error(KNNS_ERR_CUDA, "autotune copy");
         return KNNS_OK;
     };
-    // ground truth: the exact form (needs the index's TF32 copies unless the data are BF16-exact)
+    // ground truth: the exact form (needs the index's hi / lo copies unless the data are BF16-exact)
     rc = run(KNNS_PREC_EXACT, 0, exact);
     int best = 0;
     double best_recall = 0.0, last_recall = 0.0;
@@ -2651,7 +2650,7 @@ double knns_debug_host_row_bytes(int64_t N, int64_t Q, int D, int k, const knns_
     clear_error();
     if (!opt || N < 1 || Q < 1 || D < 1 || k < 1) return 0.0;
     Engine E;  // (reads the device properties alone, as below)
-    E.sms = 152;
+    E.sms = kSms;
     E.cc = 103;
     return host_row_bytes(E, N, Q, D, k, *opt);
 }

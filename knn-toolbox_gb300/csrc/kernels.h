@@ -7,6 +7,8 @@
 
 namespace knn {
 
+constexpr int kSms = 152;  // SMs of the chip that fixed grids and query counts are for (Engine::sms: the device's)
+
 // Tile geometry shared by host and device.
 constexpr int kTileQ = 128;       // queries per CTA (tensor-core M, TMEM lanes)
 constexpr int kTileN = 128;       // corpus rows per tile (tensor-core N)
@@ -70,13 +72,12 @@ struct PrepJob {
     float* scales = nullptr;
     // FP16 side: hi = fp16(s x), lo = fp16(s x - hi), s the power of two that puts the row's largest
     // |x| into [2^14, 2^15); hi / lo are [n][split_pitch(D)] FP16, zero padded, rs[0..n_pad) the
-    // reciprocals 1 / s (0 for n <= i < n_pad).  lo_flags[tile of 128 rows] and *any_lo (zeroed by
-    // the caller) become 1 when some lo is nonzero
+    // reciprocals 1 / s (0 for n <= i < n_pad).  lo_flags[tile of 128 rows] (zeroed by the caller) becomes 1 when
+    // some lo is nonzero
     void* hi = nullptr;
     void* lo = nullptr;
     float* rs = nullptr;
     uint32_t* lo_flags = nullptr;
-    uint32_t* any_lo = nullptr;
     // adaptive: the BF16 or the FP16 side per batch of rows, by *not_exact (see prep_rows_kernel);
     // done: one byte per batch (prep_batches of them), 1 when the FP16 side was written.  catch_up:
     // the FP16 side of the batches whose done byte is 0, nothing else.

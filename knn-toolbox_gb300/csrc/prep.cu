@@ -149,7 +149,7 @@ __global__ void gather_norms_kernel(const float* __restrict__ src, int64_t n, in
 //    integer, int_stats[1] = max |x| as float bits; the norm as BF16 parts;
 //  * E4M3 copy into f8[n][f8_bytes] (zero padded) with per-row absmax scales
 //    (scale = max|x| / 448, codes = satfinite(x * 448 / max|x|));
-//  * FP16 side: the split hi / lo [n][hp] with row scales and tile flags (split_pair);
+//  * FP16 side: the split hi / lo [n][hp] with row scales and tile flags (split_pair2);
 //  * row norms into norms[0..n_pad) (+inf for n <= i < n_pad): the float rounding of the double
 //    sum of x_d^2 taken in d order (the convention of norms_kernel and the CPU oracle), certified
 //    from a float-float sum -- see certified_norm -- and, for the rows that leaves open, from a
@@ -369,7 +369,8 @@ __device__ __forceinline__ float fmax3(float a, float b, float c)
     return m;
 }
 
-// split_pair with packed arithmetic (the low parts are not masked)
+// s x0, s x1 as hi + lo FP16 pairs, in packed arithmetic.  A value that is not finite leaves NaN in lo (inf - inf), so
+// its keys are NaN and enter no segment.
 __device__ __forceinline__ void split_pair2(float x0, float x1, F2 sc, uint32_t& hi, uint32_t& lo)
 {
     float y0, y1, z0, z1;
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
     const int D = p.D;
     const bool want_norms = p.norms != nullptr || p.np != nullptr;
     const bool check = p.bf != nullptr || p.not_exact != nullptr;
-    uint32_t frac = 0, bad = 0, any_lo = 0;
+    uint32_t frac = 0, bad = 0;
     float mx_all = 0.f;
     bool inexact = false;  // adaptive: *not_exact seen set
     int it = 0;
@@ -695,10 +696,8 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
             }
             if (lead) p.rs[base + g] = pick_row(inv, g);
             // a batch lies in one tile: kU divides its rows
-            if (__any_sync(0xffffffffu, (any & 0x7fff7fffu) != 0u)) {
-                any_lo = 1u;
-                if (lane == 0 && p.lo_flags) p.lo_flags[base / kTileRows] = 1u;
-            }
+            if (__any_sync(0xffffffffu, (any & 0x7fff7fffu) != 0u) && lane == 0 && p.lo_flags)
+                p.lo_flags[base / kTileRows] = 1u;
         }
         if (want_norms && !p.catch_up) {
             float f;
@@ -781,7 +780,6 @@ __global__ void __launch_bounds__(256, kChunks <= 8 ? 3 : 2)
     }
     // flags: one atomic per warp
     if (p.not_exact != nullptr && bad != 0u && lane == 0) atomicOr(p.not_exact, 1u);
-    if (p.any_lo != nullptr && any_lo != 0u && lane == 0) atomicOr(p.any_lo, 1u);
     if (p.int_stats != nullptr && !p.catch_up) {
         if (frac != 0u && lane == 0) atomicOr(p.int_stats, 1u);
         if (lane == 0 && mx_all > 0.f) atomicMax(p.int_stats + 1, __float_as_uint(mx_all));
@@ -835,7 +833,7 @@ cudaError_t launch_prep(const PrepJob& job, cudaStream_t s, const PrepJob* secon
     const int D = job.D;
     // one wave of blocks (three an SM, two for the widest rows), each warp walking its share of the rows;
     // of two jobs each gets blocks by its rows
-    const int64_t kBlocks = 152 * (D <= 1024 ? 3 : 2);
+    const int64_t kBlocks = kSms * (D <= 1024 ? 3 : 2);
     const int64_t nb = prep_batches(rows, D), nb2 = second ? prep_batches(prep_rows(*second), D) : 0;
     const int64_t want = (nb + 7) / 8, want2 = (nb2 + 7) / 8;
     int64_t b1 = std::min(want, kBlocks), b2 = want2;

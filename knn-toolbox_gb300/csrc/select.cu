@@ -322,7 +322,7 @@ constexpr int kRankSortMax = 128;
 constexpr int64_t kThrBlockQ = 1536;  // threshold mode: a warp per query above
 // Up to a query an SM: 512 threads each, which shorten one query's chain of round trips (48 queries on
 // 2,000,000 x 128: threshold from 7,813 keys 7.5 -> 4.9 us, selection 12.9 -> 11.8, the search 150 -> 145).
-constexpr int64_t kSelFewQ = 152;
+constexpr int64_t kSelFewQ = kSms;
 constexpr int64_t kSelWideQ = 384;  // up to this many queries: 256 threads each, above 128
 
 // The first k of `cur` (m packed words: key or distance above index) in ascending order to the
@@ -1544,7 +1544,7 @@ cudaError_t launch_select_small(const SmallSelect& c, cudaStream_t s)
     if (c.keys)
         return c.Q <= kSelWideQ ? run_select_small<512, kSmallDense>(c, smem, s)
                                 : run_select_small<256, kSmallDense>(c, smem, s);
-    return c.Q <= 152 ? run_select_small<1024, kSmallDirect>(c, smem, s) : run_select_small<256, kSmallDirect>(c, smem, s);
+    return c.Q <= kSms ? run_select_small<1024, kSmallDirect>(c, smem, s) : run_select_small<256, kSmallDirect>(c, smem, s);
 }
 
 size_t select_smem_bytes(int kp, int D, int rerank)

@@ -97,6 +97,7 @@ Work* work_for_device()
 }
 
 constexpr int kSortMax = 512;    // shortlist entries one warp re-ranks
+constexpr int64_t kMostBlocks = 152 * 8;  // eight an SM
 constexpr int kBruteBuf = 2048;  // candidate buffer of the brute-force kernel
 
 // x rounded to FP32 (to nearest, ties to even) in integer arithmetic, for zeros and magnitudes of FP32's
@@ -423,7 +424,7 @@ int search_device(const double* corpus, int64_t N, int64_t ldc, const double* qu
     if (rc) return rc;
     F64_CUDA(cudaMemsetAsync(W->cmax.p, 0, 8, s));
     F64_CUDA(cudaMemsetAsync(W->fails.p, 0, 4, s));
-    auto blocks = [](int64_t rows) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, 152 * 8)); };
+    auto blocks = [](int64_t rows) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((rows + 7) / 8, kMostBlocks)); };
     auto* to_f32_rows = D <= 128 ? to_f32_kernel<4> : to_f32_kernel<8>;
     to_f32_rows<<<blocks(N), 256, 0, s>>>(corpus, N, ldc, D, (float*)W->c32.p, (unsigned long long*)W->cmax.p);
     to_f32_rows<<<blocks(Q), 256, 0, s>>>(queries, Q, ldq, D, (float*)W->q32.p, nullptr);
