@@ -53,7 +53,7 @@ WORKLOADS = {
                        "L2-normalised), 2,500 queries, k=10, seed 2",
                   gen="gauss_mixture", N=1_000_000, D=96, Q=2_500, k=10, seed=2),
     # serving form: resident corpus, Poisson arrivals of requests of uneven size and k
-    "serve2m": dict(desc="serving: int-descriptor corpus 2,000,000 x 128 resident (FP32 + BF16 + FP16 hi / lo copies), "
+    "serve2m": dict(desc="serving: int-descriptor corpus 2,000,000 x 128 resident (FP32, BF16, TF32 and FP16 hi / lo copies), "
                          "Poisson arrivals, request sizes log-uniform on [1,512], k in {1,10,100}, seed 1",
                     gen="int_descriptor", N=2_000_000, D=128, Q=0, k=0, seed=1, serve=True),
     # precision form with E4M3 keys: anisotropic Gaussian N(0, diag(1/sqrt(1+j)))
